@@ -236,7 +236,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     volatile int *quit = reinterpret_cast<volatile int *>(misc + 40);          // [2] per head: a softmax thread's wait ran out, all of them leave together
     float *xch = reinterpret_cast<float *>(misc + 64);                         // what the two threads of a row tell each other
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const AttnTile tile = tiles[blockIdx.y];                                    // the host lists the tiles with the most key blocks first
     const int h0 = 2 * blockIdx.x, kh = h0 / (NH / NKV);
     const int q_last = tile.q0 + tile.q_len - 1;                                // last query row of the tile
@@ -262,7 +262,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
         // ---------------------------------------------------------- loads: both Q tiles once, then K one block ahead of Vt
         armed[0] = 0;
         mbar_expect_tx(q_full, 2 * AT_TILE_BYTES);
@@ -291,7 +291,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             tma_load_2d(v_smem(pv.stage) + AT_TILE_BYTES / 2, &tm_vt, tile.vcol0 + j * 128 + 64, kh * HD, v_full(pv.stage));
             pv.advance(AT_KV_STAGES);
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && elect_one()) {
         // ---------------------------------------------------------- MMA issuer
         // Per head and block: the value product as soon as P is written, and behind it the head's next
         // scores into the same TMEM columns (the tensor pipe runs them in the order issued, so the

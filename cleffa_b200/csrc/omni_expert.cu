@@ -312,7 +312,7 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     volatile WorkSlotX *ring = reinterpret_cast<volatile WorkSlotX *>(misc + 16 + 64);
     const uint32_t ring_u32 = misc_u32 + 16 + 64;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
     const bool leader = rank == 0;
     const bool gathering = a.gather_src != nullptr;
@@ -359,7 +359,7 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         else xtma_2d<CTAS>(dst, &tm_w, ks * BK, expert * M::OUT_COLS + m_cta * 128, bar, pol);
     };
 
-    if (warp == 0 && lane == 0 && leader) {
+    if (warp == 0 && leader && elect_one()) {
         // ---------------------------------------------------------- scheduler + weight producer
         // Claiming and decoding an item costs an atomic and two dependent global loads; they are
         // software-pipelined behind the TMA issue loop (item i+1 is decoded and item i+2 claimed
@@ -420,7 +420,7 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             cur = nxt; cur_m = nxt_m; cur_cnt = nxt_cnt;
             w1 = w2;
         }
-    } else if (warp == 0 && lane == 0) {
+    } else if (warp == 0 && !leader && elect_one()) {
         // ---------------------------------------------------------- weight producer of the second CTA
         PipeState p, wr;
         const uint64_t pol_w = l2_policy_evict_first();
@@ -535,7 +535,7 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             for (int i = 0; i < NR; i++) off[i] = off_next[i];
         }
         cp_async_wait<0>();
-    } else if (warp == 3 && lane == 0) {
+    } else if (warp == 3 && elect_one()) {
         // ---------------------------------------------------------- token producer, TMA
         PipeState p, wr;
         const uint64_t pol_t = l2_policy_evict_last();
@@ -581,7 +581,7 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 p.advance(TS);
             }
         }
-    } else if (warp == 1 && lane == 0 && leader) {
+    } else if (warp == 1 && leader && elect_one()) {
         // ---------------------------------------------------------- MMA issuer (first CTA of the pair)
         PipeState pw, pt, wr;
         bool ok = true;

@@ -99,7 +99,7 @@ router_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
     volatile int *abort_flag = reinterpret_cast<volatile int *>(misc + 4);
     volatile int *armed = reinterpret_cast<volatile int *>(misc + 8);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int row0 = blockIdx.x * NT;
 
     if (threadIdx.x == 0) {
@@ -118,7 +118,7 @@ router_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
         PipeState p;
         stamp(0);
         const uint64_t pol_w = l2_policy_evict_last();          // every CTA reads the router matrix
@@ -132,7 +132,7 @@ router_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
             p.advance(STAGES);
         }
         stamp(1);
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && elect_one()) {
         PipeState p;
         const uint32_t idesc = idesc_bf16(128, NT);
         bool ok = true;

@@ -114,7 +114,7 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     volatile int *armed_t = reinterpret_cast<volatile int *>(misc + 16 + 32);   // [8] same for the token ring
     volatile WorkSlot *ring = reinterpret_cast<volatile WorkSlot *>(misc + 16 + 64);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < WS; s++) { mbar_init(wfull_bar(s), 1); mbar_init(wempty_bar(s), 1); }
@@ -147,7 +147,7 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     const int n_tt = __ldcg(n_ttiles);
     const int n_work = tile_bounds ? min(tile_bounds[tile_group + 1], n_tt) * C::MTILES : n_tt * C::MTILES;
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
         // ---------------------------------------------------------- scheduler + weight producer
         // Claiming and decoding an item costs an atomic and two dependent global loads (~2 us).
         // They are software-pipelined behind the TMA issue loop: while item i is being loaded,
@@ -282,7 +282,7 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             for (int i = 0; i < OMNI_TILE_N / 8; i++) off[i] = off_next[i];
         }
         cp_async_wait<0>();
-    } else if (warp == 3 && lane == 0) {
+    } else if (warp == 3 && elect_one()) {
         // ---------------------------------------------------------- token producer
         PipeState p, wr;
         const uint64_t pol_t = l2_policy_evict_last();
@@ -325,7 +325,7 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 p.advance(TS);
             }
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && elect_one()) {
         // ---------------------------------------------------------- MMA issuer
         PipeState pw, pt, wr;
         bool ok = true;

@@ -412,7 +412,7 @@ def ours(args):
                     "regions": len(e2e_regions), "note": "host-buffer call clef_omni_forward_host on layer 0, pinned host memory"},
             "gpu_launches": launches * args.steps,
             "clocks": clock_summary,
-            "roofline": {"bound": "tensor", "kernel": "expert_gemm_kernel<gate_up+SwiGLU>", "achieved": achieved,
+            "roofline": {"bound": "tensor", "kernel": "expert_pair_kernel<gate_up+SwiGLU>", "achieved": achieved,
                          "peak": peaks["bf16_tflops"], "unit": "TFLOP/s", "frac": achieved / peaks["bf16_tflops"],
                          "peak_source": peaks["source"] + " burst cuBLAS bf16 figure; regime of the timed regions: " + regime(clock_summary),
                          "peak_sustained": peaks["bf16_tflops_sustained"], "frac_of_sustained": achieved / peaks["bf16_tflops_sustained"],

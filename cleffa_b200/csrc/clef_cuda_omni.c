@@ -6,7 +6,7 @@
  * becomes a CUDA stream; "encode" only enqueues work and errors surface at completion, as in
  * the reference (clef_metal.m:1591-1597).
  *
- * There is no CPU fallback: every stage is a CUDA kernel (omni_kernels.cu, omni_sm100.cu).
+ * There is no CPU fallback: every stage is a CUDA kernel (omni_kernels.cu, omni_router.cu, omni_expert.cu, omni_attn.cu).
  */
 #define _GNU_SOURCE
 #include "clef_cuda_omni.h"
@@ -28,7 +28,7 @@ typedef struct {
     float *bias;                        /* device, FP32 [128] or NULL */
     bool owned, bound;
     CUtensorMap tm_router, tm_gate_up, tm_down;
-    CUtensorMap tm_gate_up3;            /* {K, gate|up, row} view of gate_up: a box interleaves gate and up rows */
+    CUtensorMap tm_gate_up4;            /* {K, row, gate|up, block} view of gate_up: a box interleaves blocks of gate and up rows */
 } omni_layer;
 
 /* The scratch arena (clef_omni_gpu in the reference, clef_metal_omni.m:18-23). */
@@ -41,7 +41,7 @@ typedef struct {
     unsigned long long *stamps;         /* [CHUNK/128][8] optional router timestamps */
     omni_sort_state sort;
     void *xg, *h, *d;                   /* permuted rows: BF16 [ROWS][2048], [ROWS][768], [ROWS][2048] */
-    CUtensorMap tm_xg[4], tm_h[4];      /* box heights 32, 64, 128, 256 rows */
+    CUtensorMap tm_xg[OMNI_TOK_BOXES], tm_h[OMNI_TOK_BOXES];
     size_t bytes;
 } omni_arena;
 
@@ -66,10 +66,10 @@ struct clef_gpu {
     } attn[MAX_LAYERS];
     struct {
         void *p, *q, *k, *vt, *a;          /* BF16: q|k|v rows [CHUNK][5120]; Q [32][CHUNK][128]; K [4][CHUNK][128]; Vt [4][128][VPITCH]; attention output [CHUNK][4096] */
-        int32_t *tiles, *vcol, *sched;     /* device: query tiles, Vt column of every token, work counters of the two projections */
+        int32_t *tiles, *vcol;             /* device: query tiles, Vt column of every token */
         int32_t *h_tiles, *h_vcol, *h_bounds;   /* host copies; h_bounds remembers the batch the device copies describe */
         int n_tiles, last_T, last_nseq;
-        CUtensorMap tm_xn[4], tm_a[4], tm_q, tm_k, tm_vt;
+        CUtensorMap tm_xn[OMNI_TOK_BOXES], tm_a[OMNI_TOK_BOXES], tm_q, tm_k, tm_vt;
         bool ready;
     } at;
     /* route capture */
@@ -81,9 +81,8 @@ struct clef_gpu {
     int ep_fused;                       /* expert parallelism: the expert kernels move the rows themselves (default 1) */
     float router_eps;
     int gemm_impl, router_impl;         /* 0 = tcgen05, 1 = CUDA-core check kernels */
-    int expert_chain;                   /* 1: on one GPU the down kernel is chained behind gate/up per expert (default 0: worth ~1 % only while the GPU is cool) */
     int expert_kernel;                  /* tcgen05 expert products: 2 = pairs of CTAs (cta_group::2), 1 = the same kernel on
-                                           single CTAs, 0 = the earlier single-CTA kernels (two accumulators for gate/up) */
+                                           single CTAs, 0 = chosen from the number of tokens */
     int reserve_sms;                    /* SMs the persistent expert kernels leave to other streams */
     int host_pieces;                    /* clef_omni_forward_host: pieces the batch is cut into (0 = chosen from T) */
     int fused_router;                   /* the router kernel counts experts per sort segment (no histogram kernel) */
@@ -167,14 +166,15 @@ static bool make_map(clef_gpu *g, CUtensorMap *map, const void *base, uint64_t r
 }
 
 /* The gate/up matrix of the bound experts, [n_expert][gate rows 0..767 ; up rows 0..767][2048], as a
- * three-dimensional tensor {K, 2, row}: coordinate (k, 0, e*1536 + f) with box {64, 2, 64} brings
- * gate row f+i and up row f+i (i < 64) of expert e into consecutive shared-memory rows 2i, 2i+1. */
-static bool make_gate_up3(clef_gpu *g, CUtensorMap *map, const void *base, uint64_t n_expert) {
-    const cuuint64_t dims[3] = {OMNI_H, 2, n_expert * 2 * OMNI_F - OMNI_F};
-    const cuuint64_t strides[2] = {(cuuint64_t)OMNI_F * OMNI_H * 2, (cuuint64_t)OMNI_H * 2};
-    const cuuint32_t box[3] = {64, 2, 64};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    return g->encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, (void *)base, dims, strides, box, estr,
+ * four-dimensional tensor {K, row of 16, gate|up, block of 16 rows}: coordinate (k, 0, 0, e*96 + b) with box
+ * {64, 16, 2, 4} brings gate rows 16b..16b+15, up rows 16b.., gate rows 16(b+1).. and so on (64 of
+ * each) of expert e into consecutive shared-memory rows. */
+static bool make_gate_up4(clef_gpu *g, CUtensorMap *map, const void *base, uint64_t n_expert) {
+    const cuuint64_t dims[4] = {OMNI_H, 16, 2, (n_expert * 2 * OMNI_F - OMNI_F) / 16};
+    const cuuint64_t strides[3] = {(cuuint64_t)OMNI_H * 2, (cuuint64_t)OMNI_F * OMNI_H * 2, (cuuint64_t)16 * OMNI_H * 2};
+    const cuuint32_t box[4] = {64, 16, 2, 4};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    return g->encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void *)base, dims, strides, box, estr,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -200,7 +200,6 @@ bool clef_cuda_omni_open(clef_gpu **out, int device, void *stream, char *err, si
     g->fused_gather = 1;
     g->fused_router = 1;
     g->ep_fused = 1;
-    g->expert_chain = 0;
     void *fn = NULL;
     enum cudaDriverEntryPointQueryResult qres;
     e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres);
@@ -216,8 +215,7 @@ bool clef_cuda_omni_open(clef_gpu **out, int device, void *stream, char *err, si
         if (e != cudaSuccess) { set_err(err, errlen, "cuda: cannot create stream: %s", cudaGetErrorString(e)); free(g); return false; }
         g->own_stream = true;
     }
-    e = omni_sm100_configure();
-    if (e == cudaSuccess) e = omni_expert_configure();
+    e = omni_expert_configure();
     if (e == cudaSuccess) e = omni_router_configure();
     if (e == cudaSuccess) e = omni_attn_configure();
     if (e != cudaSuccess) {
@@ -310,7 +308,7 @@ bool clef_omni_reserve(clef_gpu *g, const clef_omni_config *c, int T, char *err,
         {(void **)&s->ids, (size_t)OMNI_CHUNK * OMNI_TOP * 4},
         {(void **)&s->weights, (size_t)OMNI_CHUNK * OMNI_TOP * 4},
         {(void **)&s->flag_rows, (size_t)OMNI_CHUNK * 4},
-        {(void **)&s->n_flag, 2048},       /* [0..1] flagged-row counts; from word 64: done[128], done_need[128] */
+        {(void **)&s->n_flag, 256},        /* [0..1] flagged-row counts */
         {(void **)&s->status, 256},
         {(void **)&s->sink, 256},
         {(void **)&s->stamps, (size_t)(OMNI_CHUNK / 32) * 8 * 8},
@@ -335,15 +333,14 @@ bool clef_omni_reserve(clef_gpu *g, const clef_omni_config *c, int T, char *err,
     s->sort.status = s->status;
     s->sort.n_flag = s->n_flag;
     s->sort.longest_first = 1;
+    s->sort.tile_n = OMNI_TILE_N;
     s->sort.ttiles_down = ok ? s->sort.ttiles + OMNI_MAX_TTILES : NULL;
-    s->sort.done = ok ? s->n_flag + 64 : NULL;
-    s->sort.done_need = ok ? s->n_flag + 192 : NULL;
-    for (int i = 0; i < 4 && ok; i++)
-        ok = make_map(g, &s->tm_xg[i], s->xg, OMNI_ROWS, OMNI_H, 32u << i, CU_TENSOR_MAP_L2_PROMOTION_L2_128B) &&
-             make_map(g, &s->tm_h[i], s->h, OMNI_ROWS, OMNI_F, 32u << i, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
+    for (uint32_t i = 0; i < OMNI_TOK_BOXES && ok; i++)
+        ok = make_map(g, &s->tm_xg[i], s->xg, OMNI_ROWS, OMNI_H, 16 * (i + 1), CU_TENSOR_MAP_L2_PROMOTION_L2_128B) &&
+             make_map(g, &s->tm_h[i], s->h, OMNI_ROWS, OMNI_F, 16 * (i + 1), CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
     if (ok) ok = cudaMemsetAsync(s->status, 0, 256, g->stream) == cudaSuccess &&
                  cudaMemsetAsync(s->sink, 0, 256, g->stream) == cudaSuccess &&
-                 cudaMemsetAsync(s->n_flag, 0, 2048, g->stream) == cudaSuccess &&
+                 cudaMemsetAsync(s->n_flag, 0, 256, g->stream) == cudaSuccess &&
                  cudaMemsetAsync(s->sort.n_ttiles, 0, 256, g->stream) == cudaSuccess &&
                  cudaStreamSynchronize(g->stream) == cudaSuccess;
     if (!ok) {
@@ -554,7 +551,7 @@ bool clef_omni_bind_layer(clef_gpu *g, int layer, const void *router, const void
     if (!make_map(g, &next.tm_router, next.router, OMNI_E, OMNI_H, 128, CU_TENSOR_MAP_L2_PROMOTION_L2_128B) ||
         !make_map(g, &next.tm_gate_up, next.gate_up, (uint64_t)EL * 2 * OMNI_F, OMNI_H, 128, CU_TENSOR_MAP_L2_PROMOTION_L2_256B) ||
         !make_map(g, &next.tm_down, next.down, (uint64_t)EL * OMNI_H, OMNI_F, 128, CU_TENSOR_MAP_L2_PROMOTION_L2_256B) ||
-        !make_gate_up3(g, &next.tm_gate_up3, next.gate_up, (uint64_t)EL)) {
+        !make_gate_up4(g, &next.tm_gate_up4, next.gate_up, (uint64_t)EL)) {
         free_layer(&next);
         set_err(err, errlen, "cuda: cannot describe Omni expert tensors of layer %d", layer);
         return false;
@@ -620,31 +617,25 @@ static bool run_experts(clef_gpu *g, const omni_layer *L, const void *xn, const 
                         float *x, int rows, bool have_counts) {
     omni_arena *s = g->omni;
     const int rows8 = rows * OMNI_TOP;
-    if (!launched(g, "assign", omni_launch_assign(ids, rows, s->sort, have_counts, g->stream))) return false;
+    /* pairs of CTAs unless the call says otherwise or the batch is a token or two: then eight to sixteen
+     * experts make fewer pair items (6 of 256 gate/up rows per expert) than there are pairs, and
+     * single CTAs with half the rows each spread over twice as many SMs (1 token: 16 us against 22) */
+    const int ctas = g->expert_kernel ? g->expert_kernel : rows <= 2 ? 1 : 2;
+    omni_sort_state sort = s->sort;
+    sort.tile_n = ctas == 1 ? OMNI_TILE_N1 : OMNI_TILE_N;
+    if (!launched(g, "assign", omni_launch_assign(ids, rows, sort, have_counts, g->stream))) return false;
     /* the tensor-core gate/up kernel fetches its token rows through rowmap itself; the copy
      * into expert order is only made for the check kernels (or when "fused_gather" is 0) */
     const bool fused = g->gemm_impl == 0 && g->fused_gather;
     if (!fused && !launched(g, "gather", omni_launch_gather(xn, s->sort.rowmap, rows8, s->xg, g->stream))) return false;
     stage_mark(g, 2);
-    if (g->gemm_impl == 0 && g->expert_kernel > 0) {
-        const int ctas = g->expert_kernel;
-        if (!launched(g, "gate/up experts", omni_launch_gateup_pair(ctas, &L->tm_gate_up3, s->tm_xg, s->sort, s->h, NULL, NULL, 1, fused ? xn : NULL,
-                                                                    fused ? s->sort.rowmap : NULL, NULL, NULL, g->reserve_sms == 0,
+    if (g->gemm_impl == 0) {
+        if (!launched(g, "gate/up experts", omni_launch_gateup_pair(ctas, &L->tm_gate_up4, s->tm_xg, sort, s->h, NULL, NULL, 1, fused ? xn : NULL,
+                                                                    fused ? s->sort.rowmap : NULL, NULL, NULL, g->reserve_sms == 0, 1,
                                                                     g->n_sm - g->reserve_sms, g->stream))) return false;
         stage_mark(g, 3);
-        if (!launched(g, "down experts", omni_launch_down_pair(ctas, &L->tm_down, s->tm_h, s->sort, s->d, NULL, NULL, g->reserve_sms == 0,
+        if (!launched(g, "down experts", omni_launch_down_pair(ctas, &L->tm_down, s->tm_h, sort, s->d, NULL, NULL, g->reserve_sms == 0,
                                                                g->n_sm - g->reserve_sms, g->stream))) return false;
-    } else if (g->gemm_impl == 0) {
-        /* the down kernel starts on the SMs the first gate/up blocks leave and takes an expert's rows as
-         * soon as they are complete: only when this stream's kernels are chained by dependent launch
-         * and the gate/up grid invites its successor */
-        const int chain = g->expert_chain && g->reserve_sms == 0;
-        if (!launched(g, "gate/up experts", omni_launch_gateup_sm100(&L->tm_gate_up, s->tm_xg, s->sort, s->h, NULL, NULL, 1, fused ? xn : NULL,
-                                                                     fused ? s->sort.rowmap : NULL, g->reserve_sms == 0, chain,
-                                                                     g->n_sm - g->reserve_sms, g->stream))) return false;
-        stage_mark(g, 3);
-        if (!launched(g, "down experts", omni_launch_down_sm100(&L->tm_down, s->tm_h, s->sort, s->d, NULL, 0, g->reserve_sms == 0, chain,
-                                                                g->n_sm - g->reserve_sms, g->stream))) return false;
     } else {
         if (!launched(g, "gate/up experts (check kernel)", omni_launch_gateup_simple(s->xg, L->gate_up, s->sort.offsets, rows8, s->h, g->stream))) return false;
         stage_mark(g, 3);
@@ -676,25 +667,27 @@ static bool run_experts_ep(clef_gpu *g, const omni_layer *L, const void *xn, con
     const omni_ep_peers *pe = &g->ep.peers;
     const int ctas = g->expert_kernel == 1 ? 1 : 2;
     const int n_gemm = g->n_sm - g->reserve_sms;
+    omni_sort_state sort = s->sort;
+    sort.tile_n = ctas == 1 ? OMNI_TILE_N1 : OMNI_TILE_N;
     if (g->ep_fused && !launched(g, "expert-parallel buckets", omni_launch_ep_buckets(ids, rows, pe->world, g->ep.tok_slot, g->ep.bucket_cnt,
                                                                                        g->ep.bucket_list, g->stream))) return false;
-    if (!launched(g, "assign", omni_launch_assign(ids, rows, s->sort, have_counts, g->stream))) return false;
-    if (!launched(g, "expert-parallel plan", omni_launch_ep_plan(pe, ++g->ep.epoch, s->sort, g->ep.send_base, g->ep.n_local_rows, g->ep.need,
+    if (!launched(g, "assign", omni_launch_assign(ids, rows, sort, have_counts, g->stream))) return false;
+    if (!launched(g, "expert-parallel plan", omni_launch_ep_plan(pe, ++g->ep.epoch, sort, g->ep.send_base, g->ep.n_local_rows, g->ep.need,
                                                                  g->ep.bucket_cnt, g->ep.send_cnt, g->ep.recv_base, g->ep.wait_ns, g->stream))) return false;
     if (g->ep_fused) {
         const omni_ep_send send = {g->ep.tok_slot, g->ep.bucket_list, g->ep.send_cnt, g->ep.recv_base, g->ep.send_base,
                                    s->sort.rowmap, s->sort.offsets, xn};
         stage_mark(g, 2);
         /* the token rows arrive once per source token in xg; the kernel gathers each expert's rows from there through grow */
-        if (!launched(g, "gate/up experts + dispatch", omni_launch_gateup_pair(ctas, &L->tm_gate_up3, s->tm_xg, s->sort, s->h, pe->flags[pe->rank] + OMNI_EP_READY_WORD,
+        if (!launched(g, "gate/up experts + dispatch", omni_launch_gateup_pair(ctas, &L->tm_gate_up4, s->tm_xg, s->sort, s->h, pe->flags[pe->rank] + OMNI_EP_READY_WORD,
                                                                                g->ep.need, omni_ep_group_size(pe->world), s->xg, g->ep.grow, pe, &send,
-                                                                               g->reserve_sms == 0, n_gemm, g->stream))) return false;
+                                                                               g->reserve_sms == 0, 0, n_gemm, g->stream))) return false;
     } else {
         if (!launched(g, "expert-parallel dispatch", omni_launch_ep_dispatch(pe, xn, s->sort.rowmap, s->sort.offsets, g->ep.send_base, rows8, 0, g->n_sm, g->stream))) return false;
         if (!launched(g, "expert-parallel barrier", omni_launch_ep_barrier(pe, ++g->ep.epoch, s->status, g->ep.wait_ns, g->stream))) return false;
         stage_mark(g, 2);
-        if (!launched(g, "gate/up experts", omni_launch_gateup_pair(ctas, &L->tm_gate_up3, s->tm_xg, s->sort, s->h, NULL, NULL, 1, NULL, NULL, NULL, NULL,
-                                                                    g->reserve_sms == 0, n_gemm, g->stream))) return false;
+        if (!launched(g, "gate/up experts", omni_launch_gateup_pair(ctas, &L->tm_gate_up4, s->tm_xg, s->sort, s->h, NULL, NULL, 1, NULL, NULL, NULL, NULL,
+                                                                    g->reserve_sms == 0, 0, n_gemm, g->stream))) return false;
     }
     stage_mark(g, 3);
     if (!launched(g, "down experts + return", omni_launch_down_pair(ctas, &L->tm_down, s->tm_h, s->sort, s->d, pe, g->ep.rowinfo, g->reserve_sms == 0, n_gemm, g->stream))) return false;
@@ -999,7 +992,7 @@ bool clef_omni_set_option(clef_gpu *g, const char *name, long value) {
     else if (!strcmp(name, "gemm")) { if (value < 0 || value > 1) return false; g->gemm_impl = (int)value; }
     else if (!strcmp(name, "router")) { if (value < 0 || value > 1) return false; g->router_impl = (int)value; }
     else if (!strcmp(name, "expert_kernel")) { if (value < 0 || value > 2) return false; g->expert_kernel = (int)value; }
-    else if (!strcmp(name, "expert_chain")) g->expert_chain = value != 0;
+    else if (!strcmp(name, "expert_chain")) { /* the down kernel always starts its weight loads under gate/up's tail */ }
     else if (!strcmp(name, "longest_first")) { if (!g->omni) return false; g->omni->sort.longest_first = value != 0; }
     else if (!strcmp(name, "profile")) { g->profile = value != 0; g->prof_passes = 0; }
     else if (!strcmp(name, "debug_stamps")) g->debug_stamps = value != 0;
@@ -1234,7 +1227,7 @@ bool clef_omni_assign_noalloc(const int32_t *ids, int rows, int32_t *counts, int
 enum { ATTN_VPITCH = 2 * OMNI_CHUNK, ATTN_MAX_TILES = OMNI_CHUNK / 128 + 4096 };
 
 static void attn_free(clef_gpu *g) {
-    void *dev[] = {g->at.p, g->at.q, g->at.k, g->at.vt, g->at.a, g->at.tiles, g->at.vcol, g->at.sched};
+    void *dev[] = {g->at.p, g->at.q, g->at.k, g->at.vt, g->at.a, g->at.tiles, g->at.vcol};
     for (size_t i = 0; i < sizeof dev / sizeof dev[0]; i++) if (dev[i]) cudaFree(dev[i]);
     free(g->at.h_tiles); free(g->at.h_vcol); free(g->at.h_bounds);
     memset(&g->at, 0, sizeof g->at);
@@ -1256,7 +1249,6 @@ static bool attn_reserve(clef_gpu *g, char *err, size_t errlen) {
         {&g->at.a, (size_t)OMNI_CHUNK * OMNI_NH * OMNI_HD * 2},
         {(void **)&g->at.tiles, (size_t)ATTN_MAX_TILES * 16},
         {(void **)&g->at.vcol, (size_t)OMNI_CHUNK * 4},
-        {(void **)&g->at.sched, 256},
     };
     void *xnorm = g->xnorm ? g->xnorm : dev_alloc(g, (size_t)OMNI_CHUNK * OMNI_H * 2);
     bool ok = xnorm != NULL;
@@ -1270,16 +1262,16 @@ static bool attn_reserve(clef_gpu *g, char *err, size_t errlen) {
                  cudaMemsetAsync(g->at.k, 0, (size_t)OMNI_NKV * OMNI_CHUNK * OMNI_HD * 2, g->stream) == cudaSuccess &&
                  cudaMemsetAsync(g->at.q, 0, (size_t)OMNI_NH * OMNI_CHUNK * OMNI_HD * 2, g->stream) == cudaSuccess &&
                  cudaStreamSynchronize(g->stream) == cudaSuccess;
-    for (int i = 0; i < 4 && ok; i++)
-        ok = make_map(g, &g->at.tm_xn[i], xnorm, OMNI_CHUNK, OMNI_H, 32u << i, CU_TENSOR_MAP_L2_PROMOTION_L2_128B) &&
-             make_map(g, &g->at.tm_a[i], g->at.a, OMNI_CHUNK, OMNI_NH * OMNI_HD, 32u << i, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
+    for (uint32_t i = 0; i < OMNI_TOK_BOXES && ok; i++)
+        ok = make_map(g, &g->at.tm_xn[i], xnorm, OMNI_CHUNK, OMNI_H, 16 * (i + 1), CU_TENSOR_MAP_L2_PROMOTION_L2_128B) &&
+             make_map(g, &g->at.tm_a[i], g->at.a, OMNI_CHUNK, OMNI_NH * OMNI_HD, 16 * (i + 1), CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
     if (ok) ok = make_map(g, &g->at.tm_q, g->at.q, (uint64_t)OMNI_NH * OMNI_CHUNK, OMNI_HD, 128, CU_TENSOR_MAP_L2_PROMOTION_L2_128B) &&
                  make_map(g, &g->at.tm_k, g->at.k, (uint64_t)OMNI_NKV * OMNI_CHUNK, OMNI_HD, 128, CU_TENSOR_MAP_L2_PROMOTION_L2_128B) &&
                  make_map(g, &g->at.tm_vt, g->at.vt, (uint64_t)OMNI_NKV * OMNI_HD, ATTN_VPITCH, 128, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
     if (!ok) {
         cudaGetLastError();
         if (xnorm && !g->xnorm) cudaFree(xnorm);
-        void *dev[] = {g->at.p, g->at.q, g->at.k, g->at.vt, g->at.a, g->at.tiles, g->at.vcol, g->at.sched};
+        void *dev[] = {g->at.p, g->at.q, g->at.k, g->at.vt, g->at.a, g->at.tiles, g->at.vcol};
         for (size_t i = 0; i < sizeof dev / sizeof dev[0]; i++) if (dev[i]) cudaFree(dev[i]);
         free(g->at.h_tiles); free(g->at.h_vcol); free(g->at.h_bounds);
         memset(&g->at, 0, sizeof g->at);
@@ -1401,15 +1393,14 @@ bool clef_omni_encode_attention(clef_gpu *g, int layer, float *x, const int32_t 
     if (!attn_plan(g, T, n_seq, seq_bounds, err, errlen)) return false;
     omni_arena *s = g->omni;
     bool ok = launched(g, "attention norm", omni_launch_rmsnorm(x, g->attn[layer].norm_w, g->attn[layer].eps, T, g->xnorm, g->stream)) &&
-              launched(g, "projection tiles", omni_launch_dense_tiles(T, s->sort.ttiles, s->sort.n_ttiles, g->at.sched, g->stream)) &&
-              launched(g, "q|k|v projection", omni_launch_dense_pair(0, &g->attn[layer].tm_qkv, g->at.tm_xn, s->sort, g->at.sched, g->at.p, NULL,
+              launched(g, "q|k|v projection", omni_launch_dense_pair(0, &g->attn[layer].tm_qkv, g->at.tm_xn, T, g->at.p, NULL, s->status,
                                                                        g->n_sm, g->stream)) &&
               launched(g, "attention prep", omni_launch_attn_prep(g->at.p, g->attn[layer].q_norm, g->attn[layer].k_norm, pos3, g->at.vcol, T, OMNI_CHUNK,
                                                                    ATTN_VPITCH, g->attn[layer].eps, g->attn[layer].theta, g->at.q, g->at.k, g->at.vt,
                                                                    s->status, g->stream)) &&
               launched(g, "attention", omni_launch_attention(&g->at.tm_q, &g->at.tm_k, &g->at.tm_vt, g->at.tiles, g->at.n_tiles, OMNI_CHUNK, g->at.a,
                                                              s->status, g->stream)) &&
-              launched(g, "output projection", omni_launch_dense_pair(1, &g->attn[layer].tm_out, g->at.tm_a, s->sort, g->at.sched + 1, NULL, x,
+              launched(g, "output projection", omni_launch_dense_pair(1, &g->attn[layer].tm_out, g->at.tm_a, T, NULL, x, s->status,
                                                                         g->n_sm, g->stream));
     if (!ok) { set_err(err, errlen, "%s", g->fail_msg); return false; }
     return true;

@@ -3,8 +3,6 @@
 //                       per head (reference: metal/clef.metal:2073-2130, omni_attn_prep)
 //   attention_kernel    causal grouped-query attention inside each record of the packed batch,
 //                       online softmax (reference: metal/clef.metal:2174-2319, omni_attention)
-//   dense_tiles_kernel  tile list that lets the expert-product kernel (omni_expert.cu) run the
-//                       q|k|v and the output projection as one "expert" over all token rows
 //
 // attention_kernel: one CTA per (query head, query tile of <= 128 rows of ONE record).  Both
 // products run on tcgen05 with operands in 128-byte-swizzled shared memory: S = Q K^T (128 x 128
@@ -28,15 +26,6 @@
 namespace {
 
 constexpr int HD = OMNI_HD, NH = OMNI_NH, NKV = OMNI_NKV;
-
-// ------------------------------------------------------------------ tile list of a dense projection
-__global__ void dense_tiles_kernel(int T, omni_ttile *ttiles, int32_t *n_ttiles, int32_t *counters) {
-    const int nt = (T + OMNI_TILE_N - 1) / OMNI_TILE_N;
-    const int base = T / nt, extra = T % nt;
-    for (int j = threadIdx.x; j < nt; j += blockDim.x)
-        ttiles[j] = omni_ttile{0, j * base + min(j, extra), base + (j < extra), 0 | (nt << 16)};
-    if (threadIdx.x == 0) { *n_ttiles = nt; counters[0] = 0; counters[1] = 0; }
-}
 
 // ------------------------------------------------------------------ q/k norm + rotary + layout
 // One block per token, four warps, nine heads each (32 query heads, then the 4 key heads).  A lane
@@ -491,11 +480,6 @@ extern "C" {
 
 cudaError_t omni_attn_configure(void) {
     return cudaFuncSetAttribute(attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM_BYTES);
-}
-
-cudaError_t omni_launch_dense_tiles(int T, omni_ttile *ttiles, int32_t *n_ttiles, int32_t *counters, cudaStream_t s) {
-    dense_tiles_kernel<<<1, 128, 0, s>>>(T, ttiles, n_ttiles, counters);
-    return cudaGetLastError();
 }
 
 cudaError_t omni_launch_attn_prep(const void *qkv, const float *qw, const float *kw, const int32_t *pos, const int32_t *vcol, int T,

@@ -14,12 +14,14 @@
 // tensor memory), twice buffered, so the epilogue of one item runs under the MMAs of the next.
 //
 // Gate/up: the 128 weight rows of a CTA are 64 gate rows and the 64 up rows of the same
-// intermediate columns, interleaved row by row by a three-dimensional TMA box over the
-// [gate rows; up rows] matrix of the expert.  Gate and up of one column then sit in neighbouring
-// lanes of one accumulator and SwiGLU needs one lane exchange instead of a second accumulator.
+// intermediate columns, interleaved in blocks of 16 by a four-dimensional TMA box over the
+// [gate rows; up rows] matrix of the expert.  Gate and up of one column are then 16 lanes apart in
+// one accumulator and reach the same thread's registers in the two 16-lane loads of a quadrant:
+// SwiGLU needs neither a lane exchange nor a second accumulator.
 //
-// Epilogue: TMEM -> registers -> a row-major tile in shared memory -> whole 128- or 256-byte
-// row pieces written with 16-byte stores.  With expert parallelism the down product writes each
+// Epilogue: TMEM -> registers in the layout of an 8x8 matrix fragment (tcgen05.ld.16x256b) ->
+// stmatrix.trans into a row-major tile in shared memory (four 16-byte rows per lane group instead
+// of one 2-byte store per element) -> whole 128- or 256-byte row pieces written with 16-byte stores.  With expert parallelism the down product writes each
 // row piece straight into the buffer of the rank that owns the token (plain peer stores), so
 // the way back travels under the product, tile by tile, and no separate copy kernel runs.
 //
@@ -117,6 +119,38 @@ __device__ __forceinline__ bool xwait(uint32_t bar, uint32_t parity, const Abort
 template <int CTAS>
 __device__ __forceinline__ bool xwait_item(uint32_t bar, uint32_t parity, const Abort &ab) { return xwait_impl<CTAS == 2>(bar, parity, ab); }
 
+// The same by a whole warp whose lanes stay together: the vote makes the outcome, and with it every
+// stage counter and address of the loop around it, uniform for the compiler.
+template <bool CLUSTER>
+__device__ __forceinline__ bool xwait_warp(uint32_t bar, uint32_t parity, const Abort &ab) {
+    uint64_t t0 = 0;
+    for (int i = 0;; i++) {
+        if (__all_sync(0xffffffffu, CLUSTER ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity))) return true;
+        if ((i & 63) == 63) {
+            if (__any_sync(0xffffffffu, *ab.flag)) return false;
+            const uint64_t t = globaltimer_ns();
+            if (!t0) t0 = t;
+            if (__any_sync(0xffffffffu, t - t0 > WAIT_LIMIT_NS)) {
+                if (elect_one()) ab.raise(OMNI_ST_TIMEOUT);
+                return false;
+            }
+        }
+    }
+}
+__device__ __forceinline__ int uniform_i32(int v) { return __reduce_min_sync(0xffffffffu, v); }
+
+// The same for a wait that is long as a rule and in no hurry: sleeps between polls, so that the
+// warp does not take issue slots from the epilogue warps of its scheduler.
+__device__ __forceinline__ bool xwait_lazy(uint32_t bar, uint32_t parity, const Abort &ab) {
+    const uint64_t t0 = globaltimer_ns();
+    while (!mbar_try_wait(bar, parity)) {
+        __nanosleep(100);
+        if (*ab.flag) return false;
+        if (globaltimer_ns() - t0 > WAIT_LIMIT_NS) { ab.raise(OMNI_ST_TIMEOUT); return false; }
+    }
+    return true;
+}
+
 // TMA loads whose completion is signalled on a barrier of the pair's first CTA.  Each CTA
 // issues its own loads into its own shared memory: nothing here is a multicast.
 template <int CTAS>
@@ -129,15 +163,15 @@ __device__ __forceinline__ void xtma_2d(uint32_t dst, const CUtensorMap *map, in
         tma_load_2d_hint(dst, map, x, y, bar, policy);
 }
 template <int CTAS>
-__device__ __forceinline__ void xtma_3d(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar, uint64_t policy) {
+__device__ __forceinline__ void xtma_4d(uint32_t dst, const CUtensorMap *map, int x, int y, int z, int w, uint32_t bar, uint64_t policy) {
     if (CTAS == 2)
         asm volatile(
-            "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5}], [%2], %6;"
-            ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z), "l"(policy) : "memory");
+            "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5, %6}], [%2], %7;"
+            ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(w), "l"(policy) : "memory");
     else
         asm volatile(
-            "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5}], [%2], %6;"
-            ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z), "l"(policy) : "memory");
+            "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5, %6}], [%2], %7;"
+            ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(w), "l"(policy) : "memory");
 }
 
 template <int CTAS>
@@ -183,19 +217,29 @@ __device__ __forceinline__ void named_bar_sync(int id, int threads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
+// 16 TMEM lanes x 32 columns: register 4i + {0,1} of lane t holds row t/4, columns 8i + 2(t%4) + {0,1},
+// register 4i + {2,3} row t/4 + 8 of the same columns.
+__device__ __forceinline__ void tmem_ld_16x32(uint32_t addr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+          "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(addr) : "memory");
+}
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t *>(&v);
+}
+// four 8x8 matrices, transposed: lane i supplies the address of one 16-byte row
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
 // ------------------------------------------------------------------ configuration
 enum { X_GATEUP = 0, X_DOWN = 1,
        // the two dense projections of the attention half, run as "one expert" over all token rows:
        X_QKV = 2,      // P[T][5120] = xn[T][2048] . W_qkv^T, BF16 out
        X_OPROJ = 3 };  // x[T][2048] += A[T][4096] . W_out^T, added into the FP32 residual
-#ifndef X_GU_WS
-#define X_GU_WS 7
-#define X_GU_TS 5
-#endif
-#ifndef X_DN_WS
-#define X_DN_WS 6
-#define X_DN_TS 4
-#endif
 #ifndef X_GATHER_LAG            /* stages between issuing a gathered stage and handing it to the MMA thread */
 #define X_GATHER_LAG 3
 #endif
@@ -210,13 +254,20 @@ template <> struct XMode<X_OPROJ> { static constexpr int KTOT = OMNI_NH * OMNI_H
 
 template <int MODE, int CTAS> struct XCfg {
     using M = XMode<MODE>;
-    static constexpr int TOK_ROWS = OMNI_TILE_N / CTAS;                 // token rows one CTA stages per K slab
-    static constexpr int T_BYTES = TOK_ROWS * BK * 2;                   // 32 KiB or 16 KiB
+    static constexpr int TOK_ROWS = 128;                                // token rows one CTA stages per K slab: all of a tile, or half
+    static constexpr int T_BYTES = TOK_ROWS * BK * 2;                   // 16 KiB
     static constexpr int W_BYTES = A_TILE_BYTES;                        // 16 KiB: 128 weight rows
-    static constexpr int STAGE_OUT_BYTES = OMNI_TILE_N * M::OUTC * 2;   // 32 KiB (gate/up) or 64 KiB (down)
-    // ring depths (stages of 64 K elements): weights come from HBM, token rows mostly from L2
-    static constexpr int WS = CTAS == 2 ? (MODE == X_GATEUP ? X_GU_WS : X_DN_WS) : 4;
-    static constexpr int TS = CTAS == 2 ? (MODE == X_GATEUP ? X_GU_TS : X_DN_TS) : 3;
+    // the epilogue stages 32 token rows at a time, twice buffered, per half of its warps; the
+    // output projection stores from registers
+    static constexpr int CHUNK_BYTES = 32 * M::OUTC * 2;
+    static constexpr int STAGE_OUT_BYTES = MODE == X_OPROJ ? 0 : 4 * CHUNK_BYTES;   // 16 KiB (gate/up) or 32 KiB
+    // Ring depths (stages of 64 K elements).  A slab lasts 512 clocks at 256 token rows and a load takes
+    // 1500 to 2500 under load, so everything that is not needed elsewhere goes into the rings: with
+    // a whole 64 KiB output tile in shared memory and 4 token stages the dense projections
+    // waited for tokens half of the time (847 clocks per slab).
+    // Single CTAs serve short batches, which stream weights from HBM: fewer token stages there.
+    static constexpr int TS = CTAS == 1 ? 4 : MODE == X_OPROJ ? 7 : 6;
+    static constexpr int WS = (MODE == X_GATEUP ? 13 : MODE == X_OPROJ ? 14 : 12) - TS;
     static constexpr int RING_BYTES = WS * W_BYTES + TS * T_BYTES;
     static constexpr int TOTAL_BYTES = RING_BYTES + STAGE_OUT_BYTES + 1024 + 1024;
     static constexpr int ITEMS_PER_TILE = M::MT / CTAS;
@@ -225,13 +276,12 @@ static_assert(XCfg<X_QKV, 2>::TOTAL_BYTES <= 232448 && XCfg<X_OPROJ, 2>::TOTAL_B
               XCfg<X_GATEUP, 1>::TOTAL_BYTES <= 232448 && XCfg<X_DOWN, 1>::TOTAL_BYTES <= 232448 &&
               XCfg<X_GATEUP, 2>::TOTAL_BYTES <= 232448 && XCfg<X_DOWN, 2>::TOTAL_BYTES <= 232448, "shared memory budget");
 
-constexpr int X_THREADS = 384;      // warp 0 scheduler + weight loads, 1 MMA, 2 TMEM (2+3 gather), 3 token loads, 4..11 epilogue
-constexpr int X_COPY_THREADS = 128; // with COPY: warps 12..15 move this rank's token rows to the other ranks
+constexpr int X_THREADS = 384;      // warp 0 weight loads, 1 MMA, 2 TMEM + scheduler, 3 token loads, 4..11 epilogue
+constexpr int X_GATHER_THREADS = 128;   // gate/up only: warps 12..15 fetch the token rows through the permutation
+constexpr int X_COPY_THREADS = 128; // with COPY: warps 16..19 move this rank's token rows to the other ranks
 constexpr int X_EPI_WARPS = 8;
-constexpr int X_GATHER_THREADS = 64;
+template <int MODE, bool COPY> constexpr int x_threads() { return X_THREADS + (MODE == X_GATEUP ? X_GATHER_THREADS : 0) + (COPY ? X_COPY_THREADS : 0); }
 constexpr int X_RING = 4;
-
-struct XTokMaps { CUtensorMap m[4]; };
 
 struct XArgs {
     const omni_ttile *ttiles;
@@ -256,8 +306,14 @@ struct XArgs {
     omni_ep_send send;                  // what the copy warps send from
     int need_blocks;                    // > 0: an arrival counter is complete at this value (it counts sender blocks), else at need[group]
     int early_dependents;
+    // The weights (and the work list) may be read before the kernel in front has completed: the tile
+    // list is older than that kernel, or (dense projections) there is none.
+    int early_weights;
+    int dense_rows, dense_tiles;        // dense projections: token rows, and the near-equal tiles they are cut into
 };
 
+constexpr int DENSE_MIN = 96, DENSE_ITEM = 16;    // of the choice of tile length in omni_launch_dense_pair, in rows
+constexpr int DENSE_GROUP = 16;     // token tiles (of up to 256 rows, 1 to 2 MiB) that share a sweep over the weight blocks of a dense projection
 struct WorkSlotX { int expert, row0, len, m; };
 
 // silu(g) * u with silu(g) = g * sigmoid(g) = (g/2) * (1 + tanh(g/2)): one special-function
@@ -271,13 +327,13 @@ __device__ __forceinline__ float silu_mul(float g, float u) {
 }
 
 // ====================================================================== the kernel
-// Work distribution as in the single-CTA kernels: an expert-major list of token tiles, items
+// Work distribution: an expert-major list of token tiles, items
 // (token tile, weight block) claimed one at a time from a device counter by the first CTA of the
 // pair, which hands each decoded item to the consumers of BOTH CTAs through a small ring that
 // exists in each CTA's shared memory.
 template <int MODE, int CTAS, bool COPY>
-__global__ void __launch_bounds__(X_THREADS + (COPY ? X_COPY_THREADS : 0), 1)
-expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ XTokMaps tm_tok, const __grid_constant__ XArgs a) {
+__global__ void __launch_bounds__((x_threads<MODE, COPY>()), 1)
+expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ TokMaps tm_tok, const __grid_constant__ XArgs a) {
     using C = XCfg<MODE, CTAS>;
     using M = XMode<MODE>;
     constexpr int KSTAGES = M::KTOT / BK;
@@ -301,19 +357,19 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     auto iempty_bar = [&](int r) { return bar_base + 8u * (2 * WS + 2 * TS + 5 + X_RING + r); };
     constexpr int N_BARS = 2 * WS + 2 * TS + 5 + 2 * X_RING;
     constexpr int MISC_OFF = (N_BARS * 8 + 15) & ~15;            // the item ring is written with 16-byte stores
-    static_assert(MISC_OFF + 16 + 64 + X_RING * 16 <= 1024, "barrier block");
+    static_assert(MISC_OFF + 16 + 80 + X_RING * 16 <= 1024, "barrier block");
     uint8_t *misc = smem_gen + C::RING_BYTES + C::STAGE_OUT_BYTES + MISC_OFF;
     const uint32_t misc_u32 = bar_base + MISC_OFF;
     volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(misc);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(misc + 4);
     volatile int *epi_quit = reinterpret_cast<volatile int *>(misc + 8);        // [2] a warp of this epilogue half gave up
-    volatile int *armed_w = reinterpret_cast<volatile int *>(misc + 16);        // [8] parity armed per weight stage, -1 none
-    volatile int *armed_t = reinterpret_cast<volatile int *>(misc + 16 + 32);   // [8] same for the token ring
-    volatile WorkSlotX *ring = reinterpret_cast<volatile WorkSlotX *>(misc + 16 + 64);
-    const uint32_t ring_u32 = misc_u32 + 16 + 64;
+    volatile int *armed_w = reinterpret_cast<volatile int *>(misc + 16);        // [10] parity armed per weight stage, -1 none
+    volatile int *armed_t = reinterpret_cast<volatile int *>(misc + 16 + 40);   // [10] same for the token ring
+    volatile WorkSlotX *ring = reinterpret_cast<volatile WorkSlotX *>(misc + 16 + 80);
+    const uint32_t ring_u32 = misc_u32 + 16 + 80;
 
     const int warp = warp_index(), lane = threadIdx.x & 31;
-    const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
+    const uint32_t rank = PAIR ? __shfl_sync(0xffffffffu, cluster_ctarank(), 0) : 0u;      // uniform for the compiler, like the warp index
     const bool leader = rank == 0;
     const bool gathering = a.gather_src != nullptr;
     const Abort ab{abort_flag, PAIR ? mapa_u32(misc_u32 + 4, rank ^ 1u) : 0u, a.status};
@@ -322,137 +378,136 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     auto arrive_lead = [&](uint32_t bar) { if (PAIR) mbar_arrive_remote(mapa_u32(bar, 0)); else mbar_arrive(bar); };
 
     if (threadIdx.x == 0) {
-        const int tp = gathering ? 2 : 1;                       // arrivals of a CTA's token producer per item
+        const int tp = gathering ? X_GATHER_THREADS / 32 : 1;                       // arrivals of a CTA's token producer per item
         for (int s = 0; s < WS; s++) { mbar_init(wfull_bar(s), 1); mbar_init(wempty_bar(s), 1); }
         for (int s = 0; s < TS; s++) { mbar_init(tfull_bar(s), gathering ? X_GATHER_THREADS * CTAS : 1); mbar_init(tempty_bar(s), 1); }
-        for (int s = 0; s < 8; s++) { armed_w[s] = -1; armed_t[s] = -1; }
+        for (int s = 0; s < 10; s++) { armed_w[s] = -1; armed_t[s] = -1; }
         for (int b = 0; b < 2; b++) { mbar_init(afull_bar(b), 1); mbar_init(aempty_bar(b), X_EPI_WARPS * CTAS); }
         mbar_init(drain_bar, 1);
-        // consumers of an item: token producer(s), MMA thread and epilogue warps of the first CTA;
-        // weight producer, token producer(s) and epilogue warps of the second
+        // consumers of an item: in either CTA the weight producer, the token producer(s) and the epilogue
+        // warps; in the first also the MMA thread
         for (int r = 0; r < X_RING; r++) {
             mbar_init(ifull_bar(r), 1);
-            mbar_init(iempty_bar(r), (tp + 1 + X_EPI_WARPS) + (PAIR ? 1 + tp + X_EPI_WARPS : 0));
+            mbar_init(iempty_bar(r), 1 + CTAS * (1 + tp + X_EPI_WARPS));
         }
         *abort_flag = 0;
         epi_quit[0] = 0; epi_quit[1] = 0;
         fence_mbar_init();
         prefetch_tmap(&tm_w);
-        for (int i = 0; i < 4; i++) prefetch_tmap(&tm_tok.m[i]);
+        for (int i = 0; i < OMNI_TOK_BOXES; i++) prefetch_tmap(&tm_tok.m[i]);
     }
     // the peer's barriers must exist before anything of this CTA can signal them
     if (PAIR) cluster_sync_all(); else __syncthreads();
     if (warp == 2) xtmem_alloc<CTAS>(smem_u32((const void *)tmem_slot), 512);
-    dep_wait();                 // everything above overlaps the tail of the previous kernel
+    // Everything above overlaps the tail of the previous kernel; so do the first weight loads where
+    // nothing they need comes from it: the rings fill while the previous kernel drains (and the
+    // scheduler and the weight producer wait for it before they exit, see below).
+    const bool early = a.early_weights && (warp == 0 || warp == 2);
+    if (!early) dep_wait();
     if (a.early_dependents) dep_launch();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
-    const int work_lo = 0;
-    const int n_work = *a.n_ttiles * MI;
+    const uint32_t tmem_base = (uint32_t)uniform_i32((int)*tmem_slot);
 
     // weight tile of CTA `rank` for block m of an expert, K slab ks
     auto load_weights = [&](uint32_t dst, int expert, int m, int ks, uint32_t bar, uint64_t pol) {
         const int m_cta = m * CTAS + (int)rank;
-        if (MODE == X_GATEUP) xtma_3d<CTAS>(dst, &tm_w, ks * BK, 0, expert * (2 * OMNI_F) + m_cta * 64, bar, pol);
+        if (MODE == X_GATEUP) xtma_4d<CTAS>(dst, &tm_w, ks * BK, 0, 0, expert * (2 * OMNI_F / 16) + m_cta * 4, bar, pol);
         else xtma_2d<CTAS>(dst, &tm_w, ks * BK, expert * M::OUT_COLS + m_cta * 128, bar, pol);
     };
 
-    if (warp == 0 && leader && elect_one()) {
-        // ---------------------------------------------------------- scheduler + weight producer
-        // Claiming and decoding an item costs an atomic and two dependent global loads; they are
-        // software-pipelined behind the TMA issue loop (item i+1 is decoded and item i+2 claimed
-        // while item i is being loaded).
-        PipeState p, wr;
-        const uint64_t pol_w1 = l2_policy_evict_first(), pol_keep = l2_policy_evict_last();
-        auto lookup = [&](int w, int &m, int &cnt) {          // item -> (weight block m, tile-list index)
-            const omni_ttile t0 = a.ttiles[w / MI];
-            const int first = t0.group & 0xffff;
-            cnt = t0.group >> 16;
-            const int local = w - first * MI;
-            m = local / cnt;
-            return first + local % cnt;
+    if (warp == 2 && leader && elect_one()) {
+        // ---------------------------------------------------------- scheduler
+        // Claims items and hands them, decoded, to the consumers of both CTAs.  Its own warp: an item
+        // costs an atomic, two dependent global loads and a cluster-scope release (about 2 us), which
+        // inside the weight producer's loop held up the loads of every item (12 slabs of 512 clocks in
+        // the down product).  The claim of the item after the next is in flight meanwhile.
+        constexpr bool DENSE = MODE == X_QKV || MODE == X_OPROJ;
+        PipeState wr;
+        // past L1: with early weights the list's writer has completed, but not the kernel in front
+        auto tile_at = [&](int i) {
+            const int4 v = __ldcg(reinterpret_cast<const int4 *>(a.ttiles) + i);
+            return omni_ttile{v.x, v.y, v.z, v.w};
         };
-        int cur_m = 0, cur_cnt = 1;
-        omni_ttile cur = omni_ttile{0, 0, -1, 0};
-        int w0 = work_lo + atomicAdd(a.work_counter, 1);
-        int w1 = work_lo + atomicAdd(a.work_counter, 1);
-        if (w0 < n_work) cur = a.ttiles[lookup(w0, cur_m, cur_cnt)];
+        const int n_work = (DENSE ? a.dense_tiles : __ldcg(a.n_ttiles)) * MI, n_pairs = (int)gridDim.x / CTAS;
+        int w0 = DENSE ? (int)blockIdx.x / CTAS : atomicAdd(a.work_counter, 1);
         for (;;) {
-            if (!xwait<CTAS>(iempty_bar(wr.stage), wr.phase ^ 1u, ab)) break;
-            const int len = cur.len < 0 ? -1 : cur.len;
+            const int w1 = DENSE ? w0 + n_pairs : atomicAdd(a.work_counter, 1);
+            int m = 0;
+            omni_ttile cur = omni_ttile{0, 0, -1, 0};
+            if (DENSE && w0 < n_work) {
+                // equal items, dealt out in turn: the weight blocks of a group of token tiles before the next
+                // group, so that the token rows in use stay in L2
+                const int group = w0 / (DENSE_GROUP * MI), first = group * DENSE_GROUP;
+                const int cnt = min(DENSE_GROUP, a.dense_tiles - first), local = w0 - first * MI;
+                m = local / cnt;
+                const int t = first + local % cnt, base = a.dense_rows / a.dense_tiles, extra = a.dense_rows % a.dense_tiles;
+                cur = omni_ttile{0, t * base + min(t, extra), base + (t < extra), 0};
+            } else if (w0 < n_work) {                         // item -> (weight block m, tile of the expert)
+                const omni_ttile head = tile_at(w0 / MI);
+                const int first = head.group & 0xffff, cnt = head.group >> 16, local = w0 - first * MI;
+                m = local / cnt;
+                cur = tile_at(first + local % cnt);
+            }
+            if (!xwait_lazy(iempty_bar(wr.stage), wr.phase ^ 1u, ab)) break;
             ring[wr.stage].expert = cur.expert; ring[wr.stage].row0 = cur.row0;
-            ring[wr.stage].len = len; ring[wr.stage].m = cur_m;
+            ring[wr.stage].len = cur.len; ring[wr.stage].m = m;
             mbar_arrive(ifull_bar(wr.stage));
             if (PAIR) {
-                st_cluster_v4(mapa_u32(ring_u32 + 16u * wr.stage, 1), cur.expert, cur.row0, len, cur_m);
+                st_cluster_v4(mapa_u32(ring_u32 + 16u * wr.stage, 1), cur.expert, cur.row0, cur.len, m);
                 mbar_arrive_cluster(mapa_u32(ifull_bar(wr.stage), 1));
             }
-            if (len < 0) break;                                // told the consumers to stop
+            if (cur.len < 0) break;                           // told the consumers to stop
             wr.advance(X_RING);
-            const int w2 = work_lo + atomicAdd(a.work_counter, 1);
-            const bool has_next = w1 < n_work;
-            omni_ttile head = omni_ttile{0, 0, 0, 0};
-            if (has_next) head = a.ttiles[w1 / MI];
-            int nxt_m = 0, nxt_cnt = 1;
-            // a weight tile is read once per token tile of its expert: keep it in L2 while the
-            // expert's other token tiles (claimed by neighbouring pairs) still need it
-            const uint64_t pol_w = cur_cnt > 1 ? pol_keep : pol_w1;
-            omni_ttile nxt = omni_ttile{0, 0, -1, 0};
-            bool ok = true;
-            for (int ks = 0; ks < KSTAGES; ks++) {
-                if (ks == KSTAGES / 4 && has_next) {
-                    const int first = head.group & 0xffff;
-                    nxt_cnt = head.group >> 16;
-                    const int local = w1 - first * MI;
-                    nxt_m = local / nxt_cnt;
-                    nxt = a.ttiles[first + local % nxt_cnt];
-                }
-                ok = xwait<CTAS>(wempty_bar(p.stage), p.phase ^ 1u, ab);
-                if (!ok) break;
-                armed_w[p.stage] = (int)p.phase;
-                mbar_expect_tx(wfull_bar(p.stage), CTAS * C::W_BYTES);       // this CTA's tile and the peer's
-                load_weights(smem_base + p.stage * C::W_BYTES, cur.expert, cur_m, ks, lead(wfull_bar(p.stage)), pol_w);
-                p.advance(WS);
-            }
-            if (!ok) break;
-            cur = nxt; cur_m = nxt_m; cur_cnt = nxt_cnt;
-            w1 = w2;
+            w0 = w1;
         }
-    } else if (warp == 0 && !leader && elect_one()) {
-        // ---------------------------------------------------------- weight producer of the second CTA
+    } else if (warp == 0) {
+        // ---------------------------------------------------------- weight producer (of each CTA)
+        // This warp, the token producer's and the MMA issuer's run their loops with all lanes
+        // together and elect a thread only to issue.  With the loop inside the elected branch it
+        // depended on the instantiation whether the compiler kept stages and descriptors in
+        // uniform registers; where it did not, a slab took 770 clocks to issue instead of 512.
         PipeState p, wr;
+        // evict first even when the expert has further token tiles: neighbouring pairs read those at the
+        // same time and meet in L2 all the same (kept with evict_last the weights displaced the
+        // token rows and the results: gate/up at 4096 tokens 190 us, now 179)
         const uint64_t pol_w = l2_policy_evict_first();
         bool ok = true;
         while (ok) {
-            ok = xwait_item<CTAS>(ifull_bar(wr.stage), wr.phase, ab);
+            ok = xwait_warp<PAIR>(ifull_bar(wr.stage), wr.phase, ab);
             if (!ok) break;
-            const int expert = ring[wr.stage].expert, len = ring[wr.stage].len, m = ring[wr.stage].m;
-            arrive_lead(iempty_bar(wr.stage));
+            const int expert = uniform_i32(ring[wr.stage].expert), len = uniform_i32(ring[wr.stage].len), m = uniform_i32(ring[wr.stage].m);
+            if (elect_one()) arrive_lead(iempty_bar(wr.stage));
             wr.advance(X_RING);
             if (len < 0) break;
             for (int ks = 0; ks < KSTAGES; ks++) {
-                ok = xwait<CTAS>(wempty_bar(p.stage), p.phase ^ 1u, ab);
+                ok = xwait_warp<false>(wempty_bar(p.stage), p.phase ^ 1u, ab);
                 if (!ok) break;
-                load_weights(smem_base + p.stage * C::W_BYTES, expert, m, ks, lead(wfull_bar(p.stage)), pol_w);
+                if (elect_one()) {
+                    if (leader) {
+                        armed_w[p.stage] = (int)p.phase;
+                        mbar_expect_tx(wfull_bar(p.stage), CTAS * C::W_BYTES);       // this CTA's tile and the peer's
+                    }
+                    load_weights(smem_base + p.stage * C::W_BYTES, expert, m, ks, lead(wfull_bar(p.stage)), pol_w);
+                }
                 p.advance(WS);
             }
         }
-    } else if ((warp == 2 || warp == 3) && gathering) {
+    } else if (MODE == X_GATEUP && gathering && warp >= 12 && warp < 16) {
         // ---------------------------------------------------------- token producer, gathering
-        // 64 threads fetch this CTA's share of the tile's token rows through the permutation:
+        // 128 threads fetch this CTA's share of the tile's token rows through the permutation:
         // 16-byte asynchronous copies, eight threads per 128-byte row segment, stored in the
         // 128-byte-swizzled layout the MMA descriptors expect (chunk c of row r at c ^ (r & 7)
         // inside its 8-row group).  A stage is handed to the MMA thread two stages after it was
         // issued, once the copies have landed and are ordered before the tensor core's reads.
-        constexpr int LAG = (CTAS == 2 && MODE == X_GATEUP) ? X_GATHER_LAG : 2;
+        constexpr int LAG = CTAS == 2 ? X_GATHER_LAG : 2;
         static_assert(TS > LAG, "token ring too short for the copy lag");
-        constexpr int NR = C::TOK_ROWS / 8;
+        constexpr int RSTEP = X_GATHER_THREADS / 8, NR = C::TOK_ROWS / RSTEP;
         const uint64_t pol_t = l2_policy_evict_last();
-        const int gt = threadIdx.x - 64;
-        const int c = gt & 7, rb = gt >> 3;
-        const uint32_t dst_off = (uint32_t)(rb * 128 + ((c ^ rb) << 4));
+        const int gt = threadIdx.x - X_THREADS;
+        const int c = gt & 7, rb = gt >> 3;                           // chunk of the row segment; first of this thread's rows
+        const uint32_t dst_off = (uint32_t)(rb * 128 + ((c ^ (rb & 7)) << 4));
         const char *src0 = reinterpret_cast<const char *>(a.gather_src) + c * 16;
         PipeState p, pend, wr;
         int off[NR], off_next[NR];
@@ -492,7 +547,7 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             const int first = (int)rank * share;
 #pragma unroll
             for (int i = 0; i < NR; i++) {
-                const int r = rb + 8 * i;
+                const int r = rb + RSTEP * i;
                 o[i] = (r < share && first + r < len) ? __ldcv(a.gather_rows + row0 + first + r) * (OMNI_H * 2) : -1;
             }
             return len;
@@ -517,7 +572,7 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 const char *src = src0 + ks * (BK * 2);
 #pragma unroll
                 for (int i = 0; i < NR; i++)
-                    if (off[i] >= 0) cp_async16(sb + i * 1024, src + off[i], pol_t);
+                    if (off[i] >= 0) cp_async16(sb + i * (RSTEP * 128), src + off[i], pol_t);
                 cp_async_commit();
                 p.advance(TS);
             }
@@ -535,17 +590,17 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             for (int i = 0; i < NR; i++) off[i] = off_next[i];
         }
         cp_async_wait<0>();
-    } else if (warp == 3 && elect_one()) {
+    } else if (warp == 3 && !gathering) {
         // ---------------------------------------------------------- token producer, TMA
         PipeState p, wr;
         const uint64_t pol_t = l2_policy_evict_last();
         int ready_group = -1;
         bool ok = true;
         while (ok) {
-            ok = xwait_item<CTAS>(ifull_bar(wr.stage), wr.phase, ab);
+            ok = xwait_warp<PAIR>(ifull_bar(wr.stage), wr.phase, ab);
             if (!ok) break;
-            const int row0 = ring[wr.stage].row0, len = ring[wr.stage].len, expert = ring[wr.stage].expert;
-            arrive_lead(iempty_bar(wr.stage));
+            const int row0 = uniform_i32(ring[wr.stage].row0), len = uniform_i32(ring[wr.stage].len), expert = uniform_i32(ring[wr.stage].expert);
+            if (elect_one()) arrive_lead(iempty_bar(wr.stage));
             wr.advance(X_RING);
             if (len < 0) break;
             if (a.ready && expert / a.group_size != ready_group) {
@@ -554,10 +609,10 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 const int grp = expert / a.group_size;
                 const uint32_t want = a.need_blocks ? (uint32_t)a.need_blocks : (uint32_t)a.need[grp];
                 const uint64_t t0 = globaltimer_ns();
-                while (ld_acquire_sys_u32(a.ready + grp) != want) {
+                while (!__all_sync(0xffffffffu, ld_acquire_sys_u32(a.ready + grp) == want)) {
                     __nanosleep(500);
-                    if (*abort_flag || globaltimer_ns() - t0 > WAIT_LIMIT_NS) {
-                        ab.raise(OMNI_ST_TIMEOUT | OMNI_ST_TIMEOUT_ARRIVAL);
+                    if (__any_sync(0xffffffffu, *abort_flag || globaltimer_ns() - t0 > WAIT_LIMIT_NS)) {
+                        if (elect_one()) ab.raise(OMNI_ST_TIMEOUT | OMNI_ST_TIMEOUT_ARRIVAL);
                         ok = false;
                         break;
                     }
@@ -568,62 +623,66 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             }
             const int share = ((len + 15) & ~15) / CTAS;
             const int bi = tok_box_index(share);
-            const uint32_t bytes = (32u << bi) * (BK * 2);
+            const uint32_t bytes = tok_box_bytes(bi);
             for (int ks = 0; ks < KSTAGES; ks++) {
-                ok = xwait<CTAS>(tempty_bar(p.stage), p.phase ^ 1u, ab);
+                ok = xwait_warp<false>(tempty_bar(p.stage), p.phase ^ 1u, ab);
                 if (!ok) break;
-                if (leader) {
-                    armed_t[p.stage] = (int)p.phase;
-                    mbar_expect_tx(tfull_bar(p.stage), CTAS * bytes);
+                if (elect_one()) {
+                    if (leader) {
+                        armed_t[p.stage] = (int)p.phase;
+                        mbar_expect_tx(tfull_bar(p.stage), CTAS * bytes);
+                    }
+                    xtma_2d<CTAS>(tok_base + p.stage * C::T_BYTES, &tm_tok.m[bi], ks * BK, row0 + (int)rank * share,
+                                  lead(tfull_bar(p.stage)), pol_t);
                 }
-                xtma_2d<CTAS>(tok_base + p.stage * C::T_BYTES, &tm_tok.m[bi], ks * BK, row0 + (int)rank * share,
-                              lead(tfull_bar(p.stage)), pol_t);
                 p.advance(TS);
             }
         }
-    } else if (warp == 1 && leader && elect_one()) {
+    } else if (warp == 1 && leader) {
         // ---------------------------------------------------------- MMA issuer (first CTA of the pair)
         PipeState pw, pt, wr;
         bool ok = true;
         for (int it = 0; ok; it++) {
-            ok = xwait_item<CTAS>(ifull_bar(wr.stage), wr.phase, ab);
+            ok = xwait_warp<PAIR>(ifull_bar(wr.stage), wr.phase, ab);
             if (!ok) break;
-            const int len = ring[wr.stage].len;
-            mbar_arrive(iempty_bar(wr.stage));
+            const int len = uniform_i32(ring[wr.stage].len);
+            if (elect_one()) mbar_arrive(iempty_bar(wr.stage));
             wr.advance(X_RING);
             if (len < 0) break;
             const int n_mma = (len + 15) & ~15;
             const uint32_t idesc = idesc_bf16(128 * CTAS, n_mma);
             const int buf = it & 1;
-            const uint32_t use = (uint32_t)(it >> 1);
-            ok = xwait<CTAS>(aempty_bar(buf), (use & 1u) ^ 1u, ab);
+            ok = xwait_warp<false>(aempty_bar(buf), ((uint32_t)(it >> 1) & 1u) ^ 1u, ab);
             if (!ok) break;
             tc_fence_after();
             const uint32_t d0 = tmem_base + buf * 256;
             for (int ks = 0; ks < KSTAGES; ks++) {
-                ok = xwait<CTAS>(wfull_bar(pw.stage), pw.phase, ab) && xwait<CTAS>(tfull_bar(pt.stage), pt.phase, ab);
+                ok = xwait_warp<false>(wfull_bar(pw.stage), pw.phase, ab) && xwait_warp<false>(tfull_bar(pt.stage), pt.phase, ab);
                 if (!ok) break;
                 tc_fence_after();
-                const uint64_t da = smem_desc_sw128(smem_base + pw.stage * C::W_BYTES);
-                const uint64_t db = smem_desc_sw128(tok_base + pt.stage * C::T_BYTES);
+                if (elect_one()) {
+                    const uint64_t da = smem_desc_sw128(smem_base + pw.stage * C::W_BYTES);
+                    const uint64_t db = smem_desc_sw128(tok_base + pt.stage * C::T_BYTES);
 #pragma unroll
-                for (int k = 0; k < BK / 16; k++) xmma<CTAS>(d0, da + 2u * k, db + 2u * k, idesc, (ks | k) ? 1u : 0u);
-                xcommit<CTAS>(wempty_bar(pw.stage));     // both stages are free (in both CTAs) once these MMAs have read them
-                xcommit<CTAS>(tempty_bar(pt.stage));
+                    for (int k = 0; k < BK / 16; k++) xmma<CTAS>(d0, da + 2u * k, db + 2u * k, idesc, (ks | k) ? 1u : 0u);
+                    xcommit<CTAS>(wempty_bar(pw.stage));     // both stages are free (in both CTAs) once these MMAs have read them
+                    xcommit<CTAS>(tempty_bar(pt.stage));
+                    if (ks == KSTAGES - 1) xcommit<CTAS>(afull_bar(buf));        // accumulator complete, in both CTAs
+                }
+                __syncwarp();
                 pw.advance(WS);
                 pt.advance(TS);
             }
-            if (!ok) break;
-            xcommit<CTAS>(afull_bar(buf));               // accumulator complete, in both CTAs
         }
-        // Whatever happened, wait (bounded) until every MMA issued by this thread retired
-        // before tensor memory is released.
-        xcommit<CTAS>(drain_bar);
-        {
+        // Whatever happened, wait (bounded) until every MMA issued by this warp's elected thread has
+        // retired before tensor memory is released.
+        if (elect_one()) {
+            xcommit<CTAS>(drain_bar);
             const uint64_t t0 = globaltimer_ns();
             while (!mbar_try_wait(drain_bar, 0) && globaltimer_ns() - t0 < WAIT_LIMIT_NS) {}
         }
-    } else if (COPY && warp >= 12) {
+        __syncwarp();
+    } else if (COPY && warp >= 16) {
         // ---------------------------------------------------------- dispatch of this rank's token rows
         // (expert parallelism): each token once per owner rank, plain peer stores into the owners'
         // receive buffers, group by group, each group announced on the owner's arrival counter --
@@ -631,19 +690,19 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         // the copy warps of one CTA.
         const int nvb = (int)gridDim.x - (int)gridDim.x % a.pe.world;
         if ((int)blockIdx.x < nvb)
-            ep_dispatch_dedup(a.pe, a.send, (int)blockIdx.x, nvb, warp - 12, X_COPY_THREADS / 32, lane, threadIdx.x == X_THREADS,
+            ep_dispatch_dedup(a.pe, a.send, (int)blockIdx.x, nvb, warp - 16, X_COPY_THREADS / 32, lane, threadIdx.x == X_THREADS + X_GATHER_THREADS,
                               [] { named_bar_sync(3, X_COPY_THREADS); });
     } else if (warp >= 4 && warp < 12) {
         // ---------------------------------------------------------- epilogue: TMEM -> registers -> shared -> HBM
-        // Each half stages its token rows in its own 128 rows of the shared-memory tile (which rows
-        // of an item fall to which half changes from item to item, and the halves do not wait for
-        // one another).  The four warps of a half meet at a named barrier twice per item.  A warp whose wait ran
-        // out must therefore not leave on its own: it marks the half as giving up, still joins the
-        // first barrier, and all four leave together right after it.
+        // The two halves split an item's 32-row chunks and do not wait for one another.  A half's four
+        // warps (one per TMEM quadrant, i.e. 32 accumulator rows each) write a chunk's columns into
+        // a shared-memory tile, meet at a named barrier and store whole row pieces; the next chunk
+        // uses the other of two tiles, so one barrier per chunk is enough.  They also meet before
+        // the first chunk of an item: a warp whose wait ran out marks the half there and all four
+        // leave together.
         const int q = warp & 3;                       // TMEM lane quadrant this warp may read
-        const int half = (warp - 4) >> 2;             // the two warps of a quadrant split the token rows
+        const int half = (warp - 4) >> 2;
         const int th = ((warp - 4) & 3) * 32 + lane;  // thread index inside the half (0..127)
-        unsigned short *const tile16 = reinterpret_cast<unsigned short *>(out_tile);
         PipeState wr;
         for (int it = 0;; it++) {
             int row0 = 0, len = 0, m = 0;
@@ -659,65 +718,96 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             const int nchunk = (len + 31) >> 5;
             const int c_lo = half ? (nchunk + 1) >> 1 : 0, c_hi = half ? nchunk : (nchunk + 1) >> 1;
             if (got && !stop) got = xwait<CTAS>(afull_bar(buf), (uint32_t)(it >> 1) & 1u, ab);
-            if (got && !stop) {
-                tc_fence_after();
-                const uint32_t t0 = tmem_base + ((uint32_t)(q * 32) << 16) + buf * 256;
-                for (int c = c_lo; c < c_hi; c++) {
-                    uint32_t v[32];
-                    tmem_ld32(t0 + c * 32, v);
-                    tmem_ld_wait();
-                    if (MODE == X_GATEUP) {
-                        // lanes 2i / 2i+1 hold gate / up of intermediate column i of this quadrant's
-                        // sixteen; the even lane finishes token row c*32+j, the odd one row c*32+j+1
-                        const int col = q * 16 + (lane >> 1), odd = lane & 1;
-#pragma unroll
-                        for (int j = 0; j < 32; j += 2) {
-                            const uint32_t send = odd ? v[j] : v[j + 1];
-                            const uint32_t recv = __shfl_xor_sync(0xffffffffu, send, 1);
-                            const float hv = odd ? silu_mul(__uint_as_float(recv), __uint_as_float(v[j + 1]))
-                                                 : silu_mul(__uint_as_float(v[j]), __uint_as_float(recv));
-                            tile16[(half * 128 + (c - c_lo) * 32 + j + odd) * M::OUTC + col] = __bfloat16_as_ushort(__float2bfloat16(hv));
-                        }
-                    } else if (MODE == X_OPROJ) {
-                        // added into the FP32 residual: a warp's 32 lanes are 32 consecutive columns of one row
-                        float *xr = a.resid + (long)(row0 + c * 32) * M::OUT_COLS + (m * CTAS + (int)rank) * M::OUTC + q * 32 + lane;
-#pragma unroll
-                        for (int j = 0; j < 32; j++)
-                            if (c * 32 + j < len) xr[(long)j * M::OUT_COLS] += __uint_as_float(v[j]);
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 32; j++)
-                            tile16[(half * 128 + (c - c_lo) * 32 + j) * M::OUTC + q * 32 + lane] = __bfloat16_as_ushort(__float2bfloat16(__uint_as_float(v[j])));
-                    }
-                }
-                // tensor memory goes back to the MMA thread before the stores to HBM start
+            if (!got) epi_quit[half] = 1;
+            named_bar_sync(1 + half, 128);
+            if (stop || epi_quit[half]) break;
+            tc_fence_after();
+            const uint32_t t0 = tmem_base + ((uint32_t)(q * 32) << 16) + buf * 256;
+            const int m_cta = m * CTAS + (int)rank;
+            if (c_lo == c_hi) {                       // nothing for this half: hand tensor memory back
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) arrive_lead(aempty_bar(buf));
             }
-            if (!got) epi_quit[half] = 1;
-            named_bar_sync(1 + half, 128);            // the four quadrants of this half have written their columns
-            if (stop || epi_quit[half]) break;
-            const int r_lo = c_lo * 32, r_hi = MODE == X_OPROJ ? 0 : min(len, c_hi * 32);    // the output projection has stored already
-            constexpr int LANES_PER_ROW = M::OUTC * 2 / 16;              // 8 (gate/up) or 16 (down)
-            const int sub = th % LANES_PER_ROW;
-            const int m_cta = m * CTAS + (int)rank;
-            for (int r = r_lo + th / LANES_PER_ROW; r < r_hi; r += 128 / LANES_PER_ROW) {
-                const uint4 val = *reinterpret_cast<const uint4 *>(out_tile + (half * 128 + r - r_lo) * (M::OUTC * 2) + sub * 16);
-                __nv_bfloat16 *dst_row;
-                if (MODE == X_DOWN && a.rowinfo) {
-                    const int info = __ldg(a.rowinfo + row0 + r);
-                    dst_row = reinterpret_cast<__nv_bfloat16 *>(a.pe.dret[info >> 20]) + (long)(info & 0xfffff) * M::OUT_COLS;
+            for (int c = c_lo; c < c_hi; c++) {
+                auto release = [&] {
+                    // tensor memory goes back to the MMA thread before the last stores to HBM start
+                    if (c != c_hi - 1) return;
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) arrive_lead(aempty_bar(buf));
+                };
+                if constexpr (MODE == X_OPROJ) {
+                    uint32_t v[32];
+                    tmem_ld32(t0 + c * 32, v);
+                    // added into the FP32 residual: a warp's 32 lanes are 32 consecutive columns of one row;
+                    // all loads of the chunk before its stores, so that they are in flight together
+                    float *xr = a.resid + (long)(row0 + c * 32) * M::OUT_COLS + m_cta * M::OUTC + q * 32 + lane;
+                    float old[32];
+#pragma unroll
+                    for (int j = 0; j < 32; j++) old[j] = c * 32 + j < len ? xr[(long)j * M::OUT_COLS] : 0.f;
+                    tmem_ld_wait();
+                    release();
+#pragma unroll
+                    for (int j = 0; j < 32; j++)
+                        if (c * 32 + j < len) xr[(long)j * M::OUT_COLS] = old[j] + __uint_as_float(v[j]);
                 } else {
-                    dst_row = a.out + (long)(row0 + r) * M::OUT_COLS;
+                    // Row j of the tile is token c*32 + j; its 16-byte pieces sit at piece ^ (j & 7), so that neither
+                    // the stmatrix rows (eight tokens, same piece) nor the reads below meet in a bank.
+                    constexpr int PITCH = M::OUTC * 2, PIECES = M::OUTC / 8;
+                    uint8_t *const tile = out_tile + (half * 2 + ((c - c_lo) & 1)) * C::CHUNK_BYTES;
+                    uint32_t lo[16], hi[16];
+                    tmem_ld_16x32(t0 + c * 32, lo);
+                    tmem_ld_16x32(t0 + c * 32 + (16u << 16), hi);
+                    tmem_ld_wait();
+                    release();
+                    const int tok = ((lane >> 4) << 3) | (lane & 7), sub8 = (lane >> 3) & 1;
+                    const uint32_t row_addr = smem_u32(tile) + tok * PITCH;
+                    auto store16 = [&](const uint32_t (&p)[8], int piece) {     // 16 output columns of all 32 tokens
+                        const uint32_t at = row_addr + (((piece + sub8) ^ (tok & 7)) << 4);
+                        stmatrix_x4_trans(at, p[0], p[1], p[2], p[3]);
+                        stmatrix_x4_trans(at + 16 * PITCH, p[4], p[5], p[6], p[7]);
+                    };
+                    if constexpr (MODE == X_GATEUP) {
+                        uint32_t p[8];                    // lanes 0..15 of the quadrant are gate rows, 16..31 the up rows of the same columns
+#pragma unroll
+                        for (int i = 0; i < 8; i++)
+                            p[i] = pack_bf16(silu_mul(__uint_as_float(lo[2 * i]), __uint_as_float(hi[2 * i])),
+                                             silu_mul(__uint_as_float(lo[2 * i + 1]), __uint_as_float(hi[2 * i + 1])));
+                        store16(p, q * 2);
+                    } else {
+                        uint32_t p[8];
+#pragma unroll
+                        for (int i = 0; i < 8; i++) p[i] = pack_bf16(__uint_as_float(lo[2 * i]), __uint_as_float(lo[2 * i + 1]));
+                        store16(p, q * 4);
+#pragma unroll
+                        for (int i = 0; i < 8; i++) p[i] = pack_bf16(__uint_as_float(hi[2 * i]), __uint_as_float(hi[2 * i + 1]));
+                        store16(p, q * 4 + 2);
+                    }
+                    named_bar_sync(1 + half, 128);        // the four quadrants have written their columns
+                    constexpr int LANES_PER_ROW = PIECES;                        // 8 (gate/up) or 16
+                    const int sub = th % LANES_PER_ROW;
+#pragma unroll
+                    for (int i = 0; i < 32 * LANES_PER_ROW / 128; i++) {
+                        const int rr = th / LANES_PER_ROW + i * (128 / LANES_PER_ROW), r = c * 32 + rr;
+                        if (r >= len) break;
+                        const uint4 val = *reinterpret_cast<const uint4 *>(tile + rr * PITCH + ((sub ^ (rr & 7)) << 4));
+                        __nv_bfloat16 *dst_row;
+                        if (MODE == X_DOWN && a.rowinfo) {
+                            const int info = __ldg(a.rowinfo + row0 + r);
+                            dst_row = reinterpret_cast<__nv_bfloat16 *>(a.pe.dret[info >> 20]) + (long)(info & 0xfffff) * M::OUT_COLS;
+                        } else {
+                            dst_row = a.out + (long)(row0 + r) * M::OUT_COLS;
+                        }
+                        *reinterpret_cast<uint4 *>(dst_row + m_cta * M::OUTC + sub * 8) = val;
+                    }
                 }
-                *reinterpret_cast<uint4 *>(dst_row + m_cta * M::OUTC + sub * 8) = val;
             }
-            named_bar_sync(1 + half, 128);            // the tile may be overwritten by the next item
         }
     }
 
     // ---------------------------------------------------------------- teardown
+    if (early) dep_wait();      // no thread may leave before the previous kernel has completed
     tc_fence_before();
     __syncthreads();
     if (*abort_flag && threadIdx.x == 0) {
@@ -741,12 +831,12 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
 namespace {
 
 template <int MODE, int CTAS, bool COPY>
-cudaError_t launch_pair(const CUtensorMap *tm_w, const CUtensorMap *tm_tok4, const XArgs &args, int n_sm, cudaStream_t s) {
-    XTokMaps tok;
-    for (int i = 0; i < 4; i++) tok.m[i] = tm_tok4[i];
+cudaError_t launch_pair(const CUtensorMap *tm_w, const CUtensorMap *tm_tok, const XArgs &args, int n_sm, cudaStream_t s) {
+    TokMaps tok;
+    for (int i = 0; i < OMNI_TOK_BOXES; i++) tok.m[i] = tm_tok[i];
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(n_sm - n_sm % CTAS));
-    cfg.blockDim = dim3(X_THREADS + (COPY ? X_COPY_THREADS : 0));
+    cfg.blockDim = dim3(x_threads<MODE, COPY>());
     cfg.dynamicSmemBytes = XCfg<MODE, CTAS>::TOTAL_BYTES;
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
@@ -787,26 +877,27 @@ cudaError_t omni_expert_configure(void) {
     return set_smem<X_DOWN, 2, false>();
 }
 
-cudaError_t omni_launch_gateup_pair(int ctas, const CUtensorMap *tm_w3, const CUtensorMap *tm_x4, const omni_sort_state st,
+cudaError_t omni_launch_gateup_pair(int ctas, const CUtensorMap *tm_w4, const CUtensorMap *tm_x, const omni_sort_state st,
                                     void *h, const uint32_t *ready, const int32_t *need, int group_size,
                                     const void *gather_src, const int32_t *gather_rows, const omni_ep_peers *dispatch_to,
-                                    const omni_ep_send *send, int early_dependents, int n_sm, cudaStream_t s) {
+                                    const omni_ep_send *send, int early_dependents, int early_weights, int n_sm, cudaStream_t s) {
     XArgs a = {};
     a.ttiles = st.ttiles; a.n_ttiles = st.n_ttiles; a.work_counter = st.sched; a.out = (__nv_bfloat16 *)h; a.status = st.status;
     a.ready = ready; a.need = need; a.group_size = group_size > 0 ? group_size : 1;
     a.gather_src = (const __nv_bfloat16 *)gather_src; a.gather_rows = gather_rows;
     a.early_dependents = early_dependents;
+    a.early_weights = early_weights;
     if (dispatch_to) {
         const int grid = n_sm - n_sm % ctas;
         a.pe = *dispatch_to;
         a.send = *send;
         a.need_blocks = grid - grid % dispatch_to->world;       // every rank launches the same grid
-        return ctas == 2 ? launch_pair<X_GATEUP, 2, true>(tm_w3, tm_x4, a, n_sm, s) : launch_pair<X_GATEUP, 1, true>(tm_w3, tm_x4, a, n_sm, s);
+        return ctas == 2 ? launch_pair<X_GATEUP, 2, true>(tm_w4, tm_x, a, n_sm, s) : launch_pair<X_GATEUP, 1, true>(tm_w4, tm_x, a, n_sm, s);
     }
-    return ctas == 2 ? launch_pair<X_GATEUP, 2, false>(tm_w3, tm_x4, a, n_sm, s) : launch_pair<X_GATEUP, 1, false>(tm_w3, tm_x4, a, n_sm, s);
+    return ctas == 2 ? launch_pair<X_GATEUP, 2, false>(tm_w4, tm_x, a, n_sm, s) : launch_pair<X_GATEUP, 1, false>(tm_w4, tm_x, a, n_sm, s);
 }
 
-cudaError_t omni_launch_down_pair(int ctas, const CUtensorMap *tm_w, const CUtensorMap *tm_h4, const omni_sort_state st,
+cudaError_t omni_launch_down_pair(int ctas, const CUtensorMap *tm_w, const CUtensorMap *tm_h, const omni_sort_state st,
                                   void *d, const omni_ep_peers *return_to, const int32_t *rowinfo, int early_dependents, int n_sm,
                                   cudaStream_t s) {
     XArgs a = {};
@@ -814,19 +905,30 @@ cudaError_t omni_launch_down_pair(int ctas, const CUtensorMap *tm_w, const CUten
     a.out = (__nv_bfloat16 *)d; a.status = st.status; a.group_size = 1;
     if (return_to) { a.pe = *return_to; a.rowinfo = rowinfo; }
     a.early_dependents = early_dependents;
-    return ctas == 2 ? launch_pair<X_DOWN, 2, false>(tm_w, tm_h4, a, n_sm, s) : launch_pair<X_DOWN, 1, false>(tm_w, tm_h4, a, n_sm, s);
+    a.early_weights = 1;                     // the list is older than the gate/up kernel in front
+    return ctas == 2 ? launch_pair<X_DOWN, 2, false>(tm_w, tm_h, a, n_sm, s) : launch_pair<X_DOWN, 1, false>(tm_w, tm_h, a, n_sm, s);
 }
 
-// The dense projections of the attention half on the same kernel: `st` holds a tile list that cuts
-// the T token rows into tiles of one "expert" (omni_launch_dense_tiles), tm_w is the weight matrix
-// [OUT_COLS][K] with a 64 x 128 box, tm_tok4 the token operand with boxes of 32..256 rows.
-cudaError_t omni_launch_dense_pair(int which, const CUtensorMap *tm_w, const CUtensorMap *tm_tok4, const omni_sort_state st,
-                                   int32_t *work_counter, void *out_bf16, float *resid, int n_sm, cudaStream_t s) {
+// The dense projections of the attention half on the same kernel: tm_w is the weight matrix
+// [OUT_COLS][K] with a 64 x 128 box, tm_tok the token operand.  The T token rows are cut into near-equal tiles.
+cudaError_t omni_launch_dense_pair(int which, const CUtensorMap *tm_w, const CUtensorMap *tm_tok, int T, void *out_bf16, float *resid,
+                                   uint32_t *status, int n_sm, cudaStream_t s) {
     XArgs a = {};
-    a.ttiles = st.ttiles; a.n_ttiles = st.n_ttiles; a.work_counter = work_counter;
-    a.out = (__nv_bfloat16 *)out_bf16; a.resid = resid; a.status = st.status; a.group_size = 1;
-    a.early_dependents = 1;
-    return which == 0 ? launch_pair<X_QKV, 2, false>(tm_w, tm_tok4, a, n_sm, s) : launch_pair<X_OPROJ, 2, false>(tm_w, tm_tok4, a, n_sm, s);
+    a.out = (__nv_bfloat16 *)out_bf16; a.resid = resid; a.status = status; a.group_size = 1;
+    a.early_dependents = 1; a.early_weights = 1;
+    a.dense_rows = T;
+    // Tiles: the fewest rounds of the pairs of SMs weighted by what an item of that many rows costs.  A
+    // tile of n rows takes about n/2 clocks per K step of 16 but no less than one of DENSE_MIN rows
+    // (issue and load latency).
+    const int blocks = (which == 0 ? OMNI_QKV : OMNI_H) / 256, pairs = n_sm / 2;
+    long best = -1;
+    for (int nt = (T + OMNI_TILE_N - 1) / OMNI_TILE_N; nt <= T; nt++) {
+        const int rows = ((T + nt - 1) / nt + 15) & ~15;
+        const long rounds = ((long)nt * blocks + pairs - 1) / pairs, cost = rounds * ((rows > DENSE_MIN ? rows : DENSE_MIN) + DENSE_ITEM);
+        if (best < 0 || cost < best) { best = cost; a.dense_tiles = nt; }
+        if (rows <= DENSE_MIN) break;
+    }
+    return which == 0 ? launch_pair<X_QKV, 2, false>(tm_w, tm_tok, a, n_sm, s) : launch_pair<X_OPROJ, 2, false>(tm_w, tm_tok, a, n_sm, s);
 }
 
 }  // extern "C"

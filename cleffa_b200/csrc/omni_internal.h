@@ -18,8 +18,10 @@ enum {
     OMNI_ROWS = OMNI_CHUNK * OMNI_TOP,     /* permuted rows per pass */
     OMNI_SEG = 256,                        /* assignments per sort segment (one warp) */
     OMNI_MAX_SEGS = OMNI_ROWS / OMNI_SEG,
-    OMNI_TILE_N = 256,                     /* token rows per expert-GEMM tile */
-    OMNI_MAX_TTILES = OMNI_ROWS / OMNI_TILE_N + OMNI_E,
+    OMNI_TILE_N = 256,                     /* most token rows per expert-GEMM tile on pairs of CTAs */
+    OMNI_TILE_N1 = 128,                    /* and on single CTAs */
+    OMNI_TOK_BOXES = 16,                   /* tensor maps of a token operand: box i is 16 (i + 1) rows high */
+    OMNI_MAX_TTILES = OMNI_ROWS / OMNI_TILE_N1 + OMNI_E,
 };
 
 /* status word bits (clef_omni_complete) */
@@ -60,8 +62,7 @@ typedef struct {
     int32_t *sched;        /* [8] work counters: [0] gate/up, [1..] down (one per launch group), zeroed by the scan */
     uint32_t *status;      /* [1]                                     */
     int32_t *n_flag;       /* [2] rows flagged for the exact pass: the scan moves [0] to [1] and clears [0] for the next pass */
-    int32_t *done;         /* [128] epilogue warps of the gate/up kernel that have stored their part of an expert's rows; zeroed by the scan (may be NULL) */
-    int32_t *done_need;    /* [128] what done[e] reaches when expert e's rows are complete: 8 warps x 6 weight tiles x token tiles */
+    int32_t tile_n;        /* most rows of a token tile: OMNI_TILE_N or OMNI_TILE_N1, as the expert kernels of the pass take */
     int32_t longest_first; /* tile list in order of falling tile length (else in expert order) */
     omni_ttile *ttiles_down; /* the same tiles in expert order, for the down kernel (may be NULL: it then reads ttiles) */
 } omni_sort_state;
@@ -135,8 +136,6 @@ cudaError_t omni_launch_trace(const float *logits, const float *low, const int32
 cudaError_t omni_noalloc_assign(const int32_t *ids, int rows, int32_t *counts, int32_t *offsets, int32_t *rowmap,
                                 int32_t *slots, uint32_t *status, cudaStream_t s, int *max_rows);
 
-/* ---- tcgen05 kernels (omni_sm100.cu) ---- */
-cudaError_t omni_sm100_configure(void);   /* opt-in shared-memory sizes; call once per device */
 /* ---- router (omni_router.cu) ---- */
 cudaError_t omni_router_configure(void);
 int omni_router_tile(int T, int n_sm);     /* tokens per CTA: 32 while that gives at most one CTA per SM, else 128 */
@@ -148,53 +147,40 @@ cudaError_t omni_launch_router_sm100(const CUtensorMap *tm_x, int nt, const CUte
 /* segcount (may be NULL): the kernel also writes the per-segment expert counts of the counting
  * sort for the ids it selected; omni_launch_recheck must then be given the same pointer so that
  * the rows it re-decides move their counts */
-/* tm_x4 / tm_h4: four maps of the same buffer with box heights 32, 64, 128 and 256 rows */
-/* ready/need (may be NULL): rows that have arrived / must arrive per expert before its token
- * rows may be read (expert parallelism: the rows are written by other GPUs while this runs).
- * gather_src/gather_rows (may be NULL): the kernel fetches token row i of the permuted order from
- * row gather_rows[i] of gather_src ([rows][2048] BF16) itself and tm_x4 is not used */
-cudaError_t omni_launch_gateup_sm100(const CUtensorMap *tm_w, const CUtensorMap *tm_x4, const omni_sort_state st,
-                                     void *h, const uint32_t *ready, const int32_t *need, int group_size,
-                                     const void *gather_src, const int32_t *gather_rows, int early_dependents, int announce,
-                                     int n_sm, cudaStream_t s);
-/* tile_bounds (may be NULL) + group: restrict the launch to tiles [tile_bounds[group], tile_bounds[group+1]).
- * early_dependents (both launchers): let blocks of the next kernel in the stream become resident
- * while this one runs; pass 0 when the grid leaves SMs free for kernels of another stream */
-/* announce (gate/up) + chained (down): the gate/up kernel counts, per expert, the epilogue warps
- * that have stored their rows (st.done); the down kernel launched behind it then does not wait for
- * the whole gate/up grid but, per expert, for st.done[e] to reach st.done_need[e], so its blocks
- * start on the SMs the first gate/up blocks leave while the last ones are still working. */
-cudaError_t omni_launch_down_sm100(const CUtensorMap *tm_w, const CUtensorMap *tm_h4, const omni_sort_state st,
-                                   void *d, const int32_t *tile_bounds, int group, int early_dependents, int chained,
-                                   int n_sm, cudaStream_t s);
-
 /* ---- expert products on pairs of SMs (omni_expert.cu) ---- */
 cudaError_t omni_expert_configure(void);  /* opt-in shared-memory sizes; call once per device */
-/* ctas: 2 = clusters of two CTAs driving tcgen05.mma.cta_group::2, 1 = the same code on single CTAs.
- * tm_w3: three-dimensional map of the gate/up matrix {K, gate|up, row} with box {64, 2, 64}: gate
- * and up rows of the same intermediate column arrive interleaved.  Other arguments as in
- * omni_launch_gateup_sm100. */
-cudaError_t omni_launch_gateup_pair(int ctas, const CUtensorMap *tm_w3, const CUtensorMap *tm_x4, const omni_sort_state st,
+/* ctas: 2 = clusters of two CTAs driving tcgen05.mma.cta_group::2 (st.tile_n = OMNI_TILE_N), 1 = the same
+ * code on single CTAs (OMNI_TILE_N1).
+ * tm_w4: four-dimensional map of the gate/up matrix {K, row, gate|up, block} with box {64, 16, 2, 4}:
+ * gate and up rows arrive interleaved in blocks of 16.
+ * tm_x / tm_h: OMNI_TOK_BOXES maps of the same buffer with box heights of 16, 32 .. 256 rows.
+ * ready/need (may be NULL): arrival counters per group of group_size experts, and what they must reach
+ * before a group's token rows may be read (expert parallelism: the rows are written by other GPUs
+ * while this runs).
+ * gather_src/gather_rows (may be NULL): the kernel fetches token row i of the permuted order from
+ * row gather_rows[i] of gather_src ([rows][2048] BF16) itself and tm_x is not used.
+ * early_dependents: let blocks of the next kernel in the stream become resident while this one runs;
+ * pass 0 when the grid leaves SMs free for kernels of another stream. */
+cudaError_t omni_launch_gateup_pair(int ctas, const CUtensorMap *tm_w4, const CUtensorMap *tm_x, const omni_sort_state st,
                                     void *h, const uint32_t *ready, const int32_t *need, int group_size,
                                     const void *gather_src, const int32_t *gather_rows, const omni_ep_peers *dispatch_to,
-                                    const omni_ep_send *send, int early_dependents, int n_sm, cudaStream_t s);
+                                    const omni_ep_send *send, int early_dependents, int early_weights, int n_sm, cudaStream_t s);
+/* early_weights: the weight loads need not wait for the kernel in front (st's tile list is older than it) */
 /* dispatch_to/send (may be NULL): expert parallelism -- four more warps per CTA send this rank's
  * token rows, each once per owner rank, into the owners' receive buffers (gather_src of the
  * owner) with the row map (gather_rows of the owner) and the origin tags, and count themselves on
  * the owners' arrival counters, which `ready` of every rank waits for, group by group.
  * return_to/rowinfo (may be NULL): result row i is written to row (rowinfo[i] & 0xfffff) of
  * return_to->dret[rowinfo[i] >> 20] (the rank the token came from) instead of row i of d */
-cudaError_t omni_launch_down_pair(int ctas, const CUtensorMap *tm_w, const CUtensorMap *tm_h4, const omni_sort_state st,
+cudaError_t omni_launch_down_pair(int ctas, const CUtensorMap *tm_w, const CUtensorMap *tm_h, const omni_sort_state st,
                                   void *d, const omni_ep_peers *return_to, const int32_t *rowinfo, int early_dependents, int n_sm,
                                   cudaStream_t s);
 
 /* ---- attention half (omni_attn.cu; the two projections run on the kernel of omni_expert.cu) ---- */
 cudaError_t omni_attn_configure(void);
-/* tile list that cuts T token rows into tiles of one "expert"; counters[0..1] are cleared (work counters of the two projections) */
-cudaError_t omni_launch_dense_tiles(int T, omni_ttile *ttiles, int32_t *n_ttiles, int32_t *counters, cudaStream_t s);
 /* which: 0 = q|k|v projection (out_bf16 [T][5120]), 1 = output projection (added into resid [T][2048]) */
-cudaError_t omni_launch_dense_pair(int which, const CUtensorMap *tm_w, const CUtensorMap *tm_tok4, const omni_sort_state st,
-                                   int32_t *work_counter, void *out_bf16, float *resid, int n_sm, cudaStream_t s);
+cudaError_t omni_launch_dense_pair(int which, const CUtensorMap *tm_w, const CUtensorMap *tm_tok, int T, void *out_bf16, float *resid,
+                                   uint32_t *status, int n_sm, cudaStream_t s);
 /* qkv [T][5120] BF16 -> Q [32][T][128], K [4][T][128], Vt [4][128][vpitch] (column vcol[t] for token t), BF16;
  * pos [T][3] positions (temporal, row, column); head_stride: rows between two heads of Q and K */
 cudaError_t omni_launch_attn_prep(const void *qkv, const float *qw, const float *kw, const int32_t *pos, const int32_t *vcol, int T,

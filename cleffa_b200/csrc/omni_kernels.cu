@@ -2,7 +2,8 @@
 // near-tied router rows, deterministic stable counting sort, weighted combine, the RMSNorm in
 // front of the block, plus what the default path only uses for checks or caller-supplied
 // routing: warp-level top-k selection, the stand-alone histogram, the row gather and plain
-// CUDA-core kernels for the two expert products.  The tensor-core kernels live in omni_sm100.cu.
+// CUDA-core kernels for the two expert products.  The tensor-core kernels live in omni_expert.cu,
+// omni_router.cu and omni_attn.cu.
 //
 // Reference behaviour these kernels reproduce (paths inside the reference project):
 //   selection / weights     metal/clef.metal:2347-2394  (omni_route)
@@ -205,14 +206,14 @@ __global__ void __launch_bounds__(1024) assign_scan_kernel(int nseg, omni_sort_s
 #pragma unroll
         for (int gq = 0; gq < 8; gq++) total += part[gq][e];
         rows_incl = total;
-        tiles_incl = (total + OMNI_TILE_N - 1) / OMNI_TILE_N;
+        tiles_incl = (total + st.tile_n - 1) / st.tile_n;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
             const int a = __shfl_up_sync(FULL, rows_incl, d), b = __shfl_up_sync(FULL, tiles_incl, d);
             if (lane >= d) { rows_incl += a; tiles_incl += b; }
         }
         if (lane == 31) { warp_rows[e >> 5] = rows_incl; warp_tiles[e >> 5] = tiles_incl; }
-        tile_cnt[e] = (total + OMNI_TILE_N - 1) / OMNI_TILE_N;
+        tile_cnt[e] = (total + st.tile_n - 1) / st.tile_n;
         tile_key[e] = tile_cnt[e] ? total / tile_cnt[e] : 0;
     }
     __syncthreads();
@@ -226,7 +227,7 @@ __global__ void __launch_bounds__(1024) assign_scan_kernel(int nseg, omni_sort_s
         // Expert-major tile list, the experts in order of falling tile length (ties by id): the work
         // items of the persistent expert kernels are claimed in list order, so the longest come first
         // and the short ones fill the end of the launch.  Rows and offsets stay in expert order.
-        const int nt = (n + OMNI_TILE_N - 1) / OMNI_TILE_N;
+        const int nt = (n + st.tile_n - 1) / st.tile_n;
         const int key = tile_key[e];
         int first = tiles_incl - nt;
         if (st.longest_first) {
@@ -249,9 +250,6 @@ __global__ void __launch_bounds__(1024) assign_scan_kernel(int nseg, omni_sort_s
                 st.ttiles_down[f2 + j] = omni_ttile{e, off + j * base + min(j, extra), base + (j < extra), f2 | (nt << 16)};
         }
         if (e < 8) st.sched[e] = 0;
-        // per expert: how many epilogue warps of the gate/up kernel will report (8 per work item, 6 weight
-        // tiles per token tile), and the count they report into
-        if (st.done) { st.done[e] = 0; st.done_need[e] = 8 * (OMNI_F / 128) * nt; }
         if (e == OMNI_E - 1) *st.n_ttiles = tiles_incl;
         // the router and the exact pass of this chunk are done with the flagged-row count: keep it
         // for introspection and clear it for the next router launch (no memset between passes)
@@ -633,7 +631,7 @@ cudaError_t omni_noalloc_assign(const int32_t *ids, int rows, int32_t *counts, i
     st.segcount = sc->segcount; st.ttiles = sc->ttiles; st.n_ttiles = &sc->n_ttiles; st.sched = sc->sched;
     st.status = status;
     st.n_flag = sc->n_flag;
-    st.done = nullptr; st.done_need = nullptr; st.longest_first = 0; st.ttiles_down = nullptr;
+    st.longest_first = 0; st.tile_n = OMNI_TILE_N; st.ttiles_down = nullptr;
     return omni_launch_assign(ids, rows, st, 0, s);
 }
 

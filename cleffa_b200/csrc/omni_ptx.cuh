@@ -169,11 +169,14 @@ __device__ __forceinline__ uint32_t idesc_bf16(int m, int n) {
 
 constexpr int BK = 64;                       // K elements per pipeline stage (one 128-byte swizzle row)
 constexpr int A_TILE_BYTES = 128 * BK * 2;   // 16 KiB: 128 weight rows
-// Token rows arrive in ONE TMA box per stage; four box heights (32, 64, 128, 256 rows) keep the
-// over-read of a ragged tile below 2x.  Rows past the tile belong to the next expert (or are
-// zero-filled past the buffer): they only feed accumulator columns that are never stored.
-struct TokMaps { CUtensorMap m[4]; };
-__device__ __forceinline__ int tok_box_index(int len) { return len <= 32 ? 0 : len <= 64 ? 1 : len <= 128 ? 2 : 3; }
+// Token rows arrive in ONE TMA box per stage, with a box height for every multiple of 16 rows: a
+// box that is higher than the tile costs shared-memory write bandwidth, which a 135-row tile (a
+// 4096-token batch cuts every expert of 257..300 rows into two) read as 256 rows ran out of.  Rows past
+// the tile belong to the next expert (or are zero-filled past the buffer): they only feed
+// accumulator columns that are never stored.
+struct TokMaps { CUtensorMap m[OMNI_TOK_BOXES]; };
+__device__ __forceinline__ int tok_box_index(int len) { return (len + 15) / 16 - 1; }
+__device__ __forceinline__ uint32_t tok_box_bytes(int bi) { return (uint32_t)(bi + 1) * 16 * (BK * 2); }
 
 struct PipeState {
     int stage = 0; uint32_t phase = 0;

@@ -278,13 +278,11 @@ bool clef_omni_read(clef_gpu *g, const char *what, void *dst, size_t bytes, char
  * results straight to the ranks they belong to; 0: a copy kernel and a barrier in front of the
  * gate/up kernel; same results; must be the same on every rank, as it changes the number of barriers per pass),
  * "expert_kernel" 0/1/2 (2: expert products on pairs of CTAs, tcgen05.mma.cta_group::2; 1: the same
- * kernel on single CTAs; 0: the earlier single-CTA kernels; same results),
+ * kernel on single CTAs; 0, the default: chosen from the number of tokens; same results),
  * "longest_first" 0/1 (default 1: the gate/up kernel claims its work items in order of falling tile length, the
  * short ones filling the end of the launch; 0: in expert order; same results; set after clef_omni_reserve),
- * "expert_chain" 0/1 (default 0; one GPU, single-CTA kernels: the down kernel does not wait for the
- * whole gate/up grid but starts on the SMs its first blocks leave and takes each expert's rows once
- * a per-expert counter says they are complete; same results; about 1 % faster while the GPU is
- * cool, nothing once the power limit sets the clock),
+ * "expert_chain" 0/1 (accepted and without effect: the down kernel always starts its weight loads
+ * under the gate/up kernel's tail),
  * "ep_wait_ms" N (bound on each in-pass wait for other ranks, 0 = 2000), "reserve_sms" N (the persistent expert kernels use all SMs but N, so that kernels of another
  * context on the same GPU -- another micro-batch -- are not locked out while they run),
  * "fused_gather" 0/1 (default 1: the gate/up kernel fetches its token rows through the permutation

@@ -53,6 +53,74 @@ __device__ __forceinline__ void warp_topn(double (&val)[4], int lane, double (&t
     }
 }
 
+// The same order through integer keys and the warp-wide integer reductions, for the exact pass: a
+// round of the shuffle search above costs about 300 clocks (five exchanges of a double and an id), one
+// of these about 60.  Both searches of a row together: a block of 64 to 1030 tokens went from 218.6 to
+// 216.7 us (64) and 239.6 to 238.2 (1030), two layers of 37 tokens from 451.7 to 448.2.
+__device__ __forceinline__ uint32_t ordered_key(float f) {
+    const uint32_t u = __float_as_uint(f);
+    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ float ordered_value(uint32_t k) { return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k); }
+
+// The 8th and 9th largest of the warp's 128 values (equal values count one by one).
+__device__ __forceinline__ void warp_8th_9th(const float (&val)[4], int lane, float &v8, float &v9) {
+    uint32_t k[4], top[9];
+#pragma unroll
+    for (int j = 0; j < 4; j++) k[j] = ordered_key(val[j]);
+#pragma unroll
+    for (int r = 0; r < 9; r++) {
+        const uint32_t mine = max(max(k[0], k[1]), max(k[2], k[3]));
+        top[r] = __reduce_max_sync(FULL, mine);
+        const unsigned holders = __ballot_sync(FULL, mine == top[r]);
+        if (lane == __ffs(holders) - 1) {
+            bool taken = false;
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (!taken && k[j] == mine) { k[j] = 0; taken = true; }           // below the key of every number
+        }
+    }
+    v8 = ordered_value(top[7]);
+    v9 = ordered_value(top[8]);
+}
+
+// warp_topn<8> by keys: the high words decide, the low words and then the ids only among equals.
+// Each reduction is a statement of its own: every lane has to take part, whatever its values are.
+__device__ __forceinline__ void warp_top8(const double (&val)[4], int lane, double (&top_v)[9], int (&top_id)[9]) {
+    uint64_t k[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const uint64_t u = (uint64_t)__double_as_longlong(val[j] + 0.0);           // -0 and +0 are equal
+        k[j] = (u >> 63) ? ~u : (u | 0x8000000000000000ull);
+    }
+#pragma unroll
+    for (int r = 0; r < 8; r++) {
+        uint64_t bk = k[0];
+        double bv = val[0];
+        int bj = 0;
+#pragma unroll
+        for (int j = 1; j < 4; j++) if (k[j] > bk) { bk = k[j]; bv = val[j]; bj = j; }
+        const uint32_t hi = (uint32_t)(bk >> 32), lo = (uint32_t)bk;
+        const uint32_t top_hi = __reduce_max_sync(FULL, hi);
+        bool best = hi == top_hi;
+        unsigned m = __ballot_sync(FULL, best);
+        if (m & (m - 1)) {                                                         // the same in all lanes
+            const uint32_t top_lo = __reduce_max_sync(FULL, best ? lo : 0u);
+            best = best && lo == top_lo;
+            const uint32_t id = best ? (uint32_t)(lane + 32 * bj) : 0xffffffffu;
+            const uint32_t first = __reduce_min_sync(FULL, id);
+            m = __ballot_sync(FULL, best && id == first);
+        }
+        const int src = __ffs(m) - 1;
+        top_v[r] = __shfl_sync(FULL, bv, src);
+        top_id[r] = src + 32 * __shfl_sync(FULL, bj, src);
+        if (lane == src) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) if (j == bj) k[j] = 0;
+        }
+    }
+}
+
 // Lanes 0..7 hold the selected logits; weights are softmax over the selected eight, which
 // equals softmax over all experts renormalised by the selected sum (clef.metal:2393).
 __device__ __forceinline__ void write_selection(const double (&top_v)[9], const int (&top_id)[9], int lane,
@@ -133,31 +201,30 @@ __device__ __forceinline__ void recheck_row(const __nv_bfloat16 *__restrict__ xn
                                             float *__restrict__ weights, int32_t *__restrict__ segcount,
                                             uint32_t *__restrict__ status, double *exact_s, int lane, int warp, Sync sync) {
     exact_s[warp * 32 + lane] = -CUDART_INF;
-    double val[4], approx[4];
+    float approx[4];
     float max_abs = 0.f;
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-        const float f = logits[row * OMNI_E + lane + 32 * j];
-        approx[j] = val[j] = (double)f;
-        max_abs = fmaxf(max_abs, fabsf(f));
+        approx[j] = logits[row * OMNI_E + lane + 32 * j];
+        max_abs = fmaxf(max_abs, fabsf(approx[j]));
     }
 #pragma unroll
     for (int s = 16; s > 0; s >>= 1) max_abs = fmaxf(max_abs, __shfl_xor_sync(FULL, max_abs, s));
     const double bound = (double)omni_row_eps(eps, max_abs);
     const XRow x = load_xrow(xn, row, lane);              // in flight while the threshold is found
-    double top_v[9]; int top_id[9];
-    warp_topn<9>(val, lane, top_v, top_id);               // every warp finds the same threshold
-    const double floor_v = fmin(top_v[7] - 2.0 * bound, top_v[8]);
+    float v8, v9;
+    warp_8th_9th(approx, lane, v8, v9);                   // every warp finds the same threshold
+    const double floor_v = fmin((double)v8 - 2.0 * bound, (double)v9);
     sync();
     int c = 0;
     bool off = false;
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-        unsigned m = __ballot_sync(FULL, approx[j] >= floor_v);
+        unsigned m = __ballot_sync(FULL, (double)approx[j] >= floor_v);
         while (m) {
             const int src = __ffs(m) - 1;
             m &= m - 1;
-            const double a = __shfl_sync(FULL, approx[j], src);
+            const double a = (double)__shfl_sync(FULL, approx[j], src);
             if ((c++ & 3) != warp) continue;              // candidates round-robin over the warps
             const int e = src + 32 * j;
             double v = exact_dot(x, w + (long)e * OMNI_H, lane);
@@ -178,7 +245,7 @@ __device__ __forceinline__ void recheck_row(const __nv_bfloat16 *__restrict__ xn
 #pragma unroll
         for (int j = 0; j < 4; j++) exact[j] = exact_s[lane + 32 * j];
         double fin_v[9]; int fin_id[9];
-        warp_topn<9>(exact, lane, fin_v, fin_id);         // the 9th is unused here
+        warp_top8(exact, lane, fin_v, fin_id);
         const int old_id = lane < 8 ? ids[row * 8 + lane] : 0;
         write_selection(fin_v, fin_id, lane, ids, weights, row);
         if (segcount && lane < 8) {

@@ -131,6 +131,30 @@ def test_expert_kernel_variants_give_the_same_bits(bound0, T, ctas):
         b.set_option("expert_kernel", EXPERT_KERNEL_DEFAULT)
 
 
+@pytest.mark.parametrize("T", [1, 33, 200])
+@pytest.mark.parametrize("delta", [0.0, 2.0**-8])
+def test_exact_pass_orders_paired_experts(backend, weights0, T, delta):
+    """Experts i and i + 64 have the same router row, or rows whose logits differ by 2^-28: every token
+    is decided by the exact pass, among values that are equal or share the upper half of a double.
+    The larger one comes first, equal ones by id."""
+    router, gate_up, down = weights0
+    router = router.clone()
+    router[:, 2047] = 0
+    router[64:] = router[:64]
+    router[64:, 2047] = delta
+    x = orc.make_activations(29, T)
+    x[:, 2047] = 2.0**-20
+    logits = x.double() @ router[:64].double().T
+    top = logits.sort(dim=1, descending=True)
+    assert float((top.values[:, :4] - top.values[:, 1:5]).min()) > 1e-6      # FP64 sums are good to 1e-13
+    first = top.indices[:, :4] + (64 if delta else 0)
+    want = torch.stack((first, first.remainder(64) + (0 if delta else 64)), dim=2).reshape(T, 8)
+    backend.bind_layer(1, router, gate_up, down)
+    got = run_block(backend, 1, x)
+    assert got["rechecked"] == T
+    assert np.array_equal(got["ids"], want.numpy())
+
+
 def test_golden_ids_of_config1(bound0):
     from pathlib import Path
     g = np.load(Path(__file__).resolve().parent / "golden" / "route_c1.npz")

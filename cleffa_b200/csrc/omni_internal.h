@@ -108,10 +108,13 @@ cudaError_t omni_launch_router_simple(const void *xn, const void *router, const 
 cudaError_t omni_launch_select(const float *logits, int T, float eps, int exact_all, int32_t *ids, float *weights,
                                int32_t *flag_rows, int32_t *n_flag, uint32_t *status, cudaStream_t s);
 /* logits: the approximate values on entry; on return every logit the exact pass evaluated holds
- * (float)exact, and low (may be NULL) the remainder (float)(exact - hi) */
+ * (float)exact, and low (may be NULL) the remainder (float)(exact - hi).  prefetch: memory that the
+ * kernel asks to be brought into L2 before it waits for the router, in pieces of OMNI_PREFETCH_PIECE bytes */
+#define OMNI_PREFETCH_PIECE 16384
 cudaError_t omni_launch_recheck(int32_t *segcount, const void *xn, const void *router, const float *bias, float *logits,
                                 float *low, const int32_t *flag_rows, const int32_t *n_flag, int T, float eps,
-                                int32_t *ids, float *weights, uint32_t *status, cudaStream_t s);
+                                int32_t *ids, float *weights, uint32_t *status, const void *prefetch, size_t prefetch_bytes,
+                                cudaStream_t s);
 cudaError_t omni_launch_router_exact(const void *xn, const void *router, const float *bias, int T,
                                      double *logits, cudaStream_t s);
 cudaError_t omni_launch_route_pairs(const float *hi, const float *lo, int rows, int32_t *ids, float *weights,

@@ -83,15 +83,24 @@ __global__ void __launch_bounds__(256) select_kernel(const float *__restrict__ l
     if (close && lane == 0) { const int at = atomicAdd(n_flag, 1); if (at < OMNI_CHUNK) flag_rows[at] = (int32_t)row; }
 }
 
-// One block (four warps) per flagged row.
+// One block (four warps) per flagged row; with eight warps, for fewer rounds of candidates, it measured
+// 3 to 5 us slower from 4096 tokens on.  Its blocks become resident while the router runs, when device
+// memory is idle: with `prefetch` given they ask for that much of the expert weights to be
+// brought into L2 meanwhile.  That takes blocks on every SM: 48 MiB requested by the 37 blocks of a norm
+// kernel held that kernel up by 29 us.
+template <bool PREFETCH>
 __global__ void __launch_bounds__(128) recheck_kernel(const __nv_bfloat16 *__restrict__ xn,
                                                       const __nv_bfloat16 *__restrict__ w,
                                                       const float *__restrict__ bias, float *__restrict__ logits,
                                                       float *__restrict__ low, const int32_t *__restrict__ flag_rows,
                                                       const int32_t *__restrict__ n_flag, int T, float eps,
                                                       int32_t *__restrict__ ids, float *__restrict__ weights,
-                                                      int32_t *__restrict__ segcount, uint32_t *__restrict__ status) {
+                                                      int32_t *__restrict__ segcount, uint32_t *__restrict__ status,
+                                                      const char *prefetch, int prefetch_pieces) {
     __shared__ double exact_s[OMNI_E];
+    if (PREFETCH)
+        for (int i = blockIdx.x + gridDim.x * threadIdx.x; i < prefetch_pieces; i += gridDim.x * blockDim.x)
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(prefetch + (size_t)i * OMNI_PREFETCH_PIECE), "r"(OMNI_PREFETCH_PIECE) : "memory");
     dep_wait();
     dep_launch();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -505,10 +514,13 @@ cudaError_t omni_launch_select(const float *logits, int T, float eps, int exact_
 
 cudaError_t omni_launch_recheck(int32_t *segcount, const void *xn, const void *router, const float *bias, float *logits,
                                 float *low, const int32_t *flag_rows, const int32_t *n_flag, int T, float eps, int32_t *ids,
-                                float *weights, uint32_t *status, cudaStream_t s) {
+                                float *weights, uint32_t *status, const void *prefetch, size_t prefetch_bytes, cudaStream_t s) {
     int blocks = T < 148 * 8 ? T : 148 * 8;
-    return omni_launch_chain(recheck_kernel, dim3(blocks), dim3(128), 0, s, (const __nv_bfloat16 *)xn, (const __nv_bfloat16 *)router, bias, logits,
-                             low, flag_rows, n_flag, T, eps, ids, weights, segcount, status);
+    const int pieces = (int)(prefetch_bytes / OMNI_PREFETCH_PIECE);
+    if (pieces && blocks < 148) blocks = 148;
+    return omni_launch_chain(pieces ? recheck_kernel<true> : recheck_kernel<false>, dim3(blocks), dim3(128), 0, s, (const __nv_bfloat16 *)xn,
+                             (const __nv_bfloat16 *)router, bias, logits, low, flag_rows, n_flag, T, eps, ids, weights, segcount, status,
+                             (const char *)prefetch, pieces);
 }
 
 cudaError_t omni_launch_router_exact(const void *xn, const void *router, const float *bias, int T, double *logits,

@@ -35,6 +35,7 @@
 
 #include "omni_internal.h"
 #include "omni_ep_dev.cuh"
+#include "omni_meet.cuh"
 #include "omni_pdl.cuh"
 #include "omni_ptx.cuh"
 
@@ -362,7 +363,7 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     const uint32_t misc_u32 = bar_base + MISC_OFF;
     volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(misc);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(misc + 4);
-    volatile int *epi_quit = reinterpret_cast<volatile int *>(misc + 8);        // [2] a warp of this epilogue half gave up
+    volatile short *epi_quit = reinterpret_cast<volatile short *>(misc + 8);    // [half][item parity] a warp of this epilogue half gave up
     volatile int *armed_w = reinterpret_cast<volatile int *>(misc + 16);        // [10] parity armed per weight stage, -1 none
     volatile int *armed_t = reinterpret_cast<volatile int *>(misc + 16 + 40);   // [10] same for the token ring
     volatile WorkSlotX *ring = reinterpret_cast<volatile WorkSlotX *>(misc + 16 + 80);
@@ -391,7 +392,7 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             mbar_init(iempty_bar(r), 1 + CTAS * (1 + tp + X_EPI_WARPS));
         }
         *abort_flag = 0;
-        epi_quit[0] = 0; epi_quit[1] = 0;
+        for (int i = 0; i < 4; i++) epi_quit[i] = 0;
         fence_mbar_init();
         prefetch_tmap(&tm_w);
         for (int i = 0; i < OMNI_TOK_BOXES; i++) prefetch_tmap(&tm_tok.m[i]);
@@ -698,8 +699,8 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         // warps (one per TMEM quadrant, i.e. 32 accumulator rows each) write a chunk's columns into
         // a shared-memory tile, meet at a named barrier and store whole row pieces; the next chunk
         // uses the other of two tiles, so one barrier per chunk is enough.  They also meet before
-        // the first chunk of an item: a warp whose wait ran out marks the half there and all four
-        // leave together.
+        // the first chunk of an item: a warp whose wait ran out says so there and all four leave
+        // together.
         const int q = warp & 3;                       // TMEM lane quadrant this warp may read
         const int half = (warp - 4) >> 2;
         const int th = ((warp - 4) & 3) * 32 + lane;  // thread index inside the half (0..127)
@@ -718,9 +719,7 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             const int nchunk = (len + 31) >> 5;
             const int c_lo = half ? (nchunk + 1) >> 1 : 0, c_hi = half ? nchunk : (nchunk + 1) >> 1;
             if (got && !stop) got = xwait<CTAS>(afull_bar(buf), (uint32_t)(it >> 1) & 1u, ab);
-            if (!got) epi_quit[half] = 1;
-            named_bar_sync(1 + half, 128);
-            if (stop || epi_quit[half]) break;
+            if (!warps_meet(epi_quit + 2 * half, it, got, [&] { named_bar_sync(1 + half, 128); }) || stop) break;
             tc_fence_after();
             const uint32_t t0 = tmem_base + ((uint32_t)(q * 32) << 16) + buf * 256;
             const int m_cta = m * CTAS + (int)rank;

@@ -20,6 +20,7 @@
 #include <stdint.h>
 
 #include "omni_internal.h"
+#include "omni_meet.cuh"
 #include "omni_pdl.cuh"
 #include "omni_ptx.cuh"
 
@@ -222,7 +223,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(misc);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(misc + 4);
     volatile int *armed = reinterpret_cast<volatile int *>(misc + 16);         // [5]: q, k stages, v stages (parity of the load in flight, -1 none)
-    volatile int *quit = reinterpret_cast<volatile int *>(misc + 40);          // [2] per head: a softmax thread's wait ran out, all of them leave together
+    volatile int *quit = reinterpret_cast<volatile int *>(misc + 40);          // [head][block parity]: a softmax thread's wait ran out, all of them leave together
     float *xch = reinterpret_cast<float *>(misc + 64);                         // what the two threads of a row tell each other
 
     const int warp = warp_index(), lane = threadIdx.x & 31;
@@ -238,7 +239,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             mbar_init(s_full(s), 1); mbar_init(p_full(s), 256); mbar_init(o_done(s), 1);
         }
         *abort_flag = 0;
-        quit[0] = quit[1] = 0;
+        for (int i = 0; i < 4; i++) quit[i] = 0;
         for (int i = 0; i < 5; i++) armed[i] = -1;
         fence_mbar_init();
         prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_vt);
@@ -334,8 +335,8 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         // Thread (row r, half hf) owns keys hf*64.. of every score block, the P columns that hold
         // them, and head dimensions hf*64.. of the accumulator.  The two threads of a row sit in
         // different warps and exchange their partial maxima through shared memory at the head's
-        // named barrier; a thread whose wait ran out marks `quit` and still joins that barrier,
-        // after which all threads of the head leave together.
+        // named barrier; a thread whose wait ran out says so there, after which all threads of the
+        // head leave together.
         const int x = (warp - 4) >> 3, q4 = warp & 3, hf = ((warp - 4) >> 2) & 1;
         const int r = q4 * 32 + lane;                                             // row inside the tile = TMEM lane
         const uint32_t tmem_s = tmem_base + x * 128 + ((uint32_t)(q4 * 32) << 16);
@@ -343,6 +344,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         float *xc = xch + x * 512;                                                // [parity][half][row]
         const float c = scale * 1.4426950408889634f;                              // scores to log2 units
         float m = 0.f, l = 0.f;
+        auto meet = [&](int block, bool ok) { return warps_meet(quit + 2 * x, block, ok, [&] { asm volatile("bar.sync %0, 256;" ::"r"(1 + x) : "memory"); }); };
         bool alive = true;
         for (int j = 0; j < n_blocks; j++) {
             const int par = j & 1;
@@ -370,11 +372,8 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                     pmax = fmaxf(pmax, mq);
                 }
                 xc[(par * 2 + hf) * 128 + r] = pmax;
-            } else {
-                quit[x] = 1;
             }
-            asm volatile("bar.sync %0, 256;" ::"r"(1 + x) : "memory");
-            if (quit[x]) { alive = false; break; }
+            if (!meet(j, alive)) { alive = false; break; }
             // key 0 of every block is visible to every row (tiles and blocks are both cut from the
             // record's start in steps of 128), so the block maximum is finite
             const float bm = fmaxf(pmax, xc[(par * 2 + (hf ^ 1)) * 128 + r]) * c;
@@ -426,10 +425,8 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         // the row's denominator is the sum of what its two threads added up (same reference maximum in both)
         if (alive) alive = mbar_wait(o_done(x), 0, abort_flag, status);
         alive = __all_sync(0xffffffffu, alive);
-        if (!alive) quit[x] = 1;
         xc[((n_blocks & 1) * 2 + hf) * 128 + r] = l;
-        asm volatile("bar.sync %0, 256;" ::"r"(1 + x) : "memory");
-        if (!quit[x]) {
+        if (meet(n_blocks, alive)) {
             tc_fence_after();
             const float lt = l + xc[((n_blocks & 1) * 2 + (hf ^ 1)) * 128 + r];
             const float inv = lt > 0.f ? 1.f / lt : 0.f;

@@ -1,6 +1,8 @@
-"""The meeting of an epilogue half's four warps (csrc/omni_meet.cuh), compiled for the CPU: whichever
+"""The meeting of warps that share a barrier (csrc/omni_meet.cuh), compiled for the CPU: whichever
 warp's wait runs out at whichever item, and whichever warp is held up right behind a barrier while
-the others run as far as they can, all four leave at the same item and none stays in a barrier."""
+the others run as far as they can, all leave at the same item and none stays in a barrier.  Both users:
+an epilogue half's four warps, and the eight warps of a head's softmax, which meet once more behind
+their loop, however they left it."""
 import shutil
 import subprocess
 from pathlib import Path
@@ -17,9 +19,9 @@ PROGRAM = r"""
 #include <vector>
 #include "omni_meet.cuh"
 
-enum { WARPS = 4, ITEMS = 5 };
+enum { ITEMS = 5 };                                      // WARPS and FINAL (0 or 1) come from the command line
 
-// Barrier over four warps.  A warp that has left never arrives: a meeting that can no longer be
+// Barrier over WARPS warps.  A warp that has left never arrives: a meeting that can no longer be
 // completed is given up and reported.
 struct Half {
     std::mutex m;
@@ -37,7 +39,7 @@ struct Half {
         settle();
         cv.notify_all();
         cv.wait(l, [&] { return generation != g || stuck; });
-        // held up between the barrier and what follows it until the other three have left or wait in the next barrier
+        // held up between the barrier and what follows it until all others have left or wait in the next barrier
         if (warp == slow_warp && item == slow_item) cv.wait(l, [&] { return arrived + left == WARPS - 1 || stuck; });
     }
     void leave() {
@@ -51,9 +53,9 @@ struct Half {
 int main() {
     int bad = 0;
     for (int late = 0; late < WARPS; late++)
-        for (int late_item = 0; late_item < ITEMS; late_item++)
+        for (int late_item = 0; late_item < ITEMS + FINAL; late_item++)
             for (int slow = 0; slow < WARPS; slow++)
-                for (int slow_item = 0; slow_item < ITEMS; slow_item++) {
+                for (int slow_item = 0; slow_item < ITEMS + FINAL; slow_item++) {
                     Half h;
                     h.slow_warp = slow; h.slow_item = slow_item;
                     volatile short quit[2] = {0, 0};
@@ -62,11 +64,11 @@ int main() {
                     for (int w = 0; w < WARPS; w++)
                         t.emplace_back([&, w] {
                             int it = 0;
-                            for (; it < ITEMS; it++) {
-                                const bool ok = !(w == late && it == late_item);
-                                if (!warps_meet(quit, it, ok, [&] { h.barrier(w, it); }) || h.stuck) break;
-                            }
+                            auto meet = [&](int item, bool ok) { return warps_meet(quit, item, ok, [&] { h.barrier(w, item); }); };
+                            for (; it < ITEMS; it++)
+                                if (!meet(it, !(w == late && it == late_item)) || h.stuck) break;
                             last[w] = it;
+                            if (FINAL && meet(ITEMS, it == ITEMS && !(w == late && late_item == ITEMS))) last[w] = ITEMS + 1;
                             h.leave();
                         });
                     for (auto &x : t) x.join();
@@ -80,9 +82,11 @@ int main() {
 
 
 @pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
-def test_all_warps_of_a_half_leave_at_the_same_item(tmp_path):
+@pytest.mark.parametrize("warps, final", [(4, 0), (8, 1)])
+def test_all_warps_leave_at_the_same_item(tmp_path, warps, final):
     src, exe = tmp_path / "meet.cpp", tmp_path / "meet"
     src.write_text(PROGRAM)
-    subprocess.run(["g++", "-std=c++17", "-O1", "-pthread", "-x", "c++", "-I", str(CSRC), str(src), "-o", str(exe)], check=True)
-    out = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-pthread", f"-DWARPS={warps}", f"-DFINAL={final}", "-x", "c++", "-I", str(CSRC), str(src),
+                    "-o", str(exe)], check=True)
+    out = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
     assert out.returncode == 0, f"{out.stdout.strip()} schedules leave a warp behind"

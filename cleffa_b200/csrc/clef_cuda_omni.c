@@ -643,7 +643,7 @@ static bool run_experts(clef_gpu *g, const omni_layer *L, const void *xn, const 
     stage_mark(g, 2);
     if (g->gemm_impl == 0) {
         if (!launched(g, "gate/up experts", omni_launch_gateup_pair(ctas, &L->tm_gate_up4, s->tm_xg, sort, s->h, NULL, NULL, 1, fused ? xn : NULL,
-                                                                    fused ? s->sort.rowmap : NULL, NULL, NULL, g->reserve_sms == 0, 1,
+                                                                    fused ? s->sort.rowmap : NULL, NULL, NULL, g->reserve_sms == 0,
                                                                     g->n_sm - g->reserve_sms, g->stream))) return false;
         stage_mark(g, 3);
         if (!launched(g, "down experts", omni_launch_down_pair(ctas, &L->tm_down, s->tm_h, sort, s->d, NULL, NULL, g->reserve_sms == 0,
@@ -693,13 +693,13 @@ static bool run_experts_ep(clef_gpu *g, const omni_layer *L, const void *xn, con
         /* the token rows arrive once per source token in xg; the kernel gathers each expert's rows from there through grow */
         if (!launched(g, "gate/up experts + dispatch", omni_launch_gateup_pair(ctas, &L->tm_gate_up4, s->tm_xg, s->sort, s->h, pe->flags[pe->rank] + OMNI_EP_READY_WORD,
                                                                                g->ep.need, omni_ep_group_size(pe->world), s->xg, g->ep.grow, pe, &send,
-                                                                               g->reserve_sms == 0, 0, n_gemm, g->stream))) return false;
+                                                                               g->reserve_sms == 0, n_gemm, g->stream))) return false;
     } else {
         if (!launched(g, "expert-parallel dispatch", omni_launch_ep_dispatch(pe, xn, s->sort.rowmap, s->sort.offsets, g->ep.send_base, rows8, 0, g->n_sm, g->stream))) return false;
         if (!launched(g, "expert-parallel barrier", omni_launch_ep_barrier(pe, ++g->ep.epoch, s->status, g->ep.wait_ns, g->stream))) return false;
         stage_mark(g, 2);
         if (!launched(g, "gate/up experts", omni_launch_gateup_pair(ctas, &L->tm_gate_up4, s->tm_xg, s->sort, s->h, NULL, NULL, 1, NULL, NULL, NULL, NULL,
-                                                                    g->reserve_sms == 0, 0, n_gemm, g->stream))) return false;
+                                                                    g->reserve_sms == 0, n_gemm, g->stream))) return false;
     }
     stage_mark(g, 3);
     if (!launched(g, "down experts + return", omni_launch_down_pair(ctas, &L->tm_down, s->tm_h, s->sort, s->d, pe, g->ep.rowinfo, g->reserve_sms == 0, n_gemm, g->stream))) return false;
@@ -1004,7 +1004,7 @@ bool clef_omni_set_option(clef_gpu *g, const char *name, long value) {
     else if (!strcmp(name, "gemm")) { if (value < 0 || value > 1) return false; g->gemm_impl = (int)value; }
     else if (!strcmp(name, "router")) { if (value < 0 || value > 1) return false; g->router_impl = (int)value; }
     else if (!strcmp(name, "expert_kernel")) { if (value < 0 || value > 2) return false; g->expert_kernel = (int)value; }
-    else if (!strcmp(name, "expert_chain")) { /* the down kernel always starts its weight loads under gate/up's tail */ }
+    else if (!strcmp(name, "expert_chain")) { /* belonged to kernels that are gone */ }
     else if (!strcmp(name, "longest_first")) { if (!g->omni) return false; g->omni->sort.longest_first = value != 0; }
     else if (!strcmp(name, "profile")) { g->profile = value != 0; g->prof_passes = 0; }
     else if (!strcmp(name, "debug_stamps")) g->debug_stamps = value != 0;

@@ -307,9 +307,6 @@ struct XArgs {
     omni_ep_send send;                  // what the copy warps send from
     int need_blocks;                    // > 0: an arrival counter is complete at this value (it counts sender blocks), else at need[group]
     int early_dependents;
-    // The weights (and the work list) may be read before the kernel in front has completed: the tile
-    // list is older than that kernel, or (dense projections) there is none.
-    int early_weights;
     int dense_rows, dense_tiles;        // dense projections: token rows, and the near-equal tiles they are cut into
 };
 
@@ -400,11 +397,7 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     // the peer's barriers must exist before anything of this CTA can signal them
     if (PAIR) cluster_sync_all(); else __syncthreads();
     if (warp == 2) xtmem_alloc<CTAS>(smem_u32((const void *)tmem_slot), 512);
-    // Everything above overlaps the tail of the previous kernel; so do the first weight loads where
-    // nothing they need comes from it: the rings fill while the previous kernel drains (and the
-    // scheduler and the weight producer wait for it before they exit, see below).
-    const bool early = a.early_weights && (warp == 0 || warp == 2);
-    if (!early) dep_wait();
+    dep_wait();                 // everything above overlaps the tail of the previous kernel
     if (a.early_dependents) dep_launch();
     tc_fence_before();
     __syncthreads();
@@ -426,7 +419,6 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         // the down product).  The claim of the item after the next is in flight meanwhile.
         constexpr bool DENSE = MODE == X_QKV || MODE == X_OPROJ;
         PipeState wr;
-        // past L1: with early weights the list's writer has completed, but not the kernel in front
         auto tile_at = [&](int i) {
             const int4 v = __ldcg(reinterpret_cast<const int4 *>(a.ttiles) + i);
             return omni_ttile{v.x, v.y, v.z, v.w};
@@ -806,7 +798,6 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     }
 
     // ---------------------------------------------------------------- teardown
-    if (early) dep_wait();      // no thread may leave before the previous kernel has completed
     tc_fence_before();
     __syncthreads();
     if (*abort_flag && threadIdx.x == 0) {
@@ -879,13 +870,12 @@ cudaError_t omni_expert_configure(void) {
 cudaError_t omni_launch_gateup_pair(int ctas, const CUtensorMap *tm_w4, const CUtensorMap *tm_x, const omni_sort_state st,
                                     void *h, const uint32_t *ready, const int32_t *need, int group_size,
                                     const void *gather_src, const int32_t *gather_rows, const omni_ep_peers *dispatch_to,
-                                    const omni_ep_send *send, int early_dependents, int early_weights, int n_sm, cudaStream_t s) {
+                                    const omni_ep_send *send, int early_dependents, int n_sm, cudaStream_t s) {
     XArgs a = {};
     a.ttiles = st.ttiles; a.n_ttiles = st.n_ttiles; a.work_counter = st.sched; a.out = (__nv_bfloat16 *)h; a.status = st.status;
     a.ready = ready; a.need = need; a.group_size = group_size > 0 ? group_size : 1;
     a.gather_src = (const __nv_bfloat16 *)gather_src; a.gather_rows = gather_rows;
     a.early_dependents = early_dependents;
-    a.early_weights = early_weights;
     if (dispatch_to) {
         const int grid = n_sm - n_sm % ctas;
         a.pe = *dispatch_to;
@@ -904,7 +894,6 @@ cudaError_t omni_launch_down_pair(int ctas, const CUtensorMap *tm_w, const CUten
     a.out = (__nv_bfloat16 *)d; a.status = st.status; a.group_size = 1;
     if (return_to) { a.pe = *return_to; a.rowinfo = rowinfo; }
     a.early_dependents = early_dependents;
-    a.early_weights = 1;                     // the list is older than the gate/up kernel in front
     return ctas == 2 ? launch_pair<X_DOWN, 2, false>(tm_w, tm_h, a, n_sm, s) : launch_pair<X_DOWN, 1, false>(tm_w, tm_h, a, n_sm, s);
 }
 
@@ -914,7 +903,7 @@ cudaError_t omni_launch_dense_pair(int which, const CUtensorMap *tm_w, const CUt
                                    uint32_t *status, int n_sm, cudaStream_t s) {
     XArgs a = {};
     a.out = (__nv_bfloat16 *)out_bf16; a.resid = resid; a.status = status; a.group_size = 1;
-    a.early_dependents = 1; a.early_weights = 1;
+    a.early_dependents = 1;
     a.dense_rows = T;
     // Tiles: the fewest rounds of the pairs of SMs weighted by what an item of that many rows costs.  A
     // tile of n rows takes about n/2 clocks per K step of 16 but no less than one of DENSE_MIN rows

@@ -167,8 +167,7 @@ cudaError_t omni_expert_configure(void);  /* opt-in shared-memory sizes; call on
 cudaError_t omni_launch_gateup_pair(int ctas, const CUtensorMap *tm_w4, const CUtensorMap *tm_x, const omni_sort_state st,
                                     void *h, const uint32_t *ready, const int32_t *need, int group_size,
                                     const void *gather_src, const int32_t *gather_rows, const omni_ep_peers *dispatch_to,
-                                    const omni_ep_send *send, int early_dependents, int early_weights, int n_sm, cudaStream_t s);
-/* early_weights: the weight loads need not wait for the kernel in front (st's tile list is older than it) */
+                                    const omni_ep_send *send, int early_dependents, int n_sm, cudaStream_t s);
 /* dispatch_to/send (may be NULL): expert parallelism -- four more warps per CTA send this rank's
  * token rows, each once per owner rank, into the owners' receive buffers (gather_src of the
  * owner) with the row map (gather_rows of the owner) and the origin tags, and count themselves on

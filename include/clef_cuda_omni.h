@@ -281,8 +281,8 @@ bool clef_omni_read(clef_gpu *g, const char *what, void *dst, size_t bytes, char
  * kernel on single CTAs; 0, the default: chosen from the number of tokens; same results),
  * "longest_first" 0/1 (default 1: the gate/up kernel claims its work items in order of falling tile length, the
  * short ones filling the end of the launch; 0: in expert order; same results; set after clef_omni_reserve),
- * "expert_chain" 0/1 (accepted and without effect: the down kernel always starts its weight loads
- * under the gate/up kernel's tail),
+ * "expert_chain" 0/1 (accepted and without effect: it chained the down kernel to the gate/up kernel expert by
+ * expert in kernels that CTA pairs have replaced),
  * "ep_wait_ms" N (bound on each in-pass wait for other ranks, 0 = 2000), "reserve_sms" N (the persistent expert kernels use all SMs but N, so that kernels of another
  * context on the same GPU -- another micro-batch -- are not locked out while they run),
  * "fused_gather" 0/1 (default 1: the gate/up kernel fetches its token rows through the permutation

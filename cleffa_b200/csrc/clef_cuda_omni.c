@@ -631,8 +631,9 @@ static bool run_experts(clef_gpu *g, const omni_layer *L, const void *xn, const 
     const int rows8 = rows * OMNI_TOP;
     /* pairs of CTAs unless the call says otherwise or the batch is a token or two: then eight to sixteen
      * experts make fewer pair items (6 of 256 gate/up rows per expert) than there are pairs, and
-     * single CTAs with half the rows each spread over twice as many SMs (1 token: 16 us against 22) */
-    const int ctas = g->expert_kernel ? g->expert_kernel : rows <= 2 ? 1 : 2;
+     * single CTAs with half the rows each spread over twice as many SMs (1 token: 16 us against 22);
+     * "reserve_sms" may also leave a single SM, which is no pair */
+    const int ctas = g->expert_kernel ? g->expert_kernel : rows <= 2 || g->n_sm - g->reserve_sms < 2 ? 1 : 2;
     omni_sort_state sort = s->sort;
     sort.tile_n = ctas == 1 ? OMNI_TILE_N1 : OMNI_TILE_N;
     if (!launched(g, "assign", omni_launch_assign(ids, rows, sort, have_counts, g->stream))) return false;

@@ -131,6 +131,23 @@ def test_expert_kernel_variants_give_the_same_bits(bound0, T, ctas):
         b.set_option("expert_kernel", EXPERT_KERNEL_DEFAULT)
 
 
+@pytest.mark.parametrize("T", [2, 3, 300])
+def test_reserved_sms_leave_the_same_bits(bound0, T):
+    """Whatever "reserve_sms" leaves to the expert products, down to a single SM, on which no pair of CTAs fits."""
+    b = bound0
+    x = orc.make_activations(27, T)
+    base = run_block(b, 0, x)
+    n_sm = torch.cuda.get_device_properties(0).multi_processor_count
+    try:
+        for reserve in (1, n_sm - 3, n_sm - 2, n_sm - 1):
+            b.set_option("reserve_sms", reserve)
+            other = run_block(b, 0, x)
+            for key in ("ids", "slots", "counts", "out"):
+                assert np.array_equal(base[key], other[key]), (key, reserve)
+    finally:
+        b.set_option("reserve_sms", 0)
+
+
 @pytest.mark.parametrize("T", [1, 33, 200])
 @pytest.mark.parametrize("delta", [0.0, 2.0**-8])
 def test_exact_pass_orders_paired_experts(backend, weights0, T, delta):

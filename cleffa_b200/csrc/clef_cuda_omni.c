@@ -579,12 +579,16 @@ static void stage_mark(clef_gpu *g, int i) { if (g->profile) cudaEventRecord(g->
 
 /* What the exact pass asks to have in L2 of the gate/up weights while the routing is still being found
  * and device memory is idle.  From two rows on enough of it is used (six rows touch a third of the
- * experts), and up to 1536 the gate/up product waits for its weights.  Block, us, without and with: 2 rows
- * 59.8 -> 59.3, 9 118.5 -> 115.8, 64 215.4 -> 212.4, 256 225.1 -> 220.6, 700 229.5 -> 227.1, 1030 236.3 ->
- * 237.2 (two layers 647 -> 642), 2048 264.5 -> 264.6, 3072 300.5 -> 303.0; 1 row +0.1.  48 MiB gain
- * another 1.5 us at 64 and 256 rows, but lose 2 us per pass of two layers of 12 to 200 rows. */
+ * experts); up to 512 the gate/up product waits for its weights, above that the products last longer than
+ * the stream and nothing is left to gain.  us, without and with: block of 2 rows 63.8 -> 63.8, 9 120.1 -> 117.4,
+ * 128 219.5 -> 216.6, 256 225.6 -> 223.0, 400 227.8 -> 227.4, 512 231.0 -> 231.8, 850 242.4 -> 242.7, 1030 248.3 -> 248.2,
+ * 1536 265.0 -> 266.3; clef_omni_forward_host, 64 rows 262.5 -> 258.5, 300 330.4 -> 328.0, 512 378.6 -> 375.1, 700
+ * 422.0 -> 421.4, 1030 501.5 -> 501.2; two layers of 128 rows 535.6 -> 530.4, 512 584.5 -> 583.1, 1030 678.1 -> 676.0.  The
+ * rule goes by the rows of a pass, so a short last piece of forward_host has its weights asked for too (5000
+ * rows, the last piece 392: 1569 -> 1564).
+ * 48 MiB gained another 1.5 us at 64 and 256 rows, but lost 2 us per pass of two layers of 12 to 200 rows. */
 #define PREFETCH_MIN_ROWS 2
-#define PREFETCH_MAX_ROWS 1536
+#define PREFETCH_MAX_ROWS 512
 #define PREFETCH_BYTES ((size_t)24 << 20)
 
 /* router + exact pass for one chunk; fills arena ids/weights/logits */

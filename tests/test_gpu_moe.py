@@ -194,8 +194,9 @@ def test_exact_mode_reaches_reference_weight_tolerance(bound0, weights0):
     assert np.abs(got["weights"].astype(np.float64) - w_ref.numpy()).max() < 2e-7     # tests/test_omni_moe.m:108
 
 
-@pytest.mark.parametrize("T", [1, 15, 16, 17, 31, 32, 33, 127, 128, 129, 255, 257])
+@pytest.mark.parametrize("T", [1, 2, 3, 15, 16, 17, 31, 32, 33, 127, 128, 129, 255, 257, 512, 513])
 def test_short_rows(bound0, weights0, T):
+    # single CTAs up to 2 rows; weights prefetched by the exact pass from 2 to 512
     x = orc.make_activations(100 + T, T)
     res = torch.randn(T, 2048, generator=torch.Generator().manual_seed(T))
     check_against_oracle(run_block(bound0, 0, x, residual=res), x, weights0, residual=res)

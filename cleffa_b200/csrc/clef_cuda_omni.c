@@ -317,7 +317,7 @@ bool clef_omni_reserve(clef_gpu *g, const clef_omni_config *c, int T, char *err,
         {(void **)&s->sort.rowmap, (size_t)OMNI_ROWS * 4},
         {(void **)&s->sort.slots, (size_t)OMNI_ROWS * 4},
         {(void **)&s->sort.segcount, (size_t)OMNI_MAX_SEGS * OMNI_E * 4},
-        {(void **)&s->sort.ttiles, (size_t)2 * OMNI_MAX_TTILES * sizeof(omni_ttile)},      /* the list, and the same tiles in expert order */
+        {(void **)&s->sort.ttiles, (size_t)OMNI_MAX_TTILES * sizeof(omni_ttile)},
         {(void **)&s->sort.n_ttiles, 256},
         {(void **)&s->sort.sched, 256},
         {&s->xg, (size_t)OMNI_ROWS * OMNI_H * 2},
@@ -334,7 +334,6 @@ bool clef_omni_reserve(clef_gpu *g, const clef_omni_config *c, int T, char *err,
     s->sort.n_flag = s->n_flag;
     s->sort.longest_first = 1;
     s->sort.tile_n = OMNI_TILE_N;
-    s->sort.ttiles_down = ok ? s->sort.ttiles + OMNI_MAX_TTILES : NULL;
     for (uint32_t i = 0; i < OMNI_TOK_BOXES && ok; i++)
         ok = make_map(g, &s->tm_xg[i], s->xg, OMNI_ROWS, OMNI_H, 16 * (i + 1), CU_TENSOR_MAP_L2_PROMOTION_L2_128B) &&
              make_map(g, &s->tm_h[i], s->h, OMNI_ROWS, OMNI_F, 16 * (i + 1), CU_TENSOR_MAP_L2_PROMOTION_L2_128B);

@@ -64,7 +64,6 @@ typedef struct {
     int32_t *n_flag;       /* [2] rows flagged for the exact pass: the scan moves [0] to [1] and clears [0] for the next pass */
     int32_t tile_n;        /* most rows of a token tile: OMNI_TILE_N or OMNI_TILE_N1, as the expert kernels of the pass take */
     int32_t longest_first; /* tile list in order of falling tile length (else in expert order) */
-    omni_ttile *ttiles_down; /* the same tiles in expert order, for the down kernel (may be NULL: it then reads ttiles) */
 } omni_sort_state;
 
 /* Expert parallelism: every rank's view of every rank's exchange buffers (index = rank). */

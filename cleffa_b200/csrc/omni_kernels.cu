@@ -235,7 +235,9 @@ __global__ void __launch_bounds__(1024) assign_scan_kernel(int nseg, omni_sort_s
         if (e == OMNI_E - 1) st.offsets[OMNI_E] = rows_incl;
         // Expert-major tile list, the experts in order of falling tile length (ties by id): the work
         // items of the persistent expert kernels are claimed in list order, so the longest come first
-        // and the short ones fill the end of the launch.  Rows and offsets stay in expert order.
+        // and the short ones fill the end of the launch.  Rows and offsets stay in expert order.  Both products
+        // read this list: with one in expert order for the down product a block took 437.5 us against 438 (4096
+        // tokens), 742 against 743 (8192), 1367 against 1374 (16384), 653 against 655 (8192, skewed).
         const int nt = (n + st.tile_n - 1) / st.tile_n;
         const int key = tile_key[e];
         int first = tiles_incl - nt;
@@ -252,12 +254,6 @@ __global__ void __launch_bounds__(1024) assign_scan_kernel(int nseg, omni_sort_s
         const int base = nt ? n / nt : 0, extra = nt ? n % nt : 0;
         for (int j = 0; j < nt; j++)
             st.ttiles[first + j] = omni_ttile{e, off + j * base + min(j, extra), base + (j < extra), first | (nt << 16)};
-        if (st.ttiles_down) {
-            // the down kernel measured faster on the expert-ordered list (130 against 134 us at T=4096)
-            const int f2 = tiles_incl - nt;
-            for (int j = 0; j < nt; j++)
-                st.ttiles_down[f2 + j] = omni_ttile{e, off + j * base + min(j, extra), base + (j < extra), f2 | (nt << 16)};
-        }
         if (e < 8) st.sched[e] = 0;
         if (e == OMNI_E - 1) *st.n_ttiles = tiles_incl;
         // the router and the exact pass of this chunk are done with the flagged-row count: keep it
@@ -643,7 +639,7 @@ cudaError_t omni_noalloc_assign(const int32_t *ids, int rows, int32_t *counts, i
     st.segcount = sc->segcount; st.ttiles = sc->ttiles; st.n_ttiles = &sc->n_ttiles; st.sched = sc->sched;
     st.status = status;
     st.n_flag = sc->n_flag;
-    st.longest_first = 0; st.tile_n = OMNI_TILE_N; st.ttiles_down = nullptr;
+    st.longest_first = 0; st.tile_n = OMNI_TILE_N;
     return omni_launch_assign(ids, rows, st, 0, s);
 }
 

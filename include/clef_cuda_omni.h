@@ -279,7 +279,7 @@ bool clef_omni_read(clef_gpu *g, const char *what, void *dst, size_t bytes, char
  * gate/up kernel; same results; must be the same on every rank, as it changes the number of barriers per pass),
  * "expert_kernel" 0/1/2 (2: expert products on pairs of CTAs, tcgen05.mma.cta_group::2; 1: the same
  * kernel on single CTAs; 0, the default: chosen from the number of tokens; same results),
- * "longest_first" 0/1 (default 1: the gate/up kernel claims its work items in order of falling tile length, the
+ * "longest_first" 0/1 (default 1: the expert kernels claim their work items in order of falling tile length, the
  * short ones filling the end of the launch; 0: in expert order; same results; set after clef_omni_reserve),
  * "expert_chain" 0/1 (accepted and without effect: it chained the down kernel to the gate/up kernel expert by
  * expert in kernels that CTA pairs have replaced),

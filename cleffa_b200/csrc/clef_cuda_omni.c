@@ -27,7 +27,7 @@ typedef struct {
     void *router, *gate_up, *down;      /* device, BF16 */
     float *bias;                        /* device, FP32 [128] or NULL */
     bool owned, bound;
-    CUtensorMap tm_router, tm_gate_up, tm_down;
+    CUtensorMap tm_router, tm_down;
     CUtensorMap tm_gate_up4;            /* {K, row, gate|up, block} view of gate_up: a box interleaves blocks of gate and up rows */
 } omni_layer;
 
@@ -548,7 +548,6 @@ bool clef_omni_bind_layer(clef_gpu *g, int layer, const void *router, const void
         }
     }
     if (!make_map(g, &next.tm_router, next.router, OMNI_E, OMNI_H, 128, CU_TENSOR_MAP_L2_PROMOTION_L2_128B) ||
-        !make_map(g, &next.tm_gate_up, next.gate_up, (uint64_t)EL * 2 * OMNI_F, OMNI_H, 128, CU_TENSOR_MAP_L2_PROMOTION_L2_256B) ||
         !make_map(g, &next.tm_down, next.down, (uint64_t)EL * OMNI_H, OMNI_F, 128, CU_TENSOR_MAP_L2_PROMOTION_L2_256B) ||
         !make_gate_up4(g, &next.tm_gate_up4, next.gate_up, (uint64_t)EL)) {
         free_layer(&next);

@@ -241,9 +241,6 @@ enum { X_GATEUP = 0, X_DOWN = 1,
        // the two dense projections of the attention half, run as "one expert" over all token rows:
        X_QKV = 2,      // P[T][5120] = xn[T][2048] . W_qkv^T, BF16 out
        X_OPROJ = 3 };  // x[T][2048] += A[T][4096] . W_out^T, added into the FP32 residual
-#ifndef X_GATHER_LAG            /* stages between issuing a gathered stage and handing it to the MMA thread */
-#define X_GATHER_LAG 3
-#endif
 
 // ROWS: accumulator rows (weight rows) of one CTA; OUTC: output columns one CTA produces;
 // MT: such CTA-level weight tiles per expert.
@@ -342,7 +339,7 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *const smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
     const uint32_t tok_base = smem_base + WS * C::W_BYTES;
-    uint8_t *const out_tile = smem_gen + C::RING_BYTES;                               // [256][OUTC] bf16
+    uint8_t *const out_tile = smem_gen + C::RING_BYTES; // 4 x [32][OUTC] bf16: two chunks per epilogue half, none for the output projection
     const uint32_t bar_base = smem_base + C::RING_BYTES + C::STAGE_OUT_BYTES;
     auto wfull_bar = [&](int s) { return bar_base + 8u * s; };
     auto wempty_bar = [&](int s) { return bar_base + 8u * (WS + s); };
@@ -492,9 +489,9 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         // 128 threads fetch this CTA's share of the tile's token rows through the permutation:
         // 16-byte asynchronous copies, eight threads per 128-byte row segment, stored in the
         // 128-byte-swizzled layout the MMA descriptors expect (chunk c of row r at c ^ (r & 7)
-        // inside its 8-row group).  A stage is handed to the MMA thread two stages after it was
+        // inside its 8-row group).  A stage is handed to the MMA thread LAG stages after it was
         // issued, once the copies have landed and are ordered before the tensor core's reads.
-        constexpr int LAG = CTAS == 2 ? X_GATHER_LAG : 2;
+        constexpr int LAG = CTAS == 2 ? 3 : 2;
         static_assert(TS > LAG, "token ring too short for the copy lag");
         constexpr int RSTEP = X_GATHER_THREADS / 8, NR = C::TOK_ROWS / RSTEP;
         const uint64_t pol_t = l2_policy_evict_last();
@@ -572,12 +569,9 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             if (!ok) break;
             // the next item's row indices travel while the last stages of this one land
             len = next_item(off_next);
-            static_assert(LAG >= 1 && LAG <= 6, "copy lag");
-            if (LAG >= 6) hand_over(std::integral_constant<int, 5>{});
-            if (LAG >= 5) hand_over(std::integral_constant<int, 4>{});
-            if (LAG >= 4) hand_over(std::integral_constant<int, 3>{});
-            if (LAG >= 3) hand_over(std::integral_constant<int, 2>{});
-            if (LAG >= 2) hand_over(std::integral_constant<int, 1>{});
+            static_assert(LAG == 2 || LAG == 3, "copy lag");
+            if (LAG == 3) hand_over(std::integral_constant<int, 2>{});
+            hand_over(std::integral_constant<int, 1>{});
             hand_over(std::integral_constant<int, 0>{});
 #pragma unroll
             for (int i = 0; i < NR; i++) off[i] = off_next[i];

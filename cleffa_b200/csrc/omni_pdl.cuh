@@ -12,8 +12,12 @@
 //   * dep_wait() is executed by every thread before its first access to global memory and
 //     before any exit path.  A block that left without waiting would let its grid count as
 //     complete while an earlier grid still runs, and a later kernel could overtake that one.
+//     Only memory that no kernel of the chain writes may be touched earlier, and is in two places: the
+//     exact pass asks for bound weights to be brought into L2, and the attention kernel reads its
+//     query tiles, which a copy in front of the whole pass has written.
 //   * dep_launch() follows dep_wait() directly: by then the block is resident, so waiting
-//     dependents can never hold resources a block of this grid still needs.
+//     dependents can never hold resources a block of this grid still needs.  A dependent may so count
+//     on every kernel before this one being complete, whatever it does before its own wait.
 // Both instructions do nothing in a kernel that was launched without the attribute.
 #pragma once
 #include <cuda_runtime.h>

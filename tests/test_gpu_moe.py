@@ -80,52 +80,46 @@ def test_tcgen05_and_check_kernels_agree(bound0):
 
 @pytest.mark.parametrize("T", [1, 37, 300, 2500])
 def test_launch_variants_give_the_same_bits(bound0, T):
-    """Fused or separate kernels (exact pass and histogram inside the router kernel, token
-    rows gathered by the gate/up kernel) and dependent launch on or off are ways of
+    """Fused or separate kernels (histogram inside the router kernel, token rows gathered by the
+    gate/up kernel), dependent launch on or off and the order of the work items are ways of
     scheduling the same arithmetic."""
     b = bound0
     x = orc.make_activations(17, T)
     base = run_block(b, 0, x)
-    opts = ("fused_router", "fused_gather", "dependent_launch", "expert_chain", "longest_first")
+    opts = ("fused_router", "fused_gather", "dependent_launch", "longest_first")
+    b.set_option("expert_chain", 0)           # accepted, without effect
     try:
-        # expert_chain (off by default): the down kernel starts while gate/up's last blocks still
-        # run and takes each expert's rows once they are complete; twice, so that the second pass
-        # meets the counters and the tile list of another batch at the same addresses
-        # longest_first (on by default): the order in which the gate/up kernel claims its work items
-        for combo in ((0, 1, 1, 0, 1), (1, 0, 1, 0, 1), (1, 1, 0, 0, 1), (0, 0, 0, 0, 0), (1, 1, 1, 1, 1), (1, 0, 1, 1, 0), (1, 1, 0, 1, 1),
-                      (1, 1, 1, 0, 0)):
+        # longest_first (on by default): the order in which the expert kernels claim their work items.
+        # Another batch in between: the pass meets counters and a tile list of other tokens at the same addresses.
+        for combo in ((0, 1, 1, 1), (1, 0, 1, 1), (1, 1, 0, 1), (1, 1, 1, 0), (0, 0, 1, 1), (1, 0, 1, 0), (0, 1, 0, 1), (0, 0, 0, 0)):
             for name, v in zip(opts, combo):
                 b.set_option(name, v)
-            if combo[3]:
-                run_block(b, 0, orc.make_activations(18, max(1, T // 2)))
+            run_block(b, 0, orc.make_activations(18, max(1, T // 2)))
             other = run_block(b, 0, x)
             for key in ("ids", "slots", "counts", "rechecked", "out"):
                 assert np.array_equal(base[key], other[key]), (key, combo)
     finally:
-        for name in opts[:3] + opts[4:]:
+        for name in opts:
             b.set_option(name, 1)
-        b.set_option("expert_chain", 0)
 
 
-@pytest.mark.parametrize("ctas", [1, 2])
-@pytest.mark.parametrize("T", [1, 37, 300, 2500, 4096])
-def test_expert_kernel_variants_give_the_same_bits(bound0, T, ctas):
-    """The expert products exist as two schedules of the same arithmetic: single CTAs with one
-    accumulator per gate and up tile, and CTA pairs (or single CTAs, ctas=1) on interleaved
-    gate/up rows with the output staged through shared memory.  Every element is the same K-ordered
-    FP32 sum either way, so the block's output must be the same bytes, with the token rows
-    gathered by the kernel or read from the permuted copy."""
+@pytest.mark.parametrize("T", [1, 2, 3, 37, 300, 2500, 4096])
+def test_expert_kernel_variants_give_the_same_bits(bound0, T):
+    """The expert products exist as two schedules of the same arithmetic: single CTAs with tiles of up to
+    128 token rows, and pairs of CTAs with up to 256.  Every element is the same K-ordered FP32 sum
+    either way, so the block's output must be the same bytes, with the token rows gathered by the
+    kernel or read from the permuted copy, and whichever of them the default (0) takes."""
     b = bound0
     x = orc.make_activations(23, T)
     try:
-        b.set_option("expert_kernel", 0)
+        b.set_option("expert_kernel", 1)
         base = run_block(b, 0, x)
-        for gather in (1, 0):
-            b.set_option("fused_gather", gather)
+        for ctas, gather in ((1, 0), (2, 1), (2, 0), (EXPERT_KERNEL_DEFAULT, 1)):
             b.set_option("expert_kernel", ctas)
+            b.set_option("fused_gather", gather)
             other = run_block(b, 0, x)
             for key in ("ids", "slots", "counts", "out"):
-                assert np.array_equal(base[key], other[key]), (key, gather)
+                assert np.array_equal(base[key], other[key]), (key, ctas, gather)
     finally:
         b.set_option("fused_gather", 1)
         b.set_option("expert_kernel", EXPERT_KERNEL_DEFAULT)

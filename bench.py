@@ -48,8 +48,8 @@ KERNELS_PER_PASS = 7     # router (counts the sort segments), exact pass, scan, 
 KERNELS_PER_PASS_EP = 10  # ... plus owner buckets, plan and one barrier; the expert kernels dispatch and return the rows themselves
 METRIC = "MoE-layer prefill tokens/sec at T=4096"
 # dram__bytes_read.sum + dram__bytes_write.sum of one gate/up launch at T=4096, from the ncu
-# capture summarised in profiles/ncu_full_moe_layer_T4096.md
-GATEUP_DRAM_TRAFFIC_T4096 = 864_723_456 + 46_342_144
+# capture summarised in profiles/ncu_moe_layer_T4096.md
+GATEUP_DRAM_TRAFFIC_T4096 = 842_291_456 + 10_608_896
 
 
 def measured_peaks():

@@ -3,7 +3,7 @@
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 
 One step = one pass of the block (router -> top-8 -> permutation -> gate/up+SwiGLU -> down ->
-combine) over one packed batch.  Workload at N=1: BASELINE configuration 2 -- T=4096 as eight
+combine) over one packed batch.  Workload at N=1: T=4096 as eight
 packed sequences (lengths uniform in [64,1024] rescaled to 4096), hidden 2048, 128 experts
 top-8, intermediate 768, BF16 weights N(0,0.02), BF16 activations N(0,1), seed 1.
 
@@ -16,10 +16,10 @@ The K-step timed region is repeated until at least one second of device time has
 `ms_per_step` is the median region (min and max beside it) and `clocks` are the nvidia-smi
 samples taken while those regions ran.
 
-Other workloads of BASELINE.json (each prints one JSON line of the same shape):
-    --layers 48 --tokens 16384 [--strong --gpus N]   configuration 3, the 48-layer stack
-    --bias zipf --tokens 8192 [--strong --gpus N]    configuration 4, Zipf-skewed routing
-    --sweep                                          configuration 5, T = 1 .. 256 latency table
+Other workloads (each prints one JSON line of the same shape):
+    --layers 48 --tokens 16384 [--strong --gpus N]   the 48-layer stack
+    --bias zipf --tokens 8192 [--strong --gpus N]    Zipf-skewed routing
+    --sweep                                          T = 1 .. 256 latency table
 With --strong the token count is the whole job's and every rank takes 1/N of it (strong
 scaling); without it, it is per GPU (weak scaling, the default the headline uses).
 """
@@ -604,7 +604,7 @@ def attention_bench(args):
 
 
 def sweep(args):
-    """layer latency and achieved weight-streaming bandwidth at small
+    """T = 1 .. 256: layer latency and achieved weight-streaming bandwidth at small
     batch sizes (seed 4), one GPU.  One JSON line holding the whole table."""
     import numpy as np
     import torch
@@ -638,7 +638,7 @@ def sweep(args):
             gbs = 9_437_184 * touched / (us * 1e-6) / 1e9
             rows.append({"tokens": T, "us_per_pass": us, "experts_touched": touched, "weight_gbs": gbs,
                          "frac_of_hbm_peak": gbs / peaks["hbm_gbs"], "tokens_per_s": T / (us * 1e-6)})
-    print(json.dumps({"metric": "MoE-layer latency by batch size (BASELINE configuration 5)", "unit": "us per pass", "n_gpus": 1,
+    print(json.dumps({"metric": "MoE-layer latency by batch size (T = 1 .. 256)", "unit": "us per pass", "n_gpus": 1,
                       "data": "synthetic", "dtype": "bf16", "hbm_peak_gbs": peaks["hbm_gbs"], "peak_source": peaks["source"],
                       "note": "weight_gbs = 9,437,184 B x experts touched / time; 200 passes between two CUDA events after 5 warm-up passes; "
                               "every pass streams the touched experts' weights (75 MB .. 1.21 GB), L2 is 126 MB: from T=32 on the "
@@ -656,17 +656,17 @@ def main():
     ap.add_argument("--no-cpu", action="store_true", help="skip the CPU baseline leg")
     ap.add_argument("--tokens", type=int, default=4096, help="tokens per GPU (with --strong: of the whole job); default: the headline 4096")
     ap.add_argument("--strong", action="store_true", help="strong scaling: --tokens is the whole job's and is split evenly over the GPUs")
-    ap.add_argument("--bias", default="none", choices=["none", "zipf"], help="zipf: BASELINE configuration 4 (use --tokens 8192, seed 3)")
+    ap.add_argument("--bias", default="none", choices=["none", "zipf"], help="zipf: skewed routing (use with --tokens 8192, seed 3)")
     ap.add_argument("--seed", type=int, default=None, help="workload seed (default 1; 2 with --layers, 3 with --bias zipf)")
     ap.add_argument("--min-time-ms", type=float, default=1000.0, help="repeat the K-step timed region until this much device time was timed")
     ap.add_argument("--max-regions", type=int, default=400)
     ap.add_argument("--attention", action="store_true", help="time the attention half and whole decoder layers (attention + norm + MoE); with --gpus N: records data-parallel, experts sharded (weak scaling)")
-    ap.add_argument("--sweep", action="store_true", help="BASELINE configuration 5: latency table over small batch sizes, one GPU")
+    ap.add_argument("--sweep", action="store_true", help="T = 1 .. 256: latency table over small batch sizes, one GPU")
     ap.add_argument("--sweep-tokens", type=int, nargs="+", default=[1, 8, 32, 64, 128, 256])
     ap.add_argument("--norm", action="store_true", help="with --layers: each layer normalises the residual stream itself (RMSNorm, unit weights) instead of taking a BF16 copy")
     ap.add_argument("--kernels-only", action="store_true", help="run the warm-up and the timed steps and stop (for profiler captures; one GPU)")
     ap.add_argument("--option", action="append", default=[], help="library option name=value (clef_omni_set_option), repeatable")
-    ap.add_argument("--layers", type=int, default=1, help="stack of MoE sublayers with residual adds (BASELINE configuration 3 uses 48 at --tokens 16384)")
+    ap.add_argument("--layers", type=int, default=1, help="stack of MoE sublayers with residual adds (48 at --tokens 16384 is the whole model)")
     args = ap.parse_args()
     T_TOKENS = args.tokens
     SEED = args.seed if args.seed is not None else (3 if args.bias == "zipf" else 2 if args.layers > 1 else 1)

@@ -61,7 +61,7 @@ def test_attention_half_matches_fp64_oracle(attn, bounds):
 
 
 def test_config2_T4096_eight_records(attn):
-    """The packed prefill of BASELINE configuration 2 (T=4096 as 8 records, seed 1), every row
+    """The packed prefill of the benchmark (T=4096 as 8 records, seed 1), every row
     against the FP64 oracle."""
     from cleffa_b200 import workloads
     b, w = attn
@@ -77,7 +77,7 @@ def test_config2_T4096_eight_records(attn):
 
 
 def test_config3_T16384_one_record_sampled(attn):
-    """One record of 16,384 tokens (BASELINE configuration 3's batch): 128 key blocks per query
+    """One record of 16,384 tokens (the largest batch of one pass): 128 key blocks per query
     tile.  96 sampled rows -- the first and last rows, both sides of tile and block boundaries,
     random ones -- against the FP64 oracle's rows."""
     b, w = attn

@@ -395,7 +395,7 @@ def ours(args):
         else:
             par = (f"expert parallel ep{world}, tokens data-parallel, rows exchanged by peer stores over NVLink "
                    f"from inside the expert kernels")
-        launches = (KERNELS_PER_PASS + (1 if args.norm else 0)) * n_layers if world == 1 else KERNELS_PER_PASS_EP * n_layers
+        launches = 1 + ((KERNELS_PER_PASS + (1 if args.norm else 0)) * n_layers if world == 1 else KERNELS_PER_PASS_EP * n_layers)   # 1: begin
         line = {
             "metric": METRIC if (T_TOKENS == 4096 and n_layers == 1 and not zipf) else
                       f"MoE-layer prefill tokens/sec at T={T_TOKENS}" + (f" through {n_layers} layers" if n_layers > 1 else ""),

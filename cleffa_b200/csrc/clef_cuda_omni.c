@@ -366,12 +366,8 @@ void clef_omni_begin(clef_gpu *g) {
     g->failed = false;
     g->fail_msg[0] = 0;
     g->trace_valid = false;
-    if (cudaMemsetAsync(s->status, 0, 4, g->stream) != cudaSuccess) note_failure(g, "status clear", cudaGetLastError());
-    /* a pass that failed between the router and the scan leaves its flagged-row count behind */
-    if (cudaMemsetAsync(s->n_flag, 0, 4, g->stream) != cudaSuccess) note_failure(g, "flag clear", cudaGetLastError());
-    /* likewise the bucket counters of the expert-parallel dispatch (cleared by the plan kernel in a pass that gets that far) */
-    if (g->ep.world > 1 && cudaMemsetAsync(g->ep.bucket_cnt, 0, (size_t)OMNI_EP_BUCKETS * 4, g->stream) != cudaSuccess)
-        note_failure(g, "bucket clear", cudaGetLastError());
+    const cudaError_t e = omni_launch_begin(s->status, s->n_flag, g->ep.world > 1 ? g->ep.bucket_cnt : NULL, g->stream);
+    if (e != cudaSuccess) note_failure(g, "status clear", e);
     if (g->debug_poison) {
         /* clef_metal_omni.m:152-158: every float scratch buffer starts as NaN */
         poison(g, s->logits, (size_t)OMNI_CHUNK * OMNI_E * 4, 0x7fc00000u);

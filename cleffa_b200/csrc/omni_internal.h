@@ -114,6 +114,8 @@ cudaError_t omni_launch_recheck(int32_t *segcount, const void *xn, const void *r
                                 float *low, const int32_t *flag_rows, const int32_t *n_flag, int T, float eps,
                                 int32_t *ids, float *weights, uint32_t *status, const void *prefetch, size_t prefetch_bytes,
                                 cudaStream_t s);
+/* start of a pass: clears the status word, n_flag[0] and, where given, the OMNI_EP_BUCKETS bucket counters */
+cudaError_t omni_launch_begin(uint32_t *status, int32_t *n_flag, int32_t *buckets, cudaStream_t s);
 cudaError_t omni_launch_router_exact(const void *xn, const void *router, const float *bias, int T,
                                      double *logits, cudaStream_t s);
 cudaError_t omni_launch_route_pairs(const float *hi, const float *lo, int rows, int32_t *ids, float *weights,

@@ -292,6 +292,17 @@ __global__ void __launch_bounds__(256) assign_scatter_kernel(const int32_t *__re
     }
 }
 
+// ------------------------------------------------------------------ start of a pass
+// Clears the status word, the flagged-row count that a pass which failed between the router and the sort leaves
+// behind and, with expert parallelism, the bucket counters.  One kernel of the chain: as memset nodes these
+// cost 3.5 us each, and the kernel behind a memset starts without an overlap.
+__global__ void __launch_bounds__(OMNI_EP_BUCKETS) begin_kernel(uint32_t *status, int32_t *n_flag, int32_t *buckets) {
+    dep_wait();
+    dep_launch();
+    if (threadIdx.x == 0) { *status = 0; *n_flag = 0; }
+    if (buckets) buckets[threadIdx.x] = 0;
+}
+
 // ------------------------------------------------------------------ gather (permute rows)
 // xg[row] = xn[rowmap[row]]: 4 KiB per row, one warp per row, 16-byte lanes.
 __global__ void __launch_bounds__(256) gather_kernel(const uint4 *__restrict__ xn, const int32_t *__restrict__ rowmap,
@@ -517,6 +528,10 @@ cudaError_t omni_launch_recheck(int32_t *segcount, const void *xn, const void *r
     return omni_launch_chain(pieces ? recheck_kernel<true> : recheck_kernel<false>, dim3(blocks), dim3(128), 0, s, (const __nv_bfloat16 *)xn,
                              (const __nv_bfloat16 *)router, bias, logits, low, flag_rows, n_flag, T, eps, ids, weights, segcount, status,
                              (const char *)prefetch, pieces);
+}
+
+cudaError_t omni_launch_begin(uint32_t *status, int32_t *n_flag, int32_t *buckets, cudaStream_t s) {
+    return omni_launch_chain(begin_kernel, dim3(1), dim3(OMNI_EP_BUCKETS), 0, s, status, n_flag, buckets);
 }
 
 cudaError_t omni_launch_router_exact(const void *xn, const void *router, const float *bias, int T, double *logits,

@@ -1,6 +1,6 @@
 // Device helpers shared by the routing kernels: warp-level top-k in the reference's order,
 // the selection write-out, and exact logits (FP64 sums of exact BF16 products) with the
-// re-evaluation of one near-tied router row by a group of four warps.
+// re-evaluation of one near-tied router row by a group of eight warps.
 //
 // Reference behaviour (paths inside the reference project):
 //   selection order / weights   metal/clef.metal:2347-2394  (omni_route)
@@ -121,23 +121,23 @@ __device__ __forceinline__ void warp_top8(const double (&val)[4], int lane, doub
     }
 }
 
-// Lanes 0..7 hold the selected logits; weights are softmax over the selected eight, which
+// Lanes 0..7 hold the selected logits and ids in order; weights are softmax over the selected eight, which
 // equals softmax over all experts renormalised by the selected sum (clef.metal:2393).
-__device__ __forceinline__ void write_selection(const double (&top_v)[9], const int (&top_id)[9], int lane,
-                                                int32_t *ids, float *weights, long row) {
-    double p = 0.0;
-#pragma unroll
-    for (int k = 0; k < 8; k++) if (lane == k) p = exp(top_v[k] - top_v[0]);
+__device__ __forceinline__ void write_ranked(double v, int id, int lane, int32_t *ids, float *weights, long row) {
+    const double first = __shfl_sync(FULL, v, 0);
+    const double p = lane < 8 ? exp(v - first) : 0.0;
     double sum = p;
 #pragma unroll
     for (int s = 4; s > 0; s >>= 1) sum += __shfl_xor_sync(FULL, sum, s);
-    if (lane < 8) {
-        int id = 0;
+    if (lane < 8) { ids[row * 8 + lane] = id; weights[row * 8 + lane] = (float)(p / sum); }
+}
+__device__ __forceinline__ void write_selection(const double (&top_v)[9], const int (&top_id)[9], int lane,
+                                                int32_t *ids, float *weights, long row) {
+    double v = 0.0;
+    int id = 0;
 #pragma unroll
-        for (int k = 0; k < 8; k++) if (lane == k) id = top_id[k];
-        ids[row * 8 + lane] = id;
-        weights[row * 8 + lane] = (float)(p / sum);
-    }
+    for (int k = 0; k < 8; k++) if (lane == k) { v = top_v[k]; id = top_id[k]; }
+    write_ranked(v, id, lane, ids, weights, row);
 }
 
 __device__ __forceinline__ void write_fallback(int lane, int32_t *ids, float *weights, long row, uint32_t *status) {
@@ -182,12 +182,36 @@ __device__ __forceinline__ double exact_dot(const XRow &x, const __nv_bfloat16 *
     return sum;
 }
 
-// Re-evaluates one flagged row with four warps (128 threads): exact logits for every expert
+// The same sum for the exact pass, by eight warps and for EXACT_BATCH experts at once.  A lane owns eight of
+// the 2048 K elements (its warp's 256), so the weights of all candidates of a row -- nine or ten as a
+// rule -- are in flight together; with a warp per candidate a row took three rounds of loads and sums one after
+// the other.  A BF16 weight becomes a double by moving its bits: sign and exponent field in the
+// upper word of a double stand for the value times 2^-896, denormals included, and the sum is scaled back
+// exactly (the conversion instruction runs at a quarter of the rate of the FP64 adds).  Nonfinite weights
+// do not come here: the logits of their rows are nonfinite.
+constexpr int EXACT_BATCH = 12, EXACT_WARPS = 8, EXACT_THREADS = 32 * EXACT_WARPS;
+__device__ __forceinline__ double bf16_lo_scaled(uint32_t u) {
+    return __hiloint2double((int)(((u << 16) & 0x80000000u) | ((u & 0x7fffu) << 13)), 0);
+}
+__device__ __forceinline__ double bf16_hi_scaled(uint32_t u) {
+    return __hiloint2double((int)((u & 0x80000000u) | ((u >> 3) & 0x0fffe000u)), 0);
+}
+constexpr double EXACT_UNSCALE = 0x1p896;
+
+struct ExactScratch {
+    double part[EXACT_WARPS][EXACT_BATCH];
+    double exact[OMNI_E];                  // by expert; -inf where nothing was evaluated
+    double sorted_v[8];
+    int sorted_id[8];
+    float approx[OMNI_E];                  // by candidate
+    int cand[OMNI_E];                      // expert of each candidate
+};
+
+// Re-evaluates one flagged row with eight warps (256 threads): exact logits for every expert
 // that can still reach the top eight (approximate logit within twice the row's error bound of
-// the approximate 8th) and for the approximate 9th, spread over the warps, then the final order
-// by warp 0.  `sync` is a barrier over exactly these 128 threads; `exact_s` is their scratch of
-// 128 doubles.  With `segcount` given (expert counts per 256-assignment segment, taken from the
-// ids being replaced), the counts follow the ids that change.
+// the approximate 8th) and for the approximate 9th, then the final order by warp 0.  `sync` is a barrier
+// over exactly these threads.  With `segcount` given (expert counts per 256-assignment segment, taken
+// from the ids being replaced), the counts follow the ids that change.
 //
 // What the pass learns is written back: every logit it evaluated is replaced by its exact value
 // as a float pair (hi into `logits`, the remainder into `low` when given), so that a capture of
@@ -199,65 +223,124 @@ __device__ __forceinline__ void recheck_row(const __nv_bfloat16 *__restrict__ xn
                                             const float *__restrict__ bias, float *__restrict__ logits,
                                             float *__restrict__ low, long row, float eps, int32_t *__restrict__ ids,
                                             float *__restrict__ weights, int32_t *__restrict__ segcount,
-                                            uint32_t *__restrict__ status, double *exact_s, int lane, int warp, Sync sync) {
-    exact_s[warp * 32 + lane] = -CUDART_INF;
+                                            uint32_t *__restrict__ status, ExactScratch &sc, int lane, int warp, Sync sync) {
     float approx[4];
     float max_abs = 0.f;
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        approx[j] = logits[row * OMNI_E + lane + 32 * j];
-        max_abs = fmaxf(max_abs, fabsf(approx[j]));
-    }
+    for (int j = 0; j < 4; j++) approx[j] = logits[row * OMNI_E + lane + 32 * j];
+    const int koff = warp * (OMNI_H / EXACT_WARPS) + lane * 8;
+    const uint4 xq = __ldg(reinterpret_cast<const uint4 *>(xn + row * OMNI_H + koff));
+    const int old_id = segcount && warp == 0 && lane < 8 ? ids[row * 8 + lane] : 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++) max_abs = fmaxf(max_abs, fabsf(approx[j]));
 #pragma unroll
     for (int s = 16; s > 0; s >>= 1) max_abs = fmaxf(max_abs, __shfl_xor_sync(FULL, max_abs, s));
     const double bound = (double)omni_row_eps(eps, max_abs);
-    const XRow x = load_xrow(xn, row, lane);              // in flight while the threshold is found
     float v8, v9;
     warp_8th_9th(approx, lane, v8, v9);                   // every warp finds the same threshold
     const double floor_v = fmin((double)v8 - 2.0 * bound, (double)v9);
-    sync();
-    int c = 0;
-    bool off = false;
+    int n = 0;
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-        unsigned m = __ballot_sync(FULL, (double)approx[j] >= floor_v);
-        while (m) {
-            const int src = __ffs(m) - 1;
-            m &= m - 1;
-            const double a = (double)__shfl_sync(FULL, approx[j], src);
-            if ((c++ & 3) != warp) continue;              // candidates round-robin over the warps
-            const int e = src + 32 * j;
-            double v = exact_dot(x, w + (long)e * OMNI_H, lane);
-            if (bias) v += (double)bias[e];
-            off |= fabs(v - a) > bound;
-            if (lane == 0) {
-                exact_s[e] = v;
-                const float hi = (float)v;
-                logits[row * OMNI_E + e] = hi;
-                if (low) low[row * OMNI_E + e] = (float)(v - (double)hi);
-            }
+        const bool in = (double)approx[j] >= floor_v;
+        const unsigned m = __ballot_sync(FULL, in);
+        if (warp == 0) {
+            const int at = n + __popc(m & ((1u << lane) - 1u));
+            if (in) { sc.cand[at] = lane + 32 * j; sc.approx[at] = approx[j]; }
+            sc.exact[lane + 32 * j] = -CUDART_INF;
         }
+        n += __popc(m);
     }
-    if (off && lane == 0) atomicOr(status, OMNI_ST_ROUTER_EPS);
-    sync();
-    if (warp == 0) {
-        double exact[4];
+    sync();                                               // the candidates are listed
+    double x[8];
+    {
+        const uint32_t u[4] = {xq.x, xq.y, xq.z, xq.w};
 #pragma unroll
-        for (int j = 0; j < 4; j++) exact[j] = exact_s[lane + 32 * j];
-        double fin_v[9]; int fin_id[9];
-        warp_top8(exact, lane, fin_v, fin_id);
-        const int old_id = lane < 8 ? ids[row * 8 + lane] : 0;
-        write_selection(fin_v, fin_id, lane, ids, weights, row);
-        if (segcount && lane < 8) {
-            const int new_id = ids[row * 8 + lane];       // this lane's own store
-            if (new_id != old_id) {                       // a row's eight assignments share one segment
-                int32_t *c = segcount + (row * OMNI_TOP / OMNI_SEG) * OMNI_E;
-                atomicSub(c + old_id, 1);
-                atomicAdd(c + new_id, 1);
-            }
+        for (int j = 0; j < 4; j++) {
+            x[2 * j] = (double)bf16_bits_to_float(u[j] & 0xffffu);
+            x[2 * j + 1] = (double)bf16_bits_to_float(u[j] >> 16);
         }
     }
-    sync();
+    double mine_v = 0.0;                                  // warp 0: candidate `lane` of a row with at most EXACT_BATCH of them
+    for (int b0 = 0; b0 < n; b0 += EXACT_BATCH) {
+        uint4 wq[EXACT_BATCH];
+#pragma unroll
+        for (int i = 0; i < EXACT_BATCH; i++)
+            wq[i] = b0 + i < n ? __ldg(reinterpret_cast<const uint4 *>(w + (long)sc.cand[b0 + i] * OMNI_H + koff)) : make_uint4(0, 0, 0, 0);
+        double s[EXACT_BATCH];
+#pragma unroll
+        for (int i = 0; i < EXACT_BATCH; i++) {
+            const uint32_t u[4] = {wq[i].x, wq[i].y, wq[i].z, wq[i].w};
+            s[i] = 0.0;
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                s[i] = fma(x[2 * j], bf16_lo_scaled(u[j]), s[i]);
+                s[i] = fma(x[2 * j + 1], bf16_hi_scaled(u[j]), s[i]);
+            }
+        }
+        // sums over the warp's lanes, four candidates at a time: lanes with bit 4 (then bit 3) set keep the
+        // upper half of the values and hand over the lower one, so four sums take six exchanges and not twenty
+#pragma unroll
+        for (int q = 0; q < EXACT_BATCH; q += 4) {
+            const bool h16 = lane & 16, h8 = lane & 8;
+            double a0 = h16 ? s[q + 2] : s[q], a1 = h16 ? s[q + 3] : s[q + 1];
+            const double g0 = h16 ? s[q] : s[q + 2], g1 = h16 ? s[q + 1] : s[q + 3];
+            a0 += __shfl_xor_sync(FULL, g0, 16);
+            a1 += __shfl_xor_sync(FULL, g1, 16);
+            double r = h8 ? a1 : a0;
+            r += __shfl_xor_sync(FULL, h8 ? a0 : a1, 8);
+#pragma unroll
+            for (int d = 4; d > 0; d >>= 1) r += __shfl_xor_sync(FULL, r, d);
+            if ((lane & 7) == 0) sc.part[warp][q + (lane >> 3)] = r;      // lane 8k holds candidate q + k
+        }
+        sync();
+        if (warp == 0 && lane < EXACT_BATCH && b0 + lane < n) {
+            double v = 0.0;
+#pragma unroll
+            for (int k = 0; k < EXACT_WARPS; k++) v += sc.part[k][lane];
+            v *= EXACT_UNSCALE;
+            const int e = sc.cand[b0 + lane];
+            if (bias) v += (double)bias[e];
+            if (fabs(v - (double)sc.approx[b0 + lane]) > bound) atomicOr(status, OMNI_ST_ROUTER_EPS);
+            const float hi = (float)v;
+            logits[row * OMNI_E + e] = hi;
+            if (low) low[row * OMNI_E + e] = (float)(v - (double)hi);
+            sc.exact[e] = mine_v = v;
+        }
+        if (b0 + EXACT_BATCH < n) sync();                 // the partial sums are read before the next batch's are written
+    }
+    if (warp == 0) {
+        __syncwarp();
+        double v = -CUDART_INF;
+        int id = 0;
+        if (n <= EXACT_BATCH) {
+            // order of a few candidates: each counts those in front of it
+            const int e = lane < n ? sc.cand[lane] : OMNI_E;
+            int rank = lane < n ? 0 : 32;
+            for (int j = 0; j < n; j++) {
+                const double ov = __shfl_sync(FULL, mine_v, j);
+                const int oid = __shfl_sync(FULL, e, j);
+                if (j != lane && better(ov, oid, mine_v, e)) rank++;
+            }
+            if (rank < 8) { sc.sorted_v[rank] = mine_v; sc.sorted_id[rank] = e; }
+            __syncwarp();
+            if (lane < 8) { v = sc.sorted_v[lane]; id = sc.sorted_id[lane]; }
+        } else {
+            double exact[4], fin_v[9];
+            int fin_id[9];
+#pragma unroll
+            for (int j = 0; j < 4; j++) exact[j] = sc.exact[lane + 32 * j];
+            warp_top8(exact, lane, fin_v, fin_id);
+#pragma unroll
+            for (int k = 0; k < 8; k++) if (lane == k) { v = fin_v[k]; id = fin_id[k]; }
+        }
+        write_ranked(v, id, lane, ids, weights, row);
+        if (segcount && lane < 8 && id != old_id) {       // a row's eight assignments share one segment
+            int32_t *c = segcount + (row * OMNI_TOP / OMNI_SEG) * OMNI_E;
+            atomicSub(c + old_id, 1);
+            atomicAdd(c + id, 1);
+        }
+    }
 }
 
 }  // namespace

@@ -83,13 +83,18 @@ __global__ void __launch_bounds__(256) select_kernel(const float *__restrict__ l
     if (close && lane == 0) { const int at = atomicAdd(n_flag, 1); if (at < OMNI_CHUNK) flag_rows[at] = (int32_t)row; }
 }
 
-// One block (four warps) per flagged row; with eight warps, for fewer rounds of candidates, it measured
-// 3 to 5 us slower from 4096 tokens on.  Its blocks become resident while the router runs, when device
+// This block's share of a request for memory to be brought into L2, spread over the grid.
+__device__ __forceinline__ void prefetch_share(const char *p, int pieces) {
+    for (int i = blockIdx.x + gridDim.x * threadIdx.x; i < pieces; i += gridDim.x * blockDim.x)
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p + (size_t)i * OMNI_PREFETCH_PIECE), "r"(OMNI_PREFETCH_PIECE) : "memory");
+}
+
+// One block per flagged row.  Its blocks become resident while the router runs, when device
 // memory is idle: with `prefetch` given they ask for that much of the expert weights to be
 // brought into L2 meanwhile.  That takes blocks on every SM: 48 MiB requested by the 37 blocks of a norm
 // kernel held that kernel up by 29 us.
 template <bool PREFETCH>
-__global__ void __launch_bounds__(128) recheck_kernel(const __nv_bfloat16 *__restrict__ xn,
+__global__ void __launch_bounds__(EXACT_THREADS) recheck_kernel(const __nv_bfloat16 *__restrict__ xn,
                                                       const __nv_bfloat16 *__restrict__ w,
                                                       const float *__restrict__ bias, float *__restrict__ logits,
                                                       float *__restrict__ low, const int32_t *__restrict__ flag_rows,
@@ -97,17 +102,15 @@ __global__ void __launch_bounds__(128) recheck_kernel(const __nv_bfloat16 *__res
                                                       int32_t *__restrict__ ids, float *__restrict__ weights,
                                                       int32_t *__restrict__ segcount, uint32_t *__restrict__ status,
                                                       const char *prefetch, int prefetch_pieces) {
-    __shared__ double exact_s[OMNI_E];
-    if (PREFETCH)
-        for (int i = blockIdx.x + gridDim.x * threadIdx.x; i < prefetch_pieces; i += gridDim.x * blockDim.x)
-            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(prefetch + (size_t)i * OMNI_PREFETCH_PIECE), "r"(OMNI_PREFETCH_PIECE) : "memory");
+    __shared__ ExactScratch scratch;
+    if (PREFETCH) prefetch_share(prefetch, prefetch_pieces);
     dep_wait();
     dep_launch();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int n = *n_flag;
     if (n > T) n = T;                  // a count left by a pass that failed half-way can be no larger than this
     for (int f = blockIdx.x; f < n; f += gridDim.x)
-        recheck_row(xn, w, bias, logits, low, flag_rows[f], eps, ids, weights, segcount, status, exact_s, lane, warp, [] { __syncthreads(); });
+        recheck_row(xn, w, bias, logits, low, flag_rows[f], eps, ids, weights, segcount, status, scratch, lane, warp, [] { __syncthreads(); });
 }
 
 // Exact logits for every (token, expert): tests only (tests/test_omni_router.m).
@@ -525,7 +528,7 @@ cudaError_t omni_launch_recheck(int32_t *segcount, const void *xn, const void *r
     int blocks = T < 148 * 8 ? T : 148 * 8;
     const int pieces = (int)(prefetch_bytes / OMNI_PREFETCH_PIECE);
     if (pieces && blocks < 148) blocks = 148;
-    return omni_launch_chain(pieces ? recheck_kernel<true> : recheck_kernel<false>, dim3(blocks), dim3(128), 0, s, (const __nv_bfloat16 *)xn,
+    return omni_launch_chain(pieces ? recheck_kernel<true> : recheck_kernel<false>, dim3(blocks), dim3(EXACT_THREADS), 0, s, (const __nv_bfloat16 *)xn,
                              (const __nv_bfloat16 *)router, bias, logits, low, flag_rows, n_flag, T, eps, ids, weights, segcount, status,
                              (const char *)prefetch, pieces);
 }

@@ -56,12 +56,12 @@ typedef struct {
     int32_t *offsets;      /* [E+1] exclusive prefix sum of counts    */
     int32_t *rowmap;       /* [rows*8] token of each permuted row     */
     int32_t *slots;        /* [rows*8] permuted row of assignment i   */
-    int32_t *segcount;     /* [MAX_SEGS][E] per-segment histograms, then exclusive bases */
+    int32_t *segcount;     /* [MAX_SEGS][E] per-segment histograms */
     omni_ttile *ttiles;    /* [MAX_TTILES] expert-major, an expert's rows in near-equal tiles */
     int32_t *n_ttiles;     /* [1]                                     */
-    int32_t *sched;        /* [8] work counters: [0] gate/up, [1..] down (one per launch group), zeroed by the scan */
+    int32_t *sched;        /* [8] work counters: [0] gate/up, [1..] down (one per launch group), zeroed by the sort */
     uint32_t *status;      /* [1]                                     */
-    int32_t *n_flag;       /* [2] rows flagged for the exact pass: the scan moves [0] to [1] and clears [0] for the next pass */
+    int32_t *n_flag;       /* [2] rows flagged for the exact pass: the sort moves [0] to [1] and clears [0] for the next pass */
     int32_t tile_n;        /* most rows of a token tile: OMNI_TILE_N or OMNI_TILE_N1, as the expert kernels of the pass take */
     int32_t longest_first; /* tile list in order of falling tile length (else in expert order) */
 } omni_sort_state;

@@ -177,120 +177,160 @@ __global__ void __launch_bounds__(256) assign_hist_kernel(const int32_t *__restr
     }
 }
 
-// One block, 1024 threads = 8 groups x 128 experts.  Turns segment histograms into exclusive
-// per-segment bases, writes counts/offsets and the token-tile list of the expert GEMMs.
-__global__ void __launch_bounds__(1024) assign_scan_kernel(int nseg, omni_sort_state st) {
-    __shared__ int part[8][OMNI_E];
-    __shared__ int warp_rows[4], warp_tiles[4];
-    __shared__ int tile_key[OMNI_E], tile_cnt[OMNI_E];       // per expert: rows per token tile, token tiles
-    dep_wait();
-    dep_launch();
-    const int e = threadIdx.x & (OMNI_E - 1), grp = threadIdx.x >> 7, lane = threadIdx.x & 31;
-    const int per = (nseg + 7) / 8;
-    const int s0 = grp * per, s1 = min(nseg, s0 + per);
-    // up to 16 segments per thread (4096 tokens) stay in registers between the two sweeps
-    constexpr int KEEP = 16;
-    int c[KEEP];
-    int sum = 0;
-#pragma unroll
-    for (int i = 0; i < KEEP; i++) {
-        c[i] = s0 + i < s1 ? st.segcount[(long)(s0 + i) * OMNI_E + e] : 0;
-        sum += c[i];
-    }
-    for (int s = s0 + KEEP; s < s1; s++) sum += st.segcount[(long)s * OMNI_E + e];
-    part[grp][e] = sum;
-    __syncthreads();
-    int run = 0;
-    for (int gq = 0; gq < grp; gq++) run += part[gq][e];
-#pragma unroll
-    for (int i = 0; i < KEEP; i++) {
-        if (s0 + i < s1) { st.segcount[(long)(s0 + i) * OMNI_E + e] = run; run += c[i]; }
-    }
-    for (int s = s0 + KEEP; s < s1; s++) {
-        const int v = st.segcount[(long)s * OMNI_E + e];
-        st.segcount[(long)s * OMNI_E + e] = run;
-        run += v;
-    }
+// Scan over the experts, of the kernel that places assignments; called by all threads of a block
+// (at least 128), thread e < 128 with the number of rows of expert e.  Returns the expert's offset to
+// thread e; with `publish` also writes counts, offsets and the token-tile list of the expert products
+// and resets the counters that the rest of the pass starts from.
+struct ExpertScan { int warp_rows[4], warp_tiles[4]; int4 key[OMNI_E / 4], cnt[OMNI_E / 4]; };
+
+__device__ __forceinline__ int scan_experts(ExpertScan &sm, int total, const omni_sort_state &st, bool publish) {
+    const int e = threadIdx.x, lane = threadIdx.x & 31;
     // inclusive scans over the 128 experts (rows and token tiles): shuffles inside each of the
-    // four warps of group 0, then the totals of the warps before
-    int total = 0, rows_incl = 0, tiles_incl = 0;
-    if (grp == 0) {
-#pragma unroll
-        for (int gq = 0; gq < 8; gq++) total += part[gq][e];
-        rows_incl = total;
-        tiles_incl = (total + st.tile_n - 1) / st.tile_n;
+    // first four warps, then the totals of the warps before
+    const int nt = (total + st.tile_n - 1) / st.tile_n;
+    int rows_incl = total, tiles_incl = nt;
+    // order of the tile list: falling tile length, equal ones by expert
+    const int key = nt ? total / nt * OMNI_E + (OMNI_E - 1 - e) : OMNI_E - 1 - e;
+    if (e < OMNI_E) {
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
             const int a = __shfl_up_sync(FULL, rows_incl, d), b = __shfl_up_sync(FULL, tiles_incl, d);
             if (lane >= d) { rows_incl += a; tiles_incl += b; }
         }
-        if (lane == 31) { warp_rows[e >> 5] = rows_incl; warp_tiles[e >> 5] = tiles_incl; }
-        tile_cnt[e] = (total + st.tile_n - 1) / st.tile_n;
-        tile_key[e] = tile_cnt[e] ? total / tile_cnt[e] : 0;
+        if (lane == 31) { sm.warp_rows[e >> 5] = rows_incl; sm.warp_tiles[e >> 5] = tiles_incl; }
+        reinterpret_cast<int *>(sm.key)[e] = key;
+        reinterpret_cast<int *>(sm.cnt)[e] = nt;
     }
     __syncthreads();
-    if (grp == 0) {
-        for (int q = 0; q < (e >> 5); q++) { rows_incl += warp_rows[q]; tiles_incl += warp_tiles[q]; }
-        const int n = total;
-        const int off = rows_incl - n;
-        st.counts[e] = n;
-        st.offsets[e] = off;
-        if (e == OMNI_E - 1) st.offsets[OMNI_E] = rows_incl;
-        // Expert-major tile list, the experts in order of falling tile length (ties by id): the work
-        // items of the persistent expert kernels are claimed in list order, so the longest come first
-        // and the short ones fill the end of the launch.  Rows and offsets stay in expert order.  Both products
-        // read this list: with one in expert order for the down product a block took 437.5 us against 438 (4096
-        // tokens), 742 against 743 (8192), 1367 against 1374 (16384), 653 against 655 (8192, skewed).
-        const int nt = (n + st.tile_n - 1) / st.tile_n;
-        const int key = tile_key[e];
-        int first = tiles_incl - nt;
-        if (st.longest_first) {
-            first = 0;
+    if (e >= OMNI_E) return 0;
+    for (int q = 0; q < (e >> 5); q++) { rows_incl += sm.warp_rows[q]; tiles_incl += sm.warp_tiles[q]; }
+    const int off = rows_incl - total;
+    if (!publish) return off;
+    st.counts[e] = total;
+    st.offsets[e] = off;
+    if (e == OMNI_E - 1) st.offsets[OMNI_E] = rows_incl;
+    // Expert-major tile list, the experts in order of falling tile length (ties by id): the work
+    // items of the persistent expert kernels are claimed in list order, so the longest come first
+    // and the short ones fill the end of the launch.  Rows and offsets stay in expert order.  Both products
+    // read this list: with one in expert order for the down product a block took 437.5 us against 438 (4096
+    // tokens), 742 against 743 (8192), 1367 against 1374 (16384), 653 against 655 (8192, skewed).
+    int first = tiles_incl - nt;
+    if (st.longest_first) {
+        first = 0;
 #pragma unroll 8
-            for (int o = 0; o < OMNI_E; o++) {
-                const int okey = tile_key[o];
-                if (okey > key || (okey == key && o < e)) first += tile_cnt[o];
-            }
+        for (int o = 0; o < OMNI_E / 4; o++) {
+            const int4 k = sm.key[o], c = sm.cnt[o];
+            first += (k.x > key ? c.x : 0) + (k.y > key ? c.y : 0) + (k.z > key ? c.z : 0) + (k.w > key ? c.w : 0);
         }
-        // an expert's rows are split into nt tiles of near-equal length: tiles that share a
-        // weight tile then advance at the same pace and meet in L2
-        const int base = nt ? n / nt : 0, extra = nt ? n % nt : 0;
-        for (int j = 0; j < nt; j++)
-            st.ttiles[first + j] = omni_ttile{e, off + j * base + min(j, extra), base + (j < extra), first | (nt << 16)};
-        if (e < 8) st.sched[e] = 0;
-        if (e == OMNI_E - 1) *st.n_ttiles = tiles_incl;
-        // the router and the exact pass of this chunk are done with the flagged-row count: keep it
-        // for introspection and clear it for the next router launch (no memset between passes)
-        if (e == 0 && st.n_flag) { st.n_flag[1] = st.n_flag[0]; st.n_flag[0] = 0; }
     }
+    // an expert's rows are split into nt tiles of near-equal length: tiles that share a
+    // weight tile then advance at the same pace and meet in L2
+    const int base = nt ? total / nt : 0, extra = nt ? total % nt : 0;
+    for (int j = 0; j < nt; j++)
+        st.ttiles[first + j] = omni_ttile{e, off + j * base + min(j, extra), base + (j < extra), first | (nt << 16)};
+    if (e < 8) st.sched[e] = 0;
+    if (e == OMNI_E - 1) *st.n_ttiles = tiles_incl;
+    // the router and the exact pass of this chunk are done with the flagged-row count: keep it
+    // for introspection and clear it for the next router launch (no memset between passes)
+    if (e == 0 && st.n_flag) { st.n_flag[1] = st.n_flag[0]; st.n_flag[0] = 0; }
+    return off;
 }
 
-__global__ void __launch_bounds__(256) assign_scatter_kernel(const int32_t *__restrict__ ids, int A, int nseg,
-                                                             omni_sort_state st) {
-    __shared__ int base[8][OMNI_E];
+// Counting sort behind the segment histograms: every block takes eight segments (a warp each) and works
+// out for itself where they start, from all of the histograms -- 512 bytes per segment from L2,
+// 256 KiB at 16384 tokens.  As a kernel of one block in front of the scatter that scan was a link
+// of its own in the chain of launches, and its single block took 15 us at 16384 tokens.
+constexpr int ASSIGN_SEGS = 8, ASSIGN_THREADS = 32 * ASSIGN_SEGS;
+__global__ void __launch_bounds__(ASSIGN_THREADS) assign_kernel(const int32_t *__restrict__ ids, int A, int nseg, omni_sort_state st) {
+    __shared__ ExpertScan scan;
+    __shared__ int4 all[ASSIGN_SEGS][OMNI_E / 4], front[ASSIGN_SEGS][OMNI_E / 4];     // sums of a warp's share of the segments
+    __shared__ int4 own[ASSIGN_SEGS][OMNI_E / 4];                                     // counts of this block's segments, then where they start
+    __shared__ unsigned mask[ASSIGN_SEGS][OMNI_E];
     dep_wait();
     dep_launch();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int seg = blockIdx.x * 8 + warp;
-    if (seg >= nseg) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, e = threadIdx.x;
+    const int seg0 = blockIdx.x * ASSIGN_SEGS, seg = seg0 + warp;
+    const int t = seg * 32 + lane;                                                    // a segment is the 8 assignments of 32 tokens
+    const bool have = t * OMNI_TOP < A;
+    int id[OMNI_TOP];                                                                 // loaded while the histograms are summed
+    if (have && !((uintptr_t)ids & 15)) {
+        const int4 a = *(reinterpret_cast<const int4 *>(ids) + 2 * t), b = *(reinterpret_cast<const int4 *>(ids) + 2 * t + 1);
+        id[0] = a.x; id[1] = a.y; id[2] = a.z; id[3] = a.w; id[4] = b.x; id[5] = b.y; id[6] = b.z; id[7] = b.w;
+    } else {
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        const int e = lane + 32 * j;
-        base[warp][e] = st.offsets[e] + st.segcount[(long)seg * OMNI_E + e];
+        for (int k = 0; k < OMNI_TOP; k++) id[k] = have ? ids[t * OMNI_TOP + k] : 0;
     }
-    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < OMNI_TOP; k++) id[k] &= OMNI_E - 1;
+    const int4 *hist = reinterpret_cast<const int4 *>(st.segcount) + lane;
+    auto add = [](int4 &a, const int4 &b) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; };
+    int4 mine = seg < nseg ? hist[(long)seg * (OMNI_E / 4)] : make_int4(0, 0, 0, 0), fr = make_int4(0, 0, 0, 0);
+    own[warp][lane] = mine;
+#pragma unroll 8
+    for (int s = warp; s < seg0; s += ASSIGN_SEGS) add(fr, hist[(long)s * (OMNI_E / 4)]);
+    add(mine, fr);
+#pragma unroll 8
+    for (int s = seg + ASSIGN_SEGS; s < nseg; s += ASSIGN_SEGS) add(mine, hist[(long)s * (OMNI_E / 4)]);
+    all[warp][lane] = mine;
+    front[warp][lane] = fr;
+#pragma unroll
+    for (int j = 0; j < 4; j++) mask[warp][lane + 32 * j] = 0;
+    __syncthreads();
+    // a token's experts are distinct as a rule, so the tokens of a segment that chose an expert are a mask of
+    // 32 bits and a token's rank among them a count of bits
+    bool twice = false;
+    if (have)
+#pragma unroll
+        for (int k = 0; k < OMNI_TOP; k++) twice |= (atomicOr(&mask[warp][id[k]], 1u << lane) >> lane) & 1;
+    int total = 0, run = 0;
+    if (e < OMNI_E)
+#pragma unroll
+        for (int q = 0; q < ASSIGN_SEGS; q++) {
+            total += reinterpret_cast<const int *>(all[q])[e];
+            run += reinterpret_cast<const int *>(front[q])[e];
+        }
+    run += scan_experts(scan, total, st, blockIdx.x == 0);
+    if (e < OMNI_E)
+#pragma unroll
+        for (int q = 0; q < ASSIGN_SEGS; q++) {
+            int *c = reinterpret_cast<int *>(own[q]) + e;
+            const int n = *c;
+            *c = run;
+            run += n;
+        }
+    __syncthreads();
+    if (seg >= nseg) return;
+    int *base = reinterpret_cast<int *>(own[warp]);
     const unsigned lt = (1u << lane) - 1u;
+    if (!__any_sync(FULL, twice)) {
+        if (!have) return;
+        int row[OMNI_TOP];
+#pragma unroll
+        for (int k = 0; k < OMNI_TOP; k++) {
+            row[k] = base[id[k]] + __popc(mask[warp][id[k]] & lt);
+            st.rowmap[row[k]] = t;
+        }
+        if (!((uintptr_t)st.slots & 15)) {
+            reinterpret_cast<int4 *>(st.slots)[2 * t] = make_int4(row[0], row[1], row[2], row[3]);
+            reinterpret_cast<int4 *>(st.slots)[2 * t + 1] = make_int4(row[4], row[5], row[6], row[7]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < OMNI_TOP; k++) st.slots[t * OMNI_TOP + k] = row[k];
+        }
+        return;
+    }
+    // caller-supplied ids that name an expert twice for one token: assignments in order, 32 at a time
     for (int it = 0; it < OMNI_SEG / 32; it++) {
         const int i = seg * OMNI_SEG + it * 32 + lane;
-        int e = i < A ? (ids[i] & (OMNI_E - 1)) : -1;
-        const unsigned m = __match_any_sync(FULL, e);
-        if (e >= 0) {
-            const int row = base[warp][e] + __popc(m & lt);
+        const int ei = i < A ? (ids[i] & (OMNI_E - 1)) : -1;
+        const unsigned m = __match_any_sync(FULL, ei);
+        if (ei >= 0) {
+            const int row = base[ei] + __popc(m & lt);
             st.slots[i] = row;
             st.rowmap[row] = i >> 3;
         }
         __syncwarp();
-        if (e >= 0 && lane == __ffs(m) - 1) base[warp][e] += __popc(m);
+        if (ei >= 0 && lane == __ffs(m) - 1) base[ei] += __popc(m);
         __syncwarp();
     }
 }
@@ -555,8 +595,8 @@ cudaError_t omni_launch_assign(const int32_t *ids, int rows, omni_sort_state st,
     const int blocks = (nseg + 7) / 8;
     cudaError_t e = cudaSuccess;
     if (!have_counts) e = omni_launch_chain(assign_hist_kernel, dim3(blocks), dim3(256), 0, s, ids, A, nseg, st.segcount, st.status);
-    if (e == cudaSuccess) e = omni_launch_chain(assign_scan_kernel, dim3(1), dim3(1024), 0, s, nseg, st);
-    if (e == cudaSuccess) e = omni_launch_chain(assign_scatter_kernel, dim3(blocks), dim3(256), 0, s, ids, A, nseg, st);
+    if (e == cudaSuccess)
+        e = omni_launch_chain(assign_kernel, dim3((nseg + ASSIGN_SEGS - 1) / ASSIGN_SEGS), dim3(ASSIGN_THREADS), 0, s, ids, A, nseg, st);
     return e;
 }
 

@@ -39,6 +39,25 @@ def test_assign_matches_serial_oracle_word_for_word(backend, pattern):
             assert np.array_equal(in_view.cpu().numpy(), ids.reshape(-1))
 
 
+@pytest.mark.parametrize("rows", [31, 32, 33, 255, 256, 257, 513, 2049])
+@pytest.mark.parametrize("shift", [1, 2])
+def test_assign_takes_any_word_alignment(backend, rows, shift):
+    """Ids and results at 4- and 8-byte offsets (the vector accesses need 16), around the 32 tokens of a segment and
+    the 8 segments of a block; one token names an expert twice, so its segment takes the ordered path."""
+    ids = ((np.arange(rows)[:, None] * 5 + np.arange(8) * 3) % 128).astype(np.int32)
+    ids[rows // 2, 3] = ids[rows // 2, 1]
+    want = c_oracle.assign_canonical(ids)
+    in_buf, in_view = guarded(rows * 8, shift)
+    in_view.copy_(torch.from_numpy(ids.reshape(-1)))
+    outs = [guarded(n, shift) for n in (128, 129, rows * 8, rows * 8)]
+    backend.begin()
+    backend.stage_assign(in_view.view(rows, 8), *[v for _, v in outs])
+    backend.complete()
+    for (buf, view), w in zip(outs, want):
+        assert np.array_equal(view.cpu().numpy(), w)
+        assert (buf[:GUARD].cpu() == POISON).all() and (buf[-GUARD:].cpu() == POISON).all()
+
+
 def test_assign_rejects_out_of_range_ids(backend):
     ids = torch.zeros(4, 8, dtype=torch.int32, device="cuda")
     ids[2, 3] = 128

@@ -28,6 +28,7 @@ typedef struct {
     float *bias;                        /* device, FP32 [128] or NULL */
     bool owned, bound;
     CUtensorMap tm_router, tm_down;
+    CUtensorMap tm_router_part;         /* {64, expert, K / 64} view of the router matrix for short batches */
     CUtensorMap tm_gate_up4;            /* {K, row, gate|up, block} view of gate_up: a box interleaves blocks of gate and up rows */
 } omni_layer;
 
@@ -162,6 +163,17 @@ static bool make_map(clef_gpu *g, CUtensorMap *map, const void *base, uint64_t r
     const cuuint32_t estr[2] = {1, 1};
     return g->encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void *)base, dims, strides, box, estr,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, promo,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+/* A [rows][cols] matrix as {64, row, cols / 64}: one box brings several K slabs of the same rows. */
+static bool make_slab_map(clef_gpu *g, CUtensorMap *map, const void *base, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t slabs) {
+    const cuuint64_t dims[3] = {64, rows, cols / 64};
+    const cuuint64_t strides[2] = {cols * 2, 128};
+    const cuuint32_t box[3] = {64, box_rows, slabs};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    return g->encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, (void *)base, dims, strides, box, estr,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -544,6 +556,7 @@ bool clef_omni_bind_layer(clef_gpu *g, int layer, const void *router, const void
         }
     }
     if (!make_map(g, &next.tm_router, next.router, OMNI_E, OMNI_H, 128, CU_TENSOR_MAP_L2_PROMOTION_L2_128B) ||
+        !make_slab_map(g, &next.tm_router_part, next.router, OMNI_E, OMNI_H, OMNI_PART_EXPERTS, OMNI_PART_SLABS) ||
         !make_map(g, &next.tm_down, next.down, (uint64_t)EL * OMNI_H, OMNI_F, 128, CU_TENSOR_MAP_L2_PROMOTION_L2_256B) ||
         !make_gate_up4(g, &next.tm_gate_up4, next.gate_up, (uint64_t)EL)) {
         free_layer(&next);
@@ -585,18 +598,48 @@ static void stage_mark(clef_gpu *g, int i) { if (g->profile) cudaEventRecord(g->
 #define PREFETCH_MAX_ROWS 512
 #define PREFETCH_BYTES ((size_t)24 << 20)
 
-/* router + exact pass for one chunk; fills arena ids/weights/logits */
-static bool run_router(clef_gpu *g, const omni_layer *L, const void *xn, int rows, bool *have_counts) {
+/* What the routing of a chunk leaves for the sort: nothing, the expert counts per segment, or nothing to do. */
+typedef enum { ROUTED_IDS, ROUTED_COUNTS, ROUTED_SORTED } omni_routed;
+
+static int expert_ctas(const clef_gpu *g, int rows) {
+    /* pairs of CTAs unless the call says otherwise or the batch is a token or two: then eight to sixteen
+     * experts make fewer pair items (6 of 256 gate/up rows per expert) than there are pairs, and
+     * single CTAs with half the rows each spread over twice as many SMs (1 token: 16 us against 22);
+     * "reserve_sms" may also leave a single SM, which is no pair */
+    return g->expert_kernel ? g->expert_kernel : rows <= 2 || g->n_sm - g->reserve_sms < 2 ? 1 : 2;
+}
+/* the sort's state with token tiles as the expert kernels of the pass take them */
+static omni_sort_state expert_sort(const clef_gpu *g, int ctas) {
+    omni_sort_state sort = g->omni->sort;
+    sort.tile_n = ctas == 1 ? OMNI_TILE_N1 : OMNI_TILE_N;
+    return sort;
+}
+
+/* router + exact pass for one chunk, and the sort where the same launch does it; fills arena ids/weights/logits */
+static bool run_router(clef_gpu *g, const omni_layer *L, const void *xn, int rows, omni_routed *routed) {
     omni_arena *s = g->omni;
     bool fused = false;
-    *have_counts = false;
-    /* the flagged-row count is cleared by begin and, after each chunk, by the scan kernel: no
+    *routed = ROUTED_IDS;
+    /* the flagged-row count is cleared by begin and, after each chunk, by the sort: no
      * memset node sits between the kernels of consecutive layers */
     /* the remainders of the exact logits are only read by route capture */
     float *low = g->trace ? s->logits_low : NULL;
     if (low && !launched(g, "capture reset", cudaMemsetAsync(low, 0, (size_t)rows * OMNI_E * 4, g->stream))) return false;
+    const size_t prefetch = g->ep.world <= 1 && rows >= PREFETCH_MIN_ROWS && rows <= PREFETCH_MAX_ROWS ? PREFETCH_BYTES : 0;
+    CUtensorMap tm_x;
+    /* Short batches: two launches, up to what the first one's CTAs (16 experts x 32 tokens) fit on the SMs at once. */
+    if (g->router_impl == 0 && g->fused_router && !g->debug_stamps && g->ep.world <= 1 && rows <= OMNI_ROUTE_MAX_ROWS) {
+        if (!make_slab_map(g, &tm_x, xn, (uint64_t)rows, OMNI_H, (uint32_t)omni_router_part_tile(rows), OMNI_PART_SLABS)) {
+            note_failure(g, "router activation descriptor", cudaErrorInvalidValue);
+            return false;
+        }
+        if (!launched(g, "router", omni_launch_router_part(&tm_x, &L->tm_router_part, L->bias, rows, s->logits, s->status, g->stream)) ||
+            !launched(g, "route", omni_launch_route(xn, L->router, L->bias, s->logits, low, rows, g->router_eps, g->router_exact, s->ids, s->weights,
+                                                    expert_sort(g, expert_ctas(g, rows)), L->gate_up, prefetch, g->stream))) return false;
+        *routed = ROUTED_SORTED;
+        return true;
+    }
     if (g->router_impl == 0) {
-        CUtensorMap tm_x;
         const int nt = omni_router_tile(rows, g->n_sm);
         if (!make_map(g, &tm_x, xn, (uint64_t)rows, OMNI_H, (uint32_t)nt, CU_TENSOR_MAP_L2_PROMOTION_L2_128B)) {
             note_failure(g, "router activation descriptor", cudaErrorInvalidValue);
@@ -614,27 +657,22 @@ static bool run_router(clef_gpu *g, const omni_layer *L, const void *xn, int row
         if (!launched(g, "route", omni_launch_select(s->logits, rows, g->router_eps, g->router_exact, s->ids, s->weights,
                                                      s->flag_rows, s->n_flag, s->status, g->stream))) return false;
     }
-    const size_t prefetch = g->ep.world <= 1 && rows >= PREFETCH_MIN_ROWS && rows <= PREFETCH_MAX_ROWS ? PREFETCH_BYTES : 0;
     if (!launched(g, "router exact pass", omni_launch_recheck(fused ? s->sort.segcount : NULL, xn, L->router, L->bias, s->logits, low, s->flag_rows,
                                                               s->n_flag, rows, g->router_eps, s->ids, s->weights, s->status, L->gate_up,
                                                               prefetch, g->stream))) return false;
-    *have_counts = fused;
+    *routed = fused ? ROUTED_COUNTS : ROUTED_IDS;
     return true;
 }
 
 /* permutation + expert products + combine for one chunk, routing taken from ids/weights */
 static bool run_experts(clef_gpu *g, const omni_layer *L, const void *xn, const int32_t *ids, const float *weights,
-                        float *x, int rows, bool have_counts) {
+                        float *x, int rows, omni_routed routed) {
     omni_arena *s = g->omni;
     const int rows8 = rows * OMNI_TOP;
-    /* pairs of CTAs unless the call says otherwise or the batch is a token or two: then eight to sixteen
-     * experts make fewer pair items (6 of 256 gate/up rows per expert) than there are pairs, and
-     * single CTAs with half the rows each spread over twice as many SMs (1 token: 16 us against 22);
-     * "reserve_sms" may also leave a single SM, which is no pair */
-    const int ctas = g->expert_kernel ? g->expert_kernel : rows <= 2 || g->n_sm - g->reserve_sms < 2 ? 1 : 2;
-    omni_sort_state sort = s->sort;
-    sort.tile_n = ctas == 1 ? OMNI_TILE_N1 : OMNI_TILE_N;
-    if (!launched(g, "assign", omni_launch_assign(ids, rows, sort, have_counts, g->stream))) return false;
+    const int ctas = expert_ctas(g, rows);
+    const omni_sort_state sort = expert_sort(g, ctas);
+    /* counted among the launches of a pass (fault injection) whichever kernel sorts */
+    if (!launched(g, "assign", routed == ROUTED_SORTED ? cudaSuccess : omni_launch_assign(ids, rows, sort, routed == ROUTED_COUNTS, g->stream))) return false;
     /* the tensor-core gate/up kernel fetches its token rows through rowmap itself; the copy
      * into expert order is only made for the check kernels (or when "fused_gather" is 0) */
     const bool fused = g->gemm_impl == 0 && g->fused_gather;
@@ -672,17 +710,16 @@ static bool run_experts(clef_gpu *g, const omni_layer *L, const void *xn, const 
  * ep_fused = 0 (for comparison, same bits): a copy kernel dispatches all rows and a barrier
  * follows before the gate/up kernel starts; the way back is the same as above. */
 static bool run_experts_ep(clef_gpu *g, const omni_layer *L, const void *xn, const int32_t *ids, const float *weights,
-                           float *x, int rows, bool have_counts) {
+                           float *x, int rows, omni_routed routed) {
     omni_arena *s = g->omni;
     const int rows8 = rows * OMNI_TOP;
     const omni_ep_peers *pe = &g->ep.peers;
     const int ctas = g->expert_kernel == 1 ? 1 : 2;
     const int n_gemm = g->n_sm - g->reserve_sms;
-    omni_sort_state sort = s->sort;
-    sort.tile_n = ctas == 1 ? OMNI_TILE_N1 : OMNI_TILE_N;
+    const omni_sort_state sort = expert_sort(g, ctas);
     if (g->ep_fused && !launched(g, "expert-parallel buckets", omni_launch_ep_buckets(ids, rows, pe->world, g->ep.tok_slot, g->ep.bucket_cnt,
                                                                                        g->ep.bucket_list, g->stream))) return false;
-    if (!launched(g, "assign", omni_launch_assign(ids, rows, sort, have_counts, g->stream))) return false;
+    if (!launched(g, "assign", omni_launch_assign(ids, rows, sort, routed == ROUTED_COUNTS, g->stream))) return false;
     if (!launched(g, "expert-parallel plan", omni_launch_ep_plan(pe, ++g->ep.epoch, sort, g->ep.send_base, g->ep.n_local_rows, g->ep.need,
                                                                  g->ep.bucket_cnt, g->ep.send_cnt, g->ep.recv_base, g->ep.wait_ns, g->stream))) return false;
     if (g->ep_fused) {
@@ -745,16 +782,16 @@ static bool encode_chunks(clef_gpu *g, int layer, const void *xn, float *x, int 
         const int rows = T - start < OMNI_CHUNK ? T - start : OMNI_CHUNK;
         const char *xn_c = xn ? (const char *)xn + (size_t)start * OMNI_H * 2 : (const char *)g->xnorm;
         stage_mark(g, 0);
-        bool have_counts = false;
+        omni_routed routed = ROUTED_IDS;
         bool ok = xn || launched(g, "rmsnorm", omni_launch_rmsnorm(x + (size_t)start * OMNI_H, g->norm_w[layer], g->norm_eps[layer],
                                                                    rows, g->xnorm, g->stream));
-        if (ok) ok = run_router(g, L, xn_c, rows, &have_counts);
+        if (ok) ok = run_router(g, L, xn_c, rows, &routed);
         if (ok && g->trace && layer < g->trace_layers && start + rows > g->trace_first)
             ok = launched(g, "route capture", omni_launch_trace(s->logits, s->logits_low, s->ids, s->weights, rows, start, g->trace_first,
                                                                 g->trace_rows, layer, g->trace, g->stream));
         stage_mark(g, 1);
-        if (ok) ok = g->ep.world > 1 ? run_experts_ep(g, L, xn_c, s->ids, s->weights, x + (size_t)start * OMNI_H, rows, have_counts)
-                                     : run_experts(g, L, xn_c, s->ids, s->weights, x + (size_t)start * OMNI_H, rows, have_counts);
+        if (ok) ok = g->ep.world > 1 ? run_experts_ep(g, L, xn_c, s->ids, s->weights, x + (size_t)start * OMNI_H, rows, routed)
+                                     : run_experts(g, L, xn_c, s->ids, s->weights, x + (size_t)start * OMNI_H, rows, routed);
         if (!ok) {
             if (g->ep.world > 1) g->ep.need_sync = true;     /* this rank launched fewer barriers than its peers */
             set_err(err, errlen, "%s", g->fail_msg);
@@ -961,7 +998,7 @@ bool clef_omni_stage_experts(clef_gpu *g, int layer, const void *xn, const int32
         return false;
     }
     stage_mark(g, 0); stage_mark(g, 1);
-    if (!run_experts(g, &g->layer[layer], xn, ids, weights, x, T, false)) { set_err(err, errlen, "%s", g->fail_msg); return false; }
+    if (!run_experts(g, &g->layer[layer], xn, ids, weights, x, T, ROUTED_IDS)) { set_err(err, errlen, "%s", g->fail_msg); return false; }
     book_profile(g);
     g->last_T = T;
     return true;

@@ -21,6 +21,7 @@ enum {
     OMNI_TILE_N = 256,                     /* most token rows per expert-GEMM tile on pairs of CTAs */
     OMNI_TILE_N1 = 128,                    /* and on single CTAs */
     OMNI_TOK_BOXES = 16,                   /* tensor maps of a token operand: box i is 16 (i + 1) rows high */
+    OMNI_ROUTE_MAX_ROWS = 576,             /* most tokens that the short batches' routing (omni_launch_route) takes */
     OMNI_MAX_TTILES = OMNI_ROWS / OMNI_TILE_N1 + OMNI_E,
 };
 
@@ -61,7 +62,8 @@ typedef struct {
     int32_t *n_ttiles;     /* [1]                                     */
     int32_t *sched;        /* [8] work counters: [0] gate/up, [1..] down (one per launch group), zeroed by the sort */
     uint32_t *status;      /* [1]                                     */
-    int32_t *n_flag;       /* [2] rows flagged for the exact pass: the sort moves [0] to [1] and clears [0] for the next pass */
+    int32_t *n_flag;       /* [3] rows flagged for the exact pass: the sort moves [0] to [1] and clears [0] for the next pass;
+                              [2] counts blocks inside route_kernel, zero between launches */
     int32_t tile_n;        /* most rows of a token tile: OMNI_TILE_N or OMNI_TILE_N1, as the expert kernels of the pass take */
     int32_t longest_first; /* tile list in order of falling tile length (else in expert order) */
 } omni_sort_state;
@@ -114,6 +116,10 @@ cudaError_t omni_launch_recheck(int32_t *segcount, const void *xn, const void *r
                                 float *low, const int32_t *flag_rows, const int32_t *n_flag, int T, float eps,
                                 int32_t *ids, float *weights, uint32_t *status, const void *prefetch, size_t prefetch_bytes,
                                 cudaStream_t s);
+/* routing of at most OMNI_ROUTE_MAX_ROWS tokens behind omni_launch_router_part: selection, exact pass and sort */
+cudaError_t omni_launch_route(const void *xn, const void *router, const float *bias, float *logits, float *low, int T, float eps,
+                              int exact_all, int32_t *ids, float *weights, omni_sort_state st, const void *prefetch,
+                              size_t prefetch_bytes, cudaStream_t s);
 /* start of a pass: clears the status word, n_flag[0] and, where given, the OMNI_EP_BUCKETS bucket counters */
 cudaError_t omni_launch_begin(uint32_t *status, int32_t *n_flag, int32_t *buckets, cudaStream_t s);
 cudaError_t omni_launch_router_exact(const void *xn, const void *router, const float *bias, int T,
@@ -148,6 +154,12 @@ cudaError_t omni_launch_router_sm100(const CUtensorMap *tm_x, int nt, const CUte
                                      float eps, int exact_all, float *logits, int32_t *ids, float *weights,
                                      int32_t *flag_rows, int32_t *n_flag, uint32_t *status, unsigned long long *dbg,
                                      int32_t *segcount, cudaStream_t s);
+/* The logits alone, for short batches: 16 experts x omni_router_part_tile(T) tokens per CTA.  tm_x, tm_w: maps of the
+ * activations and the router matrix as {64, row, K / 64} with boxes of {64, tile, OMNI_PART_SLABS} and {64, 16, OMNI_PART_SLABS} */
+enum { OMNI_PART_EXPERTS = 16, OMNI_PART_SLABS = 4 };
+int omni_router_part_tile(int T);
+cudaError_t omni_launch_router_part(const CUtensorMap *tm_x, const CUtensorMap *tm_w, const float *bias, int T, float *logits,
+                                    uint32_t *status, cudaStream_t s);
 /* segcount (may be NULL): the kernel also writes the per-segment expert counts of the counting
  * sort for the ids it selected; omni_launch_recheck must then be given the same pointer so that
  * the rows it re-decides move their counts */

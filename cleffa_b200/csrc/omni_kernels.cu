@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(256) assign_hist_kernel(const int32_t *__restr
     }
 }
 
-// Scan over the experts, of the kernel that places assignments; called by all threads of a block
+// Scan over the experts, shared by the two kernels that place assignments; called by all threads of a block
 // (at least 128), thread e < 128 with the number of rows of expert e.  Returns the expert's offset to
 // thread e; with `publish` also writes counts, offsets and the token-tile list of the expert products
 // and resets the counters that the rest of the pass starts from.
@@ -332,6 +332,143 @@ __global__ void __launch_bounds__(ASSIGN_THREADS) assign_kernel(const int32_t *_
         __syncwarp();
         if (ei >= 0 && lane == __ffs(m) - 1) base[ei] += __popc(m);
         __syncwarp();
+    }
+}
+
+// ------------------------------------------------------------------ routing of short batches
+// Behind router_part_kernel: selection, exact pass and counting sort of up to ROUTE_MAX_ROWS tokens in one
+// launch.  A block per token: its first warp ranks the logits and forms the weights -- the arithmetic and
+// the near-tie rule of the router kernel's own selection, bit for bit -- and all eight warps re-decide
+// the row when it is too close.  The last block to finish sorts the assignments of the whole batch.  In separate
+// launches (selection in the router, exact pass, scan, scatter) each of these steps takes 1 to 3 us and
+// the way from one to the next as much again.
+constexpr int ROUTE_SEGS = OMNI_ROUTE_MAX_ROWS / 32;
+template <bool PREFETCH>
+__global__ void __launch_bounds__(EXACT_THREADS) route_kernel(const __nv_bfloat16 *__restrict__ xn, const __nv_bfloat16 *__restrict__ w,
+                                                              const float *__restrict__ bias, float *__restrict__ logits,
+                                                              float *__restrict__ low, int T, float eps, int exact_all,
+                                                              int32_t *__restrict__ ids, float *__restrict__ weights,
+                                                              omni_sort_state st, const char *prefetch, int prefetch_pieces) {
+    __shared__ ExactScratch scratch;
+    __shared__ int s_flag;
+    if (PREFETCH) prefetch_share(prefetch, prefetch_pieces);
+    dep_wait();
+    dep_launch();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long row = blockIdx.x;
+    if (row >= T) return;                                  // blocks that only ask for weights
+    if (warp == 0) {
+        float v[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[j] = logits[row * OMNI_E + lane + 32 * j];
+        bool bad = false;
+        float max_abs = 0.f;
+        uint32_t key[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            bad |= !(fabsf(v[j]) < CUDART_INF_F);
+            max_abs = fmaxf(max_abs, fabsf(v[j]));
+            key[j] = (ordered_key(v[j]) & ~127u) | (uint32_t)(127 - (lane + 32 * j));
+        }
+        bool close = false;
+        if (__any_sync(FULL, bad)) {
+            write_fallback(lane, ids, weights, row, st.status);
+        } else {
+            max_abs = __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(max_abs)));      // not negative: ordered like its bits
+            float tv[9];
+            int my_id = 0;
+#pragma unroll
+            for (int r = 0; r < 9; r++) {
+                const uint32_t top = __reduce_max_sync(FULL, max(max(key[0], key[1]), max(key[2], key[3])));
+                const int id = 127 - (int)(top & 127u), j = id >> 5;
+                tv[r] = __shfl_sync(FULL, j == 0 ? v[0] : j == 1 ? v[1] : j == 2 ? v[2] : v[3], id & 31);
+                if (lane == r) my_id = id;
+#pragma unroll
+                for (int jj = 0; jj < 4; jj++) if (key[jj] == top) key[jj] = 0;
+            }
+            const float thr = 2.f * omni_row_eps(eps, max_abs) + fmaxf(fabsf(tv[0]), fabsf(tv[8])) * 6.1035156e-5f;   // 2^-14
+            close = exact_all != 0;
+#pragma unroll
+            for (int k = 0; k < 8; k++) close |= (tv[k] - tv[k + 1]) < thr;
+            if (!close) {
+                float mine = tv[0];
+#pragma unroll
+                for (int k = 1; k < 8; k++) if (lane == k) mine = tv[k];
+                const float p = expf(mine - tv[0]);
+                float sum = 0.f;
+#pragma unroll
+                for (int k = 0; k < 8; k++) sum += __shfl_sync(FULL, p, k);
+                const float inv = 1.f / sum;
+                if (lane < 8) { ids[row * 8 + lane] = my_id; weights[row * 8 + lane] = p * inv; }
+            } else if (lane == 0) {
+                atomicAdd(st.n_flag, 1);
+            }
+        }
+        if (lane == 0) s_flag = close;
+    }
+    __syncthreads();
+    if (s_flag)
+        recheck_row(xn, w, bias, logits, low, row, eps, ids, weights, nullptr, st.status, scratch, lane, warp, [] { __syncthreads(); });
+    __syncthreads();                                       // s_flag has been read by all
+    if (warp == 0) {
+        __threadfence();                                   // this row's ids, in front of the count
+        __syncwarp();
+        if (lane == 0) s_flag = atomicAdd(st.n_flag + 2, 1) == T - 1;
+    }
+    __syncthreads();
+    if (!s_flag) return;
+
+    // ---- the last block: counting sort of all assignments.  A token's experts are distinct, so the tokens of
+    // a segment that chose an expert are a mask of 32 bits and a token's rank among them is a count of bits.
+    __shared__ unsigned mask[ROUTE_SEGS][OMNI_E];
+    __shared__ int base[ROUTE_SEGS][OMNI_E];
+    __shared__ ExpertScan scan;
+    __threadfence();
+    const int nseg = (T + 31) / 32;
+    for (int i = threadIdx.x; i < nseg * OMNI_E; i += EXACT_THREADS) mask[0][i] = 0;
+    if (threadIdx.x == 0) st.n_flag[2] = 0;
+    constexpr int PER = (ROUTE_SEGS + EXACT_WARPS - 1) / EXACT_WARPS;
+    int4 lo[PER], hi[PER];
+#pragma unroll
+    for (int i = 0; i < PER; i++) {
+        const int t = (warp + i * EXACT_WARPS) * 32 + lane;
+        if (t < T) { lo[i] = __ldcg(reinterpret_cast<const int4 *>(ids) + 2 * t); hi[i] = __ldcg(reinterpret_cast<const int4 *>(ids) + 2 * t + 1); }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < PER; i++) {
+        const int s = warp + i * EXACT_WARPS;
+        if (s * 32 + lane < T) {
+            unsigned *m = mask[s];
+            const unsigned bit = 1u << lane;
+            atomicOr(m + lo[i].x, bit); atomicOr(m + lo[i].y, bit); atomicOr(m + lo[i].z, bit); atomicOr(m + lo[i].w, bit);
+            atomicOr(m + hi[i].x, bit); atomicOr(m + hi[i].y, bit); atomicOr(m + hi[i].z, bit); atomicOr(m + hi[i].w, bit);
+        }
+    }
+    __syncthreads();
+    int total = 0;
+    if (threadIdx.x < OMNI_E)
+#pragma unroll 4
+        for (int s = 0; s < nseg; s++) { base[s][threadIdx.x] = total; total += __popc(mask[s][threadIdx.x]); }
+    const int off = scan_experts(scan, total, st, true);
+    __shared__ int offs[OMNI_E];
+    if (threadIdx.x < OMNI_E) offs[threadIdx.x] = off;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < PER; i++) {
+        const int s = warp + i * EXACT_WARPS, t = s * 32 + lane;
+        if (t < T) {
+            const unsigned lt = (1u << lane) - 1u;
+            auto place = [&](int e) {
+                const int r = offs[e] + base[s][e] + __popc(mask[s][e] & lt);
+                st.rowmap[r] = t;
+                return r;
+            };
+            const int4 a = make_int4(place(lo[i].x), place(lo[i].y), place(lo[i].z), place(lo[i].w));
+            const int4 b = make_int4(place(hi[i].x), place(hi[i].y), place(hi[i].z), place(hi[i].w));
+            reinterpret_cast<int4 *>(st.slots)[2 * t] = a;
+            reinterpret_cast<int4 *>(st.slots)[2 * t + 1] = b;
+        }
     }
 }
 
@@ -570,6 +707,17 @@ cudaError_t omni_launch_recheck(int32_t *segcount, const void *xn, const void *r
     if (pieces && blocks < 148) blocks = 148;
     return omni_launch_chain(pieces ? recheck_kernel<true> : recheck_kernel<false>, dim3(blocks), dim3(EXACT_THREADS), 0, s, (const __nv_bfloat16 *)xn,
                              (const __nv_bfloat16 *)router, bias, logits, low, flag_rows, n_flag, T, eps, ids, weights, segcount, status,
+                             (const char *)prefetch, pieces);
+}
+
+// sort state: n_flag[0] counts the flagged rows, n_flag[2] the blocks that are done
+cudaError_t omni_launch_route(const void *xn, const void *router, const float *bias, float *logits, float *low, int T, float eps,
+                              int exact_all, int32_t *ids, float *weights, omni_sort_state st, const void *prefetch,
+                              size_t prefetch_bytes, cudaStream_t s) {
+    if (T > OMNI_ROUTE_MAX_ROWS) return cudaErrorInvalidValue;
+    const int pieces = (int)(prefetch_bytes / OMNI_PREFETCH_PIECE);
+    return omni_launch_chain(pieces ? route_kernel<true> : route_kernel<false>, dim3(pieces && T < 148 ? 148 : T), dim3(EXACT_THREADS), 0, s,
+                             (const __nv_bfloat16 *)xn, (const __nv_bfloat16 *)router, bias, logits, low, T, eps, exact_all, ids, weights, st,
                              (const char *)prefetch, pieces);
 }
 

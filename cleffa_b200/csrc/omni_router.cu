@@ -306,11 +306,129 @@ router_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
     if (warp == 2) { tc_fence_after(); tmem_dealloc(tmem_base, NT); }
 }
 
+// ------------------------------------------------------------------ logits of short batches
+// A batch of up to a few hundred tokens gives the kernel above a handful of CTAs, each of which pulls the
+// whole router matrix through its SM (640 KB with 32 tokens: 10 us from the first load to the selection).  Here a
+// CTA takes 16 experts and NT tokens: 128 to 192 KB, all of it in flight at once in
+// shared memory, on eight times as many SMs; selection is the next kernel's (route_kernel).
+// The 16 expert rows are the first rows of an M = 128 operand whose other rows are whatever follows
+// in shared memory: they feed accumulator lanes that are never read, and the logits are the bits of the
+// kernel above (same K order).
+constexpr int PT_THREADS = 128, PT_CHUNKS = OMNI_H / BK / OMNI_PART_SLABS;   // warp 0 TMA and epilogue, 1 MMA, 2 TMEM
+template <int NT> struct PtCfg {
+    static constexpr int W_SLAB = OMNI_PART_EXPERTS * BK * 2, X_SLAB = NT * BK * 2;
+    static constexpr int W_BYTES = W_SLAB * (OMNI_H / BK), X_BYTES = X_SLAB * (OMNI_H / BK);
+    static constexpr int SMEM_BYTES = W_BYTES + X_BYTES + 1024 + 8 * (PT_CHUNKS + 1) + 16;
+    // the operand of the last slab reads 128 rows: still inside the token tiles
+    static_assert(X_BYTES >= A_TILE_BYTES - W_SLAB && SMEM_BYTES <= 232448, "shared memory budget");
+};
+
+template <int NT>
+__global__ void __launch_bounds__(PT_THREADS, 1)
+router_part_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w, const float *__restrict__ bias,
+                   int T, float *__restrict__ logits, uint32_t *__restrict__ status) {
+    using C = PtCfg<NT>;
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t *const smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
+    const uint32_t x_base = smem_base + C::W_BYTES, bar_base = x_base + C::X_BYTES;
+    auto full_bar = [&](int c) { return bar_base + 8u * c; };
+    const uint32_t tfull_bar = bar_base + 8u * PT_CHUNKS;
+    uint8_t *misc = smem_gen + C::W_BYTES + C::X_BYTES + 8 * (PT_CHUNKS + 1);
+    volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(misc);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(misc + 4);
+    const int warp = warp_index(), lane = threadIdx.x & 31;
+    const int row0 = blockIdx.x * NT, e0 = blockIdx.y * OMNI_PART_EXPERTS;
+
+    if (threadIdx.x == 0) {
+        for (int c = 0; c < PT_CHUNKS; c++) mbar_init(full_bar(c), 1);
+        mbar_init(tfull_bar, 1);
+        *abort_flag = 0;
+        fence_mbar_init();
+        prefetch_tmap(&tm_x);
+        prefetch_tmap(&tm_w);
+    }
+    if (warp == 2) { tmem_alloc(smem_u32((const void *)tmem_slot), 32); tmem_relinquish(); }
+    dep_wait();
+    dep_launch();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    if (warp == 0) {
+        if (elect_one()) {
+            for (int c = 0; c < PT_CHUNKS; c++) {
+                mbar_expect_tx(full_bar(c), OMNI_PART_SLABS * (C::W_SLAB + C::X_SLAB));
+                tma_load_3d(smem_base + c * OMNI_PART_SLABS * C::W_SLAB, &tm_w, 0, e0, c * OMNI_PART_SLABS, full_bar(c));
+                tma_load_3d(x_base + c * OMNI_PART_SLABS * C::X_SLAB, &tm_x, 0, row0, c * OMNI_PART_SLABS, full_bar(c));   // rows past T read as zero
+            }
+        }
+        __syncwarp();
+        const bool have = __all_sync(0xffffffffu, mbar_wait(tfull_bar, 0, abort_flag, status));
+        if (have) {
+            tc_fence_after();
+            const int e = e0 + lane;
+            const float b = bias && lane < OMNI_PART_EXPERTS ? __ldg(bias + e) : 0.f;
+            uint32_t r[32];
+            tmem_ld32(tmem_base, r);                              // lanes 0..15: this CTA's experts; columns from NT on are not used
+            tmem_ld_wait();
+            if (lane < OMNI_PART_EXPERTS) {
+#pragma unroll
+                for (int j = 0; j < NT; j++)
+                    if (row0 + j < T) logits[(long)(row0 + j) * OMNI_E + e] = bias ? __uint_as_float(r[j]) + b : __uint_as_float(r[j]);
+            }
+        }
+    } else if (warp == 1 && elect_one()) {
+        const uint32_t idesc = idesc_bf16(128, NT);
+        bool ok = true;
+        for (int c = 0; c < PT_CHUNKS && ok; c++) {
+            ok = mbar_wait(full_bar(c), 0, abort_flag, status);
+            if (!ok) break;
+            tc_fence_after();
+#pragma unroll
+            for (int s = 0; s < OMNI_PART_SLABS; s++) {
+                const int ks = c * OMNI_PART_SLABS + s;
+                const uint64_t da = smem_desc_sw128(smem_base + ks * C::W_SLAB), db = smem_desc_sw128(x_base + ks * C::X_SLAB);
+#pragma unroll
+                for (int k = 0; k < BK / 16; k++) umma_bf16(tmem_base, da + 2u * k, db + 2u * k, idesc, (ks | k) ? 1u : 0u);
+            }
+        }
+        umma_commit(tfull_bar);
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    if (*abort_flag && threadIdx.x == 0) {
+        // a wait ran out: give the loads and the MMAs that may still be reading them a bounded chance to finish
+        for (int c = 0; c <= PT_CHUNKS; c++) {
+            const uint64_t t0 = globaltimer_ns();
+            while (!mbar_try_wait(full_bar(c), 0) && globaltimer_ns() - t0 < 50000000ull) {}
+        }
+    }
+    __syncthreads();
+    if (warp == 2) { tc_fence_after(); tmem_dealloc(tmem_base, 32); }
+}
+
 }  // namespace
 
 extern "C" {
 
+// Tokens per CTA: 16 while that gives at most one CTA per SM for each group of experts
+int omni_router_part_tile(int T) { return T <= 16 * (148 / (OMNI_E / OMNI_PART_EXPERTS)) ? 16 : 32; }
+
+cudaError_t omni_launch_router_part(const CUtensorMap *tm_x, const CUtensorMap *tm_w, const float *bias, int T, float *logits,
+                                    uint32_t *status, cudaStream_t s) {
+    const int nt = omni_router_part_tile(T);
+    const dim3 grid((T + nt - 1) / nt, OMNI_E / OMNI_PART_EXPERTS);
+    return nt == 16 ? omni_launch_chain(router_part_kernel<16>, grid, dim3(PT_THREADS), PtCfg<16>::SMEM_BYTES, s, *tm_x, *tm_w, bias, T, logits, status)
+                    : omni_launch_chain(router_part_kernel<32>, grid, dim3(PT_THREADS), PtCfg<32>::SMEM_BYTES, s, *tm_x, *tm_w, bias, T, logits, status);
+}
+
 cudaError_t omni_router_configure(void) {
+    cudaError_t p = cudaFuncSetAttribute(router_part_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, PtCfg<16>::SMEM_BYTES);
+    if (p == cudaSuccess) p = cudaFuncSetAttribute(router_part_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, PtCfg<32>::SMEM_BYTES);
+    if (p != cudaSuccess) return p;
     cudaError_t e = cudaFuncSetAttribute(router_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, RtCfg<32>::SMEM_BYTES);
     if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(router_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, RtCfg<128>::SMEM_BYTES);

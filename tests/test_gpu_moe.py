@@ -103,6 +103,38 @@ def test_launch_variants_give_the_same_bits(bound0, T):
             b.set_option(name, 1)
 
 
+@pytest.mark.parametrize("T", [1, 15, 16, 17, 31, 33, 128, 287, 288, 289, 575, 576, 577])
+def test_short_routing_gives_the_bits_of_the_general_one(bound0, weights0, T):
+    """Up to 576 tokens the logits come from CTAs of 16 experts by 16 (up to 288 tokens) or 32 tokens, and one more launch selects,
+    re-decides and sorts; with fused_router = 0 the kernels of longer batches do.  Rows as they come, every row through the exact
+    pass, and rows whose 128 logits are equal (all experts are candidates) or nonfinite."""
+    b = bound0
+    x = orc.make_activations(37, T)
+    x[T // 2] = 0                                 # all logits 0: 128 candidates
+    keys = ("ids", "weights", "logits", "slots", "counts", "offsets", "rowmap", "rechecked", "out")
+    try:
+        for exact in (0, 1):
+            b.set_option("router_exact", exact)
+            b.set_option("fused_router", 0)
+            want = run_block(b, 0, x)
+            assert want["ids"][T // 2].tolist() == list(range(8))
+            b.set_option("fused_router", 1)
+            for _ in range(2):                    # the second pass meets the counters the first one left
+                got = run_block(b, 0, x)
+                for key in keys:
+                    assert np.array_equal(want[key], got[key]), (key, exact)
+        x[T - 1, 5] = float("inf")
+        for fused in (0, 1):
+            b.set_option("fused_router", fused)
+            with pytest.raises(OmniError, match="nonfinite"):
+                run_block(b, 0, x)
+            ids = b.read("ids", T)
+            assert ids[T - 1].tolist() == list(range(8)) and not b.read("weights", T)[T - 1].any()
+    finally:
+        b.set_option("router_exact", 0)
+        b.set_option("fused_router", 1)
+
+
 @pytest.mark.parametrize("T", [1, 2, 3, 37, 300, 2500, 4096])
 def test_expert_kernel_variants_give_the_same_bits(bound0, T):
     """The expert products exist as two schedules of the same arithmetic: single CTAs with tiles of up to

@@ -411,19 +411,23 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     if (warp == 2 && leader && elect_one()) {
         // ---------------------------------------------------------- scheduler
         // Claims items and hands them, decoded, to the consumers of both CTAs.  Its own warp: an item
-        // costs an atomic, two dependent global loads and a cluster-scope release (about 2 us), which
+        // costs an atomic, up to two dependent global loads and a cluster-scope release (about 2 us), which
         // inside the weight producer's loop held up the loads of every item (12 slabs of 512 clocks in
-        // the down product).  The claim of the item after the next is in flight meanwhile.
+        // the down product).  The claim of the item after the next is in flight meanwhile.  The first item needs
+        // no claim (the counter hands out those behind one per pair), and its tile is loaded beside the length of the list.
         constexpr bool DENSE = MODE == X_QKV || MODE == X_OPROJ;
         PipeState wr;
         auto tile_at = [&](int i) {
             const int4 v = __ldcg(reinterpret_cast<const int4 *>(a.ttiles) + i);
             return omni_ttile{v.x, v.y, v.z, v.w};
         };
-        const int n_work = (DENSE ? a.dense_tiles : __ldcg(a.n_ttiles)) * MI, n_pairs = (int)gridDim.x / CTAS;
-        int w0 = DENSE ? (int)blockIdx.x / CTAS : atomicAdd(a.work_counter, 1);
-        for (;;) {
-            const int w1 = DENSE ? w0 + n_pairs : atomicAdd(a.work_counter, 1);
+        const int n_pairs = (int)gridDim.x / CTAS;
+        int w0 = (int)blockIdx.x / CTAS;
+        omni_ttile head = omni_ttile{0, 0, 0, 0};
+        if (!DENSE) head = tile_at(w0 / MI);                  // below OMNI_MAX_TTILES for any grid; only used if the list is that long
+        const int n_work = (DENSE ? a.dense_tiles : __ldcg(a.n_ttiles)) * MI;
+        for (bool first_item = true;; first_item = false) {
+            const int w1 = DENSE ? w0 + n_pairs : n_pairs + atomicAdd(a.work_counter, 1);
             int m = 0;
             omni_ttile cur = omni_ttile{0, 0, -1, 0};
             if (DENSE && w0 < n_work) {
@@ -435,10 +439,11 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 const int t = first + local % cnt, base = a.dense_rows / a.dense_tiles, extra = a.dense_rows % a.dense_tiles;
                 cur = omni_ttile{0, t * base + min(t, extra), base + (t < extra), 0};
             } else if (w0 < n_work) {                         // item -> (weight block m, tile of the expert)
-                const omni_ttile head = tile_at(w0 / MI);
+                if (!first_item) head = tile_at(w0 / MI);
                 const int first = head.group & 0xffff, cnt = head.group >> 16, local = w0 - first * MI;
                 m = local / cnt;
-                cur = tile_at(first + local % cnt);
+                const int at = first + local % cnt;
+                cur = at == w0 / MI ? head : tile_at(at);
             }
             if (!xwait_lazy(iempty_bar(wr.stage), wr.phase ^ 1u, ab)) break;
             ring[wr.stage].expert = cur.expert; ring[wr.stage].row0 = cur.row0;

@@ -21,7 +21,7 @@ enum {
     OMNI_TILE_N = 256,                     /* most token rows per expert-GEMM tile on pairs of CTAs */
     OMNI_TILE_N1 = 128,                    /* and on single CTAs */
     OMNI_TOK_BOXES = 16,                   /* tensor maps of a token operand: box i is 16 (i + 1) rows high */
-    OMNI_ROUTE_MAX_ROWS = 576,             /* most tokens that the short batches' routing (omni_launch_route) takes */
+    OMNI_ROUTE_MAX_ROWS = 384,             /* most tokens that the short batches' routing (omni_launch_route) takes */
     OMNI_MAX_TTILES = OMNI_ROWS / OMNI_TILE_N1 + OMNI_E,
 };
 

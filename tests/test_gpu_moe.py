@@ -103,9 +103,9 @@ def test_launch_variants_give_the_same_bits(bound0, T):
             b.set_option(name, 1)
 
 
-@pytest.mark.parametrize("T", [1, 15, 16, 17, 31, 33, 128, 287, 288, 289, 575, 576, 577])
+@pytest.mark.parametrize("T", [1, 15, 16, 17, 31, 33, 128, 287, 288, 289, 383, 384, 385])
 def test_short_routing_gives_the_bits_of_the_general_one(bound0, weights0, T):
-    """Up to 576 tokens the logits come from CTAs of 16 experts by 16 (up to 288 tokens) or 32 tokens, and one more launch selects,
+    """Up to 384 tokens the logits come from CTAs of 16 experts by 16 (up to 288 tokens) or 32 tokens, and one more launch selects,
     re-decides and sorts; with fused_router = 0 the kernels of longer batches do.  Rows as they come, every row through the exact
     pass, and rows whose 128 logits are equal (all experts are candidates) or nonfinite."""
     b = bound0

@@ -63,7 +63,7 @@ struct clef_gpu {
         void *qkv, *out;                   /* device BF16 [5120][2048], [2048][4096] */
         float eps; double theta;
         bool bound;
-        CUtensorMap tm_qkv, tm_out;
+        CUtensorMap tm_qkv, tm_out, tm_qkv_thin, tm_out_thin;
     } attn[MAX_LAYERS];
     struct {
         void *p, *q, *k, *vt, *a;          /* BF16: q|k|v rows [CHUNK][5120]; Q [32][CHUNK][128]; K [4][CHUNK][128]; Vt [4][128][VPITCH]; attention output [CHUNK][4096] */
@@ -71,6 +71,7 @@ struct clef_gpu {
         int32_t *h_tiles, *h_vcol, *h_bounds;   /* host copies; h_bounds remembers the batch the device copies describe */
         int n_tiles, last_T, last_nseq;
         CUtensorMap tm_xn[OMNI_TOK_BOXES], tm_a[OMNI_TOK_BOXES], tm_q, tm_k, tm_vt;
+        CUtensorMap tm_xn_thin[OMNI_THIN_BOXES], tm_a_thin[OMNI_THIN_BOXES];
         bool ready;
     } at;
     /* route capture */
@@ -229,6 +230,7 @@ bool clef_cuda_omni_open(clef_gpu **out, int device, void *stream, char *err, si
     }
     e = omni_expert_configure();
     if (e == cudaSuccess) e = omni_router_configure();
+    if (e == cudaSuccess) e = omni_dense_configure();
     if (e == cudaSuccess) e = omni_attn_configure();
     if (e != cudaSuccess) {
         set_err(err, errlen, "cuda: cannot configure sm_100a kernels: %s", cudaGetErrorString(e));
@@ -1315,6 +1317,9 @@ static bool attn_reserve(clef_gpu *g, char *err, size_t errlen) {
     for (uint32_t i = 0; i < OMNI_TOK_BOXES && ok; i++)
         ok = make_map(g, &g->at.tm_xn[i], xnorm, OMNI_CHUNK, OMNI_H, 16 * (i + 1), CU_TENSOR_MAP_L2_PROMOTION_L2_128B) &&
              make_map(g, &g->at.tm_a[i], g->at.a, OMNI_CHUNK, OMNI_NH * OMNI_HD, 16 * (i + 1), CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
+    for (uint32_t i = 0; i < OMNI_THIN_BOXES && ok; i++)
+        ok = make_slab_map(g, &g->at.tm_xn_thin[i], xnorm, OMNI_CHUNK, OMNI_H, 16 * (i + 1), OMNI_THIN_SLABS) &&
+             make_slab_map(g, &g->at.tm_a_thin[i], g->at.a, OMNI_CHUNK, OMNI_NH * OMNI_HD, 16 * (i + 1), OMNI_THIN_SLABS);
     if (ok) ok = make_map(g, &g->at.tm_q, g->at.q, (uint64_t)OMNI_NH * OMNI_CHUNK, OMNI_HD, 128, CU_TENSOR_MAP_L2_PROMOTION_L2_128B) &&
                  make_map(g, &g->at.tm_k, g->at.k, (uint64_t)OMNI_NKV * OMNI_CHUNK, OMNI_HD, 128, CU_TENSOR_MAP_L2_PROMOTION_L2_128B) &&
                  make_map(g, &g->at.tm_vt, g->at.vt, (uint64_t)OMNI_NKV * OMNI_HD, ATTN_VPITCH, 128, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
@@ -1355,9 +1360,11 @@ bool clef_omni_bind_attention(clef_gpu *g, int layer, const float *attn_norm, co
                  cudaMemcpyAsync(qkv, attn_qkv, nq, kind, g->stream) == cudaSuccess &&
                  cudaMemcpyAsync(out, attn_output, no, kind, g->stream) == cudaSuccess &&
                  cudaStreamSynchronize(g->stream) == cudaSuccess;
-    CUtensorMap tm_qkv, tm_out;
+    CUtensorMap tm_qkv, tm_out, tm_qkv_thin, tm_out_thin;
     if (ok) ok = make_map(g, &tm_qkv, qkv, OMNI_QKV, OMNI_H, 128, CU_TENSOR_MAP_L2_PROMOTION_L2_256B) &&
-                 make_map(g, &tm_out, out, OMNI_H, OMNI_NH * OMNI_HD, 128, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+                 make_map(g, &tm_out, out, OMNI_H, OMNI_NH * OMNI_HD, 128, CU_TENSOR_MAP_L2_PROMOTION_L2_256B) &&
+                 make_slab_map(g, &tm_qkv_thin, qkv, OMNI_QKV, OMNI_H, OMNI_THIN_QKV_ROWS, OMNI_THIN_SLABS) &&
+                 make_slab_map(g, &tm_out_thin, out, OMNI_H, OMNI_NH * OMNI_HD, OMNI_THIN_OPROJ_ROWS, OMNI_THIN_SLABS);
     if (!ok) {
         cudaGetLastError();
         void *w[] = {nw, qn, kn, qkv, out};
@@ -1370,6 +1377,7 @@ bool clef_omni_bind_attention(clef_gpu *g, int layer, const float *attn_norm, co
     g->attn[layer].norm_w = nw; g->attn[layer].q_norm = qn; g->attn[layer].k_norm = kn; g->attn[layer].qkv = qkv; g->attn[layer].out = out;
     g->attn[layer].eps = eps; g->attn[layer].theta = (double)rope_theta;
     g->attn[layer].tm_qkv = tm_qkv; g->attn[layer].tm_out = tm_out;
+    g->attn[layer].tm_qkv_thin = tm_qkv_thin; g->attn[layer].tm_out_thin = tm_out_thin;
     g->attn[layer].bound = true;
     return true;
 }
@@ -1442,16 +1450,19 @@ bool clef_omni_encode_attention(clef_gpu *g, int layer, float *x, const int32_t 
     if (g->failed) { set_err(err, errlen, "%s", g->fail_msg); return false; }
     if (!attn_plan(g, T, n_seq, seq_bounds, err, errlen)) return false;
     omni_arena *s = g->omni;
+    const bool thin = T <= OMNI_THIN_MAX_ROWS;        /* token rows that every CTA can afford to read whole (omni_dense.cu) */
     bool ok = launched(g, "attention norm", omni_launch_rmsnorm(x, g->attn[layer].norm_w, g->attn[layer].eps, T, g->xnorm, g->stream)) &&
-              launched(g, "q|k|v projection", omni_launch_dense_pair(0, &g->attn[layer].tm_qkv, g->at.tm_xn, T, g->at.p, NULL, s->status,
-                                                                       g->n_sm, g->stream)) &&
+              launched(g, "q|k|v projection", thin ? omni_launch_dense_thin(0, &g->attn[layer].tm_qkv_thin, g->at.tm_xn_thin, T, g->at.p, NULL, s->status, g->stream)
+                                                   : omni_launch_dense_pair(0, &g->attn[layer].tm_qkv, g->at.tm_xn, T, g->at.p, NULL, s->status,
+                                                                            g->n_sm, g->stream)) &&
               launched(g, "attention prep", omni_launch_attn_prep(g->at.p, g->attn[layer].q_norm, g->attn[layer].k_norm, pos3, g->at.vcol, T, OMNI_CHUNK,
                                                                    ATTN_VPITCH, g->attn[layer].eps, g->attn[layer].theta, g->at.q, g->at.k, g->at.vt,
                                                                    s->status, g->stream)) &&
               launched(g, "attention", omni_launch_attention(&g->at.tm_q, &g->at.tm_k, &g->at.tm_vt, g->at.tiles, g->at.n_tiles, OMNI_CHUNK, g->at.a,
                                                              s->status, g->stream)) &&
-              launched(g, "output projection", omni_launch_dense_pair(1, &g->attn[layer].tm_out, g->at.tm_a, T, NULL, x, s->status,
-                                                                        g->n_sm, g->stream));
+              launched(g, "output projection", thin ? omni_launch_dense_thin(1, &g->attn[layer].tm_out_thin, g->at.tm_a_thin, T, NULL, x, s->status, g->stream)
+                                                    : omni_launch_dense_pair(1, &g->attn[layer].tm_out, g->at.tm_a, T, NULL, x, s->status,
+                                                                             g->n_sm, g->stream));
     if (!ok) { set_err(err, errlen, "%s", g->fail_msg); return false; }
     return true;
 }

@@ -108,6 +108,17 @@ def test_records_do_not_depend_on_their_neighbours(attn):
     assert torch.equal(run(b, x, pos, bounds), packed)                 # and the pass is repeatable
 
 
+@pytest.mark.parametrize("T", [1, 15, 16, 17, 31, 33, 64, 97, 127, 128, 129])
+def test_short_batches_give_the_bits_of_long_ones(attn, T):
+    """Up to 128 tokens the projections run with all token rows in every CTA (omni_dense.cu), above that on pairs of CTAs: a
+    record alone and in front of one of 200 rows."""
+    b, w = attn
+    x = torch.randn(T + 200, 2048, generator=torch.Generator().manual_seed(T))
+    pos = ao.make_positions(T, [0, T, T + 200])
+    alone, packed = run(b, x[:T].contiguous(), pos[:, :T], [0, T]), run(b, x, pos, [0, T, T + 200])
+    assert torch.equal(alone, packed[:T])
+
+
 def test_nonfinite_projection_is_reported(attn):
     b, _ = attn
     x = torch.randn(64, 2048, generator=torch.Generator().manual_seed(6))

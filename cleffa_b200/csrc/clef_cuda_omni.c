@@ -61,7 +61,8 @@ struct clef_gpu {
     struct {
         float *norm_w, *q_norm, *k_norm;   /* device FP32 [2048], [128], [128] */
         void *qkv, *out;                   /* device BF16 [5120][2048], [2048][4096] */
-        float eps; double theta;
+        float eps;
+        double *freq;                      /* device [64]: rotary frequencies */
         bool bound;
         CUtensorMap tm_qkv, tm_out, tm_qkv_thin, tm_out_thin;
     } attn[MAX_LAYERS];
@@ -1284,7 +1285,7 @@ static void attn_free(clef_gpu *g) {
     free(g->at.h_tiles); free(g->at.h_vcol); free(g->at.h_bounds);
     memset(&g->at, 0, sizeof g->at);
     for (int l = 0; l < MAX_LAYERS; l++) {
-        void *w[] = {g->attn[l].norm_w, g->attn[l].q_norm, g->attn[l].k_norm, g->attn[l].qkv, g->attn[l].out};
+        void *w[] = {g->attn[l].norm_w, g->attn[l].q_norm, g->attn[l].k_norm, g->attn[l].qkv, g->attn[l].out, g->attn[l].freq};
         for (size_t i = 0; i < sizeof w / sizeof w[0]; i++) if (w[i]) cudaFree(w[i]);
         memset(&g->attn[l], 0, sizeof g->attn[l]);
     }
@@ -1353,12 +1354,14 @@ bool clef_omni_bind_attention(clef_gpu *g, int layer, const float *attn_norm, co
     const enum cudaMemcpyKind kind = where == CLEF_OMNI_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
     float *nw = dev_alloc(g, OMNI_H * 4), *qn = dev_alloc(g, OMNI_HD * 4), *kn = dev_alloc(g, OMNI_HD * 4);
     void *qkv = dev_alloc(g, nq), *out = dev_alloc(g, no);
-    bool ok = nw && qn && kn && qkv && out;
+    double *freq = dev_alloc(g, OMNI_HD / 2 * 8);
+    bool ok = nw && qn && kn && qkv && out && freq;
     if (ok) ok = cudaMemcpyAsync(nw, attn_norm, OMNI_H * 4, kind, g->stream) == cudaSuccess &&
                  cudaMemcpyAsync(qn, q_norm, OMNI_HD * 4, kind, g->stream) == cudaSuccess &&
                  cudaMemcpyAsync(kn, k_norm, OMNI_HD * 4, kind, g->stream) == cudaSuccess &&
                  cudaMemcpyAsync(qkv, attn_qkv, nq, kind, g->stream) == cudaSuccess &&
                  cudaMemcpyAsync(out, attn_output, no, kind, g->stream) == cudaSuccess &&
+                 omni_launch_rope_freq((double)rope_theta, freq, g->stream) == cudaSuccess &&
                  cudaStreamSynchronize(g->stream) == cudaSuccess;
     CUtensorMap tm_qkv, tm_out, tm_qkv_thin, tm_out_thin;
     if (ok) ok = make_map(g, &tm_qkv, qkv, OMNI_QKV, OMNI_H, 128, CU_TENSOR_MAP_L2_PROMOTION_L2_256B) &&
@@ -1367,15 +1370,15 @@ bool clef_omni_bind_attention(clef_gpu *g, int layer, const float *attn_norm, co
                  make_slab_map(g, &tm_out_thin, out, OMNI_H, OMNI_NH * OMNI_HD, OMNI_THIN_OPROJ_ROWS, OMNI_THIN_SLABS);
     if (!ok) {
         cudaGetLastError();
-        void *w[] = {nw, qn, kn, qkv, out};
+        void *w[] = {nw, qn, kn, qkv, out, freq};
         for (size_t i = 0; i < sizeof w / sizeof w[0]; i++) if (w[i]) cudaFree(w[i]);
         set_err(err, errlen, "cuda: cannot upload Omni attention tensors of layer %d (previous binding kept)", layer);
         return false;
     }
-    void *old[] = {g->attn[layer].norm_w, g->attn[layer].q_norm, g->attn[layer].k_norm, g->attn[layer].qkv, g->attn[layer].out};
+    void *old[] = {g->attn[layer].norm_w, g->attn[layer].q_norm, g->attn[layer].k_norm, g->attn[layer].qkv, g->attn[layer].out, g->attn[layer].freq};
     for (size_t i = 0; i < sizeof old / sizeof old[0]; i++) if (old[i]) cudaFree(old[i]);
     g->attn[layer].norm_w = nw; g->attn[layer].q_norm = qn; g->attn[layer].k_norm = kn; g->attn[layer].qkv = qkv; g->attn[layer].out = out;
-    g->attn[layer].eps = eps; g->attn[layer].theta = (double)rope_theta;
+    g->attn[layer].eps = eps; g->attn[layer].freq = freq;
     g->attn[layer].tm_qkv = tm_qkv; g->attn[layer].tm_out = tm_out;
     g->attn[layer].tm_qkv_thin = tm_qkv_thin; g->attn[layer].tm_out_thin = tm_out_thin;
     g->attn[layer].bound = true;
@@ -1455,8 +1458,8 @@ bool clef_omni_encode_attention(clef_gpu *g, int layer, float *x, const int32_t 
               launched(g, "q|k|v projection", thin ? omni_launch_dense_thin(0, &g->attn[layer].tm_qkv_thin, g->at.tm_xn_thin, T, g->at.p, NULL, s->status, g->stream)
                                                    : omni_launch_dense_pair(0, &g->attn[layer].tm_qkv, g->at.tm_xn, T, g->at.p, NULL, s->status,
                                                                             g->n_sm, g->stream)) &&
-              launched(g, "attention prep", omni_launch_attn_prep(g->at.p, g->attn[layer].q_norm, g->attn[layer].k_norm, pos3, g->at.vcol, T, OMNI_CHUNK,
-                                                                   ATTN_VPITCH, g->attn[layer].eps, g->attn[layer].theta, g->at.q, g->at.k, g->at.vt,
+              launched(g, "attention prep", omni_launch_attn_prep(g->at.p, g->attn[layer].q_norm, g->attn[layer].k_norm, pos3, g->attn[layer].freq, g->at.vcol,
+                                                                   T, OMNI_CHUNK, ATTN_VPITCH, g->attn[layer].eps, g->at.q, g->at.k, g->at.vt,
                                                                    s->status, g->stream)) &&
               launched(g, "attention", omni_launch_attention(&g->at.tm_q, &g->at.tm_k, &g->at.tm_vt, g->at.tiles, g->at.n_tiles, OMNI_CHUNK, g->at.a,
                                                              s->status, g->stream)) &&

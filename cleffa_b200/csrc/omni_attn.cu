@@ -1,6 +1,6 @@
 // Attention half of a Clef-Omni decoder layer on sm_100a: the step in front of the MoE block.
-//   attn_prep_kernel    per-head RMS norm of q and k, interleaved three-axis rotary, q/k/v laid out
-//                       per head (reference: metal/clef.metal:2073-2130, omni_attn_prep)
+//   attn_prep_kernel    per-head RMS norm of q and k, interleaved three-axis rotary, values transposed, q/k/v
+//                       laid out per head (reference: metal/clef.metal:2073-2130, omni_attn_prep)
 //   attention_kernel    causal grouped-query attention inside each record of the packed batch,
 //                       online softmax (reference: metal/clef.metal:2174-2319, omni_attention)
 //
@@ -29,50 +29,92 @@ namespace {
 constexpr int HD = OMNI_HD, NH = OMNI_NH, NKV = OMNI_NKV;
 
 // ------------------------------------------------------------------ q/k norm + rotary + layout
-// One block per token, four warps, nine heads each (32 query heads, then the 4 key heads).  A lane
+// Two jobs of one launch that read different columns of the projections: blocks below `prep_blocks` norm and
+// rotate q and k, the others transpose v.  As two launches the second waited for the first (3 us at 37
+// tokens, 12 at 16384).
+//
+// Norm and rotary: four warps per token, nine heads each (32 query heads, then the 4 key heads, dealt in turn).  A lane
 // holds four consecutive elements of the 128 of a head (one 8-byte load and store); pair p of a
 // head is (element p, element p + 64), so a lane's partners sit in lane ^ 16.  The pair's angle is
 // position[axis] * theta^(-p/64) with axis = p % 3 for p < 60 and the temporal axis above (sections
 // 24/20/20 interleaved; clef.metal:2051-2053).  The angle is formed and reduced modulo 2 pi in
-// FP64 -- FP32 loses ~pos * 6e-8 rad (clef.metal:2055-2060) -- and its cosine and sine, the same
-// for every head of the token, are computed once per warp.
-__global__ void __launch_bounds__(128) attn_prep_kernel(const __nv_bfloat16 *__restrict__ qkv, const float *__restrict__ qw,
-                                                        const float *__restrict__ kw, const int32_t *__restrict__ pos,
-                                                        int head_stride, float eps, double theta,
-                                                        __nv_bfloat16 *__restrict__ Q, __nv_bfloat16 *__restrict__ K,
-                                                        uint32_t *__restrict__ status) {
+// FP64 -- FP32 loses ~pos * 6e-8 rad (clef.metal:2055-2060) -- from frequencies that binding the layer left in
+// `freq` (rope_freq_kernel) instead of an exp2 and a log2 per token and pair.  Cosine and sine are the same for every
+// head of the token and computed once per warp (one warp for all heads of a token, which forms them once, was 8 % slower for the
+// attention half of 2048 tokens and no faster at 16384: fewer loads in flight).
+constexpr int PREP_THREADS = 256, PREP_WARPS = 4, PREP_HEADS = (NH + NKV) / PREP_WARPS;
+static_assert((NH + NKV) % PREP_WARPS == 0, "heads are dealt to the warps of a token");
+
+__global__ void __launch_bounds__(PREP_THREADS) attn_prep_kernel(const __nv_bfloat16 *__restrict__ qkv, const float *__restrict__ qw,
+                                                                 const float *__restrict__ kw, const int32_t *__restrict__ pos,
+                                                                 const double *__restrict__ freq, const int32_t *__restrict__ vcol, int T,
+                                                                 int prep_blocks, int head_stride, int vpitch, float eps,
+                                                                 __nv_bfloat16 *__restrict__ Q, __nv_bfloat16 *__restrict__ K,
+                                                                 __nv_bfloat16 *__restrict__ Vt, uint32_t *__restrict__ status) {
+    __shared__ unsigned short tile[64][HD + 2];
+    __shared__ int col[64];
     dep_wait();
     dep_launch();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const long t = blockIdx.x;
+    bool bad = false;
+    if ((int)blockIdx.x >= prep_blocks) {
+        // Values, transposed: Vt[kh][d][column of the token].  One block per (64 tokens, key/value head):
+        // rows read whole (256 bytes per token), written as 64-token runs per head dimension.
+        const int vb = blockIdx.x - prep_blocks, t0 = vb / NKV * 64, kh = vb % NKV;
+        if (threadIdx.x < 64) col[threadIdx.x] = t0 + threadIdx.x < T ? __ldg(vcol + t0 + threadIdx.x) : -1;
+#pragma unroll
+        for (int i = warp; i < 64; i += PREP_THREADS / 32) {
+            const long t = t0 + i;
+            if (t < T) {
+                const uint2 v = *reinterpret_cast<const uint2 *>(qkv + t * OMNI_QKV + (long)(NH + NKV + kh) * HD + lane * 4);
+                const unsigned short e[4] = {(unsigned short)(v.x & 0xffff), (unsigned short)(v.x >> 16), (unsigned short)(v.y & 0xffff), (unsigned short)(v.y >> 16)};
+#pragma unroll
+                for (int k = 0; k < 4; k++) { bad |= (e[k] & 0x7f80) == 0x7f80; tile[i][lane * 4 + k] = e[k]; }
+            }
+        }
+        __syncthreads();
+        unsigned short *out = reinterpret_cast<unsigned short *>(Vt) + (long)kh * HD * vpitch;
+        for (int d = warp; d < HD; d += PREP_THREADS / 32)
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                const int i = lane + 32 * k;
+                if (col[i] >= 0) out[(long)d * vpitch + col[i]] = tile[i][d];
+            }
+        if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(status, OMNI_ST_ATTN_NONFINITE);
+        return;
+    }
+    const long t = (long)blockIdx.x * (PREP_THREADS / 32 / PREP_WARPS) + warp / PREP_WARPS;
+    if (t >= T) return;
+    const int sub = warp % PREP_WARPS;
     const bool upper = lane >= 16;                                               // elements 64..127: the second of each pair
+    const __nv_bfloat16 *row = qkv + t * OMNI_QKV + 4 * lane;
+    uint2 raw[PREP_HEADS];                                // the loads of all nine heads are in flight together
+#pragma unroll
+    for (int i = 0; i < PREP_HEADS; i++) raw[i] = *reinterpret_cast<const uint2 *>(row + (long)(sub + PREP_WARPS * i) * HD);
     // the four pairs of a lane are those of lane ^ 16 too: each computes two and they swap
     float cs[4], sn[4];
 #pragma unroll
     for (int j = 0; j < 2; j++) {
         const int own = (upper ? 2 : 0) + j, pair = 4 * (lane & 15) + own, axis = pair < 60 ? pair % 3 : 0;
-        const double angle = (double)__ldg(pos + 3 * t + axis) * exp2(-(double)pair * (1.0 / 64.0) * log2(theta));
+        const double angle = (double)__ldg(pos + 3 * t + axis) * __ldg(freq + pair);
         const double turns = rint(angle * 0.15915494309189535);
         const float r = (float)fma(-turns, 6.283185307179586, angle);           // |r| <= pi, accurate to FP32 rounding
         float sj, cj;
         sincosf(r, &sj, &cj);
         const float so = __shfl_xor_sync(0xffffffffu, sj, 16), co = __shfl_xor_sync(0xffffffffu, cj, 16);
-        cs[own] = cj; sn[own] = sj;
-        cs[own ^ 2] = co; sn[own ^ 2] = so;
+        cs[j] = upper ? co : cj; cs[j + 2] = upper ? cj : co;
+        sn[j] = upper ? so : sj; sn[j + 2] = upper ? sj : so;
     }
 #pragma unroll
     for (int j = 0; j < 4; j++)
         if (!upper) sn[j] = -sn[j];                                              // lo' = lo cos - hi sin, hi' = hi cos + lo sin
     const float4 wq = __ldg(reinterpret_cast<const float4 *>(qw) + lane), wk = __ldg(reinterpret_cast<const float4 *>(kw) + lane);
-    bool bad = false;
-    static_assert((NH + NKV) % 4 == 0, "heads are dealt to four warps");
 #pragma unroll
-    for (int i = 0; i < (NH + NKV) / 4; i++) {            // unrolled: the loads of all nine heads are in flight together
-        const int h = warp + 4 * i;
+    for (int i = 0; i < PREP_HEADS; i++) {
+        const int h = sub + PREP_WARPS * i;
         const bool query = h < NH;
-        const uint2 raw = *reinterpret_cast<const uint2 *>(qkv + t * OMNI_QKV + (long)h * HD + 4 * lane);
-        float x[4] = {__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u), __uint_as_float(raw.y << 16),
-                      __uint_as_float(raw.y & 0xffff0000u)};
+        float x[4] = {__uint_as_float(raw[i].x << 16), __uint_as_float(raw[i].x & 0xffff0000u), __uint_as_float(raw[i].y << 16),
+                      __uint_as_float(raw[i].y & 0xffff0000u)};
         float sum = 0.f;
 #pragma unroll
         for (int j = 0; j < 4; j++) { bad |= !(fabsf(x[j]) < CUDART_INF_F); sum += x[j] * x[j]; }
@@ -97,38 +139,8 @@ __global__ void __launch_bounds__(128) attn_prep_kernel(const __nv_bfloat16 *__r
     if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(status, OMNI_ST_ATTN_NONFINITE);
 }
 
-// Values, transposed: Vt[kh][d][column of the token].  One block per (64 tokens, key/value head):
-// rows read whole (256 bytes per token), written as 64-token runs per head dimension.
-__global__ void __launch_bounds__(256) v_transpose_kernel(const __nv_bfloat16 *__restrict__ qkv, const int32_t *__restrict__ vcol,
-                                                          int T, int vpitch, __nv_bfloat16 *__restrict__ Vt,
-                                                          uint32_t *__restrict__ status) {
-    __shared__ unsigned short tile[64][HD + 2];
-    __shared__ int col[64];
-    dep_wait();
-    dep_launch();
-    const int t0 = blockIdx.x * 64, kh = blockIdx.y;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    bool bad = false;
-    if (threadIdx.x < 64) col[threadIdx.x] = t0 + threadIdx.x < T ? __ldg(vcol + t0 + threadIdx.x) : -1;
-    for (int i = warp; i < 64; i += 8) {
-        const long t = t0 + i;
-        if (t < T) {
-            const uint2 v = *reinterpret_cast<const uint2 *>(qkv + t * OMNI_QKV + (long)(NH + NKV + kh) * HD + lane * 4);
-            const unsigned short e[4] = {(unsigned short)(v.x & 0xffff), (unsigned short)(v.x >> 16), (unsigned short)(v.y & 0xffff), (unsigned short)(v.y >> 16)};
-#pragma unroll
-            for (int k = 0; k < 4; k++) { bad |= (e[k] & 0x7f80) == 0x7f80; tile[i][lane * 4 + k] = e[k]; }
-        }
-    }
-    __syncthreads();
-    unsigned short *out = reinterpret_cast<unsigned short *>(Vt) + (long)kh * HD * vpitch;
-    for (int d = warp; d < HD; d += 8)
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-            const int i = lane + 32 * k;
-            if (col[i] >= 0) out[(long)d * vpitch + col[i]] = tile[i][d];
-        }
-    if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(status, OMNI_ST_ATTN_NONFINITE);
-}
+// theta^(-p/64) of the 64 rotary pairs, once per bound layer
+__global__ void rope_freq_kernel(double theta, double *freq) { freq[threadIdx.x] = exp2(-(double)threadIdx.x * (1.0 / 64.0) * log2(theta)); }
 
 // ------------------------------------------------------------------ attention
 // One CTA per (pair of query heads that share a key/value head, tile of <= 128 query rows of one
@@ -479,14 +491,18 @@ cudaError_t omni_attn_configure(void) {
     return cudaFuncSetAttribute(attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM_BYTES);
 }
 
-cudaError_t omni_launch_attn_prep(const void *qkv, const float *qw, const float *kw, const int32_t *pos, const int32_t *vcol, int T,
-                                  int head_stride, int vpitch, float eps, double theta, void *Q, void *K, void *Vt, uint32_t *status,
-                                  cudaStream_t s) {
-    cudaError_t e = omni_launch_chain(attn_prep_kernel, dim3(T), dim3(128), 0, s, (const __nv_bfloat16 *)qkv, qw, kw, pos, head_stride, eps,
-                                      theta, (__nv_bfloat16 *)Q, (__nv_bfloat16 *)K, status);
-    if (e != cudaSuccess) return e;
-    return omni_launch_chain(v_transpose_kernel, dim3((T + 63) / 64, OMNI_NKV), dim3(256), 0, s, (const __nv_bfloat16 *)qkv, vcol, T, vpitch,
-                             (__nv_bfloat16 *)Vt, status);
+cudaError_t omni_launch_rope_freq(double theta, double *freq, cudaStream_t s) {
+    rope_freq_kernel<<<1, HD / 2, 0, s>>>(theta, freq);
+    return cudaGetLastError();
+}
+
+cudaError_t omni_launch_attn_prep(const void *qkv, const float *qw, const float *kw, const int32_t *pos, const double *freq,
+                                  const int32_t *vcol, int T, int head_stride, int vpitch, float eps, void *Q, void *K, void *Vt,
+                                  uint32_t *status, cudaStream_t s) {
+    const int tokens = PREP_THREADS / 32 / PREP_WARPS, prep = (T + tokens - 1) / tokens;
+    return omni_launch_chain(attn_prep_kernel, dim3(prep + (T + 63) / 64 * OMNI_NKV), dim3(PREP_THREADS), 0, s,
+                             (const __nv_bfloat16 *)qkv, qw, kw, pos, freq, vcol, T, prep, head_stride, vpitch, eps, (__nv_bfloat16 *)Q,
+                             (__nv_bfloat16 *)K, (__nv_bfloat16 *)Vt, status);
 }
 
 // tiles: [n_tiles] of {record start, first query row, rows (<= 128), Vt column of the record start}

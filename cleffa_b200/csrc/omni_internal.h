@@ -202,11 +202,13 @@ enum { OMNI_THIN_MAX_ROWS = 128, OMNI_THIN_BOXES = OMNI_THIN_MAX_ROWS / 16, OMNI
 cudaError_t omni_dense_configure(void);
 cudaError_t omni_launch_dense_thin(int which, const CUtensorMap *tm_w, const CUtensorMap *tm_x, int T, void *out_bf16, float *resid,
                                    uint32_t *status, cudaStream_t s);
+/* freq[64]: theta^(-p/64) of the rotary pairs */
+cudaError_t omni_launch_rope_freq(double theta, double *freq, cudaStream_t s);
 /* qkv [T][5120] BF16 -> Q [32][T][128], K [4][T][128], Vt [4][128][vpitch] (column vcol[t] for token t), BF16;
  * pos [T][3] positions (temporal, row, column); head_stride: rows between two heads of Q and K */
-cudaError_t omni_launch_attn_prep(const void *qkv, const float *qw, const float *kw, const int32_t *pos, const int32_t *vcol, int T,
-                                  int head_stride, int vpitch, float eps, double theta, void *Q, void *K, void *Vt, uint32_t *status,
-                                  cudaStream_t s);
+cudaError_t omni_launch_attn_prep(const void *qkv, const float *qw, const float *kw, const int32_t *pos, const double *freq,
+                                  const int32_t *vcol, int T, int head_stride, int vpitch, float eps, void *Q, void *K, void *Vt,
+                                  uint32_t *status, cudaStream_t s);
 /* tiles: [n_tiles] x {record start, first query row, rows (<= 128), Vt column of the record start}; out [T][4096] BF16 */
 cudaError_t omni_launch_attention(const CUtensorMap *tm_q, const CUtensorMap *tm_k, const CUtensorMap *tm_vt, const void *tiles,
                                   int n_tiles, int T, void *out, uint32_t *status, cudaStream_t s);

@@ -1322,8 +1322,8 @@ static bool attn_reserve(clef_gpu *g, char *err, size_t errlen) {
         ok = make_slab_map(g, &g->at.tm_xn_thin[i], xnorm, OMNI_CHUNK, OMNI_H, 16 * (i + 1), OMNI_THIN_SLABS) &&
              make_slab_map(g, &g->at.tm_a_thin[i], g->at.a, OMNI_CHUNK, OMNI_NH * OMNI_HD, 16 * (i + 1), OMNI_THIN_SLABS);
     if (ok) ok = make_map(g, &g->at.tm_q, g->at.q, (uint64_t)OMNI_NH * OMNI_CHUNK, OMNI_HD, 128, CU_TENSOR_MAP_L2_PROMOTION_L2_128B) &&
-                 make_map(g, &g->at.tm_k, g->at.k, (uint64_t)OMNI_NKV * OMNI_CHUNK, OMNI_HD, 128, CU_TENSOR_MAP_L2_PROMOTION_L2_128B) &&
-                 make_map(g, &g->at.tm_vt, g->at.vt, (uint64_t)OMNI_NKV * OMNI_HD, ATTN_VPITCH, 128, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
+                 make_map(g, &g->at.tm_k, g->at.k, (uint64_t)OMNI_NKV * OMNI_CHUNK, OMNI_HD, 64, CU_TENSOR_MAP_L2_PROMOTION_L2_128B) &&
+                 make_map(g, &g->at.tm_vt, g->at.vt, (uint64_t)OMNI_NKV * OMNI_HD, ATTN_VPITCH, 64, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
     if (!ok) {
         cudaGetLastError();
         if (xnorm && !g->xnorm) cudaFree(xnorm);
@@ -1462,7 +1462,7 @@ bool clef_omni_encode_attention(clef_gpu *g, int layer, float *x, const int32_t 
                                                                    T, OMNI_CHUNK, ATTN_VPITCH, g->attn[layer].eps, g->at.q, g->at.k, g->at.vt,
                                                                    s->status, g->stream)) &&
               launched(g, "attention", omni_launch_attention(&g->at.tm_q, &g->at.tm_k, &g->at.tm_vt, g->at.tiles, g->at.n_tiles, OMNI_CHUNK, g->at.a,
-                                                             s->status, g->stream)) &&
+                                                             s->status, g->n_sm, g->stream)) &&
               launched(g, "output projection", thin ? omni_launch_dense_thin(1, &g->attn[layer].tm_out_thin, g->at.tm_a_thin, T, NULL, x, s->status, g->stream)
                                                     : omni_launch_dense_pair(1, &g->attn[layer].tm_out, g->at.tm_a, T, NULL, x, s->status,
                                                                              g->n_sm, g->stream));

@@ -4,13 +4,9 @@
 //   attention_kernel    causal grouped-query attention inside each record of the packed batch,
 //                       online softmax (reference: metal/clef.metal:2174-2319, omni_attention)
 //
-// attention_kernel: one CTA per (query head, query tile of <= 128 rows of ONE record).  Both
-// products run on tcgen05 with operands in 128-byte-swizzled shared memory: S = Q K^T (128 x 128
-// keys, accumulator in tensor memory), softmax by 128 threads (one query row each, FP32, running
-// maximum and sum), P written back to shared memory as BF16, O_j = P V_j into a second
-// accumulator, which the same threads add into their FP32 registers with the usual rescaling.
-// Key blocks start at the record's first token, so a token sees the same blocks whether its
-// record is packed with others or runs alone.  V is kept transposed ([d][token]) so that both
+// Both products of the attention run on tcgen05 with operands in 128-byte-swizzled shared memory and
+// accumulators in tensor memory.  Key blocks start at the record's first token, so a token sees the same blocks whether
+// its record is packed with others or runs alone.  V is kept transposed ([d][token]) so that both
 // products read K-major operands; each record's columns start at a multiple of 64 tokens
 // (`vcol`), which keeps every TMA box 16-byte aligned.  Every wait is bounded.
 #include <cuda_bf16.h>
@@ -20,7 +16,7 @@
 #include <stdint.h>
 
 #include "omni_internal.h"
-#include "omni_meet.cuh"
+#include "omni_pair.cuh"
 #include "omni_pdl.cuh"
 #include "omni_ptx.cuh"
 
@@ -143,49 +139,68 @@ __global__ void __launch_bounds__(PREP_THREADS) attn_prep_kernel(const __nv_bflo
 __global__ void rope_freq_kernel(double theta, double *freq) { freq[threadIdx.x] = exp2(-(double)threadIdx.x * (1.0 / 64.0) * log2(theta)); }
 
 // ------------------------------------------------------------------ attention
-// One CTA per (pair of query heads that share a key/value head, tile of <= 128 query rows of one
-// record).  Key blocks of 128 run from the record's start to the tile's diagonal.  For each head x
-// of the pair and block j:
-//   S_x(j) = Q_x K_j^T       tcgen05, FP32 in TMEM
-//   P_x(j) = exp2(c S - m)   256 threads, two per query row (64 keys each); BF16, two keys per
-//                            column, written back over score columns the writing thread alone has
-//                            read (keys 0..63 over columns 0..31, keys 64..127 over 96..127)
-//   O_x   += P_x(j) V_j      tcgen05 with the A operand read from TMEM, accumulated over all blocks
-// The two heads run half a block apart: while one head's threads are in their exponentials the
-// tensor pipe forms the other head's value product and next scores, so neither waits for long.
-// m is the row's reference maximum.  It follows the running maximum lazily: only when a block's
-// maximum exceeds it by more than 2^8 are O and the running sum rescaled (by the softmax threads,
-// in TMEM: the scores of a block being there means the previous value product is done);
-// otherwise P simply holds values up to 256.  The accumulators never leave TMEM until the end.
+// Pairs of CTAs that stay resident (clusters of two SMs, tcgen05 cta_group::2) take work items in turn: a pair of
+// query heads that share a key/value head and a tile of <= 128 query rows of one record.  Each CTA
+// has one of the two heads; a key block of 128 is loaded once for both, half of it into each CTA.
+// Key blocks run from the record's start to the tile's diagonal.  For block g of a CTA's sequence:
+//   S(g) = Q K^T             tcgen05, FP32, into score buffer g mod 3 of tensor memory
+//   P(g) = exp2(c S - m)     by warps of group g mod 3, a thread per query row; BF16, two keys per column,
+//                            written over the upper half of the score buffer, which is in registers by then
+//   O   += P(g) V            tcgen05 with the A operand read from tensor memory, accumulated over the item's blocks
+// With three score buffers the scores of the next two blocks are complete before their softmax begins and
+// the value product of a block runs behind the softmax of the next: neither is part of a
+// chain from one block to the next.  All that passes from block to block is the row's reference maximum
+// m, handed from a group's warp to the next group's warp of the same 32 rows as soon as the block's own
+// maximum is known.  (With two heads per CTA and one score buffer each, the chain scores -> softmax -> value
+// product -> scores held a block of a head for 1870 cycles, tensor cores and special-function units 55 % busy.)
+// m follows the running maximum lazily: only when a block's maximum exceeds it by more than 2^8 is O
+// rescaled (in tensor memory, once the previous value product is done); otherwise P simply holds values up to
+// 256.  Each group sums its own blocks' probabilities against the m it last saw; the group of the item's
+// last block collects the sums, reads O and writes the rows while the others are in the next item.
+// The order of every sum goes by the block's place in its own item, so a row's bits do not depend on what the pair
+// did before.
 struct AttnTile { int32_t rec_start, q0, q_len, vcol0; };          // vcol0: Vt column of the record's first token
 
-constexpr int AT_THREADS = 640;                                    // warp 0 loads, 1 MMA, 2 TMEM, 3 spare, 4..11 softmax of head 0, 12..19 of head 1
-constexpr int AT_TILE_BYTES = 128 * 128 * 2;                       // 32 KiB: 128 rows x 128 BF16 as two 64-column halves
-constexpr int AT_KV_STAGES = 2;
-constexpr int AT_TMEM_COLS = 512;                                  // S_0, S_1, O_0, O_1 of 128 columns each
-constexpr int AT_N_BARS = 16;
-constexpr int AT_XCH_BYTES = 2 * 2 * 2 * 128 * 4;                  // [head][block parity][row half][row]
-constexpr int AT_SMEM_BYTES = AT_TILE_BYTES * (2 + 2 * AT_KV_STAGES) + 1024 + AT_N_BARS * 8 + 64 + AT_XCH_BYTES;
+constexpr int AT_THREADS = 512;                                    // warp 0 loads, 1 MMA, 2 TMEM, 3 spare, 4..7, 8..11, 12..15 softmax groups 0, 1, 2
+constexpr int AT_PAIRS_PER_TILE = NH / 2;                          // work items of a query tile
+constexpr int AT_Q_BYTES = 128 * 128 * 2;                          // 32 KiB: 128 rows x 128 BF16 as two 64-column halves
+constexpr int AT_KV_BYTES = 64 * 128 * 2;                          // 16 KiB: a CTA's half of a key or value block, as two 64-column halves
+constexpr int AT_KV_STAGES = 4, AT_BUFS = 3;
+constexpr int AT_TMEM_O = 0, AT_TMEM_S = 128, AT_P_COL = 64;       // O, then three score buffers of 128 columns; P in columns 64..127 of a buffer
+constexpr int AT_DATA_BYTES = 2 * AT_Q_BYTES + 2 * AT_KV_STAGES * AT_KV_BYTES;
+constexpr int AT_N_BARS = 4 + 4 * AT_KV_STAGES + 3 * AT_BUFS + 1 + 16 + 1;
+constexpr int AT_MISC_OFF = AT_DATA_BYTES + AT_N_BARS * 8, AT_XCH_OFF = (AT_MISC_OFF + 64 + 15) & ~15;
+constexpr int AT_SMEM_BYTES = AT_XCH_OFF + AT_BUFS * 128 * 4 + 2 * AT_BUFS * 128 * 8 + 1024;
+static_assert(AT_SMEM_BYTES <= 232448, "shared memory budget");
 constexpr float AT_LAZY = 8.f;                                     // log2 of how far a block may exceed the reference maximum
+// 128 registers per thread at launch: 80 do for the first four warps, the softmax threads take 144
+constexpr int AT_REGS_FEW = 80, AT_REGS_MANY = 144;
+static_assert(128 * AT_REGS_FEW + (AT_THREADS - 128) * AT_REGS_MANY <= AT_THREADS * 128, "registers of the block");
 
-__device__ __forceinline__ void tmem_st32(uint32_t addr, const uint32_t *r) {
+__device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&r)[16]) {
     asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(addr),
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t *r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(addr),
         "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
-        "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]),
-        "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]),
-        "r"(r[31])
+        "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
         : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// D[tmem] (+)= A[tmem] . B[smem]^T: A's rows are TMEM lanes, two BF16 of the K extent per column.
-__device__ __forceinline__ void umma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+// D[tmem] (+)= A[tmem] . B[smem]^T over both SMs: A's rows are the TMEM lanes of either CTA, two BF16 of the K extent
+// per column.
+__device__ __forceinline__ void umma_bf16_ts2(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
         ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ float ex2_approx(float x) {          // 2^x, -inf -> 0; relative error ~2^-22, far below BF16's
@@ -211,258 +226,380 @@ __device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
     return *reinterpret_cast<float2 *>(&d);
 }
 
+// The items of one pair of CTAs: the host lists the tiles with the most key blocks first; rounds over the pairs
+// alternate in direction, so that no pair gets the longer item of every round.  The entry of the item after the
+// current one is on its way meanwhile.
+struct AttnItems {
+    const AttnTile *tiles;
+    int n_items, round;
+    int4 cur, ahead;
+    __device__ __forceinline__ int index(int r) const {
+        const int pairs = (int)gridDim.x >> 1, p = (int)blockIdx.x >> 1;
+        return r * pairs + ((r & 1) ? pairs - 1 - p : p);
+    }
+    __device__ __forceinline__ AttnItems(const AttnTile *t, int n) : tiles(t), n_items(n), round(-1) { fetch(0); }
+    __device__ __forceinline__ void fetch(int r) {
+        if (index(r) < n_items) ahead = __ldg(reinterpret_cast<const int4 *>(tiles) + index(r) / AT_PAIRS_PER_TILE);
+    }
+    __device__ __forceinline__ bool more() const { return index(round + 1) < n_items; }
+    __device__ __forceinline__ bool next() {
+        const bool any = more();
+        round++;
+        cur = ahead;
+        fetch(round + 1);
+        return any;
+    }
+    __device__ __forceinline__ AttnTile tile() const { return AttnTile{cur.x, cur.y, cur.z, cur.w}; }
+    __device__ __forceinline__ int h0() const { return 2 * (index(round) % AT_PAIRS_PER_TILE); }            // first query head of the pair
+    __device__ __forceinline__ int n_blocks() const { return (cur.y + cur.z - 1 - cur.x) / 128 + 1; }        // from the record's start to the diagonal
+};
+
 __global__ void __launch_bounds__(AT_THREADS, 1)
 attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                 const __grid_constant__ CUtensorMap tm_vt, const AttnTile *__restrict__ tiles, int T, float scale,
+                 const __grid_constant__ CUtensorMap tm_vt, const AttnTile *__restrict__ tiles, int n_items, int T, float scale,
                  __nv_bfloat16 *__restrict__ out, uint32_t *__restrict__ status) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *const smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
-    auto q_smem = [&](int x) { return smem_base + AT_TILE_BYTES * x; };
-    auto k_smem = [&](int s) { return smem_base + AT_TILE_BYTES * (2 + s); };
-    auto v_smem = [&](int s) { return smem_base + AT_TILE_BYTES * (2 + AT_KV_STAGES + s); };
-    const uint32_t bar_base = smem_base + AT_TILE_BYTES * (2 + 2 * AT_KV_STAGES);
-    // barriers: q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_full[2], o_done[2]
-    const uint32_t q_full = bar_base;
-    auto k_full = [&](int s) { return bar_base + 8u * (1 + s); };
-    auto k_empty = [&](int s) { return bar_base + 8u * (3 + s); };
-    auto v_full = [&](int s) { return bar_base + 8u * (5 + s); };
-    auto v_empty = [&](int s) { return bar_base + 8u * (7 + s); };
-    auto s_full = [&](int x) { return bar_base + 8u * (9 + x); };
-    auto p_full = [&](int x) { return bar_base + 8u * (11 + x); };
-    auto o_done = [&](int x) { return bar_base + 8u * (13 + x); };
-    uint8_t *misc = smem_gen + AT_TILE_BYTES * (2 + 2 * AT_KV_STAGES) + AT_N_BARS * 8;
+    auto q_smem = [&](int b) { return smem_base + AT_Q_BYTES * b; };
+    auto k_smem = [&](int s) { return smem_base + 2 * AT_Q_BYTES + AT_KV_BYTES * s; };
+    auto v_smem = [&](int s) { return smem_base + 2 * AT_Q_BYTES + AT_KV_BYTES * (AT_KV_STAGES + s); };
+    const uint32_t bar_base = smem_base + AT_DATA_BYTES;
+    auto bar = [&](int i) { return bar_base + 8u * i; };
+    // loads are signalled on the first CTA's barriers; what the MMA thread commits arrives in both CTAs
+    auto q_full = [&](int b) { return bar(b); };
+    auto q_empty = [&](int b) { return bar(2 + b); };
+    auto k_full = [&](int s) { return bar(4 + s); };
+    auto k_empty = [&](int s) { return bar(4 + AT_KV_STAGES + s); };
+    auto v_full = [&](int s) { return bar(4 + 2 * AT_KV_STAGES + s); };
+    auto v_empty = [&](int s) { return bar(4 + 3 * AT_KV_STAGES + s); };
+    constexpr int B0 = 4 + 4 * AT_KV_STAGES;
+    auto s_full = [&](int b) { return bar(B0 + b); };
+    auto p_full = [&](int b) { return bar(B0 + AT_BUFS + b); };               // first CTA's: the four warps of the block's group, in both CTAs
+    auto pv_done = [&](int b) { return bar(B0 + 2 * AT_BUFS + b); };
+    const uint32_t o_empty = bar(B0 + 3 * AT_BUFS);                           // first CTA's: O of the previous item has been read, in both CTAs
+    auto fin_full = [&](int q, int slot) { return bar(B0 + 3 * AT_BUFS + 1 + 2 * q + slot); };
+    auto fin_empty = [&](int q, int slot) { return bar(B0 + 3 * AT_BUFS + 9 + 2 * q + slot); };
+    const uint32_t drain_bar = bar(B0 + 3 * AT_BUFS + 17);
+    uint8_t *misc = smem_gen + AT_MISC_OFF;
     volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(misc);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(misc + 4);
-    volatile int *armed = reinterpret_cast<volatile int *>(misc + 16);         // [5]: q, k stages, v stages (parity of the load in flight, -1 none)
-    volatile int *quit = reinterpret_cast<volatile int *>(misc + 40);          // [head][block parity]: a softmax thread's wait ran out, all of them leave together
-    float *xch = reinterpret_cast<float *>(misc + 64);                         // what the two threads of a row tell each other
+    volatile int *armed = reinterpret_cast<volatile int *>(misc + 16);         // [10]: q buffers, k and v stages (parity of the load in flight, -1 none)
+    float *m_sh = reinterpret_cast<float *>(smem_gen + AT_XCH_OFF);            // [group][row] reference maximum after the group's block
+    float2 *fin = reinterpret_cast<float2 *>(smem_gen + AT_XCH_OFF + AT_BUFS * 128 * 4);   // [slot][group][row] row sum of a group and the maximum it refers to
 
     const int warp = warp_index(), lane = threadIdx.x & 31;
-    const AttnTile tile = tiles[blockIdx.y];                                    // the host lists the tiles with the most key blocks first
-    const int h0 = 2 * blockIdx.x, kh = h0 / (NH / NKV);
-    const int q_last = tile.q0 + tile.q_len - 1;                                // last query row of the tile
-    const int n_blocks = (q_last - tile.rec_start) / 128 + 1;                   // key blocks from the record's start to the diagonal
+    const uint32_t rank = __shfl_sync(0xffffffffu, cluster_ctarank(), 0);
+    const bool leader = rank == 0;
+    const Abort ab{abort_flag, mapa_u32(bar_base + AT_N_BARS * 8 + 4, rank ^ 1u), status};
+    auto lead = [&](uint32_t b) { return mapa_u32(b, 0); };
+    auto give = [] { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(AT_REGS_FEW)); };
 
     if (threadIdx.x == 0) {
-        mbar_init(q_full, 1);
-        for (int s = 0; s < 2; s++) {
-            mbar_init(k_full(s), 1); mbar_init(k_empty(s), 1); mbar_init(v_full(s), 1); mbar_init(v_empty(s), 1);
-            mbar_init(s_full(s), 1); mbar_init(p_full(s), 256); mbar_init(o_done(s), 1);
+        for (int i = 0; i < AT_N_BARS; i++) {
+            const bool per_warp = (i >= B0 + AT_BUFS && i < B0 + 2 * AT_BUFS) || i == B0 + 3 * AT_BUFS;             // p_full, o_empty
+            const bool collect = i >= B0 + 3 * AT_BUFS + 1 && i < B0 + 3 * AT_BUFS + 9;                             // fin_full
+            mbar_init(bar(i), per_warp ? 8 : collect ? AT_BUFS - 1 : 1);
         }
         *abort_flag = 0;
-        for (int i = 0; i < 4; i++) quit[i] = 0;
-        for (int i = 0; i < 5; i++) armed[i] = -1;
+        for (int i = 0; i < 2 + 2 * AT_KV_STAGES; i++) armed[i] = -1;
         fence_mbar_init();
         prefetch_tmap(&tm_q); prefetch_tmap(&tm_k); prefetch_tmap(&tm_vt);
     }
-    if (warp == 2) { tmem_alloc(smem_u32((const void *)tmem_slot), AT_TMEM_COLS); tmem_relinquish(); }
+    cluster_sync_all();                       // the peer's barriers must exist before anything here can signal them
+    if (warp == 2) xtmem_alloc<2>(smem_u32((const void *)tmem_slot), 512);
     dep_wait();
     dep_launch();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = (uint32_t)uniform_i32((int)*tmem_slot);
 
-    if (warp == 0 && elect_one()) {
-        // ---------------------------------------------------------- loads: both Q tiles once, then K one block ahead of Vt
-        armed[0] = 0;
-        mbar_expect_tx(q_full, 2 * AT_TILE_BYTES);
-        for (int x = 0; x < 2; x++) {
-            tma_load_2d(q_smem(x), &tm_q, 0, (h0 + x) * T + tile.q0, q_full);                        // d 0..63
-            tma_load_2d(q_smem(x) + AT_TILE_BYTES / 2, &tm_q, 64, (h0 + x) * T + tile.q0, q_full);   // d 64..127
-        }
+    if (warp == 0) {
+        // ---------------------------------------------------------- loads of this CTA: its head's Q tile per item; of every block the
+        // key rows (head dimensions of V) that are its half.  Keys run ahead of values, as the MMAs do.
+        give();
         PipeState pk, pv;
-        auto load_k = [&](int j) {
-            if (!mbar_wait(k_empty(pk.stage), pk.phase ^ 1u, abort_flag, status)) return false;
-            const int key0 = tile.rec_start + j * 128;
-            armed[1 + pk.stage] = (int)pk.phase;
-            mbar_expect_tx(k_full(pk.stage), AT_TILE_BYTES);
-            tma_load_2d(k_smem(pk.stage), &tm_k, 0, kh * T + key0, k_full(pk.stage));
-            tma_load_2d(k_smem(pk.stage) + AT_TILE_BYTES / 2, &tm_k, 64, kh * T + key0, k_full(pk.stage));
+        AttnItems ki(tiles, n_items), vi(tiles, n_items);
+        int kj = 0, vj = 0;
+        bool ok = true;
+        bool k_left = ki.next(), v_left = vi.next();
+        auto load_k = [&] {
+            if (kj == 0) {
+                const int b = ki.round & 1;
+                const uint32_t ph = (uint32_t)(ki.round >> 1) & 1u;
+                ok = xwait_warp<false>(q_empty(b), ph ^ 1u, ab);
+                if (!ok) return;
+                if (elect_one()) {
+                    if (leader) { armed[b] = (int)ph; mbar_expect_tx(q_full(b), 2 * AT_Q_BYTES); }
+                    const int y = (ki.h0() + (int)rank) * T + ki.tile().q0;
+                    xtma_2d<2>(q_smem(b), &tm_q, 0, y, lead(q_full(b)), l2_policy_evict_first());                          // d 0..63
+                    xtma_2d<2>(q_smem(b) + AT_Q_BYTES / 2, &tm_q, 64, y, lead(q_full(b)), l2_policy_evict_first());         // d 64..127
+                }
+            }
+            ok = xwait_warp<false>(k_empty(pk.stage), pk.phase ^ 1u, ab);
+            if (!ok) return;
+            if (elect_one()) {
+                if (leader) { armed[2 + pk.stage] = (int)pk.phase; mbar_expect_tx(k_full(pk.stage), 2 * AT_KV_BYTES); }
+                const int y = ki.h0() / (NH / NKV) * T + ki.tile().rec_start + kj * 128 + (int)rank * 64;
+                xtma_2d<2>(k_smem(pk.stage), &tm_k, 0, y, lead(k_full(pk.stage)), l2_policy_evict_last());
+                xtma_2d<2>(k_smem(pk.stage) + AT_KV_BYTES / 2, &tm_k, 64, y, lead(k_full(pk.stage)), l2_policy_evict_last());
+            }
             pk.advance(AT_KV_STAGES);
-            return true;
+            if (++kj == ki.n_blocks()) { kj = 0; k_left = ki.next(); }
         };
-        bool ok = load_k(0);
-        for (int j = 0; j < n_blocks && ok; j++) {
-            if (j + 1 < n_blocks) ok = load_k(j + 1);
-            if (!ok || !mbar_wait(v_empty(pv.stage), pv.phase ^ 1u, abort_flag, status)) break;
-            armed[3 + pv.stage] = (int)pv.phase;
-            mbar_expect_tx(v_full(pv.stage), AT_TILE_BYTES);
-            tma_load_2d(v_smem(pv.stage), &tm_vt, tile.vcol0 + j * 128, kh * HD, v_full(pv.stage));            // keys 0..63 of the block
-            tma_load_2d(v_smem(pv.stage) + AT_TILE_BYTES / 2, &tm_vt, tile.vcol0 + j * 128 + 64, kh * HD, v_full(pv.stage));
+        for (int i = 0; i < AT_BUFS && k_left && ok; i++) load_k();
+        while (v_left && ok) {
+            ok = xwait_warp<false>(v_empty(pv.stage), pv.phase ^ 1u, ab);
+            if (!ok) break;
+            if (elect_one()) {
+                if (leader) { armed[2 + AT_KV_STAGES + pv.stage] = (int)pv.phase; mbar_expect_tx(v_full(pv.stage), 2 * AT_KV_BYTES); }
+                const int x = vi.tile().vcol0 + vj * 128, y = vi.h0() / (NH / NKV) * HD + (int)rank * 64;
+                xtma_2d<2>(v_smem(pv.stage), &tm_vt, x, y, lead(v_full(pv.stage)), l2_policy_evict_last());                              // keys 0..63 of the block
+                xtma_2d<2>(v_smem(pv.stage) + AT_KV_BYTES / 2, &tm_vt, x + 64, y, lead(v_full(pv.stage)), l2_policy_evict_last());
+            }
             pv.advance(AT_KV_STAGES);
+            if (++vj == vi.n_blocks()) { vj = 0; v_left = vi.next(); }
+            if (k_left) load_k();
         }
-    } else if (warp == 1 && elect_one()) {
+    } else if (warp == 1 && leader) {
         // ---------------------------------------------------------- MMA issuer
-        // Per head and block: the value product as soon as P is written, and behind it the head's next
-        // scores into the same TMEM columns (the tensor pipe runs them in the order issued, so the
-        // product has read P before the scores overwrite it).
-        const uint32_t idesc = idesc_bf16(128, 128);
-        auto scores = [&](int x, int stage) {     // S_x = Q_x K^T over the 128 head dimensions: two 64-wide halves, four K=16 steps each
-#pragma unroll
-            for (int half = 0; half < 2; half++) {
-                const uint64_t da = smem_desc_sw128(q_smem(x) + half * (AT_TILE_BYTES / 2));
-                const uint64_t db = smem_desc_sw128(k_smem(stage) + half * (AT_TILE_BYTES / 2));
-#pragma unroll
-                for (int k = 0; k < 4; k++) umma_bf16(tmem_base + x * 128, da + 2u * k, db + 2u * k, idesc, (half | k) ? 1u : 0u);
-            }
-            umma_commit(s_full(x));
-        };
-        PipeState pk, pv;
-        bool ok = mbar_wait(q_full, 0, abort_flag, status) && mbar_wait(k_full(0), 0, abort_flag, status);
-        if (ok) {
+        // Scores run AT_BUFS blocks ahead of value products; behind the value product of block g come the scores of
+        // block g + 3 into the buffer it has read P from (the tensor pipe runs them in the order issued).
+        give();
+        const uint32_t idesc = idesc_bf16(256, 128);
+        PipeState pk, pv, bs, bp;                 // stages of K and V; score buffer of the next scores and of the next value product
+        AttnItems si(tiles, n_items), pi(tiles, n_items);
+        int sj = 0, pj = 0;
+        bool ok = true;
+        bool s_left = si.next(), p_left = pi.next();
+        auto scores = [&] {
+            const int b = si.round & 1;
+            if (sj == 0) ok = xwait_warp<false>(q_full(b), (uint32_t)(si.round >> 1) & 1u, ab);
+            if (ok) ok = xwait_warp<false>(k_full(pk.stage), pk.phase, ab);
+            if (!ok) return;
             tc_fence_after();
-            scores(0, 0); scores(1, 0);
-            umma_commit(k_empty(0));
-            pk.advance(AT_KV_STAGES);
-        }
-        for (int j = 0; j < n_blocks && ok; j++) {
-            for (int x = 0; x < 2 && ok; x++) {
-                ok = mbar_wait(p_full(x), (uint32_t)j & 1u, abort_flag, status);
-                if (ok && x == 0) ok = mbar_wait(v_full(pv.stage), pv.phase, abort_flag, status);
-                if (!ok) break;
-                tc_fence_after();
-                // O_x += P_x V: the 128 keys of the block are eight K=16 steps, 8 TMEM columns of P each
-                // (keys 0..63 in columns 0..31 of the score buffer, keys 64..127 in columns 96..127)
+            if (elect_one()) {
+                const uint32_t d = tmem_base + AT_TMEM_S + bs.stage * 128;
 #pragma unroll
-                for (int k = 0; k < 8; k++) {
-                    const uint64_t db = smem_desc_sw128(v_smem(pv.stage) + (k >> 2) * (AT_TILE_BYTES / 2));
-                    umma_bf16_ts(tmem_base + 256 + x * 128, tmem_base + x * 128 + 8 * k + (k >> 2) * 64, db + 2u * (k & 3), idesc, (j | k) ? 1u : 0u);
+                for (int half = 0; half < 2; half++) {          // the 128 head dimensions: two 64-wide halves, four K=16 steps each
+                    const uint64_t da = smem_desc_sw128(q_smem(b) + half * (AT_Q_BYTES / 2));
+                    const uint64_t db = smem_desc_sw128(k_smem(pk.stage) + half * (AT_KV_BYTES / 2));
+#pragma unroll
+                    for (int k = 0; k < 4; k++) xmma<2>(d, da + 2u * k, db + 2u * k, idesc, (half | k) ? 1u : 0u);
                 }
-                if (x == 1) umma_commit(v_empty(pv.stage));
-                if (j + 1 < n_blocks) {
-                    if (x == 0) { ok = mbar_wait(k_full(pk.stage), pk.phase, abort_flag, status); if (!ok) break; tc_fence_after(); }
-                    scores(x, pk.stage);
-                    if (x == 1) umma_commit(k_empty(pk.stage));
-                } else {
-                    umma_commit(o_done(x));
-                }
+                xcommit<2>(s_full(bs.stage));
+                xcommit<2>(k_empty(pk.stage));
+                if (sj == si.n_blocks() - 1) xcommit<2>(q_empty(b));
             }
-            pv.advance(AT_KV_STAGES);
+            __syncwarp();
             pk.advance(AT_KV_STAGES);
-        }
-    } else if (warp >= 4) {
-        // ---------------------------------------------------------- softmax of one head: two threads per query row
-        // Thread (row r, half hf) owns keys hf*64.. of every score block, the P columns that hold
-        // them, and head dimensions hf*64.. of the accumulator.  The two threads of a row sit in
-        // different warps and exchange their partial maxima through shared memory at the head's
-        // named barrier; a thread whose wait ran out says so there, after which all threads of the
-        // head leave together.
-        const int x = (warp - 4) >> 3, q4 = warp & 3, hf = ((warp - 4) >> 2) & 1;
-        const int r = q4 * 32 + lane;                                             // row inside the tile = TMEM lane
-        const uint32_t tmem_s = tmem_base + x * 128 + ((uint32_t)(q4 * 32) << 16);
-        const uint32_t tmem_o = tmem_base + 256 + x * 128 + ((uint32_t)(q4 * 32) << 16) + hf * 64;
-        float *xc = xch + x * 512;                                                // [parity][half][row]
-        const float c = scale * 1.4426950408889634f;                              // scores to log2 units
-        float m = 0.f, l = 0.f;
-        auto meet = [&](int block, bool ok) { return warps_meet(quit + 2 * x, block, ok, [&] { asm volatile("bar.sync %0, 256;" ::"r"(1 + x) : "memory"); }); };
-        bool alive = true;
-        for (int j = 0; j < n_blocks; j++) {
-            const int par = j & 1;
-            if (alive) alive = mbar_wait(s_full(x), (uint32_t)par, abort_flag, status);
-            alive = __all_sync(0xffffffffu, alive);
-            const bool diagonal = j == n_blocks - 1;                              // the only block with keys after some of the rows
-            uint32_t ta[32];
-            float pmax = -CUDART_INF_F;
-            if (alive) {
-                tc_fence_after();
-                // two sweeps over the thread's 64 scores, 32 at a time: the maximum first, then the
-                // probabilities (reading TMEM twice costs less than holding the scores in registers)
+            bs.advance(AT_BUFS);
+            if (++sj == si.n_blocks()) { sj = 0; s_left = si.next(); }
+        };
+        for (int i = 0; i < AT_BUFS && s_left && ok; i++) scores();
+        while (p_left && ok) {
+            ok = xwait_warp<false>(v_full(pv.stage), pv.phase, ab);
+            if (ok && pj == 0 && pi.round > 0) ok = xwait_warp<false>(o_empty, (uint32_t)(pi.round - 1) & 1u, ab);
+            if (ok) ok = xwait_warp<false>(p_full(bp.stage), bp.phase, ab);
+            if (!ok) break;
+            tc_fence_after();
+            if (elect_one()) {
+                const uint32_t p = tmem_base + AT_TMEM_S + bp.stage * 128 + AT_P_COL;
 #pragma unroll
-                for (int q = 0; q < 2; q++) {
-                    tmem_ld32(tmem_s + hf * 64 + q * 32, ta);
-                    tmem_ld_wait();
+                for (int k = 0; k < 8; k++) {                   // the 128 keys of the block: eight K=16 steps, 8 columns of P each
+                    const uint64_t db = smem_desc_sw128(v_smem(pv.stage) + (k >> 2) * (AT_KV_BYTES / 2));
+                    umma_bf16_ts2(tmem_base + AT_TMEM_O, p + 8 * k, db + 2u * (k & 3), idesc, (pj | k) ? 1u : 0u);
+                }
+                xcommit<2>(v_empty(pv.stage));
+                xcommit<2>(pv_done(bp.stage));
+            }
+            __syncwarp();
+            pv.advance(AT_KV_STAGES);
+            bp.advance(AT_BUFS);
+            if (++pj == pi.n_blocks()) { pj = 0; p_left = pi.next(); }
+            if (s_left) scores();
+        }
+        // whatever happened, wait (bounded) until every MMA issued here has retired before tensor memory is released
+        if (elect_one()) {
+            xcommit<2>(drain_bar);
+            const uint64_t t0 = globaltimer_ns();
+            while (!mbar_try_wait(drain_bar, 0) && globaltimer_ns() - t0 < WAIT_LIMIT_NS) {}
+        }
+        __syncwarp();
+    } else if (warp < 4) {
+        give();
+    } else {
+        // ---------------------------------------------------------- softmax: a thread per query row
+        // The loop runs to its end whatever happens: a warp whose wait ran out does no more work but still meets the
+        // others at the barriers below, so none is left in them.
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(AT_REGS_MANY));
+        const int grp = (warp - 4) >> 2, q = warp & 3;
+        const int r = q * 32 + lane;                                              // row inside the tile = TMEM lane
+        const uint32_t tmem_row = tmem_base + ((uint32_t)(q * 32) << 16);
+        const float c = scale * 1.4426950408889634f;                              // scores to log2 units
+        // named barriers 1 + 4 * group + quadrant: from that group's warp to the next group's
+        const int bar_in = 1 + 4 * ((grp + AT_BUFS - 1) % AT_BUFS) + q, bar_out = 1 + 4 * grp + q;
+        const float *m_in = m_sh + (grp + AT_BUFS - 1) % AT_BUFS * 128 + r;
+        bool alive = true;
+        auto wait = [&](uint32_t b, uint32_t parity) {
+            if (alive) alive = __all_sync(0xffffffffu, xwait<2>(b, parity, ab));
+        };
+        AttnItems it(tiles, n_items);
+        int at = 0;                                                               // block of the sequence that the item starts with, mod 3
+        uint32_t phase = 0;                                                       // of this group's score buffer
+        bool first_ever = true;
+        while (it.next()) {
+            const int n_blocks = it.n_blocks();
+            const int last = (at + n_blocks - 1) % AT_BUFS;                       // group of the item's last block
+            const int slot = it.round & 1;
+            const uint32_t slot_phase = (uint32_t)(it.round >> 1) & 1u;
+            float m = -1e30f, l = 0.f;                                            // this group's sum and the maximum it refers to
+            for (int j = (grp + AT_BUFS - at) % AT_BUFS; j < n_blocks; j += AT_BUFS) {
+                const bool diagonal = j == n_blocks - 1;                          // the only block with keys after some of the rows
+                const uint32_t s_at = tmem_row + AT_TMEM_S + grp * 128;
+                uint32_t ta[32], tb[32];
+                float bm = -CUDART_INF_F;
+                wait(s_full(grp), phase);
+                // two sweeps over the row's 128 scores, the maximum first; the upper 64 stay in registers for the second
+                auto mask = [&](uint32_t (&v)[32], int key) {
                     if (diagonal) {
 #pragma unroll
                         for (int i = 0; i < 32; i++)
-                            if (hf * 64 + q * 32 + i > r) ta[i] = 0xff800000u;
+                            if (key + i > r) v[i] = 0xff800000u;
                     }
-                    float mq = fmaxf(__uint_as_float(ta[0]), __uint_as_float(ta[1]));
+                };
+                auto row_max = [&](const uint32_t (&v)[32]) {
+                    float a = max3(__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2])), b = __uint_as_float(v[3]);
 #pragma unroll
-                    for (int i = 2; i < 32; i += 2) mq = max3(mq, __uint_as_float(ta[i]), __uint_as_float(ta[i + 1]));
-                    pmax = fmaxf(pmax, mq);
-                }
-                xc[(par * 2 + hf) * 128 + r] = pmax;
-            }
-            if (!meet(j, alive)) { alive = false; break; }
-            // key 0 of every block is visible to every row (tiles and blocks are both cut from the
-            // record's start in steps of 128), so the block maximum is finite
-            const float bm = fmaxf(pmax, xc[(par * 2 + (hf ^ 1)) * 128 + r]) * c;
-            float corr = 1.f;
-            if (j == 0) m = bm;
-            else if (bm > m + AT_LAZY) { corr = ex2_approx(m - bm); m = bm; l *= corr; }
-            if (__any_sync(0xffffffffu, corr != 1.f)) {
-                // the scores of this block being complete means the previous value product is: O is at rest
-#pragma unroll
-                for (int q = 0; q < 2; q++) {
-                    uint32_t t32[32];
-                    tmem_ld32(tmem_o + q * 32, t32);
+                    for (int i = 4; i < 32; i += 4) {
+                        a = max3(a, __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
+                        b = max3(b, __uint_as_float(v[i + 2]), __uint_as_float(v[i + 3]));
+                    }
+                    bm = max3(bm, a, b);
+                };
+                if (alive) {
+                    tc_fence_after();
+                    tmem_ld32(s_at, ta);
+                    tmem_ld32(s_at + 32, tb);
                     tmem_ld_wait();
-#pragma unroll
-                    for (int i = 0; i < 32; i++) t32[i] = __float_as_uint(__uint_as_float(t32[i]) * corr);
-                    tmem_st32(tmem_o + q * 32, t32);
+                    mask(ta, 0);
+                    row_max(ta);
+                    tmem_ld32(s_at + 64, ta);
+                    mask(tb, 32);
+                    row_max(tb);
+                    tmem_ld32(s_at + 96, tb);
+                    tmem_ld_wait();
+                    mask(ta, 64);
+                    row_max(ta);
+                    mask(tb, 96);
+                    row_max(tb);
                 }
-            }
-            // P = exp2(c s - m) as BF16 (values up to 2^8 while m lags the running maximum), two keys per column
-            uint32_t pk[32];
-            float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-            const float2 c2 = make_float2(c, c), nm2 = make_float2(-m, -m);
-#pragma unroll
-            for (int q = 0; q < 2; q++) {
-                tmem_ld32(tmem_s + hf * 64 + q * 32, ta);
-                tmem_ld_wait();
-                if (diagonal) {
-#pragma unroll
-                    for (int i = 0; i < 32; i++)
-                        if (hf * 64 + q * 32 + i > r) ta[i] = 0xff800000u;
+                // key 0 of every block is visible to every row (tiles and blocks are both cut from the
+                // record's start in steps of 128), so the block maximum is finite
+                bm *= c;
+                float m_prev = bm;
+                if (at + j > 0 || !first_ever) {
+                    asm volatile("bar.sync %0, 64;" ::"r"(bar_in) : "memory");
+                    if (j > 0) m_prev = *m_in;
                 }
+                const float m_new = bm > m_prev + AT_LAZY ? bm : m_prev;
+                m_sh[grp * 128 + r] = m_new;
+                if (!diagonal || it.more()) asm volatile("bar.arrive %0, 64;" ::"r"(bar_out) : "memory");
+                if (m_new != m) { l *= ex2_approx(m - m_new); m = m_new; }
+                if (__any_sync(0xffffffffu, m_new != m_prev)) {
+                    // O may be scaled once the previous block's value product is done; this block's waits for the P below
+                    wait(pv_done((grp + AT_BUFS - 1) % AT_BUFS), grp == 0 ? phase ^ 1u : phase);
+                    if (alive) {
+                        tc_fence_after();
+                        const float corr = ex2_approx(m_prev - m_new);
+                        for (int o = 0; o < 8; o++) {
+                            uint32_t t16[16];
+                            tmem_ld16(tmem_row + AT_TMEM_O + o * 16, t16);
+                            tmem_ld_wait();
 #pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    const float2 e = ffma2(make_float2(__uint_as_float(ta[2 * i]), __uint_as_float(ta[2 * i + 1])), c2, nm2);
-                    const float2 pp = make_float2(ex2_approx(e.x), ex2_approx(e.y));
-                    acc[i & 1] = fadd2(acc[i & 1], pp);
-                    const __nv_bfloat162 bb = __floats2bfloat162_rn(pp.x, pp.y);
-                    pk[q * 16 + i] = *reinterpret_cast<const uint32_t *>(&bb);
-                }
-            }
-            l += (acc[0].x + acc[1].x) + (acc[0].y + acc[1].y);
-            // P goes over columns whose scores this thread alone read: keys 0..63 into columns 0..31,
-            // keys 64..127 into columns 96..127
-            tmem_st32(tmem_s + hf * 96, pk);
-            tmem_st_wait();
-            tc_fence_before();
-            mbar_arrive(p_full(x));
-        }
-        // the row's denominator is the sum of what its two threads added up (same reference maximum in both)
-        if (alive) alive = mbar_wait(o_done(x), 0, abort_flag, status);
-        alive = __all_sync(0xffffffffu, alive);
-        xc[((n_blocks & 1) * 2 + hf) * 128 + r] = l;
-        if (meet(n_blocks, alive)) {
-            tc_fence_after();
-            const float lt = l + xc[((n_blocks & 1) * 2 + (hf ^ 1)) * 128 + r];
-            const float inv = lt > 0.f ? 1.f / lt : 0.f;
-            const int qg = tile.q0 + r;                                           // global token index of the row
-            uint4 *dst = reinterpret_cast<uint4 *>(out + (long)qg * (NH * HD) + (h0 + x) * HD + hf * 64);
-#pragma unroll
-            for (int q = 0; q < 2; q++) {
-                uint32_t t32[32];
-                tmem_ld32(tmem_o + q * 32, t32);
-                tmem_ld_wait();
-                if (r < tile.q_len) {
-#pragma unroll
-                    for (int ch = 0; ch < 4; ch++) {
-                        uint32_t w[4];
-#pragma unroll
-                        for (int i = 0; i < 4; i++) {
-                            const __nv_bfloat162 bb = __floats2bfloat162_rn(__uint_as_float(t32[ch * 8 + 2 * i]) * inv,
-                                                                            __uint_as_float(t32[ch * 8 + 2 * i + 1]) * inv);
-                            w[i] = *reinterpret_cast<const uint32_t *>(&bb);
+                            for (int i = 0; i < 16; i++) t16[i] = __float_as_uint(__uint_as_float(t16[i]) * corr);
+                            tmem_st16(tmem_row + AT_TMEM_O + o * 16, t16);
                         }
-                        dst[q * 4 + ch] = make_uint4(w[0], w[1], w[2], w[3]);
+                    }
+                }
+                // P = exp2(c s - m) as BF16 (values up to 2^8 while m lags the running maximum), two keys per column
+                if (alive) {
+                    float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+                    const float2 c2 = make_float2(c, c), nm2 = make_float2(-m_new, -m_new);
+                    auto probs = [&](const uint32_t (&v)[32], int piece) {
+                        uint32_t pk[16];
+#pragma unroll
+                        for (int i = 0; i < 16; i++) {
+                            const float2 e = ffma2(make_float2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), c2, nm2);
+                            const float2 pp = make_float2(ex2_approx(e.x), ex2_approx(e.y));
+                            acc[i & 1] = fadd2(acc[i & 1], pp);
+                            const __nv_bfloat162 bb = __floats2bfloat162_rn(pp.x, pp.y);
+                            pk[i] = *reinterpret_cast<const uint32_t *>(&bb);
+                        }
+                        tmem_st16(s_at + AT_P_COL + piece * 16, pk);
+                    };
+                    probs(ta, 2);
+                    tmem_ld32(s_at, ta);
+                    probs(tb, 3);
+                    tmem_ld32(s_at + 32, tb);
+                    tmem_ld_wait();
+                    mask(ta, 0);
+                    probs(ta, 0);
+                    mask(tb, 32);
+                    probs(tb, 1);
+                    l += (acc[0].x + acc[1].x) + (acc[0].y + acc[1].y);
+                    tmem_st_wait();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_remote(lead(p_full(grp)));
+                }
+                phase ^= 1u;
+            }
+            first_ever = false;
+            if (grp != last) {
+                wait(fin_empty(q, slot), slot_phase ^ 1u);
+                fin[(slot * AT_BUFS + grp) * 128 + r] = make_float2(l, m);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(fin_full(q, slot));
+            } else {
+                wait(fin_full(q, slot), slot_phase);
+                const float2 f1 = fin[(slot * AT_BUFS + (grp + 1) % AT_BUFS) * 128 + r], f2 = fin[(slot * AT_BUFS + (grp + 2) % AT_BUFS) * 128 + r];
+                __syncwarp();
+                if (lane == 0) mbar_arrive(fin_empty(q, slot));
+                const float lt = l + f1.x * ex2_approx(f1.y - m) + f2.x * ex2_approx(f2.y - m);
+                const float inv = lt > 0.f ? 1.f / lt : 0.f;
+                wait(pv_done(grp), phase ^ 1u);                                   // the item's last value product
+                if (alive) {
+                    tc_fence_after();
+                    uint4 *dst = reinterpret_cast<uint4 *>(out + (long)(it.tile().q0 + r) * (NH * HD) + (it.h0() + (int)rank) * HD);
+#pragma unroll
+                    for (int o = 0; o < 4; o++) {
+                        uint32_t t32[32];
+                        tmem_ld32(tmem_row + AT_TMEM_O + o * 32, t32);
+                        tmem_ld_wait();
+                        if (o == 3) {                                             // the next item's value products may start
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive_remote(lead(o_empty));
+                        }
+                        if (r < it.tile().q_len) {
+#pragma unroll
+                            for (int ch = 0; ch < 4; ch++) {
+                                uint32_t w[4];
+#pragma unroll
+                                for (int i = 0; i < 4; i++) {
+                                    const __nv_bfloat162 bb = __floats2bfloat162_rn(__uint_as_float(t32[ch * 8 + 2 * i]) * inv,
+                                                                                    __uint_as_float(t32[ch * 8 + 2 * i + 1]) * inv);
+                                    w[i] = *reinterpret_cast<const uint32_t *>(&bb);
+                                }
+                                dst[o * 4 + ch] = make_uint4(w[0], w[1], w[2], w[3]);
+                            }
+                        }
                     }
                 }
             }
+            at = (at + n_blocks) % AT_BUFS;
         }
     }
 
@@ -470,16 +607,17 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     __syncthreads();
     if (*abort_flag && threadIdx.x == 0) {
         // a wait ran out: give loads already in flight a bounded chance to land
-        for (int s = 0; s < 5; s++) {
+        for (int s = 0; s < 2 + 2 * AT_KV_STAGES; s++) {
             const int par = armed[s];
             if (par < 0) continue;
-            const uint32_t bar = s == 0 ? q_full : s < 3 ? k_full(s - 1) : v_full(s - 3);
+            const uint32_t b = s < 2 ? q_full(s) : s < 2 + AT_KV_STAGES ? k_full(s - 2) : v_full(s - 2 - AT_KV_STAGES);
             const uint64_t t0 = globaltimer_ns();
-            while (!mbar_try_wait(bar, (uint32_t)par) && globaltimer_ns() - t0 < 50000000ull) {}
+            while (!mbar_try_wait(b, (uint32_t)par) && globaltimer_ns() - t0 < 50000000ull) {}
         }
     }
-    __syncthreads();
-    if (warp == 2) { tc_fence_after(); tmem_dealloc(tmem_base, AT_TMEM_COLS); }
+    // neither CTA may leave while the other's MMAs can still read its shared memory
+    cluster_sync_all();
+    if (warp == 2) { tc_fence_after(); xtmem_dealloc<2>(tmem_base, 512); }
 }
 
 }  // namespace
@@ -507,9 +645,22 @@ cudaError_t omni_launch_attn_prep(const void *qkv, const float *qw, const float 
 
 // tiles: [n_tiles] of {record start, first query row, rows (<= 128), Vt column of the record start}
 cudaError_t omni_launch_attention(const CUtensorMap *tm_q, const CUtensorMap *tm_k, const CUtensorMap *tm_vt, const void *tiles,
-                                  int n_tiles, int T, void *out, uint32_t *status, cudaStream_t s) {
-    return omni_launch_chain(attention_kernel, dim3(OMNI_NH / 2, n_tiles), dim3(AT_THREADS), AT_SMEM_BYTES, s, *tm_q, *tm_k, *tm_vt,
-                             (const AttnTile *)tiles, T, 1.0f / sqrtf((float)OMNI_HD), (__nv_bfloat16 *)out, status);
+                                  int n_tiles, int T, void *out, uint32_t *status, int n_sm, cudaStream_t s) {
+    const int n_items = n_tiles * AT_PAIRS_PER_TILE, pairs = n_items < n_sm / 2 ? n_items : n_sm / 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * pairs);
+    cfg.blockDim = dim3(AT_THREADS);
+    cfg.dynamicSmemBytes = AT_SMEM_BYTES;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = omni_dependent_launch_enabled() ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, attention_kernel, *tm_q, *tm_k, *tm_vt, (const AttnTile *)tiles, n_items, T, 1.0f / sqrtf((float)OMNI_HD),
+                              (__nv_bfloat16 *)out, status);
 }
 
 }  // extern "C"

@@ -211,7 +211,7 @@ cudaError_t omni_launch_attn_prep(const void *qkv, const float *qw, const float 
                                   uint32_t *status, cudaStream_t s);
 /* tiles: [n_tiles] x {record start, first query row, rows (<= 128), Vt column of the record start}; out [T][4096] BF16 */
 cudaError_t omni_launch_attention(const CUtensorMap *tm_q, const CUtensorMap *tm_k, const CUtensorMap *tm_vt, const void *tiles,
-                                  int n_tiles, int T, void *out, uint32_t *status, cudaStream_t s);
+                                  int n_tiles, int T, void *out, uint32_t *status, int n_sm, cudaStream_t s);
 
 /* Programmatic dependent launch of the pass's kernel chain (process-wide, default on) */
 void omni_set_dependent_launch(int on);

@@ -108,6 +108,33 @@ def test_records_do_not_depend_on_their_neighbours(attn):
     assert torch.equal(run(b, x, pos, bounds), packed)                 # and the pass is repeatable
 
 
+@pytest.mark.parametrize("bounds", [[0, 300], [0, 129, 640], [0, 1, 2, 130, 387]])
+def test_scores_that_outgrow_the_reference_maximum(backend, bounds):
+    """A row's scores are exponentiated against a reference maximum that is raised, and the accumulator rescaled, only when a
+    block exceeds it by more than 2^8.  Here keys are the queries of their group's first head, and the last third of each
+    record shares a direction: its scores lie 2^13 and more above those of the blocks in front."""
+    w = ao.make_attention_weights(3)
+    for kh in range(4):
+        w["w_qkv"][(32 + kh) * 128:(33 + kh) * 128] = w["w_qkv"][8 * kh * 128:(8 * kh + 1) * 128]
+    w["q_norm"], w["k_norm"] = torch.full((128,), 1.5), torch.ones(128)
+    backend.bind_attention(1, w["attn_norm"], w["w_qkv"], w["w_out"], w["q_norm"], w["k_norm"])
+    T = bounds[-1]
+    g = torch.Generator().manual_seed(T)
+    x, u = torch.randn(T, 2048, generator=g), torch.randn(2048, generator=g)
+    for lo, hi in zip(bounds[:-1], bounds[1:]):
+        x[hi - (hi - lo) // 3:hi] += 3 * u
+    pos = np.zeros((3, T), np.int32)
+    xd = x.clone().cuda()
+    backend.begin()
+    backend.encode_attention(1, xd, torch.from_numpy(np.ascontiguousarray(pos.T)).cuda(), np.asarray(bounds, np.int32))
+    backend.complete()
+    ref = ao.attention_half(x, pos, bounds, w["attn_norm"], w["w_qkv"], w["q_norm"], w["k_norm"], w["w_out"], 32, 4)
+    lo, hi = bounds[-2:]
+    scores = (ref["q"][0, hi - 1] @ ref["k"][0, lo:hi].T) * 128 ** -0.5 * 1.4427
+    assert float(scores[-20:].max() - scores[:128].max()) > 8
+    assert rel(xd.cpu().double() - x.double(), ref["out"] - x.double()) < GATE
+
+
 @pytest.mark.parametrize("T", [1, 15, 16, 17, 31, 33, 64, 97, 127, 128, 129])
 def test_short_batches_give_the_bits_of_long_ones(attn, T):
     """Up to 128 tokens the projections run with all token rows in every CTA (omni_dense.cu), above that on pairs of CTAs: a

@@ -523,6 +523,9 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         const int q = warp & 3;                       // TMEM lane quadrant this warp may read
         const int half = (warp - 4) >> 2;
         const int th = ((warp - 4) & 3) * 32 + lane;  // thread index inside the half (0..127)
+        // The combine reads d next: what of it is still in L2 then need not come back from memory.  us per block without and
+        // with: 1030 tokens 234.9 -> 234.4, 4096 432 -> 423, 8192 738 -> 727 (skewed 639 -> 630), 16384 1350 -> 1309.
+        const uint64_t pol_d = l2_policy_evict_last();
         PipeState wr;
         for (int it = 0;; it++) {
             int row0 = 0, len = 0, m = 0;
@@ -617,7 +620,8 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                         } else {
                             dst_row = a.out + (long)(row0 + r) * M::OUT_COLS;
                         }
-                        *reinterpret_cast<uint4 *>(dst_row + m_cta * M::OUTC + sub * 8) = val;
+                        if (MODE == X_DOWN && !a.rowinfo) st_global_hint(dst_row + m_cta * M::OUTC + sub * 8, val, pol_d);
+                        else *reinterpret_cast<uint4 *>(dst_row + m_cta * M::OUTC + sub * 8) = val;
                     }
                 }
             }

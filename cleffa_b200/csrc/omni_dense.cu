@@ -6,7 +6,8 @@
 // either projection.  What a CTA pays for that is the token operand, which every CTA reads whole
 // through its SM (1 MB at 128 rows of 4096), so longer batches stay on the pairs.
 //
-// The weight rows are the first rows of an M = 128 operand; its other rows are whatever follows in shared memory
+// The weight rows are the first rows of an M = 128 operand (M = 64 for the output projection: 256 instructions of K = 16 read half as
+// much of shared memory, attention half of 37 tokens 34.1 -> 32.3 us); its other rows are whatever follows in shared memory
 // and feed accumulator lanes that are never read.  K runs in the order of the pair kernel and into one
 // accumulator, so the results are its bits.  Every wait is bounded.
 #include <cuda_bf16.h>
@@ -21,8 +22,8 @@ namespace {
 
 enum { THIN_QKV = 0, THIN_OPROJ = 1 };
 template <int MODE> struct ThinCfg;
-template <> struct ThinCfg<THIN_QKV> { static constexpr int ROWS = OMNI_THIN_QKV_ROWS, K = OMNI_H, COLS = OMNI_QKV; };
-template <> struct ThinCfg<THIN_OPROJ> { static constexpr int ROWS = OMNI_THIN_OPROJ_ROWS, K = OMNI_NH * OMNI_HD, COLS = OMNI_H; };
+template <> struct ThinCfg<THIN_QKV> { static constexpr int ROWS = OMNI_THIN_QKV_ROWS, MMA_ROWS = 128, K = OMNI_H, COLS = OMNI_QKV; };
+template <> struct ThinCfg<THIN_OPROJ> { static constexpr int ROWS = OMNI_THIN_OPROJ_ROWS, MMA_ROWS = 64, K = OMNI_NH * OMNI_HD, COLS = OMNI_H; };
 
 constexpr int TN_THREADS = 256;          // warp 0 and 4 epilogue of accumulator lanes 0..31 (half of the tokens each), 1 MMA, 2 TMEM, 3 TMA, 5 epilogue of lanes 32..
 constexpr int TN_MAX_STAGES = 12, TN_RING_BYTES = 200 * 1024;
@@ -86,7 +87,7 @@ dense_thin_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
         }
     } else if (warp == 1 && elect_one()) {
         PipeState p;
-        const uint32_t idesc = idesc_bf16(128, n);
+        const uint32_t idesc = idesc_bf16(C::MMA_ROWS, n);
         for (int ks = 0; ks < STEPS; ks++) {
             if (!mbar_wait(full_bar(p.stage), p.phase, abort_flag, status)) break;
             tc_fence_after();

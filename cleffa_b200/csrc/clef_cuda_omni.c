@@ -688,7 +688,7 @@ static bool run_experts(clef_gpu *g, const omni_layer *L, const void *xn, const 
                                                                     fused ? s->sort.rowmap : NULL, NULL, NULL, g->reserve_sms == 0,
                                                                     g->n_sm - g->reserve_sms, g->stream))) return false;
         stage_mark(g, 3);
-        if (!launched(g, "down experts", omni_launch_down_pair(ctas, &L->tm_down, s->tm_h, sort, s->d, NULL, NULL, g->reserve_sms == 0,
+        if (!launched(g, "down experts", omni_launch_down_pair(ctas, &L->tm_down, s->tm_h, sort, s->d, NULL, NULL, g->reserve_sms == 0, L->down,
                                                                g->n_sm - g->reserve_sms, g->stream))) return false;
     } else {
         if (!launched(g, "gate/up experts (check kernel)", omni_launch_gateup_simple(s->xg, L->gate_up, s->sort.offsets, rows8, s->h, g->stream))) return false;
@@ -743,7 +743,7 @@ static bool run_experts_ep(clef_gpu *g, const omni_layer *L, const void *xn, con
                                                                     g->reserve_sms == 0, n_gemm, g->stream))) return false;
     }
     stage_mark(g, 3);
-    if (!launched(g, "down experts + return", omni_launch_down_pair(ctas, &L->tm_down, s->tm_h, s->sort, s->d, pe, g->ep.rowinfo, g->reserve_sms == 0, n_gemm, g->stream))) return false;
+    if (!launched(g, "down experts + return", omni_launch_down_pair(ctas, &L->tm_down, s->tm_h, s->sort, s->d, pe, g->ep.rowinfo, g->reserve_sms == 0, NULL, n_gemm, g->stream))) return false;
     stage_mark(g, 4);
     if (!launched(g, "expert-parallel barrier", omni_launch_ep_barrier(pe, ++g->ep.epoch, s->status, g->ep.wait_ns, g->stream))) return false;
     if (g->wait_residual && !launched(g, "residual upload join", cudaStreamWaitEvent(g->stream, g->residual_uploaded, 0))) return false;

@@ -132,6 +132,7 @@ struct XArgs {
     omni_ep_send send;                  // what the copy warps send from
     int need_blocks;                    // > 0: an arrival counter is complete at this value (it counts sender blocks), else at need[group]
     int early_dependents;
+    const char *weights;                // down on one GPU: the matrix behind tm_w, for prefetches
     int dense_rows, dense_tiles;        // dense projections: token rows, and the near-equal tiles they are cut into
 };
 
@@ -222,6 +223,17 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     // the peer's barriers must exist before anything of this CTA can signal them
     if (PAIR) cluster_sync_all(); else __syncthreads();
     if (warp == 2) xtmem_alloc<CTAS>(smem_u32((const void *)tmem_slot), 512);
+    if (MODE == X_DOWN && PAIR && a.weights && warp == 3 && lane < 128 * M::KTOT * 2 / OMNI_PREFETCH_PIECE) {
+        // Pairs become resident one after the other while the last items of gate/up leave memory half idle: each asks for the
+        // weights of its first item, one contiguous piece per CTA, to be brought into L2 (us per block: 3 tokens 57.5 -> 56.6,
+        // 9 109.5 -> 108.2, 37 186.0 -> 183.7, 128 203.8 -> 202.5, 2048 282 -> 279).  The tile list is older than
+        // the kernel in front (omni_pdl.cuh); whatever it held, the address stays inside the matrix.
+        const int w0 = (int)blockIdx.x / CTAS;
+        const int4 t = __ldcg(reinterpret_cast<const int4 *>(a.ttiles) + w0 / MI);
+        const int cnt = max(t.w >> 16, 1), m = ((w0 - (t.w & 0xffff) * MI) / cnt) & (MI - 1);
+        const char *p = a.weights + ((size_t)(t.x & (OMNI_E - 1)) * M::OUT_COLS + (m * CTAS + rank) * 128) * (M::KTOT * 2) + lane * OMNI_PREFETCH_PIECE;
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(OMNI_PREFETCH_PIECE) : "memory");
+    }
     dep_wait();                 // everything above overlaps the tail of the previous kernel
     if (a.early_dependents) dep_launch();
     tc_fence_before();
@@ -718,9 +730,10 @@ cudaError_t omni_launch_gateup_pair(int ctas, const CUtensorMap *tm_w4, const CU
 }
 
 cudaError_t omni_launch_down_pair(int ctas, const CUtensorMap *tm_w, const CUtensorMap *tm_h, const omni_sort_state st,
-                                  void *d, const omni_ep_peers *return_to, const int32_t *rowinfo, int early_dependents, int n_sm,
-                                  cudaStream_t s) {
+                                  void *d, const omni_ep_peers *return_to, const int32_t *rowinfo, int early_dependents,
+                                  const void *weights, int n_sm, cudaStream_t s) {
     XArgs a = {};
+    a.weights = (const char *)weights;
     a.ttiles = st.ttiles; a.n_ttiles = st.n_ttiles; a.work_counter = st.sched + 1;
     a.out = (__nv_bfloat16 *)d; a.status = st.status; a.group_size = 1;
     if (return_to) { a.pe = *return_to; a.rowinfo = rowinfo; }

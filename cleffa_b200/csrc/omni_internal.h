@@ -188,8 +188,10 @@ cudaError_t omni_launch_gateup_pair(int ctas, const CUtensorMap *tm_w4, const CU
  * return_to/rowinfo (may be NULL): result row i is written to row (rowinfo[i] & 0xfffff) of
  * return_to->dret[rowinfo[i] >> 20] (the rank the token came from) instead of row i of d */
 cudaError_t omni_launch_down_pair(int ctas, const CUtensorMap *tm_w, const CUtensorMap *tm_h, const omni_sort_state st,
-                                  void *d, const omni_ep_peers *return_to, const int32_t *rowinfo, int early_dependents, int n_sm,
-                                  cudaStream_t s);
+                                  void *d, const omni_ep_peers *return_to, const int32_t *rowinfo, int early_dependents,
+                                  const void *weights, int n_sm, cudaStream_t s);
+/* weights (may be NULL): the matrix that tm_w describes (all OMNI_E experts); pairs ask for the rows of their first item before
+ * the kernel in front is done */
 
 /* ---- attention half (omni_attn.cu; the two projections run on the kernel of omni_expert.cu) ---- */
 cudaError_t omni_attn_configure(void);

@@ -12,9 +12,9 @@
 //   * dep_wait() is executed by every thread before its first access to global memory and
 //     before any exit path.  A block that left without waiting would let its grid count as
 //     complete while an earlier grid still runs, and a later kernel could overtake that one.
-//     Only memory that no kernel of the chain writes may be touched earlier, and is in two places: the
-//     exact pass asks for bound weights to be brought into L2, and the attention kernel reads its
-//     query tiles, which a copy in front of the whole pass has written.
+//     Only memory that the kernel in front does not write may be touched earlier, and that only to
+//     ask for bound weights in L2: the exact pass (route_kernel, recheck_kernel) asks for gate/up weights, the down
+//     product for those of its first items, which it knows from the tile list, written before the kernel in front began.
 //   * dep_launch() follows dep_wait() directly: by then the block is resident, so waiting
 //     dependents can never hold resources a block of this grid still needs.  A dependent may so count
 //     on every kernel before this one being complete, whatever it does before its own wait.

@@ -136,7 +136,7 @@ struct XArgs {
     int dense_rows, dense_tiles;        // dense projections: token rows, and the near-equal tiles they are cut into
 };
 
-constexpr int DENSE_MIN = 96, DENSE_ITEM = 16;    // of the choice of tile length in omni_launch_dense_pair, in rows
+constexpr int DENSE_MIN = 96, DENSE_ITEM = 56;    // of the choice of tile length in omni_launch_dense_pair, in rows
 constexpr int DENSE_GROUP = 16;     // token tiles (of up to 256 rows, 1 to 2 MiB) that share a sweep over the weight blocks of a dense projection
 struct WorkSlotX { int expert, row0, len, m; };
 
@@ -749,14 +749,15 @@ cudaError_t omni_launch_dense_pair(int which, const CUtensorMap *tm_w, const CUt
     a.out = (__nv_bfloat16 *)out_bf16; a.resid = resid; a.status = status; a.group_size = 1;
     a.early_dependents = 1;
     a.dense_rows = T;
-    // Tiles: the fewest rounds of the pairs of SMs weighted by what an item of that many rows costs.  A
-    // tile of n rows takes about n/2 clocks per K step of 16 but no less than one of DENSE_MIN rows
-    // (issue and load latency).
+    // Tiles: the fewest rounds of the pairs of SMs weighted by what an item of that many rows costs: about n/2 clocks per K step
+    // of 16, and the weight rows, which come through the SM once per item however few tokens they meet.  (With a floor of
+    // 96 rows in place of that the q|k|v projection of 1030 tokens took three rounds of 96 rows where two of 160
+    // do: attention half 74.8 -> 69.0 us; from 4096 tokens on the choice makes no difference.)
     const int blocks = (which == 0 ? OMNI_QKV : OMNI_H) / 256, pairs = n_sm / 2;
     long best = -1;
     for (int nt = (T + OMNI_TILE_N - 1) / OMNI_TILE_N; nt <= T; nt++) {
         const int rows = ((T + nt - 1) / nt + 15) & ~15;
-        const long rounds = ((long)nt * blocks + pairs - 1) / pairs, cost = rounds * ((rows > DENSE_MIN ? rows : DENSE_MIN) + DENSE_ITEM);
+        const long rounds = ((long)nt * blocks + pairs - 1) / pairs, cost = rounds * (rows + DENSE_ITEM);
         if (best < 0 || cost < best) { best = cost; a.dense_tiles = nt; }
         if (rows <= DENSE_MIN) break;
     }

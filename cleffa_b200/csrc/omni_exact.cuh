@@ -205,53 +205,57 @@ struct ExactScratch {
     int sorted_id[8];
     float approx[OMNI_E];                  // by candidate
     int cand[OMNI_E];                      // expert of each candidate
+    int n;                                 // candidates
+    double bound;                          // the row's error bound
 };
 
-// Re-evaluates one flagged row with eight warps (256 threads): exact logits for every expert
-// that can still reach the top eight (approximate logit within twice the row's error bound of
-// the approximate 8th) and for the approximate 9th, then the final order by warp 0.  `sync` is a barrier
-// over exactly these threads.  With `segcount` given (expert counts per 256-assignment segment, taken
-// from the ids being replaced), the counts follow the ids that change.
-//
-// What the pass learns is written back: every logit it evaluated is replaced by its exact value
-// as a float pair (hi into `logits`, the remainder into `low` when given), so that a capture of
-// the row shows logits that agree with the ids chosen from them (clef_metal_omni.m:118-130
-// prints hi+lo).  And the assumed error bound is checked on the way: an approximate logit
-// further than the bound from its exact value raises OMNI_ST_ROUTER_EPS.
-template <typename Sync>
-__device__ __forceinline__ void recheck_row(const __nv_bfloat16 *__restrict__ xn, const __nv_bfloat16 *__restrict__ w,
-                                            const float *__restrict__ bias, float *__restrict__ logits,
-                                            float *__restrict__ low, long row, float eps, int32_t *__restrict__ ids,
-                                            float *__restrict__ weights, int32_t *__restrict__ segcount,
-                                            uint32_t *__restrict__ status, ExactScratch &sc, int lane, int warp, Sync sync) {
-    float approx[4];
+// One warp lists the candidates of a row: every expert that can still reach the top eight (approximate
+// logit within twice the row's error bound of the approximate 8th) and the approximate 9th.
+__device__ __forceinline__ void recheck_list(const float (&approx)[4], float eps, int lane, ExactScratch &sc) {
     float max_abs = 0.f;
 #pragma unroll
-    for (int j = 0; j < 4; j++) approx[j] = logits[row * OMNI_E + lane + 32 * j];
-    const int koff = warp * (OMNI_H / EXACT_WARPS) + lane * 8;
-    const uint4 xq = __ldg(reinterpret_cast<const uint4 *>(xn + row * OMNI_H + koff));
-    const int old_id = segcount && warp == 0 && lane < 8 ? ids[row * 8 + lane] : 0;
-#pragma unroll
     for (int j = 0; j < 4; j++) max_abs = fmaxf(max_abs, fabsf(approx[j]));
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) max_abs = fmaxf(max_abs, __shfl_xor_sync(FULL, max_abs, s));
+    max_abs = __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(max_abs)));          // not negative: ordered like its bits
     const double bound = (double)omni_row_eps(eps, max_abs);
     float v8, v9;
-    warp_8th_9th(approx, lane, v8, v9);                   // every warp finds the same threshold
+    warp_8th_9th(approx, lane, v8, v9);
     const double floor_v = fmin((double)v8 - 2.0 * bound, (double)v9);
     int n = 0;
 #pragma unroll
     for (int j = 0; j < 4; j++) {
         const bool in = (double)approx[j] >= floor_v;
         const unsigned m = __ballot_sync(FULL, in);
-        if (warp == 0) {
-            const int at = n + __popc(m & ((1u << lane) - 1u));
-            if (in) { sc.cand[at] = lane + 32 * j; sc.approx[at] = approx[j]; }
-            sc.exact[lane + 32 * j] = -CUDART_INF;
-        }
+        const int at = n + __popc(m & ((1u << lane) - 1u));
+        if (in) { sc.cand[at] = lane + 32 * j; sc.approx[at] = approx[j]; }
+        sc.exact[lane + 32 * j] = -CUDART_INF;
         n += __popc(m);
     }
-    sync();                                               // the candidates are listed
+    if (lane == 0) { sc.n = n; sc.bound = bound; }
+}
+
+// Re-evaluates one flagged row with eight warps (256 threads): exact logits of the candidates that recheck_list has
+// left in the scratch (behind a barrier), then the final order by warp 0.  `xq`: this lane's part of the row
+// (recheck_x).  `sync` is a barrier over exactly these threads.  With `segcount` given (expert counts per 256-assignment
+// segment, taken from the ids being replaced), the counts follow the ids that change.
+//
+// What the pass learns is written back: every logit it evaluated is replaced by its exact value
+// as a float pair (hi into `logits`, the remainder into `low` when given), so that a capture of
+// the row shows logits that agree with the ids chosen from them (clef_metal_omni.m:118-130
+// prints hi+lo).  And the assumed error bound is checked on the way: an approximate logit
+// further than the bound from its exact value raises OMNI_ST_ROUTER_EPS.
+__device__ __forceinline__ int recheck_k(int lane, int warp) { return warp * (OMNI_H / EXACT_WARPS) + lane * 8; }
+__device__ __forceinline__ uint4 recheck_x(const __nv_bfloat16 *xn, long row, int lane, int warp) {
+    return __ldg(reinterpret_cast<const uint4 *>(xn + row * OMNI_H + recheck_k(lane, warp)));
+}
+
+template <typename Sync>
+__device__ __forceinline__ void recheck_row(const uint4 &xq, const __nv_bfloat16 *__restrict__ w,
+                                            const float *__restrict__ bias, float *__restrict__ logits,
+                                            float *__restrict__ low, long row, int32_t *__restrict__ ids,
+                                            float *__restrict__ weights, int32_t *__restrict__ segcount,
+                                            uint32_t *__restrict__ status, ExactScratch &sc, int lane, int warp, Sync sync) {
+    const int koff = recheck_k(lane, warp), n = sc.n;
+    const int old_id = segcount && warp == 0 && lane < 8 ? ids[row * 8 + lane] : 0;
     double x[8];
     {
         const uint32_t u[4] = {xq.x, xq.y, xq.z, xq.w};
@@ -301,7 +305,7 @@ __device__ __forceinline__ void recheck_row(const __nv_bfloat16 *__restrict__ xn
             v *= EXACT_UNSCALE;
             const int e = sc.cand[b0 + lane];
             if (bias) v += (double)bias[e];
-            if (fabs(v - (double)sc.approx[b0 + lane]) > bound) atomicOr(status, OMNI_ST_ROUTER_EPS);
+            if (fabs(v - (double)sc.approx[b0 + lane]) > sc.bound) atomicOr(status, OMNI_ST_ROUTER_EPS);
             const float hi = (float)v;
             logits[row * OMNI_E + e] = hi;
             if (low) low[row * OMNI_E + e] = (float)(v - (double)hi);

@@ -109,8 +109,19 @@ __global__ void __launch_bounds__(EXACT_THREADS) recheck_kernel(const __nv_bfloa
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int n = *n_flag;
     if (n > T) n = T;                  // a count left by a pass that failed half-way can be no larger than this
-    for (int f = blockIdx.x; f < n; f += gridDim.x)
-        recheck_row(xn, w, bias, logits, low, flag_rows[f], eps, ids, weights, segcount, status, scratch, lane, warp, [] { __syncthreads(); });
+    for (int f = blockIdx.x; f < n; f += gridDim.x) {
+        const long row = flag_rows[f];
+        const uint4 xq = recheck_x(xn, row, lane, warp);
+        __syncthreads();                                   // the row before is done with the scratch
+        if (warp == 0) {
+            float v[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) v[j] = logits[row * OMNI_E + lane + 32 * j];
+            recheck_list(v, eps, lane, scratch);
+        }
+        __syncthreads();
+        recheck_row(xq, w, bias, logits, low, row, ids, weights, segcount, status, scratch, lane, warp, [] { __syncthreads(); });
+    }
 }
 
 // Exact logits for every (token, expert): tests only (tests/test_omni_router.m).
@@ -357,10 +368,13 @@ __global__ void __launch_bounds__(EXACT_THREADS) route_kernel(const __nv_bfloat1
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long row = blockIdx.x;
     if (row >= T) return;                                  // blocks that only ask for weights
-    if (warp == 0) {
-        float v[4];
+    const uint4 xq = recheck_x(xn, row, lane, warp);
+    float v[4];
+    if (warp < 2)
 #pragma unroll
         for (int j = 0; j < 4; j++) v[j] = logits[row * OMNI_E + lane + 32 * j];
+    if (warp == 1) recheck_list(v, eps, lane, scratch);    // beside the selection, in case the row is too close
+    if (warp == 0) {
         bool bad = false;
         float max_abs = 0.f;
         uint32_t key[4];
@@ -408,7 +422,7 @@ __global__ void __launch_bounds__(EXACT_THREADS) route_kernel(const __nv_bfloat1
     }
     __syncthreads();
     if (s_flag)
-        recheck_row(xn, w, bias, logits, low, row, eps, ids, weights, nullptr, st.status, scratch, lane, warp, [] { __syncthreads(); });
+        recheck_row(xq, w, bias, logits, low, row, ids, weights, nullptr, st.status, scratch, lane, warp, [] { __syncthreads(); });
     __syncthreads();                                       // s_flag has been read by all
     if (warp == 0) {
         __threadfence();                                   // this row's ids, in front of the count

@@ -188,35 +188,43 @@ __global__ void __launch_bounds__(256) assign_hist_kernel(const int32_t *__restr
     }
 }
 
-// Scan over the experts, shared by the two kernels that place assignments; called by all threads of a block
-// (at least 128), thread e < 128 with the number of rows of expert e.  Returns the expert's offset to
-// thread e; with `publish` also writes counts, offsets and the token-tile list of the expert products
-// and resets the counters that the rest of the pass starts from.
+// Scan over the experts, shared by the two kernels that place assignments; called by all 256 threads of a
+// block with the number of rows of expert tid % 128.  Returns the expert's offset to the first 128 threads. With
+// `publish` the other 128 also write counts, offsets and the token-tile list of the expert products and reset the
+// counters that the rest of the pass starts from: off the path of the threads that go on to place assignments
+// (3600 clocks while those did it themselves).
 struct ExpertScan { int warp_rows[4], warp_tiles[4]; int4 key[OMNI_E / 4], cnt[OMNI_E / 4]; };
 
 __device__ __forceinline__ int scan_experts(ExpertScan &sm, int total, const omni_sort_state &st, bool publish) {
-    const int e = threadIdx.x, lane = threadIdx.x & 31;
-    // inclusive scans over the 128 experts (rows and token tiles): shuffles inside each of the
-    // first four warps, then the totals of the warps before
+    const int e = threadIdx.x & (OMNI_E - 1), lane = threadIdx.x & 31;
+    const bool publisher = threadIdx.x >= OMNI_E;
+    // the router and the exact pass of this chunk are done with the flagged-row count: keep it
+    // for introspection and clear it for the next router launch (no memset between passes)
+    const int flagged = publisher && publish && e == 0 && st.n_flag ? st.n_flag[0] : 0;
+    // inclusive scans over the 128 experts (rows and token tiles): shuffles inside each of
+    // four warps (both halves of the block hold the same numbers), then the totals of the warps before
     const int nt = (total + st.tile_n - 1) / st.tile_n;
     int rows_incl = total, tiles_incl = nt;
-    // order of the tile list: falling tile length, equal ones by expert
-    const int key = nt ? total / nt * OMNI_E + (OMNI_E - 1 - e) : OMNI_E - 1 - e;
-    if (e < OMNI_E) {
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int a = __shfl_up_sync(FULL, rows_incl, d), b = __shfl_up_sync(FULL, tiles_incl, d);
-            if (lane >= d) { rows_incl += a; tiles_incl += b; }
-        }
-        if (lane == 31) { sm.warp_rows[e >> 5] = rows_incl; sm.warp_tiles[e >> 5] = tiles_incl; }
+    for (int d = 1; d < 32; d <<= 1) {
+        const int a = __shfl_up_sync(FULL, rows_incl, d), b = __shfl_up_sync(FULL, tiles_incl, d);
+        if (lane >= d) { rows_incl += a; tiles_incl += b; }
+    }
+    // order of the tile list: falling tile length, equal ones by expert
+    int key = 0;
+    if (!publisher) {
+        if (lane == 31) sm.warp_rows[e >> 5] = rows_incl;
+    } else {
+        key = (nt ? total / nt * OMNI_E : 0) + OMNI_E - 1 - e;
+        if (lane == 31) sm.warp_tiles[e >> 5] = tiles_incl;
         reinterpret_cast<int *>(sm.key)[e] = key;
         reinterpret_cast<int *>(sm.cnt)[e] = nt;
     }
     __syncthreads();
-    if (e >= OMNI_E) return 0;
-    for (int q = 0; q < (e >> 5); q++) { rows_incl += sm.warp_rows[q]; tiles_incl += sm.warp_tiles[q]; }
+#pragma unroll
+    for (int q = 0; q < 3; q++) if (q < (e >> 5)) { rows_incl += sm.warp_rows[q]; tiles_incl += sm.warp_tiles[q]; }
     const int off = rows_incl - total;
-    if (!publish) return off;
+    if (!publisher || !publish) return off;
     st.counts[e] = total;
     st.offsets[e] = off;
     if (e == OMNI_E - 1) st.offsets[OMNI_E] = rows_incl;
@@ -241,9 +249,7 @@ __device__ __forceinline__ int scan_experts(ExpertScan &sm, int total, const omn
         st.ttiles[first + j] = omni_ttile{e, off + j * base + min(j, extra), base + (j < extra), first | (nt << 16)};
     if (e < 8) st.sched[e] = 0;
     if (e == OMNI_E - 1) *st.n_ttiles = tiles_incl;
-    // the router and the exact pass of this chunk are done with the flagged-row count: keep it
-    // for introspection and clear it for the next router launch (no memset between passes)
-    if (e == 0 && st.n_flag) { st.n_flag[1] = st.n_flag[0]; st.n_flag[0] = 0; }
+    if (e == 0 && st.n_flag) { st.n_flag[1] = flagged; st.n_flag[0] = 0; }
     return off;
 }
 
@@ -252,6 +258,7 @@ __device__ __forceinline__ int scan_experts(ExpertScan &sm, int total, const omn
 // 256 KiB at 16384 tokens.  As a kernel of one block in front of the scatter that scan was a link
 // of its own in the chain of launches, and its single block took 15 us at 16384 tokens.
 constexpr int ASSIGN_SEGS = 8, ASSIGN_THREADS = 32 * ASSIGN_SEGS;
+static_assert(ASSIGN_THREADS == 2 * OMNI_E && EXACT_THREADS == 2 * OMNI_E, "scan_experts: half of the threads publish");
 __global__ void __launch_bounds__(ASSIGN_THREADS) assign_kernel(const int32_t *__restrict__ ids, int A, int nseg, omni_sort_state st) {
     __shared__ ExpertScan scan;
     __shared__ int4 all[ASSIGN_SEGS][OMNI_E / 4], front[ASSIGN_SEGS][OMNI_E / 4];     // sums of a warp's share of the segments
@@ -259,7 +266,7 @@ __global__ void __launch_bounds__(ASSIGN_THREADS) assign_kernel(const int32_t *_
     __shared__ unsigned mask[ASSIGN_SEGS][OMNI_E];
     dep_wait();
     dep_launch();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, e = threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, e = threadIdx.x & (OMNI_E - 1);
     const int seg0 = blockIdx.x * ASSIGN_SEGS, seg = seg0 + warp;
     const int t = seg * 32 + lane;                                                    // a segment is the 8 assignments of 32 tokens
     const bool have = t * OMNI_TOP < A;
@@ -294,14 +301,13 @@ __global__ void __launch_bounds__(ASSIGN_THREADS) assign_kernel(const int32_t *_
 #pragma unroll
         for (int k = 0; k < OMNI_TOP; k++) twice |= (atomicOr(&mask[warp][id[k]], 1u << lane) >> lane) & 1;
     int total = 0, run = 0;
-    if (e < OMNI_E)
 #pragma unroll
-        for (int q = 0; q < ASSIGN_SEGS; q++) {
-            total += reinterpret_cast<const int *>(all[q])[e];
-            run += reinterpret_cast<const int *>(front[q])[e];
-        }
+    for (int q = 0; q < ASSIGN_SEGS; q++) {
+        total += reinterpret_cast<const int *>(all[q])[e];
+        run += reinterpret_cast<const int *>(front[q])[e];
+    }
     run += scan_experts(scan, total, st, blockIdx.x == 0);
-    if (e < OMNI_E)
+    if (threadIdx.x < OMNI_E)
 #pragma unroll
         for (int q = 0; q < ASSIGN_SEGS; q++) {
             int *c = reinterpret_cast<int *>(own[q]) + e;
@@ -424,20 +430,22 @@ __global__ void __launch_bounds__(EXACT_THREADS) route_kernel(const __nv_bfloat1
     if (s_flag)
         recheck_row(xq, w, bias, logits, low, row, ids, weights, nullptr, st.status, scratch, lane, warp, [] { __syncthreads(); });
     __syncthreads();                                       // s_flag has been read by all
-    if (warp == 0) {
-        __threadfence();                                   // this row's ids, in front of the count
-        __syncwarp();
-        if (lane == 0) s_flag = atomicAdd(st.n_flag + 2, 1) == T - 1;
+    if (T > 1) {                                           // a single block needs no count
+        if (warp == 0) {
+            __threadfence();                               // this row's ids, in front of the count
+            __syncwarp();
+            if (lane == 0) s_flag = atomicAdd(st.n_flag + 2, 1) == T - 1;
+        }
+        __syncthreads();
+        if (!s_flag) return;
+        __threadfence();
     }
-    __syncthreads();
-    if (!s_flag) return;
 
     // ---- the last block: counting sort of all assignments.  A token's experts are distinct, so the tokens of
     // a segment that chose an expert are a mask of 32 bits and a token's rank among them is a count of bits.
     __shared__ unsigned mask[ROUTE_SEGS][OMNI_E];
     __shared__ int base[ROUTE_SEGS][OMNI_E];
     __shared__ ExpertScan scan;
-    __threadfence();
     const int nseg = (T + 31) / 32;
     for (int i = threadIdx.x; i < nseg * OMNI_E; i += EXACT_THREADS) mask[0][i] = 0;
     if (threadIdx.x == 0) st.n_flag[2] = 0;
@@ -461,9 +469,12 @@ __global__ void __launch_bounds__(EXACT_THREADS) route_kernel(const __nv_bfloat1
     }
     __syncthreads();
     int total = 0;
-    if (threadIdx.x < OMNI_E)
+    const int e128 = threadIdx.x & (OMNI_E - 1);
 #pragma unroll 4
-        for (int s = 0; s < nseg; s++) { base[s][threadIdx.x] = total; total += __popc(mask[s][threadIdx.x]); }
+    for (int s = 0; s < nseg; s++) {
+        if (threadIdx.x < OMNI_E) base[s][e128] = total;
+        total += __popc(mask[s][e128]);
+    }
     const int off = scan_experts(scan, total, st, true);
     __shared__ int offs[OMNI_E];
     if (threadIdx.x < OMNI_E) offs[threadIdx.x] = off;

@@ -223,9 +223,9 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     // the peer's barriers must exist before anything of this CTA can signal them
     if (PAIR) cluster_sync_all(); else __syncthreads();
     if (warp == 2) xtmem_alloc<CTAS>(smem_u32((const void *)tmem_slot), 512);
-    if (MODE == X_DOWN && PAIR && a.weights && warp == 3 && lane < 128 * M::KTOT * 2 / OMNI_PREFETCH_PIECE) {
-        // Pairs become resident one after the other while the last items of gate/up leave memory half idle: each asks for the
-        // weights of its first item, one contiguous piece per CTA, to be brought into L2 (us per block: 3 tokens 57.5 -> 56.6,
+    if (MODE == X_DOWN && a.weights && warp == 3 && lane < 128 * M::KTOT * 2 / OMNI_PREFETCH_PIECE) {
+        // CTAs become resident one after the other while the last items of gate/up leave memory half idle: each asks for the
+        // weights of its first item, one contiguous piece, to be brought into L2 (us per block: 1 token 36.6 -> 35.7, 3 57.5 -> 56.6,
         // 9 109.5 -> 108.2, 37 186.0 -> 183.7, 128 203.8 -> 202.5, 2048 282 -> 279).  The tile list is older than
         // the kernel in front (omni_pdl.cuh); whatever it held, the address stays inside the matrix.
         const int w0 = (int)blockIdx.x / CTAS;

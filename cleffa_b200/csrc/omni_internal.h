@@ -190,7 +190,7 @@ cudaError_t omni_launch_gateup_pair(int ctas, const CUtensorMap *tm_w4, const CU
 cudaError_t omni_launch_down_pair(int ctas, const CUtensorMap *tm_w, const CUtensorMap *tm_h, const omni_sort_state st,
                                   void *d, const omni_ep_peers *return_to, const int32_t *rowinfo, int early_dependents,
                                   const void *weights, int n_sm, cudaStream_t s);
-/* weights (may be NULL): the matrix that tm_w describes (all OMNI_E experts); pairs ask for the rows of their first item before
+/* weights (may be NULL): the matrix that tm_w describes (all OMNI_E experts); CTAs ask for the rows of their first item before
  * the kernel in front is done */
 
 /* ---- attention half (omni_attn.cu; the two projections run on the kernel of omni_expert.cu) ---- */

@@ -49,7 +49,7 @@ KERNELS_PER_PASS_EP = 9   # ... plus owner buckets, plan and one barrier; the ex
 METRIC = "MoE-layer prefill tokens/sec at T=4096"
 # dram__bytes_read.sum + dram__bytes_write.sum of one gate/up launch at T=4096, from the ncu
 # capture summarised in profiles/ncu_moe_layer_T4096.md
-GATEUP_DRAM_TRAFFIC_T4096 = 842_291_456 + 10_608_896
+GATEUP_DRAM_TRAFFIC_T4096 = 850_602_240 + 11_229_696
 
 
 def measured_peaks():

@@ -1,5 +1,5 @@
-// How warps that share a barrier agree, once per work item, whether to go on: the four of an epilogue half
-// (omni_expert.cu), the eight that form the softmax of a head, per key block (omni_attn.cu).
+// How the four warps of an epilogue half, which share a barrier, agree once per work item whether to go on
+// (omni_expert.cu).
 // Plain C++ besides the barrier it is given, so that the order of its accesses is tested on the CPU.
 #pragma once
 

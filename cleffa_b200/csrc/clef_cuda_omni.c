@@ -1310,7 +1310,8 @@ static bool attn_reserve(clef_gpu *g, char *err, size_t errlen) {
     g->at.h_vcol = malloc((size_t)OMNI_CHUNK * 4);
     g->at.h_bounds = malloc((size_t)(OMNI_CHUNK + 2) * 4);
     ok = ok && g->at.h_tiles && g->at.h_vcol && g->at.h_bounds;
-    /* the padding columns of Vt are multiplied by probabilities that are exactly zero: they must stay finite */
+    /* columns of Vt outside a record's own are multiplied by probabilities that are exactly zero and must be finite: zero at
+     * first, and attn_prep_kernel writes nothing else */
     if (ok) ok = cudaMemsetAsync(g->at.vt, 0, (size_t)OMNI_NKV * OMNI_HD * ATTN_VPITCH * 2, g->stream) == cudaSuccess &&
                  cudaMemsetAsync(g->at.k, 0, (size_t)OMNI_NKV * OMNI_CHUNK * OMNI_HD * 2, g->stream) == cudaSuccess &&
                  cudaMemsetAsync(g->at.q, 0, (size_t)OMNI_NH * OMNI_CHUNK * OMNI_HD * 2, g->stream) == cudaSuccess &&

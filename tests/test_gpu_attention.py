@@ -5,6 +5,8 @@ Gates: what the half adds to the residual stream within relative L2 1e-2 of FP64
 the tensor cores, FP32 softmax and accumulation; measured ~4e-3), the intermediate q|k|v projections
 and attention outputs within the same bound, a record's rows bitwise independent of what it is
 packed with, nonfinite inputs reported through the status word."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -35,7 +37,6 @@ def run(b, x, pos, bounds):
 
 def bf16_rows(b, what, T, cols):
     raw = np.empty((T, cols), np.uint16)
-    import ctypes as C
     ok = b.lib.clef_omni_read(b._g, what.encode(), C.c_void_p(raw.ctypes.data), raw.nbytes, b._err, 512)
     assert ok, b._err.value
     return torch.from_numpy(raw.view(np.int16)).view(torch.bfloat16).double()
@@ -156,6 +157,24 @@ def test_nonfinite_projection_is_reported(attn):
     b.encode_attention(0, xd, pd)
     with pytest.raises(OmniError, match="nonfinite Omni attention or router values"):
         b.complete()
+
+
+@pytest.mark.parametrize("bad, bounds", [(110, [0, 100]), (100, [0, 60]), (127, [0, 64]), (100, [0, 30, 60]), (150, [0, 30, 60]), (190, [0, 30, 90]),
+                                         (114, [0, 1])])
+def test_values_of_a_failed_pass_stay_out_of_a_later_one(attn, bad, bounds):
+    """The last key block of a record reaches past its tokens, into columns that another batch may have filled: `bad` is the
+    column of a nonfinite value there, in the record's own padding, the next record's or behind the last one."""
+    b, _ = attn
+    T = bounds[-1]
+    x = torch.randn(T, 2048, generator=torch.Generator().manual_seed(T))
+    pos = ao.make_positions(T, bounds)
+    want = run(b, x, pos, bounds)
+    assert torch.isfinite(want).all()
+    failing = torch.randn(200, 2048, generator=torch.Generator().manual_seed(6))
+    failing[bad, 100] = float("inf")
+    with pytest.raises(OmniError, match="nonfinite Omni attention or router values"):
+        run(b, failing, np.zeros((3, 200), np.int32), [0, 200])
+    assert torch.equal(run(b, x, pos, bounds), want)
 
 
 def test_invalid_attention_dispatch_is_refused(attn):

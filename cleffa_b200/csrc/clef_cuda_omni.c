@@ -86,7 +86,7 @@ struct clef_gpu {
     int gemm_impl, router_impl;         /* 0 = tcgen05, 1 = CUDA-core check kernels */
     int expert_kernel;                  /* tcgen05 expert products: 2 = pairs of CTAs (cta_group::2), 1 = the same kernel on
                                            single CTAs, 0 = chosen from the number of tokens */
-    int reserve_sms;                    /* SMs the persistent expert kernels leave to other streams */
+    int reserve_sms;                    /* SMs that the kernels whose blocks stay for the whole launch leave to other streams */
     int host_pieces;                    /* clef_omni_forward_host: pieces the batch is cut into (0 = chosen from T) */
     int fused_router;                   /* the router kernel counts experts per sort segment (no histogram kernel) */
     int fused_gather;                   /* gate/up fetches its token rows through rowmap (no gather kernel) */
@@ -1432,6 +1432,12 @@ static bool attn_plan(clef_gpu *g, int T, int n_seq, const int32_t *seq_bounds, 
     return true;
 }
 
+/* SMs for the attention half's kernels of pairs of CTAs that stay for the whole launch: what "reserve_sms" leaves, and one pair at least */
+static int resident_sms(const clef_gpu *g) {
+    const int n = g->n_sm - g->reserve_sms;
+    return n < 2 ? 2 : n;
+}
+
 bool clef_omni_encode_attention(clef_gpu *g, int layer, float *x, const int32_t *pos3, int T, int n_seq,
                                 const int32_t *seq_bounds, char *err, size_t errlen) {
     if (!g || !g->omni || layer < 0 || layer >= MAX_LAYERS || !g->attn[layer].bound) {
@@ -1463,7 +1469,7 @@ bool clef_omni_encode_attention(clef_gpu *g, int layer, float *x, const int32_t 
                                                                    T, OMNI_CHUNK, ATTN_VPITCH, g->attn[layer].eps, g->at.q, g->at.k, g->at.vt,
                                                                    s->status, g->stream)) &&
               launched(g, "attention", omni_launch_attention(&g->at.tm_q, &g->at.tm_k, &g->at.tm_vt, g->at.tiles, g->at.n_tiles, OMNI_CHUNK, g->at.a,
-                                                             s->status, g->n_sm, g->stream)) &&
+                                                             s->status, g->reserve_sms == 0, resident_sms(g), g->stream)) &&
               launched(g, "output projection", thin ? omni_launch_dense_thin(1, &g->attn[layer].tm_out_thin, g->at.tm_a_thin, T, NULL, x, s->status, g->stream)
                                                     : omni_launch_dense_pair(1, &g->attn[layer].tm_out, g->at.tm_a, T, NULL, x, s->status,
                                                                              g->n_sm, g->stream));

@@ -266,7 +266,7 @@ struct AttnItems {
 __global__ void __launch_bounds__(AT_THREADS, 1)
 attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_vt, const AttnTile *__restrict__ tiles, int n_items, int T, float scale,
-                 __nv_bfloat16 *__restrict__ out, uint32_t *__restrict__ status) {
+                 __nv_bfloat16 *__restrict__ out, int early_dependents, uint32_t *__restrict__ status) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *const smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -318,7 +318,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     cluster_sync_all();                       // the peer's barriers must exist before anything here can signal them
     if (warp == 2) xtmem_alloc<2>(smem_u32((const void *)tmem_slot), 512);
     dep_wait();
-    dep_launch();
+    if (early_dependents) dep_launch();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -654,7 +654,7 @@ cudaError_t omni_launch_attn_prep(const void *qkv, const float *qw, const float 
 
 // tiles: [n_tiles] of {record start, first query row, rows (<= 128), Vt column of the record start}
 cudaError_t omni_launch_attention(const CUtensorMap *tm_q, const CUtensorMap *tm_k, const CUtensorMap *tm_vt, const void *tiles,
-                                  int n_tiles, int T, void *out, uint32_t *status, int n_sm, cudaStream_t s) {
+                                  int n_tiles, int T, void *out, uint32_t *status, int early_dependents, int n_sm, cudaStream_t s) {
     const int n_items = n_tiles * AT_PAIRS_PER_TILE, pairs = n_items < n_sm / 2 ? n_items : n_sm / 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * pairs);
@@ -669,7 +669,7 @@ cudaError_t omni_launch_attention(const CUtensorMap *tm_q, const CUtensorMap *tm
     cfg.attrs = attr;
     cfg.numAttrs = omni_dependent_launch_enabled() ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, attention_kernel, *tm_q, *tm_k, *tm_vt, (const AttnTile *)tiles, n_items, T, 1.0f / sqrtf((float)OMNI_HD),
-                              (__nv_bfloat16 *)out, status);
+                              (__nv_bfloat16 *)out, early_dependents, status);
 }
 
 }  // extern "C"

@@ -211,9 +211,10 @@ cudaError_t omni_launch_rope_freq(double theta, double *freq, cudaStream_t s);
 cudaError_t omni_launch_attn_prep(const void *qkv, const float *qw, const float *kw, const int32_t *pos, const double *freq,
                                   const int32_t *vcol, int T, int head_stride, int vpitch, float eps, void *Q, void *K, void *Vt,
                                   uint32_t *status, cudaStream_t s);
-/* tiles: [n_tiles] x {record start, first query row, rows (<= 128), Vt column of the record start}; out [T][4096] BF16 */
+/* tiles: [n_tiles] x {record start, first query row, rows (<= 128), Vt column of the record start}; out [T][4096] BF16.
+ * The pairs of CTAs stay for the whole launch: n_sm SMs at most, and early_dependents as for the expert products */
 cudaError_t omni_launch_attention(const CUtensorMap *tm_q, const CUtensorMap *tm_k, const CUtensorMap *tm_vt, const void *tiles,
-                                  int n_tiles, int T, void *out, uint32_t *status, int n_sm, cudaStream_t s);
+                                  int n_tiles, int T, void *out, uint32_t *status, int early_dependents, int n_sm, cudaStream_t s);
 
 /* Programmatic dependent launch of the pass's kernel chain (process-wide, default on) */
 void omni_set_dependent_launch(int on);

@@ -11,7 +11,7 @@ import numpy as np
 import pytest
 import torch
 
-from cleffa_b200 import OmniError
+from cleffa_b200 import OmniBackend, OmniError
 from oracle import omni_attn_oracle as ao
 from oracle import omni_oracle as orc
 
@@ -226,3 +226,60 @@ def test_a_layer_is_attention_then_norm_and_moe(attn, weights0):
     b.encode_layer(2, one, pd, np.asarray(bounds, np.int32))
     b.complete()
     assert torch.equal(one, xd)
+
+
+class KernelNode(C.Structure):
+    """CUDA_KERNEL_NODE_PARAMS of the driver."""
+    _fields_ = [("func", C.c_void_p), ("grid", C.c_uint * 3), ("block", C.c_uint * 3), ("smem", C.c_uint), ("params", C.c_void_p),
+                ("extra", C.c_void_p), ("kern", C.c_void_p), ("ctx", C.c_void_p)]
+
+
+def captured_grids(stream, call):
+    """Name -> blocks of the kernels that `call` launches on the stream, from a capture that is not run."""
+    cu = C.CDLL("libcuda.so.1")
+    graph, n = C.c_void_p(), C.c_size_t()
+    assert cu.cuStreamBeginCapture_v2(C.c_void_p(stream), 1) == 0
+    try:
+        call()
+    finally:
+        assert cu.cuStreamEndCapture(C.c_void_p(stream), C.byref(graph)) == 0
+    assert cu.cuGraphGetNodes(graph, None, C.byref(n)) == 0
+    nodes, out = (C.c_void_p * n.value)(), {}
+    assert cu.cuGraphGetNodes(graph, nodes, C.byref(n)) == 0
+    for node in nodes:
+        kind, k, name = C.c_int(), KernelNode(), C.c_char_p()
+        assert cu.cuGraphNodeGetType(C.c_void_p(node), C.byref(kind)) == 0
+        if kind.value == 0:
+            assert cu.cuGraphKernelNodeGetParams_v2(C.c_void_p(node), C.byref(k)) == 0
+            assert (cu.cuFuncGetName(C.byref(name), C.c_void_p(k.func)) if k.func else cu.cuKernelGetName(C.byref(name), C.c_void_p(k.kern))) == 0
+            out[name.value.decode()] = k.grid[0] * k.grid[1] * k.grid[2]
+    assert cu.cuGraphDestroy(graph) == 0
+    return out
+
+
+def test_reserved_sms_hold_for_the_attention_half():
+    """Kernels whose blocks stay for the whole launch keep to the SMs that "reserve_sms" leaves, or to one pair, with the same bits."""
+    w = ao.make_attention_weights(0)
+    stream = torch.cuda.Stream()
+    n_sm = torch.cuda.get_device_properties(0).multi_processor_count
+    T, bounds = 1030, np.array([0, 500, 1030], np.int32)
+    x = torch.randn(T, 2048, generator=torch.Generator().manual_seed(11)).cuda()
+    pos = torch.from_numpy(np.ascontiguousarray(ao.make_positions(11, bounds).T)).cuda()
+    torch.cuda.synchronize()
+    with OmniBackend(0, stream=stream.cuda_stream) as b:
+        b.reserve(1)
+        b.bind_attention(0, w["attn_norm"], w["w_qkv"], w["w_out"], w["q_norm"], w["k_norm"])
+        want = None
+        for reserve in (0, 40, n_sm - 3, n_sm - 2, n_sm - 1):
+            b.set_option("reserve_sms", reserve)
+            out = x.clone()
+            torch.cuda.synchronize()
+            b.begin()
+            b.encode_attention(0, out, pos, bounds)
+            b.complete()
+            want = out if want is None else want
+            assert torch.equal(out, want), reserve
+            grids = captured_grids(stream.cuda_stream, lambda: b.encode_attention(0, out, pos, bounds))
+            resident = {k: v for k, v in grids.items() if "attention_kernel" in k}
+            assert len(resident) == 1
+            assert all(v <= max(2, n_sm - reserve) for v in resident.values()), (reserve, resident)

@@ -1432,12 +1432,6 @@ static bool attn_plan(clef_gpu *g, int T, int n_seq, const int32_t *seq_bounds, 
     return true;
 }
 
-/* SMs for the attention half's kernels of pairs of CTAs that stay for the whole launch: what "reserve_sms" leaves, and one pair at least */
-static int resident_sms(const clef_gpu *g) {
-    const int n = g->n_sm - g->reserve_sms;
-    return n < 2 ? 2 : n;
-}
-
 bool clef_omni_encode_attention(clef_gpu *g, int layer, float *x, const int32_t *pos3, int T, int n_seq,
                                 const int32_t *seq_bounds, char *err, size_t errlen) {
     if (!g || !g->omni || layer < 0 || layer >= MAX_LAYERS || !g->attn[layer].bound) {
@@ -1461,18 +1455,20 @@ bool clef_omni_encode_attention(clef_gpu *g, int layer, float *x, const int32_t 
     if (!attn_plan(g, T, n_seq, seq_bounds, err, errlen)) return false;
     omni_arena *s = g->omni;
     const bool thin = T <= OMNI_THIN_MAX_ROWS;        /* token rows that every CTA can afford to read whole (omni_dense.cu) */
+    /* the attention and the projections on pairs of CTAs stay for the whole launch: they take what "reserve_sms" leaves, one pair at least */
+    const int early = g->reserve_sms == 0, n_sm = g->n_sm - g->reserve_sms < 2 ? 2 : g->n_sm - g->reserve_sms;
     bool ok = launched(g, "attention norm", omni_launch_rmsnorm(x, g->attn[layer].norm_w, g->attn[layer].eps, T, g->xnorm, g->stream)) &&
               launched(g, "q|k|v projection", thin ? omni_launch_dense_thin(0, &g->attn[layer].tm_qkv_thin, g->at.tm_xn_thin, T, g->at.p, NULL, s->status, g->stream)
                                                    : omni_launch_dense_pair(0, &g->attn[layer].tm_qkv, g->at.tm_xn, T, g->at.p, NULL, s->status,
-                                                                            g->n_sm, g->stream)) &&
+                                                                            early, n_sm, g->stream)) &&
               launched(g, "attention prep", omni_launch_attn_prep(g->at.p, g->attn[layer].q_norm, g->attn[layer].k_norm, pos3, g->attn[layer].freq, g->at.vcol,
                                                                    T, OMNI_CHUNK, ATTN_VPITCH, g->attn[layer].eps, g->at.q, g->at.k, g->at.vt,
                                                                    s->status, g->stream)) &&
               launched(g, "attention", omni_launch_attention(&g->at.tm_q, &g->at.tm_k, &g->at.tm_vt, g->at.tiles, g->at.n_tiles, OMNI_CHUNK, g->at.a,
-                                                             s->status, g->reserve_sms == 0, resident_sms(g), g->stream)) &&
+                                                             s->status, early, n_sm, g->stream)) &&
               launched(g, "output projection", thin ? omni_launch_dense_thin(1, &g->attn[layer].tm_out_thin, g->at.tm_a_thin, T, NULL, x, s->status, g->stream)
                                                     : omni_launch_dense_pair(1, &g->attn[layer].tm_out, g->at.tm_a, T, NULL, x, s->status,
-                                                                             g->n_sm, g->stream));
+                                                                             early, n_sm, g->stream));
     if (!ok) { set_err(err, errlen, "%s", g->fail_msg); return false; }
     return true;
 }

@@ -744,10 +744,10 @@ cudaError_t omni_launch_down_pair(int ctas, const CUtensorMap *tm_w, const CUten
 // The dense projections of the attention half on the same kernel: tm_w is the weight matrix
 // [OUT_COLS][K] with a 64 x 128 box, tm_tok the token operand.  The T token rows are cut into near-equal tiles.
 cudaError_t omni_launch_dense_pair(int which, const CUtensorMap *tm_w, const CUtensorMap *tm_tok, int T, void *out_bf16, float *resid,
-                                   uint32_t *status, int n_sm, cudaStream_t s) {
+                                   uint32_t *status, int early_dependents, int n_sm, cudaStream_t s) {
     XArgs a = {};
     a.out = (__nv_bfloat16 *)out_bf16; a.resid = resid; a.status = status; a.group_size = 1;
-    a.early_dependents = 1;
+    a.early_dependents = early_dependents;
     a.dense_rows = T;
     // Tiles: the fewest rounds of the pairs of SMs weighted by what an item of that many rows costs: about n/2 clocks per K step
     // of 16, and the weight rows, which come through the SM once per item however few tokens they meet.  (With a floor of

@@ -197,7 +197,7 @@ cudaError_t omni_launch_down_pair(int ctas, const CUtensorMap *tm_w, const CUten
 cudaError_t omni_attn_configure(void);
 /* which: 0 = q|k|v projection (out_bf16 [T][5120]), 1 = output projection (added into resid [T][2048]) */
 cudaError_t omni_launch_dense_pair(int which, const CUtensorMap *tm_w, const CUtensorMap *tm_tok, int T, void *out_bf16, float *resid,
-                                   uint32_t *status, int n_sm, cudaStream_t s);
+                                   uint32_t *status, int early_dependents, int n_sm, cudaStream_t s);
 /* the same for at most OMNI_THIN_MAX_ROWS token rows (omni_dense.cu).  tm_w: the weights as {64, row, K / 64} with a box of
  * {64, OMNI_THIN_QKV_ROWS or OMNI_THIN_OPROJ_ROWS, OMNI_THIN_SLABS}; tm_x: such maps of the token operand, box i with 16 (i + 1) rows */
 enum { OMNI_THIN_MAX_ROWS = 128, OMNI_THIN_BOXES = OMNI_THIN_MAX_ROWS / 16, OMNI_THIN_SLABS = 2, OMNI_THIN_QKV_ROWS = 40, OMNI_THIN_OPROJ_ROWS = 16 };

@@ -284,9 +284,9 @@ bool clef_omni_read(clef_gpu *g, const char *what, void *dst, size_t bytes, char
  * "expert_chain" 0/1 (accepted and without effect: it chained the down kernel to the gate/up kernel expert by
  * expert in kernels that CTA pairs have replaced),
  * "ep_wait_ms" N (bound on each in-pass wait for other ranks, 0 = 2000), "reserve_sms" N (the kernels whose
- * blocks stay for the whole launch -- expert products, attention -- use all SMs but N, so that kernels of another
- * context on the same GPU -- another micro-batch -- are not locked out while they run; the attention runs on pairs of SMs and takes
- * one pair at least),
+ * blocks stay for the whole launch -- expert products, attention and its projections -- use all SMs but N, so that kernels of another
+ * context on the same GPU -- another micro-batch -- are not locked out while they run; the attention half runs on pairs of SMs and
+ * takes one pair at least),
  * "fused_gather" 0/1 (default 1: the gate/up kernel fetches its token rows through the permutation
  * itself instead of reading a copy in expert order made by a separate kernel; same results),
  * "fused_router" 0/1 (default 1: the router kernel counts the experts per segment of the counting sort,

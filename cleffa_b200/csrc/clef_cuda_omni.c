@@ -634,13 +634,14 @@ static bool run_router(clef_gpu *g, const omni_layer *L, const void *xn, int row
      * 9 108.9 -> 106.8, 37 186.6 -> 185.2, 128 207.5 -> 203.5, 256 215.0 -> 213.3, 400 218.4 -> 218.9, 511 220.5 -> 221.5,
      * 576 223.6 -> 226.0. */
     if (g->router_impl == 0 && g->fused_router && !g->debug_stamps && g->ep.world <= 1 && rows <= OMNI_ROUTE_MAX_ROWS) {
-        if (!make_slab_map(g, &tm_x, xn, (uint64_t)rows, OMNI_H, (uint32_t)omni_router_part_tile(rows), OMNI_PART_SLABS)) {
+        const int nt = omni_router_part_tile(rows, g->n_sm);
+        if (!make_slab_map(g, &tm_x, xn, (uint64_t)rows, OMNI_H, (uint32_t)nt, OMNI_PART_SLABS)) {
             note_failure(g, "router activation descriptor", cudaErrorInvalidValue);
             return false;
         }
-        if (!launched(g, "router", omni_launch_router_part(&tm_x, &L->tm_router_part, L->bias, rows, s->logits, s->status, g->stream)) ||
+        if (!launched(g, "router", omni_launch_router_part(&tm_x, nt, &L->tm_router_part, L->bias, rows, s->logits, s->status, g->stream)) ||
             !launched(g, "route", omni_launch_route(xn, L->router, L->bias, s->logits, low, rows, g->router_eps, g->router_exact, s->ids, s->weights,
-                                                    expert_sort(g, expert_ctas(g, rows)), L->gate_up, prefetch, g->stream))) return false;
+                                                    expert_sort(g, expert_ctas(g, rows)), L->gate_up, prefetch, g->n_sm, g->stream))) return false;
         *routed = ROUTED_SORTED;
         return true;
     }
@@ -664,7 +665,7 @@ static bool run_router(clef_gpu *g, const omni_layer *L, const void *xn, int row
     }
     if (!launched(g, "router exact pass", omni_launch_recheck(fused ? s->sort.segcount : NULL, xn, L->router, L->bias, s->logits, low, s->flag_rows,
                                                               s->n_flag, rows, g->router_eps, s->ids, s->weights, s->status, L->gate_up,
-                                                              prefetch, g->stream))) return false;
+                                                              prefetch, g->n_sm, g->stream))) return false;
     *routed = fused ? ROUTED_COUNTS : ROUTED_IDS;
     return true;
 }

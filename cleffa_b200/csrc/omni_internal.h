@@ -110,16 +110,17 @@ cudaError_t omni_launch_select(const float *logits, int T, float eps, int exact_
                                int32_t *flag_rows, int32_t *n_flag, uint32_t *status, cudaStream_t s);
 /* logits: the approximate values on entry; on return every logit the exact pass evaluated holds
  * (float)exact, and low (may be NULL) the remainder (float)(exact - hi).  prefetch: memory that the
- * kernel asks to be brought into L2 before it waits for the router, in pieces of OMNI_PREFETCH_PIECE bytes */
+ * kernel asks to be brought into L2 before it waits for the router, in pieces of OMNI_PREFETCH_PIECE bytes, from a block on each
+ * of n_sm SMs at least */
 #define OMNI_PREFETCH_PIECE 16384
 cudaError_t omni_launch_recheck(int32_t *segcount, const void *xn, const void *router, const float *bias, float *logits,
                                 float *low, const int32_t *flag_rows, const int32_t *n_flag, int T, float eps,
                                 int32_t *ids, float *weights, uint32_t *status, const void *prefetch, size_t prefetch_bytes,
-                                cudaStream_t s);
+                                int n_sm, cudaStream_t s);
 /* routing of at most OMNI_ROUTE_MAX_ROWS tokens behind omni_launch_router_part: selection, exact pass and sort */
 cudaError_t omni_launch_route(const void *xn, const void *router, const float *bias, float *logits, float *low, int T, float eps,
                               int exact_all, int32_t *ids, float *weights, omni_sort_state st, const void *prefetch,
-                              size_t prefetch_bytes, cudaStream_t s);
+                              size_t prefetch_bytes, int n_sm, cudaStream_t s);
 /* start of a pass: clears the status word, n_flag[0] and, where given, the OMNI_EP_BUCKETS bucket counters */
 cudaError_t omni_launch_begin(uint32_t *status, int32_t *n_flag, int32_t *buckets, cudaStream_t s);
 cudaError_t omni_launch_router_exact(const void *xn, const void *router, const float *bias, int T,
@@ -154,11 +155,11 @@ cudaError_t omni_launch_router_sm100(const CUtensorMap *tm_x, int nt, const CUte
                                      float eps, int exact_all, float *logits, int32_t *ids, float *weights,
                                      int32_t *flag_rows, int32_t *n_flag, uint32_t *status, unsigned long long *dbg,
                                      int32_t *segcount, cudaStream_t s);
-/* The logits alone, for short batches: 16 experts x omni_router_part_tile(T) tokens per CTA.  tm_x, tm_w: maps of the
- * activations and the router matrix as {64, row, K / 64} with boxes of {64, tile, OMNI_PART_SLABS} and {64, 16, OMNI_PART_SLABS} */
+/* The logits alone, for short batches: 16 experts x nt = omni_router_part_tile(T, n_sm) tokens per CTA.  tm_x, tm_w: maps of the
+ * activations and the router matrix as {64, row, K / 64} with boxes of {64, nt, OMNI_PART_SLABS} and {64, 16, OMNI_PART_SLABS} */
 enum { OMNI_PART_EXPERTS = 16, OMNI_PART_SLABS = 4 };
-int omni_router_part_tile(int T);
-cudaError_t omni_launch_router_part(const CUtensorMap *tm_x, const CUtensorMap *tm_w, const float *bias, int T, float *logits,
+int omni_router_part_tile(int T, int n_sm);
+cudaError_t omni_launch_router_part(const CUtensorMap *tm_x, int nt, const CUtensorMap *tm_w, const float *bias, int T, float *logits,
                                     uint32_t *status, cudaStream_t s);
 /* segcount (may be NULL): the kernel also writes the per-segment expert counts of the counting
  * sort for the ids it selected; omni_launch_recheck must then be given the same pointer so that

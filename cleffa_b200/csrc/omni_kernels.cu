@@ -726,10 +726,10 @@ cudaError_t omni_launch_select(const float *logits, int T, float eps, int exact_
 
 cudaError_t omni_launch_recheck(int32_t *segcount, const void *xn, const void *router, const float *bias, float *logits,
                                 float *low, const int32_t *flag_rows, const int32_t *n_flag, int T, float eps, int32_t *ids,
-                                float *weights, uint32_t *status, const void *prefetch, size_t prefetch_bytes, cudaStream_t s) {
-    int blocks = T < 148 * 8 ? T : 148 * 8;
+                                float *weights, uint32_t *status, const void *prefetch, size_t prefetch_bytes, int n_sm, cudaStream_t s) {
+    int blocks = T < n_sm * 8 ? T : n_sm * 8;
     const int pieces = (int)(prefetch_bytes / OMNI_PREFETCH_PIECE);
-    if (pieces && blocks < 148) blocks = 148;
+    if (pieces && blocks < n_sm) blocks = n_sm;
     return omni_launch_chain(pieces ? recheck_kernel<true> : recheck_kernel<false>, dim3(blocks), dim3(EXACT_THREADS), 0, s, (const __nv_bfloat16 *)xn,
                              (const __nv_bfloat16 *)router, bias, logits, low, flag_rows, n_flag, T, eps, ids, weights, segcount, status,
                              (const char *)prefetch, pieces);
@@ -738,10 +738,10 @@ cudaError_t omni_launch_recheck(int32_t *segcount, const void *xn, const void *r
 // sort state: n_flag[0] counts the flagged rows, n_flag[2] the blocks that are done
 cudaError_t omni_launch_route(const void *xn, const void *router, const float *bias, float *logits, float *low, int T, float eps,
                               int exact_all, int32_t *ids, float *weights, omni_sort_state st, const void *prefetch,
-                              size_t prefetch_bytes, cudaStream_t s) {
+                              size_t prefetch_bytes, int n_sm, cudaStream_t s) {
     if (T > OMNI_ROUTE_MAX_ROWS) return cudaErrorInvalidValue;
     const int pieces = (int)(prefetch_bytes / OMNI_PREFETCH_PIECE);
-    return omni_launch_chain(pieces ? route_kernel<true> : route_kernel<false>, dim3(pieces && T < 148 ? 148 : T), dim3(EXACT_THREADS), 0, s,
+    return omni_launch_chain(pieces ? route_kernel<true> : route_kernel<false>, dim3(pieces && T < n_sm ? n_sm : T), dim3(EXACT_THREADS), 0, s,
                              (const __nv_bfloat16 *)xn, (const __nv_bfloat16 *)router, bias, logits, low, T, eps, exact_all, ids, weights, st,
                              (const char *)prefetch, pieces);
 }

@@ -414,12 +414,12 @@ router_part_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
 
 extern "C" {
 
-// Tokens per CTA: 16 while that gives at most one CTA per SM for each group of experts
-int omni_router_part_tile(int T) { return T <= 16 * (148 / (OMNI_E / OMNI_PART_EXPERTS)) ? 16 : 32; }
+// Tokens per CTA: 16 while that gives at most one CTA per SM, with a row of CTAs for each group of experts (288 tokens on 148 SMs)
+int omni_router_part_tile(int T, int n_sm) { return (T + 15) / 16 * (OMNI_E / OMNI_PART_EXPERTS) <= n_sm ? 16 : 32; }
 
-cudaError_t omni_launch_router_part(const CUtensorMap *tm_x, const CUtensorMap *tm_w, const float *bias, int T, float *logits,
+// tm_x: map of the activations with boxes of `nt` rows (nt = omni_router_part_tile)
+cudaError_t omni_launch_router_part(const CUtensorMap *tm_x, int nt, const CUtensorMap *tm_w, const float *bias, int T, float *logits,
                                     uint32_t *status, cudaStream_t s) {
-    const int nt = omni_router_part_tile(T);
     const dim3 grid((T + nt - 1) / nt, OMNI_E / OMNI_PART_EXPERTS);
     return nt == 16 ? omni_launch_chain(router_part_kernel<16>, grid, dim3(PT_THREADS), PtCfg<16>::SMEM_BYTES, s, *tm_x, *tm_w, bias, T, logits, status)
                     : omni_launch_chain(router_part_kernel<32>, grid, dim3(PT_THREADS), PtCfg<32>::SMEM_BYTES, s, *tm_x, *tm_w, bias, T, logits, status);

@@ -93,3 +93,10 @@ def test_integration_stub_builds_against_the_reference_headers(tmp_path, lib):
     subprocess.run(["gcc", "-std=c11", "-D_GNU_SOURCE", "-Wall", "-Wextra", "-Werror", "-I", str(reference_dir()), "-I", str(ROOT / "include"),
                     str(stub), str(main), "-L", str(libdir), "-lclef_cuda_omni", f"-Wl,-rpath,{libdir}", "-o", str(exe)], check=True)
     subprocess.run([str(exe)], check=True)
+
+
+@pytest.mark.parametrize("n_sm", [7, 132, 148, 160])
+def test_short_routing_takes_its_tile_from_the_number_of_sms(lib, n_sm):
+    """16 tokens per CTA, with CTAs for each of eight groups of experts, while no SM gets two of them, else 32."""
+    for T in range(1, 385):
+        assert lib.omni_router_part_tile(T, n_sm) == (16 if -(-T // 16) * 8 <= n_sm else 32), T

@@ -44,12 +44,21 @@ H, F, E, TOP = 2048, 768, 128, 8
 GATEUP_FLOP_PER_TOKEN = 2 * H * (2 * F) * TOP          # 50,331,648
 EXPERT_FLOP_PER_TOKEN = GATEUP_FLOP_PER_TOKEN + 2 * F * H * TOP   # 75,497,472
 WEIGHT_BYTES = (E * H + E * 2 * F * H + E * H * F) * 2
-KERNELS_PER_PASS = 6     # router (counts the sort segments), exact pass, sort, gate/up (gathers its rows), down, combine
-KERNELS_PER_PASS_EP = 9   # ... plus owner buckets, plan and one barrier; the expert kernels dispatch and return the rows themselves
+ARENA_TOKENS = 16384      # a longer batch runs in pieces of this many
+SHORT_TOKENS = 384        # most tokens whose routing takes two launches
+KERNELS_SHORT = 5         # logits, routing (selection, exact pass, sort), gate/up (gathers its rows), down, combine
+KERNELS = 6               # router (counts the sort segments), exact pass, sort, gate/up, down, combine
+KERNELS_EP = 9            # ... plus owner buckets, plan and one barrier; the expert kernels dispatch and return the rows themselves
 METRIC = "MoE-layer prefill tokens/sec at T=4096"
 # dram__bytes_read.sum + dram__bytes_write.sum of one gate/up launch at T=4096, from the ncu
 # capture summarised in profiles/ncu_moe_layer_T4096.md
 GATEUP_DRAM_TRAFFIC_T4096 = 850_602_240 + 11_229_696
+
+
+def kernel_launches(tokens, world, n_layers, norm):
+    """Launches of this repository's kernels in one step: `begin`, then each layer's pieces, with the norm in front where it runs."""
+    pieces = [ARENA_TOKENS] * (tokens // ARENA_TOKENS) + [t for t in [tokens % ARENA_TOKENS] if t]
+    return 1 + n_layers * sum((KERNELS_EP if world > 1 else KERNELS_SHORT if t <= SHORT_TOKENS else KERNELS) + bool(norm) for t in pieces)
 
 
 def measured_peaks():
@@ -395,7 +404,7 @@ def ours(args):
         else:
             par = (f"expert parallel ep{world}, tokens data-parallel, rows exchanged by peer stores over NVLink "
                    f"from inside the expert kernels")
-        launches = 1 + ((KERNELS_PER_PASS + (1 if args.norm else 0)) * n_layers if world == 1 else KERNELS_PER_PASS_EP * n_layers)   # 1: begin
+        launches = kernel_launches(T, world, n_layers, args.norm)
         line = {
             "metric": METRIC if (T_TOKENS == 4096 and n_layers == 1 and not zipf) else
                       f"MoE-layer prefill tokens/sec at T={T_TOKENS}" + (f" through {n_layers} layers" if n_layers > 1 else ""),

@@ -1,6 +1,7 @@
 """The benchmark's reference arm on the host cores, launched the way the N>1 runs are: rank 0
 alone measures and prints one JSON line, the other ranks leave without work."""
 import json
+import re
 import subprocess
 import sys
 from pathlib import Path
@@ -23,3 +24,15 @@ def test_reference_arm_under_two_ranks_prints_one_line():
     cb = d["cpu_baseline"]
     assert cb["kind"] in ("reference", "port") and cb["cores"] >= 1 and cb["value"] == d["value"] and cb["sample"]
     assert "workload" in d["config"] and "model" not in d["config"]
+
+
+def test_launches_are_counted_by_the_kernels_of_each_size():
+    """Routing takes two launches up to OMNI_ROUTE_MAX_ROWS tokens on one GPU and three above; longer batches run in arena pieces."""
+    sys.path.insert(0, str(ROOT))
+    import bench
+    source = (ROOT / "cleffa_b200" / "csrc" / "omni_internal.h").read_text()
+    assert bench.SHORT_TOKENS == int(re.search(r"OMNI_ROUTE_MAX_ROWS = (\d+)", source)[1])
+    assert bench.ARENA_TOKENS == int(re.search(r"OMNI_CHUNK = (\d+)", source)[1])
+    assert [bench.kernel_launches(T, 1, 1, False) for T in (1, 384, 385, 4096, 16384, 16385, 32768)] == [6, 6, 7, 7, 7, 12, 13]
+    assert bench.kernel_launches(4096, 8, 1, False) == 10 and bench.kernel_launches(100, 8, 1, False) == 10
+    assert bench.kernel_launches(4096, 1, 48, True) == 1 + 48 * 7

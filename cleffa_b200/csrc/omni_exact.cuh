@@ -12,6 +12,7 @@
 #include <stdint.h>
 
 #include "omni_internal.h"
+#include "omni_select.cuh"
 
 namespace {
 
@@ -57,10 +58,6 @@ __device__ __forceinline__ void warp_topn(double (&val)[4], int lane, double (&t
 // round of the shuffle search above costs about 300 clocks (five exchanges of a double and an id), one
 // of these about 60.  Both searches of a row together: a block of 64 to 1030 tokens went from 218.6 to
 // 216.7 us (64) and 239.6 to 238.2 (1030), two layers of 37 tokens from 451.7 to 448.2.
-__device__ __forceinline__ uint32_t ordered_key(float f) {
-    const uint32_t u = __float_as_uint(f);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
 __device__ __forceinline__ float ordered_value(uint32_t k) { return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k); }
 
 // The 8th and 9th largest of the warp's 128 values (equal values count one by one).

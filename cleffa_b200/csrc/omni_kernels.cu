@@ -354,8 +354,8 @@ __global__ void __launch_bounds__(ASSIGN_THREADS) assign_kernel(const int32_t *_
 
 // ------------------------------------------------------------------ routing of short batches
 // Behind router_part_kernel: selection, exact pass and counting sort of up to ROUTE_MAX_ROWS tokens in one
-// launch.  A block per token: its first warp ranks the logits and forms the weights -- the arithmetic and
-// the near-tie rule of the router kernel's own selection, bit for bit -- and all eight warps re-decide
+// launch.  A block per token: its first warp ranks the logits and forms the weights -- the rules and, in
+// rank order, the sums of the router kernel's own selection, bit for bit -- and all eight warps re-decide
 // the row when it is too close.  The last block to finish sorts the assignments of the whole batch.  In separate
 // launches (selection in the router, exact pass, scan, scatter) each of these steps takes 1 to 3 us and
 // the way from one to the next as much again.
@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(EXACT_THREADS) route_kernel(const __nv_bfloat1
         for (int j = 0; j < 4; j++) {
             bad |= !(fabsf(v[j]) < CUDART_INF_F);
             max_abs = fmaxf(max_abs, fabsf(v[j]));
-            key[j] = (ordered_key(v[j]) & ~127u) | (uint32_t)(127 - (lane + 32 * j));
+            key[j] = ranking_key(v[j], lane + 32 * j);
         }
         bool close = false;
         if (__any_sync(FULL, bad)) {
@@ -400,16 +400,13 @@ __global__ void __launch_bounds__(EXACT_THREADS) route_kernel(const __nv_bfloat1
 #pragma unroll
             for (int r = 0; r < 9; r++) {
                 const uint32_t top = __reduce_max_sync(FULL, max(max(key[0], key[1]), max(key[2], key[3])));
-                const int id = 127 - (int)(top & 127u), j = id >> 5;
+                const int id = ranked_expert(top), j = id >> 5;
                 tv[r] = __shfl_sync(FULL, j == 0 ? v[0] : j == 1 ? v[1] : j == 2 ? v[2] : v[3], id & 31);
                 if (lane == r) my_id = id;
 #pragma unroll
                 for (int jj = 0; jj < 4; jj++) if (key[jj] == top) key[jj] = 0;
             }
-            const float thr = 2.f * omni_row_eps(eps, max_abs) + fmaxf(fabsf(tv[0]), fabsf(tv[8])) * 6.1035156e-5f;   // 2^-14
-            close = exact_all != 0;
-#pragma unroll
-            for (int k = 0; k < 8; k++) close |= (tv[k] - tv[k + 1]) < thr;
+            close = exact_all != 0 || near_tie(tv, eps, max_abs);
             if (!close) {
                 float mine = tv[0];
 #pragma unroll

@@ -19,6 +19,7 @@
 #include "omni_internal.h"
 #include "omni_pdl.cuh"
 #include "omni_ptx.cuh"
+#include "omni_select.cuh"
 
 namespace {
 
@@ -182,9 +183,7 @@ router_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
                     const float v = col[(q * 32 + i) * PITCH + lane];
                     bad |= !(fabsf(v) < CUDART_INF_F);
                     max_abs = fmaxf(max_abs, fabsf(v));
-                    const uint32_t u = __float_as_uint(v);
-                    const uint32_t ord = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-                    key[i] = (ord & ~127u) | (uint32_t)(127 - (q * 32 + i));
+                    key[i] = ranking_key(v, q * 32 + i);
                 }
                 sort16_desc<0>(key); sort16_desc<16>(key);
                 merge_top16<0, 16>(key);
@@ -228,9 +227,7 @@ router_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
                     const float v = col[i * PITCH + et];
                     bad |= !(fabsf(v) < CUDART_INF_F);
                     max_abs = fmaxf(max_abs, fabsf(v));
-                    const uint32_t u = __float_as_uint(v);
-                    const uint32_t ord = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-                    key[i] = (ord & ~127u) | (uint32_t)(127 - i);
+                    key[i] = ranking_key(v, i);
                 }
             }
             int4 *ip = reinterpret_cast<int4 *>(ids + row * 8);
@@ -249,13 +246,8 @@ router_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ 
                 }
                 float tv[9]; int ti[9];
 #pragma unroll
-                for (int r = 0; r < 9; r++) { ti[r] = 127 - (int)(key[r] & 127u); tv[r] = col[ti[r] * PITCH + et]; }
-                // near-tie threshold: the row's assumed accumulation error (it grows with the
-                // row's largest |logit|) plus what the borrowed key bits can hide
-                const float thr = 2.f * omni_row_eps(eps, max_abs) + fmaxf(fabsf(tv[0]), fabsf(tv[8])) * 6.1035156e-5f;   // 2^-14
-                bool close = exact_all != 0;
-#pragma unroll
-                for (int k = 0; k < 8; k++) close |= (tv[k] - tv[k + 1]) < thr;
+                for (int r = 0; r < 9; r++) { ti[r] = ranked_expert(key[r]); tv[r] = col[ti[r] * PITCH + et]; }
+                const bool close = exact_all != 0 || near_tie(tv, eps, max_abs);
                 float p[8], sum = 0.f;
 #pragma unroll
                 for (int k = 0; k < 8; k++) { p[k] = expf(tv[k] - tv[0]); sum += p[k]; }

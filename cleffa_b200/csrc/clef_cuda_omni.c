@@ -88,7 +88,8 @@ struct clef_gpu {
                                            single CTAs, 0 = chosen from the number of tokens */
     int reserve_sms;                    /* SMs that the kernels whose blocks stay for the whole launch leave to other streams */
     int host_pieces;                    /* clef_omni_forward_host: pieces the batch is cut into (0 = chosen from T) */
-    int fused_router;                   /* the router kernel counts experts per sort segment (no histogram kernel) */
+    int fused_router;                   /* the router kernel counts experts per sort segment (no histogram kernel), and short batches
+                                           are routed in two launches */
     int fused_gather;                   /* gate/up fetches its token rows through rowmap (no gather kernel) */
     long alloc_fail_at, alloc_count;    /* host-side fault injection */
     long launch_fail_at, launch_count;
@@ -323,7 +324,7 @@ bool clef_omni_reserve(clef_gpu *g, const clef_omni_config *c, int T, char *err,
         {(void **)&s->ids, (size_t)OMNI_CHUNK * OMNI_TOP * 4},
         {(void **)&s->weights, (size_t)OMNI_CHUNK * OMNI_TOP * 4},
         {(void **)&s->flag_rows, (size_t)OMNI_CHUNK * 4},
-        {(void **)&s->n_flag, 256},        /* [0..1] flagged-row counts */
+        {(void **)&s->n_flag, 256},        /* [0..1] flagged-row counts, [2] blocks that are done in route_kernel (zero between launches) */
         {(void **)&s->status, 256},
         {(void **)&s->sink, 256},
         {(void **)&s->stamps, (size_t)(OMNI_CHUNK / 32) * 8 * 8},
@@ -630,9 +631,10 @@ static bool run_router(clef_gpu *g, const omni_layer *L, const void *xn, int row
     if (low && !launched(g, "capture reset", cudaMemsetAsync(low, 0, (size_t)rows * OMNI_E * 4, g->stream))) return false;
     const size_t prefetch = g->ep.world <= 1 && rows >= PREFETCH_MIN_ROWS && rows <= PREFETCH_MAX_ROWS ? PREFETCH_BYTES : 0;
     CUtensorMap tm_x;
-    /* Short batches: two launches.  us per block with the general routing and with this one: 1 token 50.1 -> 38.5,
-     * 9 108.9 -> 106.8, 37 186.6 -> 185.2, 128 207.5 -> 203.5, 256 215.0 -> 213.3, 400 218.4 -> 218.9, 511 220.5 -> 221.5,
-     * 576 223.6 -> 226.0. */
+    /* Short batches: two launches.  us per block with the general routing and with this one, both in turn: 1 token 39.7 -> 35.4,
+     * 9 109.1 -> 102.1, 37 189.2 -> 180.3, 128 208.1 -> 199.2, 256 213.7 -> 204.9, 384 220.0 -> 211.1.  The line was drawn where they
+     * were equal before the exact pass had its candidates listed beside the selection; with a later one: 448 215.9 -> 212.8,
+     * 511 220.9 -> 217.9, 576 219.7 -> 221.2, 640 220.4 -> 229.2. */
     if (g->router_impl == 0 && g->fused_router && !g->debug_stamps && g->ep.world <= 1 && rows <= OMNI_ROUTE_MAX_ROWS) {
         const int nt = omni_router_part_tile(rows, g->n_sm);
         if (!make_slab_map(g, &tm_x, xn, (uint64_t)rows, OMNI_H, (uint32_t)nt, OMNI_PART_SLABS)) {

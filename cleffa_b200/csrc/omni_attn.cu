@@ -10,7 +10,6 @@
 // products read K-major operands; each record's columns start at a multiple of 64 tokens
 // (`vcol`), which keeps every TMA box 16-byte aligned.  Every wait is bounded.
 #include <cuda_bf16.h>
-#include <type_traits>
 #include <cuda_runtime.h>
 #include <math_constants.h>
 #include <stdint.h>

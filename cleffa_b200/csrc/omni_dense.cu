@@ -4,10 +4,12 @@
 // rows and the output projection 8: 40 and 16 of 148 SMs stream 21 and 17 MB of weights, 11.5 and 16.5 us
 // where the memory would need 3.  Here a CTA takes 40 (16) weight rows and all token rows: 128 CTAs for
 // either projection.  What a CTA pays for that is the token operand, which every CTA reads whole
-// through its SM (1 MB at 128 rows of 4096), so longer batches stay on the pairs.
+// through its SM (1 MB at 128 rows of 4096), so longer batches stay on the pairs.  Attention half on pairs and here, both in
+// turn: 1 token 41.4 -> 27.0 us, 37 44.5 -> 29.2, 100 45.3 -> 34.8, 128 46.0 -> 37.1; the line lies at the longest token operand of one
+// CTA here, not where the two would be equal.
 //
 // The weight rows are the first rows of an M = 128 operand (M = 64 for the output projection: 256 instructions of K = 16 read half as
-// much of shared memory, attention half of 37 tokens 34.1 -> 32.3 us); its other rows are whatever follows in shared memory
+// much of shared memory, attention half of 37 tokens 31.0 -> 28.9 us, 128 38.0 -> 36.8); its other rows are whatever follows in shared memory
 // and feed accumulator lanes that are never read.  K runs in the order of the pair kernel and into one
 // accumulator, so the results are its bits.  Every wait is bounded.
 #include <cuda_bf16.h>

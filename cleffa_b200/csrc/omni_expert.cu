@@ -225,8 +225,8 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     if (warp == 2) xtmem_alloc<CTAS>(smem_u32((const void *)tmem_slot), 512);
     if (MODE == X_DOWN && a.weights && warp == 3 && lane < 128 * M::KTOT * 2 / OMNI_PREFETCH_PIECE) {
         // CTAs become resident one after the other while the last items of gate/up leave memory half idle: each asks for the
-        // weights of its first item, one contiguous piece, to be brought into L2 (us per block: 1 token 36.6 -> 35.7, 3 57.5 -> 56.6,
-        // 9 109.5 -> 108.2, 37 186.0 -> 183.7, 128 203.8 -> 202.5, 2048 282 -> 279).  The tile list is older than
+        // weights of its first item, one contiguous piece, to be brought into L2 (us per block, both in turn: 1 token 36.7 -> 35.3, 3 55.6 ->
+        // 54.5, 9 108.4 -> 103.5, 37 183.4 -> 180.6, 128 202.1 -> 200.8, 511 and 1030 the same, 2048 284.0 -> 281.6).  The tile list is older than
         // the kernel in front (omni_pdl.cuh); whatever it held, the address stays inside the matrix.
         const int w0 = (int)blockIdx.x / CTAS;
         const int4 t = __ldcg(reinterpret_cast<const int4 *>(a.ttiles) + w0 / MI);
@@ -536,7 +536,8 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         const int half = (warp - 4) >> 2;
         const int th = ((warp - 4) & 3) * 32 + lane;  // thread index inside the half (0..127)
         // The combine reads d next: what of it is still in L2 then need not come back from memory.  us per block without and
-        // with: 1030 tokens 234.9 -> 234.4, 4096 432 -> 423, 8192 738 -> 727 (skewed 639 -> 630), 16384 1350 -> 1309.
+        // with, both in turn under the power limit: 1030 and 2048 tokens the same, 4096 437.9 -> 436.4, 12000 1048.7 -> 1039.8, 16384
+        // 1380 -> 1370.
         const uint64_t pol_d = l2_policy_evict_last();
         PipeState wr;
         for (int it = 0;; it++) {
@@ -752,7 +753,7 @@ cudaError_t omni_launch_dense_pair(int which, const CUtensorMap *tm_w, const CUt
     // Tiles: the fewest rounds of the pairs of SMs weighted by what an item of that many rows costs: about n/2 clocks per K step
     // of 16, and the weight rows, which come through the SM once per item however few tokens they meet.  (With a floor of
     // 96 rows in place of that the q|k|v projection of 1030 tokens took three rounds of 96 rows where two of 160
-    // do: attention half 74.8 -> 69.0 us; from 4096 tokens on the choice makes no difference.)
+    // do: attention half 74.0 -> 69.0 us, both in turn; 300, 2048 and 4096 tokens the same within 1 %.)
     const int blocks = (which == 0 ? OMNI_QKV : OMNI_H) / 256, pairs = n_sm / 2;
     long best = -1;
     for (int nt = (T + OMNI_TILE_N - 1) / OMNI_TILE_N; nt <= T; nt++) {

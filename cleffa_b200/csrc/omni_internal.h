@@ -150,7 +150,10 @@ cudaError_t omni_noalloc_assign(const int32_t *ids, int rows, int32_t *counts, i
 /* ---- router (omni_router.cu) ---- */
 cudaError_t omni_router_configure(void);
 int omni_router_tile(int T, int n_sm);     /* tokens per CTA: 32 while that gives at most one CTA per SM, else 128 */
-/* tm_x: the activations with a box of 64 K elements x nt rows (nt = omni_router_tile(T, n_sm)) */
+/* tm_x: the activations with a box of 64 K elements x nt rows (nt = omni_router_tile(T, n_sm)).
+ * segcount (may be NULL): the kernel also writes the per-segment expert counts of the counting
+ * sort for the ids it selected; omni_launch_recheck must then be given the same pointer so that
+ * the rows it re-decides move their counts */
 cudaError_t omni_launch_router_sm100(const CUtensorMap *tm_x, int nt, const CUtensorMap *tm_w, const float *bias, int T,
                                      float eps, int exact_all, float *logits, int32_t *ids, float *weights,
                                      int32_t *flag_rows, int32_t *n_flag, uint32_t *status, unsigned long long *dbg,
@@ -161,9 +164,6 @@ enum { OMNI_PART_EXPERTS = 16, OMNI_PART_SLABS = 4 };
 int omni_router_part_tile(int T, int n_sm);
 cudaError_t omni_launch_router_part(const CUtensorMap *tm_x, int nt, const CUtensorMap *tm_w, const float *bias, int T, float *logits,
                                     uint32_t *status, cudaStream_t s);
-/* segcount (may be NULL): the kernel also writes the per-segment expert counts of the counting
- * sort for the ids it selected; omni_launch_recheck must then be given the same pointer so that
- * the rows it re-decides move their counts */
 /* ---- expert products on pairs of SMs (omni_expert.cu) ---- */
 cudaError_t omni_expert_configure(void);  /* opt-in shared-memory sizes; call once per device */
 /* ctas: 2 = clusters of two CTAs driving tcgen05.mma.cta_group::2 (st.tile_n = OMNI_TILE_N), 1 = the same

@@ -290,7 +290,8 @@ bool clef_omni_read(clef_gpu *g, const char *what, void *dst, size_t bytes, char
  * "fused_gather" 0/1 (default 1: the gate/up kernel fetches its token rows through the permutation
  * itself instead of reading a copy in expert order made by a separate kernel; same results),
  * "fused_router" 0/1 (default 1: the router kernel counts the experts per segment of the counting sort,
- * so no histogram kernel runs; same results),
+ * so no histogram kernel runs, and up to 384 tokens on one GPU routing and sort are two launches; 0: the kernels of longer
+ * batches for all sizes, with a histogram kernel; same results),
  * "dependent_launch" 0/1 (default 1, process-wide: the kernels of a pass are launched so that each one's
  * prologue overlaps the tail of the one before),
  * "alloc_fail_at" N / "launch_fail_at" N (host-side fault injection, 0 = off). */
@@ -298,7 +299,8 @@ bool clef_omni_set_option(clef_gpu *g, const char *name, long value);
 /* With "profile" on every pass records stage marks on the stream without waiting.  This call
  * waits for the stream and returns the mean device milliseconds per pass over the passes
  * recorded since the previous call (at most the last 64), in the order router, permute
- * (histogram + sort + gather), gate_up, down, combine, total; then restarts the count. */
+ * (histogram + sort + gather), gate_up, down, combine, total; then restarts the count.  Up to 384 tokens the
+ * sort runs in the launch that routes and its time is in "router"; "permute" is then next to nothing. */
 bool clef_omni_profile(clef_gpu *g, float ms[6]);
 /* Arena bytes currently reserved (0 when not reserved). */
 size_t clef_omni_arena_bytes(const clef_gpu *g);

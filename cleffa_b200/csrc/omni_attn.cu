@@ -451,7 +451,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         const float *m_in = m_sh + (grp + AT_BUFS - 1) % AT_BUFS * 128 + r;
         bool alive = true;
         auto wait = [&](uint32_t b, uint32_t parity) {
-            if (alive) alive = __all_sync(0xffffffffu, xwait<2>(b, parity, ab));
+            if (alive) alive = xwait_warp<false>(b, parity, ab);
         };
         AttnItems it(tiles, n_items);
         int at = 0;                                                               // block of the sequence that the item starts with, mod 3

@@ -17,6 +17,7 @@
 #include <stdint.h>
 
 #include "omni_internal.h"
+#include "omni_pair.cuh"
 #include "omni_pdl.cuh"
 #include "omni_ptx.cuh"
 
@@ -58,6 +59,7 @@ dense_thin_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     volatile int *armed = reinterpret_cast<volatile int *>(misc + 16);
     const int warp = warp_index(), lane = threadIdx.x & 31;
     const int col0 = blockIdx.x * C::ROWS;
+    const Abort ab{abort_flag, 0u, status};
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < TN_MAX_STAGES; s++) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); armed[s] = -1; }
@@ -121,7 +123,7 @@ dense_thin_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
                     const int t = (c0 + i) * 32 + j;
                     old[i][j] = mine && c0 + i < c1 && t < T ? xr[(long)t * C::COLS] : 0.f;
                 }
-            if (__all_sync(0xffffffffu, mbar_wait(done_bar, 0, abort_flag, status))) {
+            if (xwait_warp<false>(done_bar, 0, ab)) {
                 tc_fence_after();
 #pragma unroll
                 for (int i = 0; i < 2; i++) {
@@ -137,7 +139,7 @@ dense_thin_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
                     }
                 }
             }
-        } else if (__all_sync(0xffffffffu, mbar_wait(done_bar, 0, abort_flag, status))) {
+        } else if (xwait_warp<false>(done_bar, 0, ab)) {
             tc_fence_after();
             for (int c = c0; c < c1; c++) {
                 uint32_t v[32];

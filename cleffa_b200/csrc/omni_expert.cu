@@ -348,7 +348,7 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         int off[NR], off_next[NR];
         int ready_group = -1;
         auto next_item = [&](int (&o)[NR]) -> int {
-            if (!xwait_item<CTAS>(ifull_bar(wr.stage), wr.phase, ab)) return -1;
+            if (!xwait_warp<PAIR>(ifull_bar(wr.stage), wr.phase, ab)) return -1;
             const int row0 = ring[wr.stage].row0, len = ring[wr.stage].len, expert = ring[wr.stage].expert;
             __syncwarp();
             if (lane == 0) arrive_lead(iempty_bar(wr.stage));
@@ -401,7 +401,7 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 // hand over before blocking on a free stage: the MMA thread must never wait for
                 // this loop to issue further copies
                 if (ks >= LAG) hand_over(std::integral_constant<int, LAG - 1>{});
-                ok = xwait<CTAS>(tempty_bar(p.stage), p.phase ^ 1u, ab);
+                ok = xwait_warp<false>(tempty_bar(p.stage), p.phase ^ 1u, ab);
                 if (!ok) break;
                 const uint32_t sb = tok_base + p.stage * C::T_BYTES + dst_off;
                 const char *src = src0 + ks * (BK * 2);
@@ -542,7 +542,7 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         PipeState wr;
         for (int it = 0;; it++) {
             int row0 = 0, len = 0, m = 0;
-            bool got = xwait_item<CTAS>(ifull_bar(wr.stage), wr.phase, ab);
+            bool got = xwait_warp<PAIR>(ifull_bar(wr.stage), wr.phase, ab);
             if (got) {
                 row0 = ring[wr.stage].row0; len = ring[wr.stage].len; m = ring[wr.stage].m;
                 __syncwarp();
@@ -553,7 +553,7 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             const int buf = it & 1;
             const int nchunk = (len + 31) >> 5;
             const int c_lo = half ? (nchunk + 1) >> 1 : 0, c_hi = half ? nchunk : (nchunk + 1) >> 1;
-            if (got && !stop) got = xwait<CTAS>(afull_bar(buf), (uint32_t)(it >> 1) & 1u, ab);
+            if (got && !stop) got = xwait_warp<false>(afull_bar(buf), (uint32_t)(it >> 1) & 1u, ab);
             if (!warps_meet(epi_quit + 2 * half, it, got, [&] { named_bar_sync(1 + half, 128); }) || stop) break;
             tc_fence_after();
             const uint32_t t0 = tmem_base + ((uint32_t)(q * 32) << 16) + buf * 256;

@@ -91,9 +91,10 @@ template <int MODE, int CTAS> struct XCfg {
     // 1500 to 2500 under load, so everything that is not needed elsewhere goes into the rings: with
     // a whole 64 KiB output tile in shared memory and 4 token stages the dense projections
     // waited for tokens half of the time (847 clocks per slab).
-    // Single CTAs serve short batches, which stream weights from HBM: fewer token stages there.
+    // Single CTAs serve short batches, which stream weights from HBM: fewer token stages there.  On pairs both rings are
+    // equally deep (JOINT in the kernel); the seventh weight stage that gate/up gave up for that was worth nothing.
     static constexpr int TS = CTAS == 1 ? 4 : MODE == X_OPROJ ? 7 : 6;
-    static constexpr int WS = (MODE == X_GATEUP ? 13 : MODE == X_OPROJ ? 14 : 12) - TS;
+    static constexpr int WS = CTAS == 1 ? (MODE == X_GATEUP ? 13 : 12) - TS : TS;
     static constexpr int RING_BYTES = WS * W_BYTES + TS * T_BYTES;
     static constexpr int TOTAL_BYTES = RING_BYTES + STAGE_OUT_BYTES + 1024 + 1024;
     static constexpr int ITEMS_PER_TILE = M::MT / CTAS;
@@ -163,6 +164,13 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     constexpr int KSTAGES = M::KTOT / BK;
     constexpr int WS = C::WS, TS = C::TS, MI = C::ITEMS_PER_TILE;
     constexpr bool PAIR = CTAS == 2;
+    // Rings of one depth (pairs): a stage of weights and one of tokens share their two barriers, so that the MMA warp waits and commits
+    // once per slab.  Its loop costs about 400 clocks per slab with two waits and two commits, more than the MMAs of a
+    // tile of up to ~190 rows, and 300 with one of each.  us, two rings of barriers -> one, in turn, each alone under its own
+    // clock: block of 9 tokens 97.5 -> 96.3, 128 to 1030 the same, 2048 273.3 -> 270.4, 4096 416.8 -> 406.4, 8192 715 -> 701, 16384 1301 -> 1296;
+    // attention half of 129 tokens 46.6 -> 43.3, 300 48.4 -> 45.3, 700 57.2 -> 54.5, 1030 in 6 records 64.7 -> 63.0, 4096 in 8 204.8 -> 202.9.
+    // (Two slabs per turn of the loop, or a look at the next slab's barrier ahead of the MMAs: up to 2 % slower, and no change.)
+    constexpr bool JOINT = WS == TS;
 
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -172,8 +180,8 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     const uint32_t bar_base = smem_base + C::RING_BYTES + C::STAGE_OUT_BYTES;
     auto wfull_bar = [&](int s) { return bar_base + 8u * s; };
     auto wempty_bar = [&](int s) { return bar_base + 8u * (WS + s); };
-    auto tfull_bar = [&](int s) { return bar_base + 8u * (2 * WS + s); };
-    auto tempty_bar = [&](int s) { return bar_base + 8u * (2 * WS + TS + s); };
+    auto tfull_bar = [&](int s) { return bar_base + 8u * (JOINT ? s : 2 * WS + s); };
+    auto tempty_bar = [&](int s) { return bar_base + 8u * (JOINT ? WS + s : 2 * WS + TS + s); };
     auto afull_bar = [&](int b) { return bar_base + 8u * (2 * WS + 2 * TS + b); };
     auto aempty_bar = [&](int b) { return bar_base + 8u * (2 * WS + 2 * TS + 2 + b); };
     const uint32_t drain_bar = bar_base + 8u * (2 * WS + 2 * TS + 4);
@@ -203,8 +211,10 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
 
     if (threadIdx.x == 0) {
         const int tp = gathering ? X_GATHER_THREADS / 32 : 1;                       // arrivals of a CTA's token producer per item
-        for (int s = 0; s < WS; s++) { mbar_init(wfull_bar(s), 1); mbar_init(wempty_bar(s), 1); }
-        for (int s = 0; s < TS; s++) { mbar_init(tfull_bar(s), gathering ? X_GATHER_THREADS * CTAS : 1); mbar_init(tempty_bar(s), 1); }
+        const int tok_arrivals = gathering ? X_GATHER_THREADS * CTAS : 1;
+        for (int s = 0; s < WS; s++) { mbar_init(wfull_bar(s), JOINT ? 1 + tok_arrivals : 1); mbar_init(wempty_bar(s), 1); }
+        if (!JOINT)
+            for (int s = 0; s < TS; s++) { mbar_init(tfull_bar(s), tok_arrivals); mbar_init(tempty_bar(s), 1); }
         for (int s = 0; s < 10; s++) { armed_w[s] = -1; armed_t[s] = -1; }
         for (int b = 0; b < 2; b++) { mbar_init(afull_bar(b), 1); mbar_init(aempty_bar(b), X_EPI_WARPS * CTAS); }
         mbar_init(drain_bar, 1);
@@ -489,7 +499,7 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             tc_fence_after();
             const uint32_t d0 = tmem_base + buf * 256;
             for (int ks = 0; ks < KSTAGES; ks++) {
-                ok = xwait_warp<false>(wfull_bar(pw.stage), pw.phase, ab) && xwait_warp<false>(tfull_bar(pt.stage), pt.phase, ab);
+                ok = xwait_warp<false>(wfull_bar(pw.stage), pw.phase, ab) && (JOINT || xwait_warp<false>(tfull_bar(pt.stage), pt.phase, ab));
                 if (!ok) break;
                 tc_fence_after();
                 if (elect_one()) {
@@ -497,13 +507,13 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                     const uint64_t db = smem_desc_sw128(tok_base + pt.stage * C::T_BYTES);
 #pragma unroll
                     for (int k = 0; k < BK / 16; k++) xmma<CTAS>(d0, da + 2u * k, db + 2u * k, idesc, (ks | k) ? 1u : 0u);
-                    xcommit<CTAS>(wempty_bar(pw.stage));     // both stages are free (in both CTAs) once these MMAs have read them
-                    xcommit<CTAS>(tempty_bar(pt.stage));
+                    xcommit<CTAS>(wempty_bar(pw.stage));     // what was staged is free (in both CTAs) once these MMAs have read it
+                    if (!JOINT) xcommit<CTAS>(tempty_bar(pt.stage));
                     if (ks == KSTAGES - 1) xcommit<CTAS>(afull_bar(buf));        // accumulator complete, in both CTAs
                 }
                 __syncwarp();
                 pw.advance(WS);
-                pt.advance(TS);
+                if (JOINT) pt = pw; else pt.advance(TS);
             }
         }
         // Whatever happened, wait (bounded) until every MMA issued by this warp's elected thread has

@@ -700,7 +700,7 @@ static bool run_experts(clef_gpu *g, const omni_layer *L, const void *xn, const 
     }
     stage_mark(g, 4);
     if (g->wait_residual && !launched(g, "residual upload join", cudaStreamWaitEvent(g->stream, g->residual_uploaded, 0))) return false;
-    if (!launched(g, "combine", omni_launch_combine(s->d, ids, weights, s->sort.slots, x, rows, g->stream))) return false;
+    if (!launched(g, "combine", omni_launch_combine(s->d, ids, weights, s->sort.slots, x, rows, 1, g->stream))) return false;
     stage_mark(g, 5);
     return true;
 }
@@ -750,7 +750,7 @@ static bool run_experts_ep(clef_gpu *g, const omni_layer *L, const void *xn, con
     stage_mark(g, 4);
     if (!launched(g, "expert-parallel barrier", omni_launch_ep_barrier(pe, ++g->ep.epoch, s->status, g->ep.wait_ns, g->stream))) return false;
     if (g->wait_residual && !launched(g, "residual upload join", cudaStreamWaitEvent(g->stream, g->residual_uploaded, 0))) return false;
-    if (!launched(g, "combine", omni_launch_combine(g->ep.dret, ids, weights, s->sort.slots, x, rows, g->stream))) return false;
+    if (!launched(g, "combine", omni_launch_combine(g->ep.dret, ids, weights, s->sort.slots, x, rows, 0, g->stream))) return false;
     stage_mark(g, 5);
     return true;
 }

@@ -133,7 +133,8 @@ cudaError_t omni_launch_assign(const int32_t *ids, int rows, omni_sort_state st,
 cudaError_t omni_launch_rmsnorm(const float *x, const float *w, float eps, int rows, void *xn, cudaStream_t s);
 cudaError_t omni_launch_gather(const void *xn, const int32_t *rowmap, int rows8, void *xg, cudaStream_t s);
 cudaError_t omni_launch_combine(const void *d, const int32_t *ids, const float *weights, const int32_t *slots,
-                                float *x, int T, cudaStream_t s);
+                                float *x, int T, int dead, cudaStream_t s);
+/* dead: d is not needed after this and may be dropped from L2 unwritten */
 cudaError_t omni_launch_gateup_simple(const void *xg, const void *gate_up, const int32_t *offsets, int rows8, void *h,
                                       cudaStream_t s);
 cudaError_t omni_launch_down_simple(const void *h, const void *down, const int32_t *offsets, int rows8, void *d,

@@ -327,6 +327,24 @@ def test_config4_T8192_zipf_skew_sampled(backend, weights0):
     permutation_properties(got, T)
 
 
+@pytest.mark.parametrize("T", [447, 448, 449, 2559, 2560, 2561])
+def test_expert_rows_dropped_from_l2_were_all_read(bound0, T):
+    """From 448 to 2560 tokens the combine discards the experts' rows it has read.  A token's result does not depend on the batch, so the
+    first rows are those of a batch without that; passes follow one another on the same memory."""
+    x = orc.make_activations(41, T)
+    res = torch.randn(T, 2048, generator=torch.Generator().manual_seed(2))
+    n = 300
+    want = run_block(bound0, 0, x[:n], residual=res[:n])["out"]
+    first = run_block(bound0, 0, x, residual=res)["out"]
+    xd, outs = x.cuda(), [res.cuda() for _ in range(3)]
+    torch.cuda.synchronize()                      # the library's passes run on a stream of their own
+    bound0.begin()
+    for out in outs:
+        bound0.encode_moe(0, xd, out)
+    bound0.complete()
+    assert torch.equal(first[:n], want) and all(torch.equal(out.cpu(), first) for out in outs)
+
+
 @pytest.mark.parametrize("T", [300, 1537, 3000])
 def test_forward_host_equals_device_path(bound0, T):
     # above 1536 tokens the host call cuts the batch into pieces whose copies and kernels overlap

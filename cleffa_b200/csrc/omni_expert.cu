@@ -91,11 +91,8 @@ template <int MODE, int CTAS> struct XCfg {
     // 1500 to 2500 under load, so everything that is not needed elsewhere goes into the rings: with
     // a whole 64 KiB output tile in shared memory and 4 token stages the dense projections
     // waited for tokens half of the time (847 clocks per slab).
-    // Single CTAs serve short batches, which stream weights from HBM: fewer token stages there.  On pairs both rings are
-    // equally deep (JOINT in the kernel); the seventh weight stage that gate/up gave up for that was worth nothing.
-    static constexpr int TS = CTAS == 1 ? 4 : MODE == X_OPROJ ? 7 : 6;
-    static constexpr int WS = CTAS == 1 ? (MODE == X_GATEUP ? 13 : 12) - TS : TS;
-    static constexpr int RING_BYTES = WS * W_BYTES + TS * T_BYTES;
+    static constexpr int STAGES = MODE == X_OPROJ ? 7 : 6;
+    static constexpr int RING_BYTES = STAGES * (W_BYTES + T_BYTES);
     static constexpr int TOTAL_BYTES = RING_BYTES + STAGE_OUT_BYTES + 1024 + 1024;
     static constexpr int ITEMS_PER_TILE = M::MT / CTAS;
 };
@@ -162,32 +159,29 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     using C = XCfg<MODE, CTAS>;
     using M = XMode<MODE>;
     constexpr int KSTAGES = M::KTOT / BK;
-    constexpr int WS = C::WS, TS = C::TS, MI = C::ITEMS_PER_TILE;
+    constexpr int STAGES = C::STAGES, MI = C::ITEMS_PER_TILE;
     constexpr bool PAIR = CTAS == 2;
-    // Rings of one depth (pairs): a stage of weights and one of tokens share their two barriers, so that the MMA warp waits and commits
-    // once per slab.  Its loop costs about 400 clocks per slab with two waits and two commits, more than the MMAs of a
-    // tile of up to ~190 rows, and 300 with one of each.  us, two rings of barriers -> one, in turn, each alone under its own
-    // clock: block of 9 tokens 97.5 -> 96.3, 128 to 1030 the same, 2048 273.3 -> 270.4, 4096 416.8 -> 406.4, 8192 715 -> 701, 16384 1301 -> 1296;
-    // attention half of 129 tokens 46.6 -> 43.3, 300 48.4 -> 45.3, 700 57.2 -> 54.5, 1030 in 6 records 64.7 -> 63.0, 4096 in 8 204.8 -> 202.9.
-    // (Two slabs per turn of the loop, or a look at the next slab's barrier ahead of the MMAs: up to 2 % slower, and no change.)
-    constexpr bool JOINT = WS == TS;
-
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *const smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
-    const uint32_t tok_base = smem_base + WS * C::W_BYTES;
+    const uint32_t tok_base = smem_base + STAGES * C::W_BYTES;
     uint8_t *const out_tile = smem_gen + C::RING_BYTES; // 4 x [32][OUTC] bf16: two chunks per epilogue half, none for the output projection
     const uint32_t bar_base = smem_base + C::RING_BYTES + C::STAGE_OUT_BYTES;
-    auto wfull_bar = [&](int s) { return bar_base + 8u * s; };
-    auto wempty_bar = [&](int s) { return bar_base + 8u * (WS + s); };
-    auto tfull_bar = [&](int s) { return bar_base + 8u * (JOINT ? s : 2 * WS + s); };
-    auto tempty_bar = [&](int s) { return bar_base + 8u * (JOINT ? WS + s : 2 * WS + TS + s); };
-    auto afull_bar = [&](int b) { return bar_base + 8u * (2 * WS + 2 * TS + b); };
-    auto aempty_bar = [&](int b) { return bar_base + 8u * (2 * WS + 2 * TS + 2 + b); };
-    const uint32_t drain_bar = bar_base + 8u * (2 * WS + 2 * TS + 4);
-    auto ifull_bar = [&](int r) { return bar_base + 8u * (2 * WS + 2 * TS + 5 + r); };
-    auto iempty_bar = [&](int r) { return bar_base + 8u * (2 * WS + 2 * TS + 5 + X_RING + r); };
-    constexpr int N_BARS = 2 * WS + 2 * TS + 5 + 2 * X_RING;
+    // A stage of weights and one of tokens share their two barriers, so that the MMA warp waits and commits
+    // once per slab.  Its loop costs about 400 clocks per slab with two waits and two commits, more than the MMAs of a
+    // tile of up to ~190 rows, and 300 with one of each.  us, two rings of barriers -> one, in turn, each alone under its own
+    // clock: block of 1 token 33.9 -> 32.0 (single CTAs, whose nine and eight weight stages became six), 2 47.2 -> 46.4, 9 97.5 -> 96.3, 128 to
+    // 1030 the same, 2048 273.3 -> 270.4, 4096 416.8 -> 406.4, 8192 715 -> 701, 16384 1301 -> 1296; attention half of 129 tokens 46.6 -> 43.3,
+    // 300 48.4 -> 45.3, 700 57.2 -> 54.5, 1030 in 6 records 64.7 -> 63.0, 4096 in 8 204.8 -> 202.9.
+    // (Two slabs per turn of the loop, or a look at the next slab's barrier ahead of the MMAs: up to 2 % slower, and no change.)
+    auto full_bar = [&](int s) { return bar_base + 8u * s; };
+    auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
+    auto afull_bar = [&](int b) { return bar_base + 8u * (2 * STAGES + b); };
+    auto aempty_bar = [&](int b) { return bar_base + 8u * (2 * STAGES + 2 + b); };
+    const uint32_t drain_bar = bar_base + 8u * (2 * STAGES + 4);
+    auto ifull_bar = [&](int r) { return bar_base + 8u * (2 * STAGES + 5 + r); };
+    auto iempty_bar = [&](int r) { return bar_base + 8u * (2 * STAGES + 5 + X_RING + r); };
+    constexpr int N_BARS = 2 * STAGES + 5 + 2 * X_RING;
     constexpr int MISC_OFF = (N_BARS * 8 + 15) & ~15;            // the item ring is written with 16-byte stores
     static_assert(MISC_OFF + 16 + 80 + X_RING * 16 <= 1024, "barrier block");
     uint8_t *misc = smem_gen + C::RING_BYTES + C::STAGE_OUT_BYTES + MISC_OFF;
@@ -212,9 +206,7 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     if (threadIdx.x == 0) {
         const int tp = gathering ? X_GATHER_THREADS / 32 : 1;                       // arrivals of a CTA's token producer per item
         const int tok_arrivals = gathering ? X_GATHER_THREADS * CTAS : 1;
-        for (int s = 0; s < WS; s++) { mbar_init(wfull_bar(s), JOINT ? 1 + tok_arrivals : 1); mbar_init(wempty_bar(s), 1); }
-        if (!JOINT)
-            for (int s = 0; s < TS; s++) { mbar_init(tfull_bar(s), tok_arrivals); mbar_init(tempty_bar(s), 1); }
+        for (int s = 0; s < STAGES; s++) { mbar_init(full_bar(s), 1 + tok_arrivals); mbar_init(empty_bar(s), 1); }
         for (int s = 0; s < 10; s++) { armed_w[s] = -1; armed_t[s] = -1; }
         for (int b = 0; b < 2; b++) { mbar_init(afull_bar(b), 1); mbar_init(aempty_bar(b), X_EPI_WARPS * CTAS); }
         mbar_init(drain_bar, 1);
@@ -327,16 +319,16 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             wr.advance(X_RING);
             if (len < 0) break;
             for (int ks = 0; ks < KSTAGES; ks++) {
-                ok = xwait_warp<false>(wempty_bar(p.stage), p.phase ^ 1u, ab);
+                ok = xwait_warp<false>(empty_bar(p.stage), p.phase ^ 1u, ab);
                 if (!ok) break;
                 if (elect_one()) {
                     if (leader) {
                         armed_w[p.stage] = (int)p.phase;
-                        mbar_expect_tx(wfull_bar(p.stage), CTAS * C::W_BYTES);       // this CTA's tile and the peer's
+                        mbar_expect_tx(full_bar(p.stage), CTAS * C::W_BYTES);       // this CTA's tile and the peer's
                     }
-                    load_weights(smem_base + p.stage * C::W_BYTES, expert, m, ks, lead(wfull_bar(p.stage)), pol_w);
+                    load_weights(smem_base + p.stage * C::W_BYTES, expert, m, ks, lead(full_bar(p.stage)), pol_w);
                 }
-                p.advance(WS);
+                p.advance(STAGES);
             }
         }
     } else if (MODE == X_GATEUP && gathering && warp >= 12 && warp < 16) {
@@ -347,7 +339,7 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         // inside its 8-row group).  A stage is handed to the MMA thread LAG stages after it was
         // issued, once the copies have landed and are ordered before the tensor core's reads.
         constexpr int LAG = CTAS == 2 ? 3 : 2;
-        static_assert(TS > LAG, "token ring too short for the copy lag");
+        static_assert(STAGES > LAG, "token ring too short for the copy lag");
         constexpr int RSTEP = X_GATHER_THREADS / 8, NR = C::TOK_ROWS / RSTEP;
         const uint64_t pol_t = l2_policy_evict_last();
         const int gt = threadIdx.x - X_THREADS;
@@ -401,8 +393,8 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         auto hand_over = [&](auto left) {
             cp_async_wait<decltype(left)::value>();
             fence_proxy_async_smem();
-            arrive_lead(tfull_bar(pend.stage));
-            pend.advance(TS);
+            arrive_lead(full_bar(pend.stage));
+            pend.advance(STAGES);
         };
         int len = next_item(off);
         while (len >= 0) {
@@ -411,7 +403,7 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 // hand over before blocking on a free stage: the MMA thread must never wait for
                 // this loop to issue further copies
                 if (ks >= LAG) hand_over(std::integral_constant<int, LAG - 1>{});
-                ok = xwait_warp<false>(tempty_bar(p.stage), p.phase ^ 1u, ab);
+                ok = xwait_warp<false>(empty_bar(p.stage), p.phase ^ 1u, ab);
                 if (!ok) break;
                 const uint32_t sb = tok_base + p.stage * C::T_BYTES + dst_off;
                 const char *src = src0 + ks * (BK * 2);
@@ -419,7 +411,7 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
                 for (int i = 0; i < NR; i++)
                     if (off[i] >= 0) cp_async16(sb + i * (RSTEP * 128), src + off[i], pol_t);
                 cp_async_commit();
-                p.advance(TS);
+                p.advance(STAGES);
             }
             if (!ok) break;
             // the next item's row indices travel while the last stages of this one land
@@ -467,22 +459,22 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             const int bi = tok_box_index(share);
             const uint32_t bytes = tok_box_bytes(bi);
             for (int ks = 0; ks < KSTAGES; ks++) {
-                ok = xwait_warp<false>(tempty_bar(p.stage), p.phase ^ 1u, ab);
+                ok = xwait_warp<false>(empty_bar(p.stage), p.phase ^ 1u, ab);
                 if (!ok) break;
                 if (elect_one()) {
                     if (leader) {
                         armed_t[p.stage] = (int)p.phase;
-                        mbar_expect_tx(tfull_bar(p.stage), CTAS * bytes);
+                        mbar_expect_tx(full_bar(p.stage), CTAS * bytes);
                     }
                     xtma_2d<CTAS>(tok_base + p.stage * C::T_BYTES, &tm_tok.m[bi], ks * BK, row0 + (int)rank * share,
-                                  lead(tfull_bar(p.stage)), pol_t);
+                                  lead(full_bar(p.stage)), pol_t);
                 }
-                p.advance(TS);
+                p.advance(STAGES);
             }
         }
     } else if (warp == 1 && leader) {
         // ---------------------------------------------------------- MMA issuer (first CTA of the pair)
-        PipeState pw, pt, wr;
+        PipeState p, wr;
         bool ok = true;
         for (int it = 0; ok; it++) {
             ok = xwait_warp<PAIR>(ifull_bar(wr.stage), wr.phase, ab);
@@ -499,21 +491,19 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             tc_fence_after();
             const uint32_t d0 = tmem_base + buf * 256;
             for (int ks = 0; ks < KSTAGES; ks++) {
-                ok = xwait_warp<false>(wfull_bar(pw.stage), pw.phase, ab) && (JOINT || xwait_warp<false>(tfull_bar(pt.stage), pt.phase, ab));
+                ok = xwait_warp<false>(full_bar(p.stage), p.phase, ab);
                 if (!ok) break;
                 tc_fence_after();
                 if (elect_one()) {
-                    const uint64_t da = smem_desc_sw128(smem_base + pw.stage * C::W_BYTES);
-                    const uint64_t db = smem_desc_sw128(tok_base + pt.stage * C::T_BYTES);
+                    const uint64_t da = smem_desc_sw128(smem_base + p.stage * C::W_BYTES);
+                    const uint64_t db = smem_desc_sw128(tok_base + p.stage * C::T_BYTES);
 #pragma unroll
                     for (int k = 0; k < BK / 16; k++) xmma<CTAS>(d0, da + 2u * k, db + 2u * k, idesc, (ks | k) ? 1u : 0u);
-                    xcommit<CTAS>(wempty_bar(pw.stage));     // what was staged is free (in both CTAs) once these MMAs have read it
-                    if (!JOINT) xcommit<CTAS>(tempty_bar(pt.stage));
+                    xcommit<CTAS>(empty_bar(p.stage));     // what was staged is free (in both CTAs) once these MMAs have read it
                     if (ks == KSTAGES - 1) xcommit<CTAS>(afull_bar(buf));        // accumulator complete, in both CTAs
                 }
                 __syncwarp();
-                pw.advance(WS);
-                if (JOINT) pt = pw; else pt.advance(TS);
+                p.advance(STAGES);
             }
         }
         // Whatever happened, wait (bounded) until every MMA issued by this warp's elected thread has
@@ -656,10 +646,10 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     __syncthreads();
     if (*abort_flag && threadIdx.x == 0) {
         // a wait ran out: give copies already in flight a bounded chance to land
-        for (int s = 0; s < WS + TS; s++) {
-            const int par = s < WS ? armed_w[s] : armed_t[s - WS];
+        for (int s = 0; s < 2 * STAGES; s++) {
+            const int par = s < STAGES ? armed_w[s] : armed_t[s - STAGES];
             if (par < 0) continue;
-            const uint32_t bar = s < WS ? wfull_bar(s) : tfull_bar(s - WS);
+            const uint32_t bar = full_bar(s % STAGES);
             const uint64_t t0 = globaltimer_ns();
             while (!mbar_try_wait(bar, (uint32_t)par) && globaltimer_ns() - t0 < 50000000ull) {}
         }

@@ -15,6 +15,7 @@
 #include <stdint.h>
 
 #include "omni_internal.h"
+#include "omni_land.cuh"
 #include "omni_pair.cuh"
 #include "omni_pdl.cuh"
 #include "omni_ptx.cuh"
@@ -614,14 +615,11 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     tc_fence_before();
     __syncthreads();
     if (*abort_flag && threadIdx.x == 0) {
-        // a wait ran out: give loads already in flight a bounded chance to land
-        for (int s = 0; s < 2 + 2 * AT_KV_STAGES; s++) {
-            const int par = armed[s];
-            if (par < 0) continue;
-            const uint32_t b = s < 2 ? q_full(s) : s < 2 + AT_KV_STAGES ? k_full(s - 2) : v_full(s - 2 - AT_KV_STAGES);
-            const uint64_t t0 = globaltimer_ns();
-            while (!mbar_try_wait(b, (uint32_t)par) && globaltimer_ns() - t0 < 50000000ull) {}
-        }
+        // a wait ran out; both CTAs' loads are announced here, in the first one
+        copies_land(armed, 2 + 2 * AT_KV_STAGES, [&](int i, int parity) {
+            const uint32_t b = i < 2 ? q_full(i) : i < 2 + AT_KV_STAGES ? k_full(i - 2) : v_full(i - 2 - AT_KV_STAGES);
+            return mbar_try_wait(b, (uint32_t)parity) != 0;
+        }, globaltimer_ns, LAND_LIMIT_NS);
     }
     // neither CTA may leave while the other's MMAs can still read its shared memory
     cluster_sync_all();

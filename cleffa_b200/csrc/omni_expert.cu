@@ -35,6 +35,7 @@
 
 #include "omni_internal.h"
 #include "omni_ep_dev.cuh"
+#include "omni_land.cuh"
 #include "omni_meet.cuh"
 #include "omni_pair.cuh"
 #include "omni_pdl.cuh"
@@ -106,6 +107,7 @@ constexpr int X_COPY_THREADS = 128; // with COPY: warps 16..19 move this rank's 
 constexpr int X_EPI_WARPS = 8;
 template <int MODE, bool COPY> constexpr int x_threads() { return X_THREADS + (MODE == X_GATEUP ? X_GATHER_THREADS : 0) + (COPY ? X_COPY_THREADS : 0); }
 constexpr int X_RING = 4;
+constexpr int X_MAX_STAGES = 8;     // of the rings; 64 bytes of announced parities
 
 struct XArgs {
     const omni_ttile *ttiles;
@@ -183,16 +185,17 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     auto iempty_bar = [&](int r) { return bar_base + 8u * (2 * STAGES + 5 + X_RING + r); };
     constexpr int N_BARS = 2 * STAGES + 5 + 2 * X_RING;
     constexpr int MISC_OFF = (N_BARS * 8 + 15) & ~15;            // the item ring is written with 16-byte stores
-    static_assert(MISC_OFF + 16 + 80 + X_RING * 16 <= 1024, "barrier block");
+    constexpr int RING_OFF = 16 + 2 * X_MAX_STAGES * 4;
+    static_assert(STAGES <= X_MAX_STAGES && RING_OFF % 16 == 0 && MISC_OFF + RING_OFF + X_RING * 16 <= 1024, "barrier block");
     uint8_t *misc = smem_gen + C::RING_BYTES + C::STAGE_OUT_BYTES + MISC_OFF;
     const uint32_t misc_u32 = bar_base + MISC_OFF;
     volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(misc);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(misc + 4);
     volatile short *epi_quit = reinterpret_cast<volatile short *>(misc + 8);    // [half][item parity] a warp of this epilogue half gave up
-    volatile int *armed_w = reinterpret_cast<volatile int *>(misc + 16);        // [10] parity armed per weight stage, -1 none
-    volatile int *armed_t = reinterpret_cast<volatile int *>(misc + 16 + 40);   // [10] same for the token ring
-    volatile WorkSlotX *ring = reinterpret_cast<volatile WorkSlotX *>(misc + 16 + 80);
-    const uint32_t ring_u32 = misc_u32 + 16 + 80;
+    volatile int *armed_w = reinterpret_cast<volatile int *>(misc + 16);        // [STAGES] parity with which weights were announced last, -1 none
+    volatile int *armed_t = armed_w + STAGES;                                   // [STAGES] the same for tokens that come by TMA
+    volatile WorkSlotX *ring = reinterpret_cast<volatile WorkSlotX *>(misc + RING_OFF);
+    const uint32_t ring_u32 = misc_u32 + RING_OFF;
 
     const int warp = warp_index(), lane = threadIdx.x & 31;
     const uint32_t rank = PAIR ? __shfl_sync(0xffffffffu, cluster_ctarank(), 0) : 0u;      // uniform for the compiler, like the warp index
@@ -207,7 +210,7 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
         const int tp = gathering ? X_GATHER_THREADS / 32 : 1;                       // arrivals of a CTA's token producer per item
         const int tok_arrivals = gathering ? X_GATHER_THREADS * CTAS : 1;
         for (int s = 0; s < STAGES; s++) { mbar_init(full_bar(s), 1 + tok_arrivals); mbar_init(empty_bar(s), 1); }
-        for (int s = 0; s < 10; s++) { armed_w[s] = -1; armed_t[s] = -1; }
+        for (int s = 0; s < 2 * STAGES; s++) armed_w[s] = -1;
         for (int b = 0; b < 2; b++) { mbar_init(afull_bar(b), 1); mbar_init(aempty_bar(b), X_EPI_WARPS * CTAS); }
         mbar_init(drain_bar, 1);
         // consumers of an item: in either CTA the weight producer, the token producer(s) and the epilogue
@@ -645,14 +648,9 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     tc_fence_before();
     __syncthreads();
     if (*abort_flag && threadIdx.x == 0) {
-        // a wait ran out: give copies already in flight a bounded chance to land
-        for (int s = 0; s < 2 * STAGES; s++) {
-            const int par = s < STAGES ? armed_w[s] : armed_t[s - STAGES];
-            if (par < 0) continue;
-            const uint32_t bar = full_bar(s % STAGES);
-            const uint64_t t0 = globaltimer_ns();
-            while (!mbar_try_wait(bar, (uint32_t)par) && globaltimer_ns() - t0 < 50000000ull) {}
-        }
+        // a wait ran out; both CTAs' copies are announced here, in the first one
+        copies_land(armed_w, 2 * STAGES, [&](int i, int parity) { return mbar_try_wait(full_bar(i % STAGES), (uint32_t)parity) != 0; },
+                    globaltimer_ns, LAND_LIMIT_NS);
     }
     // neither CTA of a pair may leave while the other's MMAs can still read its shared memory
     if (PAIR) cluster_sync_all(); else __syncthreads();

@@ -615,11 +615,11 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     tc_fence_before();
     __syncthreads();
     if (*abort_flag && threadIdx.x == 0) {
-        // a wait ran out; both CTAs' loads are announced here, in the first one
+        // a wait ran out; the first CTA knows what both announced
         copies_land(armed, 2 + 2 * AT_KV_STAGES, [&](int i, int parity) {
             const uint32_t b = i < 2 ? q_full(i) : i < 2 + AT_KV_STAGES ? k_full(i - 2) : v_full(i - 2 - AT_KV_STAGES);
             return mbar_try_wait(b, (uint32_t)parity) != 0;
-        }, globaltimer_ns, LAND_LIMIT_NS);
+        }, globaltimer_ns, LAND_LIMIT_NS, LAND_SETTLE_NS);
     }
     // neither CTA may leave while the other's MMAs can still read its shared memory
     cluster_sync_all();

@@ -648,9 +648,9 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     tc_fence_before();
     __syncthreads();
     if (*abort_flag && threadIdx.x == 0) {
-        // a wait ran out; both CTAs' copies are announced here, in the first one
+        // a wait ran out; of a pair the first CTA knows what both announced
         copies_land(armed_w, 2 * STAGES, [&](int i, int parity) { return mbar_try_wait(full_bar(i % STAGES), (uint32_t)parity) != 0; },
-                    globaltimer_ns, LAND_LIMIT_NS);
+                    globaltimer_ns, LAND_LIMIT_NS, LAND_SETTLE_NS);
     }
     // neither CTA of a pair may leave while the other's MMAs can still read its shared memory
     if (PAIR) cluster_sync_all(); else __syncthreads();

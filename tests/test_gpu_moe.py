@@ -329,20 +329,26 @@ def test_config4_T8192_zipf_skew_sampled(backend, weights0):
 
 @pytest.mark.parametrize("T", [447, 448, 449, 2559, 2560, 2561])
 def test_expert_rows_dropped_from_l2_were_all_read(bound0, T):
-    """From 448 to 2560 tokens the combine discards the experts' rows it has read.  A token's result does not depend on the batch, so the
-    first rows are those of a batch without that; passes follow one another on the same memory."""
-    x = orc.make_activations(41, T)
-    res = torch.randn(T, 2048, generator=torch.Generator().manual_seed(2))
-    n = 300
-    want = run_block(bound0, 0, x[:n], residual=res[:n])["out"]
-    first = run_block(bound0, 0, x, residual=res)["out"]
-    xd, outs = x.cuda(), [res.cuda() for _ in range(3)]
+    """From 448 to 2560 tokens the combine discards the experts' rows it has read.  A token's result does not depend on the batch, so all rows
+    are those of batches without that, of 400 tokens at most.  Two batches take turns on the same memory: a row that was dropped too early, or after the
+    next pass had written it, is another batch's row then, or the poison that the passes begin with."""
+    batches = [(orc.make_activations(seed, T), torch.randn(T, 2048, generator=torch.Generator().manual_seed(seed))) for seed in (41, 42)]
+    cuts = list(range(0, T, 400)) + [T]
+    want = [torch.cat([run_block(bound0, 0, x[lo:hi], residual=res[lo:hi])["out"] for lo, hi in zip(cuts, cuts[1:])]) for x, res in batches]
+    assert not torch.equal(want[0], want[1])
+    xs = [x.cuda() for x, _ in batches]
+    outs = [batches[i % 2][1].cuda() for i in range(5)]
     torch.cuda.synchronize()                      # the library's passes run on a stream of their own
-    bound0.begin()
-    for out in outs:
-        bound0.encode_moe(0, xd, out)
-    bound0.complete()
-    assert torch.equal(first[:n], want) and all(torch.equal(out.cpu(), first) for out in outs)
+    bound0.set_option("debug_poison", 1)
+    try:
+        bound0.begin()
+        for i, out in enumerate(outs):
+            bound0.encode_moe(0, xs[i % 2], out)
+        bound0.complete()
+    finally:
+        bound0.set_option("debug_poison", 0)
+    for i, out in enumerate(outs):
+        assert torch.equal(out.cpu(), want[i % 2]), i
 
 
 @pytest.mark.parametrize("T", [300, 1537, 3000])

@@ -170,11 +170,15 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     uint8_t *const out_tile = smem_gen + C::RING_BYTES; // 4 x [32][OUTC] bf16: two chunks per epilogue half, none for the output projection
     const uint32_t bar_base = smem_base + C::RING_BYTES + C::STAGE_OUT_BYTES;
     // A stage of weights and one of tokens share their two barriers, so that the MMA warp waits and commits
-    // once per slab.  Its loop costs about 400 clocks per slab with two waits and two commits, more than the MMAs of a
-    // tile of up to ~190 rows, and 300 with one of each.  us, two rings of barriers -> one, in turn, each alone under its own
-    // clock: block of 1 token 33.9 -> 32.0 (single CTAs, whose nine and eight weight stages became six), 2 47.2 -> 46.4, 9 97.5 -> 96.3, 128 to
-    // 1030 the same, 2048 273.3 -> 270.4, 4096 416.8 -> 406.4, 8192 715 -> 701, 16384 1301 -> 1296; attention half of 129 tokens 46.6 -> 43.3,
-    // 300 48.4 -> 45.3, 700 57.2 -> 54.5, 1030 in 6 records 64.7 -> 63.0, 4096 in 8 204.8 -> 202.9.
+    // once per slab.  Its loop costs about 400 clocks per slab with two waits (70 to 90 each, also when the phase is complete) and two
+    // commits, more than the MMAs of a tile of up to ~190 rows.  us, two rings of barriers -> one, in turn, each alone under its own
+    // clock, on two boxes: block of 9 tokens 97.5 -> 96.3 and 98.6 -> 97.4, 128 and 1030 the same, 2048 273.3 -> 270.4 and 283.4 -> 282.7, 4096
+    // 416.8 -> 406.4 and 445 -> 436, 8192 715 -> 701 and 770 -> 759, 16384 1301 -> 1296 and 1368 -> 1354; attention half of 37 tokens the same, 129
+    // 46.6 -> 43.3 and 45.8 -> 43.7, 300 48.4 -> 45.3 and 47.6 -> 45.3, 700 57.2 -> 54.5 and 56.4 -> 54.4, 1030 in 6 records 64.7 -> 63.0 and 64.6 -> 62.7,
+    // 4096 in 8 204.8 -> 202.9 and the same.
+    // On single CTAs nine (gate/up) and eight (down) stages of weights and four of tokens became six of both.  A layer whose experts stay in
+    // L2, and 16 layers in turn (1.2 GB of touched experts, from memory): 1 token 35.4 -> 33.3 and 35.8 -> 34.1, 2 tokens 47.2 -> 46.7 and
+    // 49.9 -> 48.8; longer batches on single CTAs, 9 tokens 111.7 -> 106.6, 128 200.1 -> 199.6, 1030 246 -> 238, 4096 578 -> 548.
     // (Two slabs per turn of the loop, or a look at the next slab's barrier ahead of the MMAs: up to 2 % slower, and no change.)
     auto full_bar = [&](int s) { return bar_base + 8u * s; };
     auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };

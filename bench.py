@@ -52,7 +52,7 @@ KERNELS_EP = 9            # ... plus owner buckets, plan and one barrier; the ex
 METRIC = "MoE-layer prefill tokens/sec at T=4096"
 # dram__bytes_read.sum + dram__bytes_write.sum of one gate/up launch at T=4096, from the ncu
 # capture summarised in profiles/ncu_moe_layer_T4096.md
-GATEUP_DRAM_TRAFFIC_T4096 = 850_602_240 + 11_229_696
+GATEUP_DRAM_TRAFFIC_T4096 = 863_890_176 + 12_117_248
 
 
 def kernel_launches(tokens, world, n_layers, norm):

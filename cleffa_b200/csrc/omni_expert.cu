@@ -172,7 +172,7 @@ expert_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     // A stage of weights and one of tokens share their two barriers, so that the MMA warp waits and commits
     // once per slab.  Its loop costs about 400 clocks per slab with two waits (70 to 90 each, also when the phase is complete) and two
     // commits, more than the MMAs of a tile of up to ~190 rows.  us, two rings of barriers -> one, in turn, each alone under its own
-    // clock, on two boxes: block of 9 tokens 97.5 -> 96.3 and 98.6 -> 97.4, 128 and 1030 the same, 2048 273.3 -> 270.4 and 283.4 -> 282.7, 4096
+    // clock, on two GPUs: block of 9 tokens 97.5 -> 96.3 and 98.6 -> 97.4, 128 and 1030 the same, 2048 273.3 -> 270.4 and 283.4 -> 282.7, 4096
     // 416.8 -> 406.4 and 445 -> 436, 8192 715 -> 701 and 770 -> 759, 16384 1301 -> 1296 and 1368 -> 1354; attention half of 37 tokens the same, 129
     // 46.6 -> 43.3 and 45.8 -> 43.7, 300 48.4 -> 45.3 and 47.6 -> 45.3, 700 57.2 -> 54.5 and 56.4 -> 54.4, 1030 in 6 records 64.7 -> 63.0 and 64.6 -> 62.7,
     // 4096 in 8 204.8 -> 202.9 and the same.

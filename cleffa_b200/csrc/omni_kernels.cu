@@ -564,7 +564,7 @@ constexpr int DISCARD_MIN = 448, DISCARD_MAX = 2560;     // tokens
 // HBM bound: 32 KiB of d and 16 KiB of x per token.  DISCARD: d is dead once it has been read, and what of it is still in L2 then
 // need not go to memory (up to 32 KiB per token that compete with the weights of the next pass).  The line, in tokens for the 126 MB of L2 of the one
 // device this is built for: up to 448 tokens it gains nothing and costs nothing, above 2560 (84 MB) part of d has left L2 before it is read, and
-// discarding such lines costs.  us per block, without and with, each alone under its own clock, on two boxes: 400 tokens 213.0 -> 212.8, 448 208.3 -> 208.1,
+// discarding such lines costs.  us per block, without and with, each alone under its own clock, on two GPUs: 400 tokens 213.0 -> 212.8, 448 208.3 -> 208.1,
 // 511 218.6 -> 217.4 and 211.5 -> 210.0, 1030 237.0 -> 234.7 and 228.6 -> 223.9, 1536 258.6 -> 253.6 and 246.7 -> 242.0, 2048 280.5 -> 276.7 and
 // 266.5 -> 261.7, 2500 301.2 -> 299.1, 2560 286.8 -> 283.9; beyond: 3000 327.7 -> 328.6, 4096 between 1.1 % faster and 0.8 % slower, 16384 2 % slower.
 template <bool DISCARD>

@@ -66,7 +66,7 @@ struct Abort {
 // ordinary stores (the item ring); everything else is signalled by the asynchronous units.
 // The lanes stay together: the vote makes the outcome, and with it every stage counter and address of the loop around it, uniform for
 // the compiler, and nothing is called.  us, waits lane by lane with a function behind the first polls, in the epilogue, gather and softmax
-// warps -> these, in turn, each alone under its own clock, on two boxes: attention half of 37 tokens 29.1 -> 28.7 and 28.9 -> 28.7, 300 48.5 -> 47.4
+// warps -> these, in turn, each alone under its own clock, on two GPUs: attention half of 37 tokens 29.1 -> 28.7 and 28.9 -> 28.7, 300 48.5 -> 47.4
 // and 48.3 -> 47.6, 1030 in 6 records 64.9 -> 64.3 and 65.2 -> 64.6, 16384 in 16 839 -> 827 and 860 -> 849; MoE block the same within 0.7 %.
 // (Spills are not the reason: the expert kernels have none either way, and attention_kernel reloads 120 bytes where it reloaded 52.)
 template <bool CLUSTER>

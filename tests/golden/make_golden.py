@@ -20,7 +20,7 @@ What is stored (small .npz files, committed):
 * route_small.npz-- `route()` of the reference on small random FP64 problems (4 experts
                     top-2 and 16 experts top-4), inputs included.
 
-The GPU box has no reference checkout; the tests only read the .npz files.
+The tests only read the .npz files and need no reference checkout.
 """
 from __future__ import annotations
 

@@ -5,8 +5,8 @@
 Calls `text_attention`, `rotary` and `attention` of the reference's ref/omni_fp64.py (FP64, CPU) on
 a small seeded problem (hidden 64, 4 query heads, 2 key/value heads, head width 16, rotary
 sections 4/2/2, 37 tokens) and stores inputs and outputs.  tests/test_oracle.py checks that
-oracle/omni_attn_oracle.py reproduces them; the GPU box has no reference checkout and only reads
-the .npz file.
+oracle/omni_attn_oracle.py reproduces them; it only reads the .npz file and needs no reference
+checkout.
 """
 from __future__ import annotations
 
